@@ -12,12 +12,31 @@
 // codeword 255's): a free pass proposes the closing state, pinned passes start from it until
 // the path's pre-state of step 0 and its last state both equal the pin (at most max_pins passes).
 //
-// One CTA of 1024 threads per tile: a thread owns the bases (s' >> K) i + 1024 m and writes the
-// 2^K successor states of each.  The two cost arrays
-// (2 x 512 KiB of float64) and the back-pointers (one byte per base and step, in a 16 MiB area) live in
-// a workspace slot of the CTA and stay in L2; the cost arrays are read and written with
-// cache-global accesses because every step reads what other threads of the CTA wrote in the
-// step before.  The only synchronisation is the CTA barrier: nothing waits on another CTA.
+// The 2^K successors of a base b = s' >> K share their predecessors, so all that a step hands on is
+// the cheapest predecessor cost of every base: m[b], 2^(16-K) numbers instead of 65,536.
+//   m_t+1[b'] = min_j ( m_t[(b' >> K) | (j << (16-2K))] + (codebook(b' | j << (16-K)) - w_t)^2 )
+// For K >= 2 they fit the SM's shared memory and a tile is searched by one CTA without leaving it;
+// only the back-pointers (one byte per base and step) go to L2.
+//   * A thread owns the same 128 of the 65,536 (b', j) pairs in every step and keeps their codebook
+//     values in registers.  The bases with the same b' >> K read the same 2^K costs, so a thread's
+//     bases are taken from one such group where K allows.
+//   * The minimum over j is found in fp32 (two values per instruction) on keys with j in their low
+//     bits, relative to a lower bound of all costs, together with the gap to the runner-up; the
+//     winner's cost is then computed in float64 as the reference does.  Where the gap is inside the
+//     error bound of the fp32 keys (about one base in a thousand; exact ties too) the thread takes the
+//     minimum over all j in float64.  fp32 rounding therefore never reaches a result.
+//   * K = 2 has 16,384 bases, 192 KiB for one set of costs: the group of a thread (four reads, four
+//     writes) is updated in place, which rotates the address of a base by K bits per step.
+//   * K = 1 (32,768 bases, 384 KiB) keeps its costs in L2 and compares its two predecessors in float64.
+//   * The walk over the back-pointers reads two steps per L2 round trip: while the warp fetches step
+//     t's pointer its lanes fetch step t - 1's for every value that pointer can have.
+// Tiles are handed out by a counter, because the number of passes differs from tile to tile.
+//
+// Bound: instruction issue, 8 to 9 warp instructions per 32 states and step, two thirds of the logic
+// pipe's slots busy (the keys, their minimum and the gap are three of them).  592 tiles of a 256 x 592
+// matrix, K = 4: 98.7 -> 10.0 ms (59,000 tiles/s) against a version that kept all 65,536 float64 costs
+// of a tile in L2 and moved 1 MiB per step through it; 148 tiles at K = 2 32 -> 13 ms, K = 8 77 -> 13 ms.
+
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -29,128 +48,486 @@
 namespace exl3 {
 
 constexpr int kEncStates = 65536;
-constexpr size_t kEncSlotBytes = 2 * (size_t)kEncStates * sizeof(double) + 256 * (size_t)kEncStates;
+constexpr int kEncThreads = 512;
+constexpr size_t kEncCounterBytes = 256;                 // tile counter in front of the slots
+constexpr size_t kEncBackBytes = 256 * (size_t)(kEncStates / 2);
+constexpr size_t kEncCostBytes = 2 * (size_t)(kEncStates / 2) * sizeof(double);   // K = 1 only
+constexpr size_t kEncSlotBytes = kEncBackBytes + kEncCostBytes;
 
 struct EncodeArgs {
     const float* w;        // (n_tiles, 256) codeword order
     int64_t n_tiles;
-    int k, max_pins;
+    int max_pins;
     uint16_t* states;      // (n_tiles, 256) the 16-bit window of every codeword
     uint32_t* packed;      // NULL or (n_tiles, 8K) packed tile words
+    unsigned* counter;     // tiles handed out so far
     uint8_t* slots;        // gridDim.x workspace slots
 };
 
-template <int CB>
-__global__ void __launch_bounds__(1024) encode_kernel(const EncodeArgs a)
+struct EncodeShared {
+    double red_c[32];
+    int red_s[32];
+    float w[256];
+    uint16_t states[256];
+    uint32_t words[64];
+    unsigned smin[3];
+    int fin, pin, done;
+    unsigned tile;
+};
+
+__device__ __forceinline__ double sq_err(double c, double w)
 {
-    __shared__ float sh_w[256];
-    __shared__ uint16_t sh_states[256];
-    __shared__ double red_c[32];
-    __shared__ int red_s[32];
-    __shared__ uint32_t sh_words[64];
-    __shared__ int sh_fin, sh_pin, sh_done;
+    const double d = c - w;
+    return __dmul_rn(d, d);
+}
+// fp16 -> float64 with integer operations (a value of the codebook is finite): the conversion
+// instructions run at an eighth of the rate.
+__device__ __forceinline__ double half_as_f64(__half h)
+{
+    const uint32_t f = __float_as_uint(__half2float(h));       // at most eleven significant bits
+    const uint32_t hi = (f & 0x7FFFFFFFu) ? (f & 0x80000000u) | (((f & 0x7FFFFFFFu) >> 3) + 0x38000000u) : f;
+    return __hiloint2double((int)hi, 0);
+}
+template <int CB> __device__ __forceinline__ float codebook_f32(uint32_t s) { return __half2float(decode_one<CB>(s)); }
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int k = a.k, kk = 1 << k;
-    uint8_t* slot = a.slots + (size_t)blockIdx.x * kEncSlotBytes;
-    double* cost0 = reinterpret_cast<double*>(slot);
-    double* cost1 = cost0 + kEncStates;
-    uint8_t* back = slot + 2 * (size_t)kEncStates * sizeof(double);
+// The cheapest final state, the lowest index among equals, over the CTA; (bc, bs) is the thread's own.
+__device__ __forceinline__ void final_state(EncodeShared& sh, double bc, int bs, int warps)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const double oc = __shfl_down_sync(0xFFFFFFFFu, bc, off);
+        const int os = __shfl_down_sync(0xFFFFFFFFu, bs, off);
+        if (oc < bc || (oc == bc && os < bs)) { bc = oc; bs = os; }
+    }
+    if (lane == 0) { sh.red_c[warp] = bc; sh.red_s[warp] = bs; }
+    __syncthreads();
+    if (warp == 0) {
+        bc = sh.red_c[lane < warps ? lane : 0];
+        bs = sh.red_s[lane < warps ? lane : 0];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const double oc = __shfl_down_sync(0xFFFFFFFFu, bc, off);
+            const int os = __shfl_down_sync(0xFFFFFFFFu, bs, off);
+            if (oc < bc || (oc == bc && os < bs)) { bc = oc; bs = os; }
+        }
+        if (lane == 0) sh.fin = bs;
+    }
+    __syncthreads();
+}
 
-    for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
-        if (tid < 256) sh_w[tid] = a.w[tile * 256 + tid];
-        if (tid == 0) { sh_pin = -1; sh_done = 0; }
+// Walk of one warp over the back-pointers, two steps per round trip to L2.
+template <int K> __device__ __forceinline__ void walk_back(EncodeShared& sh, const uint8_t* back, int pass)
+{
+    constexpr int NB = kEncStates >> K, J = 1 << K, R = (J + 31) / 32;
+    const int lane = threadIdx.x & 31;
+    uint32_t s = (uint32_t)sh.fin;
+    for (int t = 255; t >= 0; t -= 2) {
+        const uint32_t j0 = __ldcg(back + (size_t)t * NB + (s >> K));
+        uint32_t v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const uint32_t j = (uint32_t)(lane + 32 * r) & (J - 1);
+            v[r] = __ldcg(back + (size_t)(t - 1) * NB + ((s | (j << 16)) >> (2 * K)));
+        }
+        if (lane == 0) sh.states[t] = (uint16_t)s;
+        s = (s >> K) | (j0 << (16 - K));
+        if (lane == 0) sh.states[t - 1] = (uint16_t)s;
+        uint32_t j1 = v[0];
+#pragma unroll
+        for (int r = 1; r < R; r++)
+            if ((int)(j0 >> 5) == r) j1 = v[r];
+        j1 = __shfl_sync(0xFFFFFFFFu, j1, (int)(j0 & 31));
+        s = (s >> K) | (j1 << (16 - K));
+    }
+    __syncwarp();
+    if (lane == 0) {
+        const int last = sh.states[255];
+        if (pass > 0 && (int)s == sh.pin && last == sh.pin) sh.done = 1;
+        sh.pin = last;
+    }
+}
+
+// States and, when asked for, the packed tile: the low K bits of every codeword, MSB first in codeword
+// order, as little-endian 32-bit words (ponyexl3/ref/trellis.py:12-50).
+template <int K> __device__ __forceinline__ void store_tile(EncodeShared& sh, const EncodeArgs& a, int64_t tile)
+{
+    const int tid = threadIdx.x;
+    if (tid < 256) a.states[tile * 256 + tid] = sh.states[tid];
+    if (a.packed) {
+        if (tid < 64) sh.words[tid] = 0u;
         __syncthreads();
+        if (tid < 256) {
+            const uint32_t v = sh.states[tid] & (uint32_t)((1 << K) - 1);
+            for (int b = 0; b < K; b++)
+                if ((v >> (K - 1 - b)) & 1u) {
+                    const int pos = tid * K + b;
+                    atomicOr(&sh.words[pos >> 5], 1u << (31 - (pos & 31)));
+                }
+        }
+        __syncthreads();
+        if (tid < 8 * K) a.packed[tile * 8 * K + tid] = sh.words[tid];
+    }
+    __syncthreads();
+}
+
+// The next tile for this CTA (n_tiles or more: none left), its weights in shared memory.
+__device__ __forceinline__ int64_t next_tile(EncodeShared& sh, const EncodeArgs& a)
+{
+    const int tid = threadIdx.x;
+    if (tid == 0) sh.tile = atomicAdd(a.counter, 1u);
+    __syncthreads();
+    const int64_t tile = sh.tile;
+    if (tile < a.n_tiles) {
+        if (tid < 256) sh.w[tid] = a.w[tile * 256 + tid];
+        if (tid == 0) { sh.pin = -1; sh.done = 0; }
+    }
+    __syncthreads();
+    return tile;
+}
+
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi)
+{
+    return (uint64_t)__float_as_uint(lo) | ((uint64_t)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// (k & ~(J - 1)) | j as one three-input operation (written in C, ptxas made two of it).
+template <int J> __device__ __forceinline__ uint32_t key_with_index(uint32_t k, uint32_t j)
+{
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(k), "n"(~(J - 1)), "r"(j));
+    return r;
+}
+
+// How the 65,536 (b', j) pairs of a step are dealt to the threads.
+template <int K> struct EncodeSplit {
+    static constexpr int NB = kEncStates >> K;           // bases
+    static constexpr int J = 1 << K;
+    static constexpr int JT = J < 128 ? J : 128;         // j values per thread and base (K = 8: two threads a base)
+    static constexpr int BPT = 128 / JT;                 // bases per thread
+    static constexpr int L = BPT < J ? BPT : J;          // ... of them in one group (same b' >> K)
+    static constexpr int G = BPT / L;                    // groups per thread
+    static constexpr int JC = JT < 16 ? JT : 16;         // j values per turn
+    static constexpr bool kInPlace = K == 2;
+    static constexpr size_t kSmem = (size_t)NB * (kInPlace ? 1 : 2) * (sizeof(double) + sizeof(float));
+};
+
+template <int K, int CB>
+__global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs a)
+{
+    using E = EncodeSplit<K>;
+    constexpr int NB = E::NB, J = E::J, L = E::L, G = E::G, JC = E::JC, LB = 16 - K;
+    // Two fp32 keys whose bit patterns differ by less than this may be in the wrong order: the low K
+    // bits hold j (2^K units), the arithmetic before is off by at most four units on either side; twice
+    // that, rounded up.
+    constexpr uint32_t kGap = 4u * J + 32u;
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ EncodeShared sh;
+    double* md0 = reinterpret_cast<double*>(smem);
+    float* mf0 = reinterpret_cast<float*>(md0 + (E::kInPlace ? 1 : 2) * NB);
+    const int tid = threadIdx.x;
+    uint8_t* back = a.slots + (size_t)blockIdx.x * kEncSlotBytes;
+
+    // this thread's bases: groups h(g) = h0 + 512 g, bases (h << K) | (l0 + i)
+    constexpr int TPG = K == 8 ? 512 : J / L;            // threads per group
+    const uint32_t h0 = (uint32_t)(tid / TPG);
+    const uint32_t l0 = K == 8 ? (uint32_t)(tid >> 1) : (uint32_t)(tid % TPG) * L;
+    const uint32_t j_first = K == 8 ? 128u * (tid & 1) : 0u;
+
+    uint32_t cbr[G * L][E::JT / 2];
+#pragma unroll
+    for (int g = 0; g < G; g++)
+#pragma unroll
+        for (int i = 0; i < L; i++)
+#pragma unroll
+            for (int q = 0; q < E::JT / 2; q++) {
+                const uint32_t b = ((h0 + 512u * g) << K) | (l0 + i), j = j_first + 2 * q;
+                cbr[g * L + i][q] = decode_pair<CB>(b | (j << LB), b | ((j + 1) << LB));
+            }
+
+    // Address of base b.  Its low four bits are XOR-ed with the next four, so that a warp's stores (a
+    // few consecutive bases per thread) fall into different banks.  In place, b is first rotated by
+    // the bits of the steps taken so far and the XOR takes all its nibbles, because sixteen neighbours
+    // are then at any power-of-two stride.
+    auto slot = [&](uint32_t b, int rot) -> uint32_t {
+        if (E::kInPlace) {
+            b = ((b >> rot) | (b << (LB - rot))) & (NB - 1);
+            return b ^ (((b >> 4) ^ (b >> 8) ^ (b >> 12)) & 15u);
+        }
+        return b ^ ((b >> 4) & 15u);
+    };
+    // ... of the j-th predecessor base of group h (hs = slot(h)): the high bits pass through the XOR
+    // unless they are among the eight low ones
+    auto pred_slot = [&](uint32_t h, uint32_t hs, uint32_t j, int rot) -> uint32_t {
+        if (!E::kInPlace && LB - K >= 8) return hs + (j << (LB - K));
+        return slot(h | (j << (LB - K)), rot);
+    };
+    for (;;) {
+        const int64_t tile = next_tile(sh, a);
+        if (tile >= a.n_tiles) return;
         for (int pass = 0; pass <= a.max_pins; pass++) {
-            const int pin = sh_pin;
-            for (int s = tid; s < kEncStates; s += 1024) __stcg(cost0 + s, (pin < 0 || s == pin) ? 0.0 : 1e30);
+            const int pin = sh.pin;
+            for (int b = tid; b < NB; b += kEncThreads) {
+                const bool home = pin >= 0 && b == (pin & (NB - 1));
+                const double m = pin < 0 || home ? 0.0 : 1e30;
+                const uint32_t at = slot((uint32_t)b, 0);
+                md0[at] = m;
+                mf0[at] = (float)m;
+                __stcg(back + b, (uint8_t)(home ? pin >> LB : 0));
+            }
+            if (tid == 0) sh.smin[1] = 0x7F800000u;
+            __syncthreads();
+            double off = 0.0;                            // lower bound of every m_t[b]
+            for (int t = 0; t < 255; t++) {
+                const int cur = E::kInPlace ? 0 : (t & 1), nxt = E::kInPlace ? 0 : cur ^ 1;
+                const int rot = E::kInPlace ? (K * t) % LB : 0;
+                const double* mdc = md0 + cur * NB;
+                const float* mfc = mf0 + cur * NB;
+                double* mdn = md0 + nxt * NB;
+                float* mfn = mf0 + nxt * NB;
+                const float w = sh.w[t];
+                const bool tame = fabsf(w) < 1e6f;
+                // costs in mfc are relative to the bound of the step before
+                const float near = (float)off * 9.3e-10f;   // 2^-30: closer than this, float64 roundings decide
+                if (t > 0) {
+                    const float low = __uint_as_float(sh.smin[t % 3]);
+                    if (low < 1e29f) off += (double)low * (1.0 - 2.4e-7);
+                }
+                if (tid == 0) sh.smin[(t + 2) % 3] = 0x7F800000u;
+                const uint64_t nw = pack_f32x2(-w, -w);
+                uint32_t low_new = 0x7F800000u;
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    const uint32_t h = h0 + 512u * g, hs = slot(h, 0);
+                    uint32_t m1[L], m2[L];
+#pragma unroll
+                    for (int c = 0; c < E::JT / JC; c++) {
+                        uint64_t mf2[JC / 2];
+#pragma unroll
+                        for (int q = 0; q < JC / 2; q++) {
+                            const uint32_t j = j_first + c * JC + 2 * q;
+                            mf2[q] = pack_f32x2(mfc[pred_slot(h, hs, j, rot)], mfc[pred_slot(h, hs, j + 1, rot)]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < L; i++) {
+                            uint32_t key[JC];
+#pragma unroll
+                            for (int q = 0; q < JC / 2; q++) {
+                                uint32_t pair = cbr[g * L + i][c * (JC / 2) + q];
+                                asm volatile("" : "+r"(pair));   // converted here: hoisted, 128 floats spill
+                                const float2 cf = __half22float2(u32_as_h2(pair));
+                                const uint64_t d = add_f32x2(pack_f32x2(cf.x, cf.y), nw);
+                                const uint64_t k2 = fma_f32x2(d, d, mf2[q]);
+                                const uint32_t j = c * JC + 2 * q;
+                                key[2 * q] = key_with_index<J>((uint32_t)k2, j);
+                                key[2 * q + 1] = key_with_index<J>((uint32_t)(k2 >> 32), j + 1);
+                            }
+                            uint32_t lo = key[0];
+#pragma unroll
+                            for (int q = 1; q < JC; q++) lo = min(lo, key[q]);
+                            // gap to the runner-up: the winner itself wraps to the largest number
+                            uint32_t gap = 0xFFFFFFFFu;
+#pragma unroll
+                            for (int q = 0; q < JC; q++) gap = __viaddmin_u32(key[q], ~lo, gap);
+                            const uint32_t up = lo + 1u + gap;
+                            if (c == 0) {
+                                m1[i] = lo;
+                                m2[i] = up;
+                            } else {
+                                m2[i] = min(max(m1[i], lo), min(m2[i], up));
+                                m1[i] = min(m1[i], lo);
+                            }
+                        }
+                    }
+                    // the winners' costs in float64, all bases at once; then the bases where fp32 could not decide
+                    double val[L];
+                    uint32_t bj[L], unsure = 0;
+                    const double wd = (double)w;
+#pragma unroll
+                    for (int i = 0; i < L; i++) {
+                        uint32_t lo = m1[i], up = m2[i];
+                        if (K == 8) {                    // the other half of the j values
+                            lo |= j_first;               // (the low bits hold 0 .. 127 so far)
+                            up |= j_first;
+                            const uint32_t lo2 = __shfl_xor_sync(0xFFFFFFFFu, lo, 1), up2 = __shfl_xor_sync(0xFFFFFFFFu, up, 1);
+                            up = min(max(lo, lo2), min(up, up2));
+                            lo = min(lo, lo2);
+                        }
+                        bj[i] = lo & (J - 1);
+                        const uint32_t s = ((h << K) | (l0 + i)) | (bj[i] << LB);
+                        val[i] = __dadd_rn(mdc[pred_slot(h, hs, bj[i], rot)], sq_err(half_as_f64(decode_one<CB>(s)), wd));
+                        if (up - lo < kGap || __uint_as_float(up) < near) unsure |= 1u << i;
+                    }
+                    if (unsure) {
+#pragma unroll
+                        for (int i = 0; i < L; i++) {
+                            if (!((unsure >> i) & 1u)) continue;
+                            const uint32_t b = (h << K) | (l0 + i);
+                            bj[i] = 0;
+                            if (val[i] >= 9e29 && tame) {   // not reachable from the pinned state yet: all exactly 1e30
+                                val[i] = 1e30;
+                                continue;
+                            }
+                            val[i] = __dadd_rn(mdc[pred_slot(h, hs, 0, rot)], sq_err(half_as_f64(decode_one<CB>(b)), wd));
+#pragma unroll 1
+                            for (int q = 1; q < J; q++) {
+                                const uint32_t sq = b | ((uint32_t)q << LB);
+                                const double v = __dadd_rn(mdc[pred_slot(h, hs, (uint32_t)q, rot)], sq_err(half_as_f64(decode_one<CB>(sq)), wd));
+                                if (v < val[i]) { val[i] = v; bj[i] = q; }
+                            }
+                        }
+                    }
+                    if (K != 8 || (tid & 1) == 0) {
+#pragma unroll
+                        for (int i = 0; i < L; i++) {
+                            const uint32_t b = (h << K) | (l0 + i);
+                            // in place, base b' = (h << K) | l of the next step takes the address of h | l << (LB - K)
+                            const uint32_t at = E::kInPlace ? slot(h | (i << (LB - K)), rot) : slot(b, 0);
+                            const float rel = fmaxf((float)(val[i] - off), 0.f);
+                            mdn[at] = val[i];
+                            mfn[at] = rel;
+                            low_new = min(low_new, __float_as_uint(rel));
+                        }
+                        uint8_t* bp = back + (size_t)(t + 1) * NB + ((h << K) | l0);
+                        uint32_t pk[(L + 3) / 4];
+#pragma unroll
+                        for (int i = 0; i < (L + 3) / 4; i++) pk[i] = 0u;
+#pragma unroll
+                        for (int i = 0; i < L; i++) pk[i >> 2] |= bj[i] << (8 * (i & 3));
+                        if constexpr (L == 8) __stcg(reinterpret_cast<uint2*>(bp), make_uint2(pk[0], pk[1]));
+                        else if constexpr (L == 4) __stcg(reinterpret_cast<uint32_t*>(bp), pk[0]);
+                        else if constexpr (L == 2) __stcg(reinterpret_cast<uint16_t*>(bp), (uint16_t)pk[0]);
+                        else __stcg(bp, (uint8_t)pk[0]);
+                    }
+                }
+                low_new = __reduce_min_sync(0xFFFFFFFFu, low_new);
+                if ((tid & 31) == 0) atomicMin(&sh.smin[(t + 1) % 3], low_new);
+                __syncthreads();
+            }
+            // step 255: every final state in float64
+            {
+                const int cur = E::kInPlace ? 0 : 1, rot = E::kInPlace ? (K * 255) % LB : 0;
+                const double* mdc = md0 + cur * NB;
+                const double wd = (double)sh.w[255];
+                double bc = 0.0;
+                int bs = -1;
+#pragma unroll 4
+                for (int s = tid; s < kEncStates; s += kEncThreads) {
+                    const double v = __dadd_rn(mdc[slot((uint32_t)s >> K, rot)], sq_err((double)codebook_f32<CB>((uint32_t)s), wd));
+                    if (bs < 0 || v < bc) { bc = v; bs = s; }
+                }
+                final_state(sh, bc, bs, kEncThreads / 32);
+            }
+            if (tid < 32) walk_back<K>(sh, back, pass);
+            __syncthreads();
+            if (sh.done) break;
+        }
+        store_tile<K>(sh, a, tile);
+    }
+}
+
+// K = 1: 32,768 bases of two predecessors; the costs stay in L2.
+constexpr int kEncThreads1 = 1024;
+template <int CB> __global__ void __launch_bounds__(kEncThreads1) encode_kernel_k1(const EncodeArgs a)
+{
+    constexpr int NB = kEncStates / 2;
+    __shared__ EncodeShared sh;
+    const int tid = threadIdx.x;
+    uint8_t* back = a.slots + (size_t)blockIdx.x * kEncSlotBytes;
+    double* cost0 = reinterpret_cast<double*>(back + kEncBackBytes);
+    double* cost1 = cost0 + NB;
+    for (;;) {
+        const int64_t tile = next_tile(sh, a);
+        if (tile >= a.n_tiles) return;
+        for (int pass = 0; pass <= a.max_pins; pass++) {
+            const int pin = sh.pin;
+            for (int b = tid; b < NB; b += kEncThreads1) {
+                const bool home = pin >= 0 && b == (pin & (NB - 1));
+                __stcg(cost0 + b, pin < 0 || home ? 0.0 : 1e30);
+                __stcg(back + b, (uint8_t)(home ? pin >> 15 : 0));
+            }
             __syncthreads();
             double* cur = cost0;
             double* nxt = cost1;
-            for (int t = 0; t < 256; t++) {
-                const double wt = (double)sh_w[t];
-                uint8_t* bt = back + (size_t)t * kEncStates;
-                // The 2^K successors of one base (s' >> K) share their predecessor set, hence its
-                // cheapest member: every cost of the step before is read exactly once.
-                for (uint32_t base = tid; base < (uint32_t)(kEncStates >> k); base += 1024) {
-                    double cb = __ldcg(cur + base);
-                    int best = 0;
-                    for (int j = 1; j < kk; j++) {
-                        const double c = __ldcg(cur + (base | ((uint32_t)j << (16 - k))));
-                        if (c < cb) { cb = c; best = j; }
+            for (int t = 0; t < 255; t++) {
+                const double wd = (double)sh.w[t];
+                uint8_t* bp = back + (size_t)(t + 1) * NB;
+                // bases 2h and 2h + 1 share the predecessor bases h and h + 2^14
+#pragma unroll 4
+                for (int h = tid; h < NB / 2; h += kEncThreads1) {
+                    const double c0 = __ldcg(cur + h), c1 = __ldcg(cur + h + NB / 2);
+                    double m[2];
+                    uint32_t bj = 0;
+#pragma unroll
+                    for (int l = 0; l < 2; l++) {
+                        const uint32_t b = 2 * h + l;
+                        const double v0 = __dadd_rn(c0, sq_err((double)codebook_f32<CB>(b), wd));
+                        const double v1 = __dadd_rn(c1, sq_err((double)codebook_f32<CB>(b | 0x8000u), wd));
+                        m[l] = v1 < v0 ? v1 : v0;
+                        if (v1 < v0) bj |= 1u << (8 * l);
                     }
-                    __stcg(bt + base, (uint8_t)best);          // one back-pointer for all 2^K successors
-                    for (int low = 0; low < kk; low += 2) {
-                        const uint32_t s = (base << k) | (uint32_t)low;
-                        const double d0 = (double)__half2float(decode_one<CB>(s)) - wt;
-                        const double d1 = (double)__half2float(decode_one<CB>(s + 1)) - wt;
-                        __stcg(reinterpret_cast<double2*>(nxt + s),
-                               make_double2(__dadd_rn(cb, __dmul_rn(d0, d0)), __dadd_rn(cb, __dmul_rn(d1, d1))));
-                    }
+                    __stcg(reinterpret_cast<double2*>(nxt + 2 * h), make_double2(m[0], m[1]));
+                    __stcg(reinterpret_cast<uint16_t*>(bp + 2 * h), (uint16_t)bj);
                 }
                 __syncthreads();
                 double* tmp = cur; cur = nxt; nxt = tmp;
             }
-            // the cheapest final state, the lowest index among equals
-            double bc = __ldcg(cur + tid);
-            int bs = tid;
-            for (int s = tid + 1024; s < kEncStates; s += 1024) {
-                const double c = __ldcg(cur + s);
-                if (c < bc) { bc = c; bs = s; }
+            const double wd = (double)sh.w[255];
+            double bc = 0.0;
+            int bs = -1;
+#pragma unroll 4
+            for (int s = tid; s < kEncStates; s += kEncThreads1) {
+                const double v = __dadd_rn(__ldcg(cur + (s >> 1)), sq_err((double)codebook_f32<CB>((uint32_t)s), wd));
+                if (bs < 0 || v < bc) { bc = v; bs = s; }
             }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const double oc = __shfl_down_sync(0xFFFFFFFFu, bc, off);
-                const int os = __shfl_down_sync(0xFFFFFFFFu, bs, off);
-                if (oc < bc || (oc == bc && os < bs)) { bc = oc; bs = os; }
-            }
-            if (lane == 0) { red_c[warp] = bc; red_s[warp] = bs; }
+            final_state(sh, bc, bs, kEncThreads1 / 32);
+            if (tid < 32) walk_back<1>(sh, back, pass);
             __syncthreads();
-            if (warp == 0) {
-                bc = red_c[lane];
-                bs = red_s[lane];
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    const double oc = __shfl_down_sync(0xFFFFFFFFu, bc, off);
-                    const int os = __shfl_down_sync(0xFFFFFFFFu, bs, off);
-                    if (oc < bc || (oc == bc && os < bs)) { bc = oc; bs = os; }
-                }
-                if (lane == 0) sh_fin = bs;
-            }
-            __syncthreads();
-            if (tid == 0) {
-                // walk the back-pointers (the stores of this CTA are visible after the barriers)
-                uint32_t s = (uint32_t)sh_fin;
-                for (int t = 255; t >= 0; t--) {
-                    sh_states[t] = (uint16_t)s;
-                    const uint32_t j = __ldcg(back + (size_t)t * kEncStates + (s >> k));
-                    s = (s >> k) | (j << (16 - k));
-                }
-                const int last = sh_states[255];
-                if (pass > 0 && (int)s == pin && last == pin) sh_done = 1;
-                sh_pin = last;
-            }
-            __syncthreads();
-            if (sh_done) break;
+            if (sh.done) break;
         }
-        if (tid < 256) a.states[tile * 256 + tid] = sh_states[tid];
-        if (a.packed) {
-            // the low K bits of every codeword, MSB first in codeword order, as little-endian
-            // 32-bit words (ponyexl3/ref/trellis.py:12-50)
-            if (tid < 64) sh_words[tid] = 0u;
-            __syncthreads();
-            if (tid < 256) {
-                const uint32_t v = sh_states[tid] & (uint32_t)(kk - 1);
-                for (int b = 0; b < k; b++)
-                    if ((v >> (k - 1 - b)) & 1u) {
-                        const int pos = tid * k + b;
-                        atomicOr(&sh_words[pos >> 5], 1u << (31 - (pos & 31)));
-                    }
-            }
-            __syncthreads();
-            if (tid < 8 * k) a.packed[tile * 8 * k + tid] = sh_words[tid];
+        store_tile<1>(sh, a, tile);
+    }
+}
+
+template <int K, int CB> static int launch_encode(const EncodeArgs& a, unsigned slots, cudaStream_t s)
+{
+    if constexpr (K == 1) {
+        encode_kernel_k1<CB><<<slots, kEncThreads1, 0, s>>>(a);
+        return check_launch();
+    } else {
+        static bool attr_set[kMaxDevices] = {};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev < 0 || dev >= kMaxDevices) return EXL3_E_UNSUPPORTED;
+        if (!attr_set[dev]) {
+            const cudaError_t e = cudaFuncSetAttribute(encode_kernel<K, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)EncodeSplit<K>::kSmem);
+            if (e != cudaSuccess) return note_cuda(e);
+            attr_set[dev] = true;
         }
-        __syncthreads();
+        encode_kernel<K, CB><<<slots, kEncThreads, EncodeSplit<K>::kSmem, s>>>(a);
+        return check_launch();
+    }
+}
+
+template <int K> static int launch_encode_k(const EncodeArgs& a, int cb, unsigned slots, cudaStream_t s)
+{
+    switch (cb) {
+        case CB_3INST: return launch_encode<K, CB_3INST>(a, slots, s);
+        case CB_MCG: return launch_encode<K, CB_MCG>(a, slots, s);
+        default: return launch_encode<K, CB_MUL1>(a, slots, s);
     }
 }
 
@@ -164,7 +541,7 @@ extern "C" size_t exl3_encode_workspace_bytes(int64_t n_tiles)
     int64_t slots = device_sm_count();
     if (slots < 1) slots = 1;
     if (n_tiles < slots) slots = n_tiles;
-    return (size_t)slots * kEncSlotBytes;
+    return kEncCounterBytes + (size_t)slots * kEncSlotBytes;
 }
 
 extern "C" int exl3_encode_tiles(const float* w, int64_t n_tiles, int k, int cb, int max_pins, uint16_t* states,
@@ -173,28 +550,40 @@ extern "C" int exl3_encode_tiles(const float* w, int64_t n_tiles, int k, int cb,
     if (!w || !states) return EXL3_E_NULL;
     if (k < 1 || k > 8) return EXL3_E_K;
     if (cb < 0 || cb > 2) return EXL3_E_CODEBOOK;
+    // the tile counter is 32 bits wide
     if (n_tiles < 0 || n_tiles > ((int64_t)1 << 32) || max_pins < 0 || max_pins > 64) return EXL3_E_RANGE;
     if ((reinterpret_cast<uintptr_t>(w) & 3) || (reinterpret_cast<uintptr_t>(states) & 1) ||
         (packed && (reinterpret_cast<uintptr_t>(packed) & 3)))
         return EXL3_E_ALIGN;
-    if (!workspace || workspace_bytes < kEncSlotBytes) return EXL3_E_WORKSPACE;
+    if (!workspace || workspace_bytes < kEncCounterBytes + kEncSlotBytes) return EXL3_E_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(workspace) & 255) return EXL3_E_ALIGN;
     if (n_tiles == 0) return EXL3_OK;
-    int64_t slots = (int64_t)(workspace_bytes / kEncSlotBytes);
-    slots = std::min<int64_t>(slots, std::min<int64_t>(n_tiles, 4 * (int64_t)device_sm_count()));
+    int64_t slots = (int64_t)((workspace_bytes - kEncCounterBytes) / kEncSlotBytes);
+    slots = std::min<int64_t>(slots, std::min<int64_t>(n_tiles, (int64_t)device_sm_count()));
     EncodeArgs a;
-    a.w = w;
-    a.n_tiles = n_tiles;
-    a.k = k;
     a.max_pins = max_pins;
-    a.states = states;
-    a.packed = reinterpret_cast<uint32_t*>(packed);
-    a.slots = static_cast<uint8_t*>(workspace);
+    a.counter = static_cast<unsigned*>(workspace);
+    a.slots = static_cast<uint8_t*>(workspace) + kEncCounterBytes;
     cudaStream_t s = (cudaStream_t)stream;
-    switch (cb) {
-        case CB_3INST: encode_kernel<CB_3INST><<<(unsigned)slots, 1024, 0, s>>>(a); break;
-        case CB_MCG: encode_kernel<CB_MCG><<<(unsigned)slots, 1024, 0, s>>>(a); break;
-        default: encode_kernel<CB_MUL1><<<(unsigned)slots, 1024, 0, s>>>(a); break;
+    constexpr int64_t kMost = (int64_t)1 << 31;      // tiles per launch: the counter must not wrap
+    for (int64_t t0 = 0; t0 < n_tiles; t0 += kMost) {
+        a.w = w + t0 * 256;
+        a.n_tiles = std::min<int64_t>(kMost, n_tiles - t0);
+        a.states = states + t0 * 256;
+        a.packed = packed ? reinterpret_cast<uint32_t*>(packed) + t0 * 8 * k : nullptr;
+        int rc = note_cuda(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), s));
+        if (rc) return rc;
+        switch (k) {
+            case 1: rc = launch_encode_k<1>(a, cb, (unsigned)slots, s); break;
+            case 2: rc = launch_encode_k<2>(a, cb, (unsigned)slots, s); break;
+            case 3: rc = launch_encode_k<3>(a, cb, (unsigned)slots, s); break;
+            case 4: rc = launch_encode_k<4>(a, cb, (unsigned)slots, s); break;
+            case 5: rc = launch_encode_k<5>(a, cb, (unsigned)slots, s); break;
+            case 6: rc = launch_encode_k<6>(a, cb, (unsigned)slots, s); break;
+            case 7: rc = launch_encode_k<7>(a, cb, (unsigned)slots, s); break;
+            default: rc = launch_encode_k<8>(a, cb, (unsigned)slots, s); break;
+        }
+        if (rc) return rc;
     }
-    return check_launch();
+    return EXL3_OK;
 }

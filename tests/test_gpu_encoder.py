@@ -50,6 +50,24 @@ def test_encoder_matches_the_oracle_on_random_tiles(ops, oracle, k, cb):
         assert (_u16(packed)[t] == oracle.pack_trellis_tile((want & ((1 << k) - 1)).astype(np.uint16), k)).all()
 
 
+@pytest.mark.parametrize("k,cb", [(1, 0), (1, 2), (2, 1), (4, 1), (5, 2), (6, 0), (7, 1), (8, 0), (8, 2)])
+def test_encoder_where_fp32_keys_cannot_decide(ops, oracle, k, cb):
+    """Exact ties, weights that are codebook values, and magnitudes at which neighbouring costs are
+    closer than fp32 resolves: every split of the bases over the threads takes the float64 path."""
+    rng = np.random.default_rng(40 + k)
+    w = rng.standard_normal((6, 256)).astype(np.float32)
+    w[0] = 0.0
+    w[1] = w[1].astype(np.float16).astype(np.float32)
+    w[2] *= 1e4
+    w[3] = np.sign(w[3]) * 0.5
+    w[4] *= 1e-6
+    states, packed = ops.quantize_tiles(torch.from_numpy(w).cuda(), k, cb)
+    for t in range(6):
+        want, _ = oracle.quantize_tile(w[t], k, cb)
+        assert (_u16(states)[t] == want).all(), f"tile {t}"
+        assert (_u16(packed)[t] == oracle.pack_trellis_tile((want & ((1 << k) - 1)).astype(np.uint16), k)).all()
+
+
 def test_quantised_matrix_decodes_to_the_chosen_codebook_values(ops, oracle):
     k, cb = 3, 0
     rng = np.random.default_rng(3)
