@@ -53,25 +53,6 @@ template <int K> struct LaneWords {
     }
 };
 
-// The eight codewords of a lane from its (up to) three words a, b, c, taken in
-// stream order.  Output values are zero-extended 16-bit windows.
-template <int K> EXL3_HD void lane_codewords(uint32_t a, uint32_t b, uint32_t c, uint32_t sh,
-                                             uint32_t (&cw)[8])
-{
-    // Left-align the lane's 7K+16 bits: n[0] bit 31 is stream bit p0.
-    uint32_t n[3];
-    n[0] = funnel_l(b, a, sh);
-    n[1] = LaneWords<K>::kThree ? funnel_l(c, b, sh) : (b << sh);
-    n[2] = LaneWords<K>::kThree ? (c << sh) : 0u;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int off = j * K;                    // window j = bits [off, off+16) of n
-        const int q = off >> 5, r = off & 31;
-        if (r + 16 <= 32) cw[j] = (n[q] >> (16 - r)) & 0xFFFFu;
-        else cw[j] = funnel_l(n[q + 1 > 2 ? 2 : q + 1], n[q], (uint32_t)r) >> 16;
-    }
-}
-
 // Byte permute of the register pair (b:a) — selector nibble i picks the source byte of
 // result byte i (0-3 from a, 4-7 from b).
 EXL3_HD uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t sel)
@@ -84,6 +65,39 @@ EXL3_HD uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t sel)
     for (int i = 0; i < 4; i++) r |= (uint32_t)((v >> (8 * ((sel >> (4 * i)) & 7))) & 0xFF) << (8 * i);
     return r;
 #endif
+}
+
+// Bits [r, r + 16) of w, counted from its top: a byte permute when they are whole bytes, else a left
+// shift (a multiplication, off the logic pipe) and a byte permute.  A right shift and a mask would be two
+// logic-pipe operations, the shift at half the rate of the others.
+template <int R> EXL3_HD uint32_t window16(uint32_t w)
+{
+    static_assert(R >= 0 && R <= 16, "window inside one word");
+    if (R == 16) return byte_perm(w, 0u, 0x4410);
+    if (R == 8) return byte_perm(w, 0u, 0x4421);
+    return byte_perm(R == 0 ? w : w << R, 0u, 0x4432);
+}
+
+// The eight codewords of a lane from its (up to) three words a, b, c, taken in
+// stream order.  Output values are zero-extended 16-bit windows.
+template <int K, int J> EXL3_HD void lane_window(const uint32_t (&n)[5], uint32_t (&cw)[8])
+{
+    // n[i] holds stream bits [16 i, 16 i + 32): window J starts in its first 17 bits
+    constexpr int off = J * K, i = off <= 16 ? 0 : (off - 1) / 16;
+    cw[J] = window16<off - 16 * i>(n[i]);
+    if constexpr (J < 7) lane_window<K, J + 1>(n, cw);
+}
+template <int K> EXL3_HD void lane_codewords(uint32_t a, uint32_t b, uint32_t c, uint32_t sh,
+                                             uint32_t (&cw)[8])
+{
+    // Left-align the lane's 7K+16 bits: n[0] bit 31 is stream bit p0.
+    uint32_t n[5];
+    n[0] = funnel_l(b, a, sh);
+    n[2] = LaneWords<K>::kThree ? funnel_l(c, b, sh) : (b << sh);
+    n[4] = LaneWords<K>::kThree ? (c << sh) : 0u;
+    n[1] = byte_perm(n[2], n[0], 0x5432);
+    n[3] = byte_perm(n[4], n[2], 0x5432);
+    lane_window<K, 0>(n, cw);
 }
 
 // 64-bit a * b + (c_hi << 32), returned as (lo, hi).  On the device this is one
