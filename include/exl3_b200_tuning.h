@@ -21,14 +21,9 @@ extern "C" {
  * is the maximum; 0 always uses the separate rotation kernel). */
 EXL3_API void exl3_tune_gemv(int max_grid, int fuse_x_bytes);
 
-/* one_acc_rows: 128 (default) = an output tile of the prefill GEMM with at most 128 rows loads,
- * multiplies and drains only its first accumulator; 0 = every tile uses both (for comparison).
- * + 256: a dense layer's short last wave of tiles is NOT cut into 128-column half tiles. */
+/* Without effect: they chose between variants of the prefill GEMM (accumulators per tile, pairs of
+ * SMs), which is one kernel for every shape now.  Kept for callers that link against them. */
 EXL3_API void exl3_tune_gemm(int one_acc_rows);
-
-/* on: 1 = dense prefill GEMMs of 1024 rows and more run on pairs of SMs
- * (tcgen05.mma.cta_group::2, 512-row output tiles); 0 (default) = the one-CTA kernel for every
- * shape, which is a little faster on the shapes measured so far. */
 EXL3_API void exl3_tune_gemm_pairs(int on);
 
 #ifdef __cplusplus

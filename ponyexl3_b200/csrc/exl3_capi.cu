@@ -479,11 +479,17 @@ int exl3_gemv_blocks_counted(const void* x, int x_dtype, int64_t x_row_stride, i
                             workspace, workspace_bytes, flags, stream);
 }
 
+// Where the partial sums of shared tiles start: after the rotated activations, on a 256-byte boundary.
+static size_t gemm_partial_offset(int64_t rows, int64_t in)
+{
+    return ((size_t)kWsScratch + (size_t)rows * (size_t)in * 2 + 255) & ~(size_t)255;
+}
+
 size_t exl3_gemm_workspace_bytes(int64_t rows, int64_t in)
 {
     if (rows < 1) rows = 1;
     if (in < 128) in = 128;
-    return ((size_t)kWsScratch + (size_t)rows * (size_t)in * 2 + 255) & ~(size_t)255;
+    return gemm_partial_offset(rows, in) + gemm_partial_bytes(rows);
 }
 
 int exl3_gemm(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, const uint16_t* trellis,
@@ -507,7 +513,8 @@ int exl3_gemm(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, co
         return EXL3_E_ALIGN;
     if (!workspace) return EXL3_E_WORKSPACE;
     if (!aligned(workspace, 256)) return EXL3_E_ALIGN;
-    if (workspace_bytes < exl3_gemm_workspace_bytes(rows, in)) return EXL3_E_WORKSPACE;
+    const size_t part_off = gemm_partial_offset(rows, in);     // without room behind it tiles are not shared
+    if (workspace_bytes < part_off) return EXL3_E_WORKSPACE;
 
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     __half* xh = reinterpret_cast<__half*>(ws + kWsScratch);
@@ -525,6 +532,9 @@ int exl3_gemm(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, co
     a.xh_rows = (int)rows;
     a.t_in = (int)t_in;
     a.t_out = (int)t_out;
+    a.ts_partials = reinterpret_cast<float*>(ws + part_off);
+    a.ts_partial_bytes = workspace_bytes - part_off;
+    a.ts_ctr = reinterpret_cast<unsigned*>(ws + kWsSplitCtr);
     a.y_wide = (y_row_stride % 16 == 0 && aligned(y, 32)) ? 1 : 0;   // 32-byte stores in the epilogue
     return launch_gemm(a, k, cb, xh, reinterpret_cast<const uint32_t*>(trellis), s);
 }
@@ -561,7 +571,7 @@ static int gemm_tiles_impl(const void* x, int x_dtype, int64_t x_row_stride, int
     if ((suh && !aligned(suh, 8)) || (svh && !aligned(svh, 16))) return EXL3_E_ALIGN;
     if (!workspace) return EXL3_E_WORKSPACE;
     if (!aligned(workspace, 256)) return EXL3_E_ALIGN;
-    if (workspace_bytes < exl3_gemm_workspace_bytes(xh_rows, in)) return EXL3_E_WORKSPACE;
+    if (workspace_bytes < gemm_partial_offset(xh_rows, in)) return EXL3_E_WORKSPACE;
     if (peers.n < 0 || peers.n > kMaxPeers) return EXL3_E_RANGE;
     if (peers.n > 0 && (!peers.y || !peers.ctr || peers.rows_per_peer < 1 || peers.rows_per_peer > (1 << 30) || !y_row_map))
         return EXL3_E_NULL;
@@ -652,14 +662,8 @@ void exl3_tune_gemv(int max_grid, int fuse_x_bytes)
     gemv_set_tuning(max_grid, fuse_x_bytes);
 }
 
-void exl3_tune_gemm(int one_acc_rows)
-{
-    gemm_set_tuning(one_acc_rows);
-}
-
-void exl3_tune_gemm_pairs(int on)
-{
-    gemm_set_pairs(on);
-}
+// The GEMM these two chose variants of is one kernel now; the names stay for callers that set them.
+void exl3_tune_gemm(int one_acc_rows) { (void)one_acc_rows; }
+void exl3_tune_gemm_pairs(int on) { (void)on; }
 
 }  // extern "C"

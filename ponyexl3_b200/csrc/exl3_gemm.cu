@@ -1,19 +1,8 @@
-// Host-side dispatch of the prefill GEMM over K; the kernel template (exl3_gemm.cuh) is
+// Host side of the tensor-core GEMM: the launch plan and the dispatch over K; the kernel template (exl3_gemm.cuh) is
 // instantiated in exl3_gemm_k12.cu .. exl3_gemm_k78.cu.
-#include "exl3_internal.h"
+#include "exl3_gemm.cuh"
 
 namespace exl3 {
-
-int g_gemm_one_acc_rows = 128;
-int g_gemm_split_last_wave = 1;
-void gemm_set_tuning(int one_acc_rows)
-{
-    g_gemm_one_acc_rows = (one_acc_rows & 255) == 0 ? 0 : 128;
-    g_gemm_split_last_wave = (one_acc_rows & 256) ? 0 : 1;     // + 256: whole tiles only
-}
-// Off: measured on 8192 x 5120 x 5120 the pair kernel is at 0.43 ms against 0.40 ms (see exl3_gemm2.cuh).
-int g_gemm_pairs = 0;
-void gemm_set_pairs(int on) { g_gemm_pairs = on ? 1 : 0; }
 
 template <int K>
 int launch_gemm_k(const GemmArgs& a, int cb, const __half* xh, const uint32_t* trellis, cudaStream_t s);
@@ -21,6 +10,50 @@ int launch_gemm_k(const GemmArgs& a, int cb, const __half* xh, const uint32_t* t
     extern template int launch_gemm_k<K>(const GemmArgs&, int, const __half*, const uint32_t*, cudaStream_t);
 EXL3_DECL(1) EXL3_DECL(2) EXL3_DECL(3) EXL3_DECL(4) EXL3_DECL(5) EXL3_DECL(6) EXL3_DECL(7) EXL3_DECL(8)
 #undef EXL3_DECL
+
+// How many CTAs a dense launch of `tiles` output tiles of nks k-steps gets, and whether they share tiles.
+// Cost in k-steps of the slowest CTA: its k-steps, and for each of its segments the hand-over and the
+// epilogue, measured at about ten k-steps.  Whole tiles are the case of every segment being one; for
+// shared tiles a count that lets ranges end on tile boundaries saves a segment per CTA, so all counts
+// down to half of the SMs are looked at.  The choice is remembered per shape.
+int ts_plan(int64_t tiles, int nks, int sms, int64_t rows, size_t partial_bytes, int* split)
+{
+    constexpr double kSegment = 10.0;
+    struct Memo { int64_t tiles; int nks, sms, room, grid, split; };
+    static thread_local Memo memo[32] = {};
+    static thread_local int memo_next = 0;
+    sms = std::min(sms, kGemvMaxGrid);
+    const int room = partial_bytes >= gemm_tile_partial_bytes(rows, sms) ? 1 : 0;
+    for (const Memo& m : memo)
+        if (m.tiles == tiles && m.nks == nks && m.sms == sms && m.room == room) {
+            *split = m.split;
+            return m.grid;
+        }
+    const int whole = (int)std::min<int64_t>(tiles, sms);
+    int best = whole, best_split = 0;
+    double best_cost = (double)((tiles + whole - 1) / whole) * (nks + kSegment);
+    const int64_t units = tiles * nks;
+    if (room && tiles < 64 * sms && units >= 4) {
+        const int most = (int)std::min<int64_t>(sms, units / 4);
+        for (int g = most; g >= std::max(1, most / 2); g--) {
+            double worst = 0;
+            for (int c = 0; c < g; c++) {
+                int64_t u = units * c / g;
+                const int64_t u1 = units * (c + 1) / g;
+                double t = (double)(u1 - u);
+                for (; u < u1; u = (u / nks + 1) * nks) t += kSegment;
+                worst = std::max(worst, t);
+            }
+            if (worst < best_cost - 1e-9) { best_cost = worst; best = g; best_split = 1; }
+        }
+    }
+    memo[memo_next] = Memo{tiles, nks, sms, room, best, best_split};
+    memo_next = (memo_next + 1) % 32;
+    *split = best_split;
+    return best;
+}
+
+size_t gemm_partial_bytes(int64_t rows) { return gemm_tile_partial_bytes(rows, std::min(device_sm_count(), kGemvMaxGrid)); }
 
 int launch_gemm(const GemmArgs& a, int k, int cb, const __half* xh, const uint32_t* trellis,
                 cudaStream_t s)

@@ -1,38 +1,34 @@
-// Prefill GEMM on the 5th-generation tensor cores: y = had( fp16( xh @ W ) ) * svh + bias
-// for many rows (tokens), W decoded on the fly from the packed trellis — never materialised
-// in global memory.
+// GEMM for more than a handful of rows on the 5th-generation tensor cores, weights in tensor memory:
+//   y = had( fp16( xh @ W ) ) * svh + bias,  W decoded on the fly from the packed trellis.
 //
-// One persistent CTA per SM walks output tiles of 256 tokens x 256 columns.  Per 64-wide
-// k-step and ring stage:
-//   * warp 0 (one lane) issues TMA loads: two 128-token x 64-k boxes of the rotated fp16
-//     activations (128B-swizzled, the canonical K-major operand layout) and one 3-D box with
-//     the 16 x 4 packed tiles of the step (2*K KiB);
-//   * warps 2..9 decode those tiles in registers (the same window / codebook code as the
-//     GEMV, bit-exact) and store fp16 pairs into the 128B-swizzled K-major B operand tile
-//     (conflict-free 4-byte stores: the packed tile order puts 8 rows x 4 k-pairs in a warp);
-//   * warp 1 (one lane) issues tcgen05.mma (M = 128 tokens, N = 256 columns, K = 16) for BOTH
-//     token halves against the same decoded B tile, accumulating in two 128 x 256 fp32
-//     accumulators that fill the SM's 512 tensor-memory columns; tcgen05.commit frees the
-//     stage.  Sharing B between two accumulators halves the decode work per FLOP.
-// When a tile's k-loop is done the decode warps become the epilogue: each thread owns one
-// token (tensor-memory lane) and 128 columns, loads them with tcgen05.ld, rounds to fp16 as
-// the reference does, runs the 128-point Hadamard entirely in registers, applies svh and
-// bias, and writes 256 contiguous bytes (32 bytes per store when the rows are 32-byte aligned).
-// A grouped launch may spread its output rows over several GPUs: the epilogue then stores each
-// row into the buffer of the GPU that owns it and the last CTA announces the grid to every peer.
+// The product is computed transposed, D[outs x tokens] = W^T x^T: the decoded weights are the A operand
+// of tcgen05.mma, which may live in tensor memory.  The packed order of a 16x16 tile is the fragment
+// order of W^T, and that is the register layout of tcgen05.st.16x128b, so a decoded tile goes from
+// registers to tensor memory with one store and no address arithmetic, and shared memory carries only
+// the activations (operand B) and the packed words.  Decoding into a swizzled operand tile in shared
+// memory instead costs four scattered stores per tile and 96 bytes of operand reads per clock.
 //
-// Measured on 8192 x 5120 x 5120 (K = 4) by switching parts off with all barriers and copies
-// intact: the kernel is bound by shared-memory bandwidth and by the latency of a ring turn, not
-// by the tensor pipe (about half active) nor by the number of decode warps — per k-step an SM
-// reads 96 KiB of MMA operands (B once per accumulator), takes 40 KiB of TMA data and moves
-// about 48 KiB of decode loads and stores.  Sixteen decode warps (with the epilogue's first
-// Hadamard half parked in tensor memory to fit the registers) and rings of separate depth for
-// packed tiles, activations and B were measured equal and slower respectively, and are not kept.
+// Output tile: 128 columns (the width of the output rotation) x up to 256 tokens, k-step 64.
+//   warp 0      packed tiles: one 3-D TMA box of 8 x 4 tiles per k-step (ring w, eight stages)
+//   warp 1      activations: a 128B-swizzled TMA box per k-step (ring x)
+//   warp 2      issues the MMAs: A from tensor memory (eight 32-column stages), B from ring x
+//   warps 4-19  decode, four sets of four warps (a warp may touch the quarter of the tensor-memory
+//               lanes that its index names); the sets take the k-steps in turn
+// then the 16 decode warps finish the tile:
+//   1. D (fp32, lane = column, register = token) is rounded to fp16 as the reference does and parked in
+//      shared memory as Y[token][column] in the MN-major operand layout;
+//   2. the output rotation is one more product on the tensor cores, D2[token x column] = Y H with the
+//      +-1 Sylvester matrix H (exact in fp16, fp32 sums), into D's own columns;
+//   3. D2 (lane = token) is scaled by 1/sqrt(128) svh, biased, and stored as 64-byte row pieces.
 //
-// fp16 operands are exact for the decoded weights (|w| < 4) and equal to the reference's
-// fp16 rounding of the rotated activations; accumulation is fp32.
-// Every mbarrier wait is bounded; a wait that gives up sets ST_TC_TIMEOUT in the status
-// word, every role leaves its loop, and the tensor memory is freed before the CTA exits.
+// Work is dealt in k-steps: CTA c takes the k-steps [U c/G, U (c+1)/G) of the tiles laid end to end, so a
+// layer with few tiles still uses every SM.  A tile that several CTAs share is finished by the one that
+// ends last: each writes its fp32 sums to its own slot of the workspace and counts itself; the last
+// one adds the slots in CTA order, so the result does not depend on who came last.  Grouped launches
+// (a tile table) take whole tiles in turn.
+//
+// Every mbarrier wait is bounded; a wait that gives up sets ST_TC_TIMEOUT, the thread stops waiting (so
+// named barriers still meet) and the tensor memory is freed at the end.
 #pragma once
 #include <algorithm>
 
@@ -42,33 +38,89 @@
 
 namespace exl3 {
 
-constexpr int kGemmThreads = 320;          // TMA warp, MMA warp, 8 decode / epilogue warps
-constexpr int kGemmDecodeWarps = 8;
-constexpr int kTileM = 256, kTileN = 256, kStepK = 64;
-constexpr int kABytes = 128 * kStepK * 2;  // one 128-token activation box
-constexpr int kBBytes = kTileN * kStepK * 2;
-constexpr int kGemmCtrlBytes = 1024;
+constexpr int kTsThreads = 640;
+constexpr int kTsDecodeWarps = 16, kTsFirstDecodeWarp = 4, kTsSets = 4;
+constexpr int kTsOuts = 128, kTsMaxTok = 256, kTsStepTiles = 4;      // k-step: 4 tile rows
+constexpr int kTsAStages = 8, kTsACol0 = 256;       // tensor memory: D in columns 0..255, A stages behind it
+constexpr int kTsMaxXStages = 8;
+constexpr int kTsCtrlBytes = 1024;
+constexpr int kTsHBytes = 128 * 128 * 2, kTsYBytes = 128 * 128 * 2;
+constexpr int kTsHOff = kTsCtrlBytes, kTsYOff = kTsHOff + kTsHBytes, kTsWOff = kTsYOff + kTsYBytes;
+constexpr int kTsSmemBytes = 227 * 1024;
 
-template <int K> struct GemmLayout {
+template <int K> struct TsLayout {
     static constexpr int kTileWords = 8 * K;
-    static constexpr int kWBytes = 64 * kTileWords * 4;                  // 16 x 4 packed tiles
-    static constexpr int kStageBytes = 2 * kABytes + kBBytes + kWBytes;  // 64 KiB + 2K KiB
-    static constexpr int kStages = (227 * 1024 - kGemmCtrlBytes) / kStageBytes >= 3 ? 3 : 2;
-    static constexpr int kSmemBytes = kGemmCtrlBytes + kStages * kStageBytes;
+    static constexpr int kWBytes = 32 * kTileWords * 4;                 // 8 x 4 packed tiles: K KiB
+    static constexpr int kXOff = kTsWOff + kTsAStages * kWBytes;
+    static constexpr int kXRoom = kTsSmemBytes - kXOff;
+    // tokens per tile of a dense launch: at least four stages of activations have to fit
+    static constexpr int kTok = kXRoom / 512 >= kTsMaxTok ? kTsMaxTok : kXRoom / 512 / 16 * 16;
 };
 
-// Two codewords -> (w_a, w_b) fp16, with the XOR constant as a run-time value (one LOP3).
-template <int CB> __device__ __forceinline__ uint32_t decode_pair_rt(uint32_t cw_a, uint32_t cw_b, uint32_t xc)
-{
-    const uint32_t xa = codebook_word_rt<CB>(cw_a, xc);
-    const uint32_t xb = codebook_word_rt<CB>(cw_b, xc);
-    if (CB == CB_MUL1) {
-        const uint32_t s = xa | (xb << 16);
-        return h2_as_u32(__hfma2(u32_as_h2(s), u32_as_h2(0x1EEE1EEEu), u32_as_h2(0xC931C931u)));
+// Bounded wait.  It has no result, so that the code behind it stays warp-uniform for the compiler; a
+// wait that gives up raises the CTA's abort word, which ends all later waits at once, and the kernel
+// runs to its end without meaning.  Nothing here legitimately waits for longer than the kernels in
+// front of it in the stream run.
+struct TsWait {
+    volatile int* abort_word;      // shared memory
+    int* status;
+    __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity) const
+    {
+        const uint32_t b = smem_u32(bar);
+        if (mbar_try_wait(b, parity)) return;
+#pragma unroll 1
+        for (uint32_t i = 0; i < kWaitSpins; i++) {
+            if (mbar_try_wait(b, parity)) return;
+            if ((i & 15u) == 15u && *abort_word) return;
+        }
+        *abort_word = 1;
+        atomicOr(status, ST_TC_TIMEOUT);
     }
-    const uint32_t lo = __byte_perm(xa, xb, 0x5410);
-    const uint32_t hi = __byte_perm(xa, xb, 0x7632);
-    return h2_as_u32(__hadd2(u32_as_h2(lo), u32_as_h2(hi)));
+};
+
+// ---- tensor memory as an operand and as a destination of registers ------------------------------------
+// D[tmem] (+)= A[tmem] * B[smem]; issued by ONE thread.
+__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                              uint32_t accumulate)
+{
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// 16 lanes x 32 columns: register 4 t + {0, 1, 2, 3} of lane l is column 8 t + {0, 0, 4, 4} + l % 4 of tensor-
+// memory lane l / 4 + {0, 8, 0, 8}: four 16x16 fp16 fragments side by side.
+__device__ __forceinline__ void tmem_st_16x32cols(uint32_t taddr, const uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(
+            taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+// 16 consecutive fp32 columns of this thread's tensor-memory lane.
+__device__ __forceinline__ void tmem_ld_16cols(uint32_t taddr, float (&v)[16])
+{
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
 // One 32-byte store (sm_100: 256-bit vector stores); p must be 32-byte aligned.
@@ -79,271 +131,394 @@ __device__ __forceinline__ void st_global_256(void* p, const uint4& a, const uin
                  : "memory");
 }
 
-// In-register 128-point Sylvester Hadamard (un-normalised).
-__device__ __forceinline__ void had128_regs(float (&v)[128])
+// Two codewords -> (w_a, w_b) fp16, with the XOR constant as a run-time value (one LOP3).  Each word's
+// halves are added by a broadcasting HADD2 and one byte permute joins the two sums.  Gathering the halves
+// with two byte permutes and adding once is one operation on either side too, but the logic pipe bounds
+// the decode (14 of its clocks per tile that way, 11 this way) and the multiplier pipe is half empty.
+template <int CB> __device__ __forceinline__ uint32_t decode_pair_rt(uint32_t cw_a, uint32_t cw_b, uint32_t xc)
 {
-#pragma unroll
-    for (int h = 1; h < 128; h <<= 1)
-#pragma unroll
-        for (int i = 0; i < 128; i += 2 * h)
-#pragma unroll
-            for (int j = i; j < i + h; j++) {
-                const float a = v[j], b = v[j + h];
-                v[j] = a + b;
-                v[j + h] = a - b;
-            }
-}
-
-// One output tile: rows [m0, m_end) of the rotated activations against 256 trellis columns
-// starting at tile column tn0; outputs go to y rows (row + y_row_delta), columns y_col.. ;
-// svh / bias are read at sv_off.  Dense layers derive it from the tile index; grouped (MoE)
-// launches read it from a device table of 8 ints per tile, where m0 >= m_end marks an unused
-// slot that every role skips.
-struct GemmTile {
-    int m0, m_end, tn0, sv_off, y_col, ncols, y_row_delta;
-    int half;      // -1: all 256 columns; 0 / 1: only the first / second 128 columns of the packed box
-};
-// Dense layers: the first a.n_full_tiles work items are whole tiles; the tiles that would make up
-// a short last wave are cut into two 128-column halves each (half the decode, half the MMAs), so
-// that the last wave keeps more SMs busy for half as long.
-__device__ __forceinline__ GemmTile gemm_tile(const GemmArgs& a, int item)
-{
-    GemmTile t;
-    if (a.tile_tab) {
-        const int4 u = reinterpret_cast<const int4*>(a.tile_tab)[2 * item];
-        const int4 v = reinterpret_cast<const int4*>(a.tile_tab)[2 * item + 1];
-        t.m0 = u.x; t.m_end = u.y; t.tn0 = u.z; t.sv_off = u.w;
-        t.y_col = v.x; t.ncols = v.y; t.y_row_delta = v.z;
-        t.half = -1;
-    } else {
-        int tile = item, h = -1;
-        if (item >= a.n_full_tiles) {
-            const int j = item - a.n_full_tiles;
-            tile = a.n_full_tiles + (j >> 1);
-            h = j & 1;
-        }
-        const int n0 = (tile % a.tiles_n) * kTileN;
-        t.m0 = (tile / a.tiles_n) * kTileM;
-        t.m_end = a.m;
-        t.tn0 = n0 / 16;
-        t.half = h;
-        const int c0 = n0 + (h > 0 ? 128 : 0);
-        t.sv_off = c0;
-        t.y_col = c0;
-        t.ncols = h < 0 ? a.t_out * 16 - n0 : min(128, a.t_out * 16 - c0);
-        t.y_row_delta = 0;
-        if (t.ncols <= 0) t.m_end = t.m0;      // a second half beyond the last column: nothing to do
+    const uint32_t xa = codebook_word_rt<CB>(cw_a, xc), xb = codebook_word_rt<CB>(cw_b, xc);
+    if (CB == CB_MUL1) {
+        const uint32_t s = xa | (xb << 16);
+        return h2_as_u32(__hfma2(u32_as_h2(s), u32_as_h2(0x1EEE1EEEu), u32_as_h2(0xC931C931u)));
     }
-    return t;
+    const __half2 ha = u32_as_h2(xa), hb = u32_as_h2(xb);
+    return __byte_perm(h2_as_u32(__hadd2(__low2half2(ha), __high2half2(ha))),
+                       h2_as_u32(__hadd2(__low2half2(hb), __high2half2(hb))), 0x5410);
 }
 
-template <int K, int CB>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-    gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x,
-                const __grid_constant__ CUtensorMap tm_w)
+// MN-major operand in the 128-byte-swizzled layout: 64 elements of the M (or N) index per 128-byte row,
+// one row per k, 8-row groups 1024 bytes apart, the next 64 elements 128 rows (16 KiB) further on.
+__device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t smem_addr)
 {
-    using L = GemmLayout<K>;
-    constexpr int NS = L::kStages;
-    extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* a_full = reinterpret_cast<uint64_t*>(smem);      // activations + packed tiles landed
-    uint64_t* b_full = a_full + 4;                             // decoded B tile written
-    uint64_t* empty = b_full + 4;                              // MMAs that read the stage are done
-    uint64_t* tmem_full = empty + 4;                           // accumulators complete
-    uint64_t* tmem_empty = tmem_full + 1;                      // accumulators drained
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 1);
-    uint8_t* stage0 = smem + kGemmCtrlBytes;
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(16384 >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+constexpr uint32_t kIdescMajorA = 1u << 15;          // A is MN-major
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nks = a.t_in / 4;                                // 64-wide k-steps
-    const int n_tiles = a.n_items;                             // work items: tiles, or tiles and half tiles
+// One stretch of k-steps of one output tile.
+struct TsSeg {
+    int m0, rows;            // first row of xh, rows in use
+    int tn0;                 // first tile column of the trellis
+    int sv_off, y_col, y_row_delta;
+    int k0, k1;              // k-steps
+    int tile;                // tile number (dense launches)
+    int first;               // first segment of this CTA's range
+};
+
+// The segments of one CTA, the same sequence for every role.
+template <bool TABLE> struct TsWalk {
+    // the same value in every lane already; the broadcast tells the compiler
+    static __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+    int64_t u, u1, u0;
+    int item;
+    __device__ __forceinline__ void start(const GemmArgs& a)
+    {
+        item = (int)blockIdx.x;
+        const int64_t g = gridDim.x, c = blockIdx.x, nks = a.t_in >> 2;
+        if (a.ts_split) {
+            u0 = a.n_items * nks * c / g;
+            u1 = a.n_items * nks * (c + 1) / g;
+        } else {
+            u0 = a.n_items * c / g * nks;
+            u1 = a.n_items * (c + 1) / g * nks;
+        }
+        u = u0;
+    }
+    __device__ __forceinline__ bool next(const GemmArgs& a, TsSeg& s)
+    {
+        const int nks = a.t_in >> 2;
+        if (TABLE) {
+            for (; item < a.n_items; item += gridDim.x) {
+                const int h = item & 1;
+                int4 p = reinterpret_cast<const int4*>(a.tile_tab)[item & ~1];
+                int4 q = reinterpret_cast<const int4*>(a.tile_tab)[item | 1];
+                p.x = uniform(p.x); p.y = uniform(p.y); p.z = uniform(p.z); p.w = uniform(p.w);
+                q.x = uniform(q.x); q.y = uniform(q.y); q.z = uniform(q.z);
+                if (p.x >= p.y || 128 * h >= q.y) continue;
+                s.m0 = p.x; s.rows = p.y - p.x;
+                s.tn0 = p.z + 8 * h; s.sv_off = p.w + 128 * h;
+                s.y_col = q.x + 128 * h; s.y_row_delta = q.z;
+                s.k0 = 0; s.k1 = nks; s.tile = item; s.first = 1;
+                item += gridDim.x;
+                return true;
+            }
+            return false;
+        }
+        if (u >= u1) return false;
+        s.first = u == u0;
+        s.tile = uniform((int)(u / nks));
+        s.k0 = uniform((int)(u - (int64_t)s.tile * nks));
+        s.k1 = uniform((int)min((int64_t)nks, s.k0 + (u1 - u)));
+        u += s.k1 - s.k0;
+        const int tn = uniform(s.tile / a.tiles_m), tm = s.tile - tn * a.tiles_m;
+        s.m0 = tm * a.ts_tok;
+        s.rows = min(a.ts_tok, a.m - s.m0);
+        s.tn0 = 8 * tn;
+        s.sv_off = s.y_col = 128 * tn;
+        s.y_row_delta = 0;
+        return true;
+    }
+};
+
+template <int K, int CB, bool TABLE>
+__global__ void __launch_bounds__(kTsThreads, 1)
+    gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w)
+{
+    using L = TsLayout<K>;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t* w_full = reinterpret_cast<uint64_t*>(smem);      // packed tiles landed                      [8]
+    uint64_t* w_empty = w_full + kTsAStages;                   // ... read by the set's four warps          [8]
+    uint64_t* full = w_empty + kTsAStages;                     // weights decoded AND activations landed    [8]
+    uint64_t* empty = full + kTsAStages;                       // the k-step's MMAs are done                [8]
+    uint64_t* d_full = empty + kTsAStages;                   // the segment's sums are complete
+    uint64_t* d_empty = d_full + 1;                            // ... and drained
+    uint64_t* h_full = d_empty + 1;                            // the rotated tile is complete
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(h_full + 1);
+    volatile int* handoff = reinterpret_cast<volatile int*>(tmem_slot + 2);
+    const TsWait wait{reinterpret_cast<volatile int*>(tmem_slot + 1), a.status};
+    uint8_t* h_mat = smem + kTsHOff;
+    uint8_t* y_buf = smem + kTsYOff;
+    uint8_t* w_ring = smem + kTsWOff;
+    uint8_t* x_ring = smem + L::kXOff;
+
+    const int tid = threadIdx.x, warp = TsWalk<TABLE>::uniform(tid >> 5), lane = tid & 31;
+    const int nx = a.stages, x_bytes = a.ts_x_bytes;           // depth and stage size of ring x
+    TsWalk<TABLE> walk;
+    walk.start(a);
+    TsSeg sg;
 
     if (tid == 0) {
-        for (int s = 0; s < NS; s++) {
-            mbar_init(smem_u32(&a_full[s]), 1);
-            mbar_init(smem_u32(&b_full[s]), kGemmDecodeWarps);
+        *wait.abort_word = 0;
+        for (int s = 0; s < kTsAStages; s++) {
+            mbar_init(smem_u32(&w_full[s]), 1);
+            mbar_init(smem_u32(&w_empty[s]), 4);
+            mbar_init(smem_u32(&full[s]), 5);                  // a set's four warps and the activations' copy
             mbar_init(smem_u32(&empty[s]), 1);
         }
-        mbar_init(smem_u32(tmem_full), 1);
-        mbar_init(smem_u32(tmem_empty), kGemmDecodeWarps);
+        mbar_init(smem_u32(d_full), 1);
+        mbar_init(smem_u32(d_empty), kTsDecodeWarps);
+        mbar_init(smem_u32(h_full), 1);
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
+    if (warp == 2) tmem_alloc(smem_u32(tmem_slot), 512);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = (uint32_t)TsWalk<TABLE>::uniform((int)*tmem_slot);
+    griddep_launch_dependents();
 
+    // The three single-issuer roles run as whole warps with one elected lane issuing: loop control,
+    // addresses and descriptors then stay in uniform registers, where TMA and tcgen05.mma take them.
+    // Written as one lane's code, an MMA k-step took 570 clocks to issue and a TMA box about 200.
     if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer ----
-        if (lane == 0) {
-            tma_prefetch_desc(&tm_x);
-            tma_prefetch_desc(&tm_w);
-            int s = 0;
-            uint32_t parity = 0;
-            bool first_pass = true;
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-                const GemmTile ti = gemm_tile(a, tile);
-                if (ti.m0 >= ti.m_end) continue;
-                const int m0 = ti.m0, tn0 = ti.tn0;
-                const bool two = ti.m_end - ti.m0 > a.one_acc_rows;   // tiles of up to 128 rows use one accumulator
-                for (int ks = 0; ks < nks; ks++) {
-                    if (!first_pass && !mbar_wait(smem_u32(&empty[s]), parity ^ 1u)) {
-                        atomicOr(a.status, ST_TC_TIMEOUT);
-                        goto done;
-                    }
-                    uint8_t* st = stage0 + (size_t)s * L::kStageBytes;
-                    const uint32_t bar = smem_u32(&a_full[s]);
-                    mbar_arrive_expect_tx(bar, (two ? 2 : 1) * kABytes + L::kWBytes);
-                    tma_load_2d(smem_u32(st), &tm_x, ks * kStepK, m0, bar);
-                    if (two) tma_load_2d(smem_u32(st + kABytes), &tm_x, ks * kStepK, m0 + 128, bar);
-                    tma_load_3d(smem_u32(st + 2 * kABytes + kBBytes), &tm_w, 0, tn0, 4 * ks, bar);
-                    if (++s == NS) { s = 0; parity ^= 1u; first_pass = false; }
+        // ------------------------------------------------------------------ packed tiles ----
+        const bool leader = elect_one();
+        if (leader) tma_prefetch_desc(&tm_w);
+        if (TABLE) griddep_wait();                        // the table belongs to an earlier kernel
+        int s = 0;
+        uint32_t parity = 1;                                   // (a wait for the phase before the first passes)
+        while (walk.next(a, sg)) {
+            for (int ks = sg.k0; ks < sg.k1; ks++) {
+                wait(&w_empty[s], parity);
+                if (leader) {
+                    const uint32_t bar = smem_u32(&w_full[s]);
+                    mbar_arrive_expect_tx(bar, L::kWBytes);
+                    tma_load_3d(smem_u32(w_ring) + s * L::kWBytes, &tm_w, 0, sg.tn0, kTsStepTiles * ks, bar);
                 }
+                if (++s == kTsAStages) { s = 0; parity ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        // -------------------------------------------------------------------- MMA issuer ----
-        if (lane == 0) {
-            int s = 0;
-            uint32_t parity = 0, tile_parity = 0;
-            bool first_tile = true;
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-                bool two;
-                uint32_t idesc;
-                {
-                    const GemmTile ti = gemm_tile(a, tile);
-                    if (ti.m0 >= ti.m_end) continue;
-                    two = ti.m_end - ti.m0 > a.one_acc_rows;
-                    idesc = ti.half < 0 ? mma_idesc_f16(128, kTileN) : mma_idesc_f16(128, 128);
+        // ------------------------------------------------------------------- activations ----
+        const bool leader = elect_one();
+        if (leader) tma_prefetch_desc(&tm_x);
+        griddep_wait();
+        const int box_rows = a.ts_box_rows, box_bytes = box_rows * 128;
+        // The copy counts on the barrier of the k-step's tensor-memory stage.  A stage of this ring is free
+        // when the MMAs of the k-step nx before are done (nx <= 8: that barrier cannot be a turn ahead).
+        int s = 0, v = 0;
+        while (walk.next(a, sg)) {
+            const int boxes = (sg.rows + box_rows - 1) / box_rows;
+            for (int ks = sg.k0; ks < sg.k1; ks++, v++) {
+                const int u = v - nx;
+                if (u >= 0) wait(&empty[u & (kTsAStages - 1)], (uint32_t)(u / kTsAStages) & 1u);
+                if (leader) {
+                    const uint32_t bar = smem_u32(&full[v & (kTsAStages - 1)]);
+                    const uint32_t dst = smem_u32(x_ring) + (uint32_t)(s * x_bytes);
+                    mbar_arrive_expect_tx(bar, (uint32_t)(boxes * box_bytes));
+                    tma_load_2d(dst, &tm_x, ks * 64, sg.m0, bar);
+                    for (int b = 1; b < boxes; b++)
+                        tma_load_2d(dst + b * box_bytes, &tm_x, ks * 64, sg.m0 + box_rows * b, bar);
                 }
-                if (!first_tile) {   // the epilogue of the previous tile must have drained D
-                    if (!mbar_wait(smem_u32(tmem_empty), tile_parity ^ 1u)) {
-                        atomicOr(a.status, ST_TC_TIMEOUT);
-                        goto done;
-                    }
-                }
-                tc_fence_after_sync();
-                for (int ks = 0; ks < nks; ks++) {
-                    if (!mbar_wait(smem_u32(&a_full[s]), parity) ||
-                        !mbar_wait(smem_u32(&b_full[s]), parity)) {
-                        atomicOr(a.status, ST_TC_TIMEOUT);
-                        goto done;
-                    }
-                    tc_fence_after_sync();
-                    const uint32_t sa = smem_u32(stage0 + (size_t)s * L::kStageBytes);
-#pragma unroll
-                    for (int kk = 0; kk < kStepK / 16; kk++) {
-                        const uint64_t da0 = smem_desc_sw128(sa + kk * 32);
-                        const uint64_t da1 = smem_desc_sw128(sa + kABytes + kk * 32);
-                        const uint64_t db = smem_desc_sw128(sa + 2 * kABytes + kk * 32);
-                        const uint32_t accum = (ks | kk) != 0 ? 1u : 0u;
-                        tc_mma_f16(tmem_base, da0, db, idesc, accum);
-                        if (two) tc_mma_f16(tmem_base + kTileN, da1, db, idesc, accum);
-                    }
-                    tc_commit(smem_u32(&empty[s]));
-                    if (++s == NS) { s = 0; parity ^= 1u; }
-                }
-                tc_commit(smem_u32(tmem_full));
-                first_tile = false;
-                tile_parity ^= 1u;
+                if (++s == nx) s = 0;
             }
         }
-    } else {
-        // ------------------------------------------------------- decode, then epilogue ----
-        const int dw = warp - 2;
-        const int g = lane >> 2, q = lane & 3;
+    } else if (warp == 2) {
+        // -------------------------------------------------------------------- MMA issuer ----
+        const bool leader = elect_one();
+        if (TABLE) griddep_wait();
+        int xs = 0, as = 0;
+        uint32_t parity = 0, dpar = 1;
+        const uint32_t x0 = smem_u32(x_ring);
+        while (walk.next(a, sg)) {
+            wait(d_empty, dpar);
+            dpar ^= 1u;
+            tc_fence_after_sync();
+            const uint32_t idesc = mma_idesc_f16(128, (sg.rows + 15) & ~15);
+            uint32_t accum = 0;
+            for (int ks = sg.k0; ks < sg.k1; ks++) {
+                const uint32_t at = tmem_base + kTsACol0 + 32 * as;
+                const uint64_t xd = smem_desc_sw128(x0 + (uint32_t)(xs * x_bytes));
+                wait(&full[as], parity);
+                tc_fence_after_sync();
+                if (leader) {                                  // 16 k = 8 columns of A, 32 bytes of B
+                    tc_mma_f16_ts(tmem_base, at, xd, idesc, accum);
+                    tc_mma_f16_ts(tmem_base, at + 8, xd + 2, idesc, 1u);
+                    tc_mma_f16_ts(tmem_base, at + 16, xd + 4, idesc, 1u);
+                    tc_mma_f16_ts(tmem_base, at + 24, xd + 6, idesc, 1u);
+                    tc_commit(smem_u32(&empty[as]));
+                }
+                accum = 1u;
+                if (++xs == nx) xs = 0;
+                if (++as == kTsAStages) { as = 0; parity ^= 1u; }
+            }
+            if (leader) tc_commit(smem_u32(d_full));
+        }
+    } else if (warp >= kTsFirstDecodeWarp) {
+        // -------------------------------------------------------- decode, then finish ----
+        const int dt = tid - 32 * kTsFirstDecodeWarp;
+        const int q = warp & 3, set = (warp - kTsFirstDecodeWarp) >> 2;
         const int prev_word = (lane + 31) & 31;
         const uint32_t xc = a.cb_xor;
+        const int nks = a.t_in >> 2;
         LaneWords<K> lw;
         lw.init(lane);
-        int s = 0;
-        uint32_t parity = 0, tile_parity = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            const GemmTile ti = gemm_tile(a, tile);
-            if (ti.m0 >= ti.m_end) continue;
-            const int m0 = ti.m0;
-            for (int ks = 0; ks < nks; ks++) {
-                // all lanes take the same decision: the tensor-memory loads below are warp-wide
-                if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&a_full[s]), parity))) {
-                    if (lane == 0) atomicOr(a.status, ST_TC_TIMEOUT);
-                    goto done;
-                }
-                uint8_t* st = stage0 + (size_t)s * L::kStageBytes;
-                uint8_t* bt = st + 2 * kABytes;
-                const uint32_t* wt = reinterpret_cast<const uint32_t*>(bt + kBBytes);
-                // All packed words of the warp's eight tiles are fetched before the first store: the
-                // stores into the B tile could alias the packed words as far as the compiler knows,
-                // so loads written after them would wait for them, tile after tile.
-                // Whole tile: this warp decodes tile columns 2 dw, 2 dw + 1 of all four tile rows; half
-                // tile: column 8 half + dw of the box, stored as column dw of a 128-column B tile.
-                const int n_mine = ti.half < 0 ? 8 : 4;
-                uint32_t pw[8][3];
+        // H[n][k] = (-1)^popcount(n & k), K-major: two 64-wide halves of k, 128 rows of 128 bytes each
+        {
+            uint32_t w4[4];                                        // the low three bits of k: the same for all of a thread's pieces
+            const int n_low = (dt >> 3) & 7;
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (i < n_mine) {
-                        const int tk = ti.half < 0 ? i >> 1 : i;
-                        const int tn = ti.half < 0 ? 2 * dw + (i & 1) : 8 * ti.half + dw;
-                        const uint32_t* tw = wt + (tk * 16 + tn) * L::kTileWords;
+            for (int j = 0; j < 4; j++)
+                w4[j] = 0x3C003C00u | ((__popc(n_low & (2 * j)) & 1) ? 0x8000u : 0u) | ((__popc(n_low & (2 * j + 1)) & 1) ? 0x80000000u : 0u);
+#pragma unroll
+            for (int i = dt; i < 2048; i += 512) {
+                const int kh = i >> 10, n = (i >> 3) & 127, ch = i & 7;
+                const uint32_t flip = (__popc(n & (64 * kh + 8 * ch)) & 1) ? 0x80008000u : 0u;
+                *reinterpret_cast<uint4*>(h_mat + kh * 16384 + n * 128 + ((ch ^ (n & 7)) << 4)) =
+                    make_uint4(w4[0] ^ flip, w4[1] ^ flip, w4[2] ^ flip, w4[3] ^ flip);
+            }
+        }
+        if (TABLE) griddep_wait();
+        int kc = 0;                                                // k-steps of this CTA so far
+        uint32_t dpar = 0, hpar = 0;
+        while (walk.next(a, sg)) {
+            const int n_steps = sg.k1 - sg.k0;
+            for (int v = kc + ((set - kc) & 3); v < kc + n_steps; v += kTsSets) {
+                // Eight stages, four sets: a stage of ring w always belongs to the same set.  (With another number a
+                // set could look at a barrier two phases early and read a stale parity.)
+                const int st = v & (kTsAStages - 1);
+                const uint32_t parity = (uint32_t)(v / kTsAStages) & 1u;
+                wait(&w_full[st], parity);
+                // tile columns 2q, 2q + 1 of all four tile rows: words first, so that the slot can be refilled
+                const uint32_t* wt = reinterpret_cast<const uint32_t*>(w_ring + st * L::kWBytes) + 2 * q * L::kTileWords;
+                uint32_t pw[2][4][K == 4 ? 4 : 3];
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int tk = 0; tk < 4; tk++) {
+                        const uint32_t* tw = wt + (tk * 8 + h) * L::kTileWords;
                         if (K == 4) {
-                            pw[i][0] = tw[lane];
-                            pw[i][1] = tw[prev_word];
-                            pw[i][2] = 0u;
+                            pw[h][tk][0] = tw[lane];
+                            pw[h][tk][1] = tw[prev_word];
+                            pw[h][tk][2] = reinterpret_cast<const uint16_t*>(tw)[2 * lane];        // the two 16-bit aligned
+                            pw[h][tk][3] = reinterpret_cast<const uint16_t*>(tw)[2 * lane + 1];    // windows
                         } else {
-                            pw[i][0] = tw[lw.i0];
-                            pw[i][1] = tw[lw.i1];
-                            pw[i][2] = LaneWords<K>::kThree ? tw[lw.i2] : 0u;
+                            pw[h][tk][0] = tw[lw.i0];
+                            pw[h][tk][1] = tw[lw.i1];
+                            pw[h][tk][2] = LaneWords<K>::kThree ? tw[lw.i2] : 0u;
                         }
                     }
-                }
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (i < n_mine) {
-                        const int tk = ti.half < 0 ? i >> 1 : i;
-                        const int tn = ti.half < 0 ? 2 * dw + (i & 1) : dw;
-                        uint32_t cw[8];
-                        if (K == 4) lane_codewords_k4(pw[i][0], pw[i][1], cw);
-                        else lane_codewords<K>(pw[i][0], pw[i][1], pw[i][2], lw.sh, cw);
-                        // B[n][k] K-major, 128B swizzle: n = 16 tn + g (+8), k = 16 tk + 2q (+8)
-                        uint8_t* row = bt + (2 * tn) * 1024 + g * 128 + 4 * q;
-                        const int c0 = ((2 * tk) ^ g) << 4, c1 = ((2 * tk + 1) ^ g) << 4;
-                        *reinterpret_cast<uint32_t*>(row + c0) = decode_pair_rt<CB>(cw[0], cw[1], xc);
-                        *reinterpret_cast<uint32_t*>(row + 1024 + c0) = decode_pair_rt<CB>(cw[4], cw[5], xc);
-                        *reinterpret_cast<uint32_t*>(row + c1) = decode_pair_rt<CB>(cw[2], cw[3], xc);
-                        *reinterpret_cast<uint32_t*>(row + 1024 + c1) = decode_pair_rt<CB>(cw[6], cw[7], xc);
-                    }
-                }
-                fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&b_full[s]));
-                if (++s == NS) { s = 0; parity ^= 1u; }
-            }
-
-            // ---- epilogue of this tile ----
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(tmem_full), tile_parity))) {
-                if (lane == 0) atomicOr(a.status, ST_TC_TIMEOUT);
-                goto done;
-            }
-            tile_parity ^= 1u;
-            tc_fence_after_sync();
-            const int quarter = warp & 3, chalf = dw >> 2;
-            const int col0 = ti.y_col + 128 * chalf, sv0 = ti.sv_off + 128 * chalf;
-            if (128 * chalf < ti.ncols) {
-#pragma unroll 1
-                for (int acc = 0; acc < (ti.m_end - m0 > a.one_acc_rows ? 2 : 1); acc++) {
-                    const int row = m0 + 128 * acc + 32 * quarter + lane;
-                    const uint32_t taddr =
-                        tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(kTileN * acc + 128 * chalf);
-                    float v[128];
+                if (lane == 0) mbar_arrive(smem_u32(&w_empty[st]));
+                wait(&empty[st], parity ^ 1u);
+                tc_fence_after_sync();
 #pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        float t32[32];
-                        tmem_ld_32cols(taddr + 32 * c, t32);
+                for (int h = 0; h < 2; h++) {
+                    uint32_t frag[16];
 #pragma unroll
-                        for (int i = 0; i < 32; i++) v[32 * c + i] = __half2float(__float2half_rn(t32[i]));
+                    for (int tk = 0; tk < 4; tk++) {
+                        uint32_t cw[8];
+                        if constexpr (K == 4) lane_codewords_k4_halves(pw[h][tk][0], pw[h][tk][1], pw[h][tk][2], pw[h][tk][3], cw);
+                        else lane_codewords<K>(pw[h][tk][0], pw[h][tk][1], pw[h][tk][2], lw.sh, cw);
+                        frag[4 * tk + 0] = decode_pair_rt<CB>(cw[0], cw[1], xc);
+                        frag[4 * tk + 1] = decode_pair_rt<CB>(cw[4], cw[5], xc);
+                        frag[4 * tk + 2] = decode_pair_rt<CB>(cw[2], cw[3], xc);
+                        frag[4 * tk + 3] = decode_pair_rt<CB>(cw[6], cw[7], xc);
                     }
-                    had128_regs(v);
-                    if (row < ti.m_end) {
-                        const int orow = a.y_row_map ? a.y_row_map[row + ti.y_row_delta] : row + ti.y_row_delta;
+                    tmem_st_16x32cols(tmem_base + ((uint32_t)(32 * q + 16 * h) << 16) + kTsACol0 + 32 * st, frag);
+                }
+                tmem_st_wait();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&full[st]));
+            }
+            kc += n_steps;
+
+            // ---- the segment's sums are complete ----
+            wait(d_full, dpar);
+            dpar ^= 1u;
+            tc_fence_after_sync();
+            const uint32_t lane_base = tmem_base + ((uint32_t)(32 * q) << 16);
+            const int out = 32 * q + lane;                         // this thread's column of the tile
+            const int n16 = (sg.rows + 15) >> 4;
+            const size_t slot_floats = (size_t)kTsOuts * a.ts_tok;
+            bool finish = true;
+            int c_first = 0, n_contrib = 1, slot_first = 0;
+            if (n_steps != nks) {
+                float* part = a.ts_partials + (size_t)(2 * blockIdx.x + (sg.first ? 0 : 1)) * slot_floats + out;
+                for (int ch = set; ch < n16; ch += kTsSets) {
+                    float v[16];
+                    tmem_ld_16cols(lane_base + 16 * ch, v);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) __stcg(part + (16 * ch + i) * kTsOuts, v[i]);
+                }
+                named_bar_sync(1, 512);
+                if (dt == 0) {
+                    // as in the streamed GEMV: the barrier orders the CTA's stores before this release, the
+                    // count wraps to zero with the last arrival and is an acquire for the reads below
+                    const int64_t U = (int64_t)a.n_items * nks, G = gridDim.x, f = (int64_t)sg.tile * nks;
+                    const int cf = (int)(((f + 1) * G - 1) / U), cl = (int)(((f + nks) * G - 1) / U);
+                    unsigned old;
+                    asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;"
+                                 : "=r"(old) : "l"(a.ts_ctr + cf), "r"((unsigned)(cl - cf)) : "memory");
+                    handoff[0] = old == (unsigned)(cl - cf) ? 1 : 0;
+                    handoff[1] = cf;
+                    handoff[2] = cl - cf + 1;
+                    handoff[3] = U * cf / G == f ? 0 : 1;
+                }
+                named_bar_sync(1, 512);
+                finish = handoff[0] != 0;
+                c_first = handoff[1];
+                n_contrib = handoff[2];
+                slot_first = handoff[3];
+            }
+            if (finish) {
+                for (int tg = 0; 128 * tg < sg.rows; tg++) {
+                    const int ch1 = min(8 * tg + 8, n16);
+                    for (int ch = 8 * tg + set; ch < ch1; ch += kTsSets) {
+                        float v[16];
+                        if (n_steps == nks) {
+                            tmem_ld_16cols(lane_base + 16 * ch, v);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 16; i++) v[i] = 0.f;
+#pragma unroll 2
+                            for (int j = 0; j < n_contrib; j++) {  // in CTA order
+                                const float* p = a.ts_partials + (size_t)(2 * (c_first + j) + (j == 0 ? slot_first : 0)) * slot_floats +
+                                                 out + (size_t)(16 * ch) * kTsOuts;
+#pragma unroll
+                                for (int i = 0; i < 16; i++) v[i] += __ldcg(p + i * kTsOuts);
+                            }
+                        }
+                        uint32_t hv[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) hv[i] = h2_as_u32(__floats2half2_rn(v[2 * i], v[2 * i + 1]));
+                        const int c16 = ch & 7;                    // 16 tokens = two 16-byte pieces of a 64-token row
+                        uint8_t* row = y_buf + (c16 >> 2) * 16384 + out * 128;
+                        const int piece = 2 * (c16 & 3), sw = out & 7;
+                        *reinterpret_cast<uint4*>(row + ((piece ^ sw) << 4)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+                        *reinterpret_cast<uint4*>(row + (((piece + 1) ^ sw) << 4)) = make_uint4(hv[4], hv[5], hv[6], hv[7]);
+                    }
+                    fence_proxy_async_smem();
+                    tc_fence_before_sync();
+                    named_bar_sync(1, 512);
+                    if (dt == 0) {
+                        tc_fence_after_sync();
+                        const uint32_t ya = smem_u32(y_buf), hb = smem_u32(h_mat);
+#pragma unroll
+                        for (int kk = 0; kk < 8; kk++)
+                            tc_mma_f16(tmem_base + 128 * tg, smem_desc_mn_sw128(ya + kk * 2048),
+                                       smem_desc_sw128(hb + (kk >> 2) * 16384 + (kk & 3) * 32),
+                                       mma_idesc_f16(128, 128) | kIdescMajorA, kk > 0 ? 1u : 0u);
+                        tc_commit(smem_u32(h_full));
+                    }
+                    __syncwarp();
+                    wait(h_full, hpar);
+                    hpar ^= 1u;
+                    tc_fence_after_sync();
+                    float v[32];
+                    tmem_ld_32cols(lane_base + 128 * tg + 32 * set, v);
+                    const int row = 128 * tg + 32 * q + lane;      // lane = token now
+                    if (row < sg.rows) {
+                        const int grow = sg.m0 + row + sg.y_row_delta;
+                        const int orow = a.y_row_map ? a.y_row_map[grow] : grow;
+                        const int col0 = sg.y_col + 32 * set, sv0 = sg.sv_off + 32 * set;
                         __half* yp;
                         if (a.n_peer > 0) {      // the row belongs to the GPU that holds its token
                             const int pr = orow / a.rows_per_peer;
@@ -353,7 +528,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                         }
                         uint4 held = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-                        for (int c = 0; c < 16; c++) {
+                        for (int c = 0; c < 4; c++) {
                             float o[8];
 #pragma unroll
                             for (int i = 0; i < 8; i++) o[i] = v[8 * c + i] * EXL3_HAD_SCALE;
@@ -376,15 +551,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
                                 for (int i = 0; i < 4; i++) h[i] = __hadd2(h[i], u32_as_h2(bw[i]));
                             }
-                            uint4 ov;
-                            ov.x = h2_as_u32(h[0]); ov.y = h2_as_u32(h[1]);
-                            ov.z = h2_as_u32(h[2]); ov.w = h2_as_u32(h[3]);
+                            const uint4 ov = make_uint4(h2_as_u32(h[0]), h2_as_u32(h[1]), h2_as_u32(h[2]), h2_as_u32(h[3]));
                             if (!a.y_wide) {
                                 *reinterpret_cast<uint4*>(yp + 8 * c) = ov;
                             } else if (c & 1) {
-                                // 32-byte stores (whole sectors): what a row stored into another GPU's
-                                // memory travels as
-                                st_global_256(yp + 8 * (c - 1), held, ov);
+                                st_global_256(yp + 8 * (c - 1), held, ov);   // whole sectors, also into another GPU
                             } else {
                                 held = ov;
                             }
@@ -393,22 +564,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 }
             }
             tc_fence_before_sync();
+            // handoff and y_buf are read by all warps before any of them comes here again: the next use is
+            // behind the named barrier of the next shared tile
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(tmem_empty));
+            if (lane == 0) mbar_arrive(smem_u32(d_empty));
         }
     }
-done:
+    __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) {
+    if (warp == 2) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
     if (a.n_peer > 0 && tid == 0) {
         // Rows were stored into other GPUs' memory: every CTA is counted on a local counter (the
         // barrier above orders the CTA's stores before this thread's fence), and the CTA that
-        // completes the count announces this GPU's rows to every peer — one system-scope fence
-        // and one arrival per peer for the whole grid.
+        // completes the count announces this GPU's rows to every peer.
         __threadfence();
         const unsigned done = atomicAdd(a.done_ctr, 1u) + 1u;
         if (done == gridDim.x) {
@@ -422,55 +594,81 @@ done:
 
 // ---- host side ----------------------------------------------------------------------------------
 
-extern int g_gemm_one_acc_rows;   // exl3_gemm.cu: 128, or 0 from the benchmark hook (always two accumulators)
-extern int g_gemm_split_last_wave;   // exl3_gemm.cu: 1, or 0 from the benchmark hook
+// Bytes of partial sums a dense launch may use: two slots of 128 columns x (tokens of a tile) per CTA.
+inline size_t gemm_tile_partial_bytes(int64_t rows, int ctas)
+{
+    const int64_t tiles = (rows + kTsMaxTok - 1) / kTsMaxTok;
+    const int64_t tok = ((rows + tiles - 1) / tiles + 15) / 16 * 16;
+    return (size_t)ctas * 2 * kTsOuts * (size_t)tok * sizeof(float);
+}
 
-template <int K, int CB>
+int ts_plan(int64_t tiles, int nks, int sms, int64_t rows, size_t partial_bytes, int* split);   // exl3_gemm.cu
+
+template <int K, int CB, bool TABLE>
 static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, cudaStream_t s)
 {
-    using L = GemmLayout<K>;
+    using L = TsLayout<K>;
     static bool attr_set[kMaxDevices] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxDevices) return EXL3_E_UNSUPPORTED;
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_kernel<K, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             L::kSmemBytes);
+        cudaError_t e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             kTsSmemBytes);
         if (e != cudaSuccess) return note_cuda(e);
         attr_set[dev] = true;
     }
+    a.cb_xor = 0x3B603B60u;
+    const int sms = device_sm_count(), nks = a.t_in / kTsStepTiles;
+    int grid;
+    a.ts_split = 0;
+    if (TABLE) {
+        a.ts_tok = kTsMaxTok;
+        a.ts_box_rows = 64;
+        a.n_items = 2 * a.n_tiles_tab;
+        grid = std::min(a.n_items, sms);
+    } else {
+        a.tiles_m = (a.m + L::kTok - 1) / L::kTok;
+        a.ts_tok = ((a.m + a.tiles_m - 1) / a.tiles_m + 15) / 16 * 16;
+        a.tiles_m = (a.m + a.ts_tok - 1) / a.ts_tok;
+        a.ts_box_rows = a.ts_tok;
+        a.tiles_n = a.t_out / 8;
+        a.n_items = a.tiles_m * a.tiles_n;
+        grid = ts_plan(a.n_items, nks, sms, a.m, a.ts_partial_bytes, &a.ts_split);
+    }
+    a.ts_x_bytes = (a.ts_tok + a.ts_box_rows - 1) / a.ts_box_rows * a.ts_box_rows * 128;
+    a.stages = std::min(kTsMaxXStages, L::kXRoom / a.ts_x_bytes);
     CUtensorMap tm_x, tm_w;
     {
         const uint64_t in = (uint64_t)a.t_in * 16;
         const uint64_t xdims[2] = {in, (uint64_t)a.xh_rows};
         const uint64_t xstrides[1] = {in * 2};
-        const uint32_t xbox[2] = {(uint32_t)kStepK, 128u};
+        const uint32_t xbox[2] = {64u, (uint32_t)a.ts_box_rows};
         int rc = make_tensor_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, xh, xdims, xstrides, xbox,
                                  CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
         const uint64_t dims[3] = {(uint64_t)L::kTileWords, (uint64_t)a.t_out, (uint64_t)a.t_in};
         const uint64_t strides[2] = {(uint64_t)L::kTileWords * 4, (uint64_t)a.t_out * L::kTileWords * 4};
-        const uint32_t box[3] = {(uint32_t)L::kTileWords, 16u, 4u};
+        const uint32_t box[3] = {(uint32_t)L::kTileWords, 8u, (uint32_t)kTsStepTiles};
         rc = make_tensor_map(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, trellis, dims, strides, box,
                              CU_TENSOR_MAP_SWIZZLE_NONE);
         if (rc) return rc;
     }
-    a.tiles_m = (a.m + kTileM - 1) / kTileM;
-    a.tiles_n = (a.t_out * 16 + kTileN - 1) / kTileN;
-    a.cb_xor = 0x3B603B60u;
-    a.one_acc_rows = g_gemm_one_acc_rows;
-    const int sms = device_sm_count();
-    if (a.tile_tab) {
-        a.n_full_tiles = a.n_items = a.n_tiles_tab;
-    } else {
-        // a last wave that would fill at most half of the SMs is run as half tiles
-        const int n = a.tiles_m * a.tiles_n, rest = n % sms;
-        a.n_full_tiles = (n > sms && rest > 0 && 2 * rest <= sms && g_gemm_split_last_wave) ? n - rest : n;
-        a.n_items = a.n_full_tiles + 2 * (n - a.n_full_tiles);
+    return launch_kernel(gemm_kernel<K, CB, TABLE>, dim3((unsigned)grid), dim3(kTsThreads), kTsSmemBytes, s, true, a, tm_x, tm_w);
+}
+
+template <int K>
+int launch_gemm_k(const GemmArgs& a, int cb, const __half* xh, const uint32_t* trellis, cudaStream_t s)
+{
+    switch (cb) {
+        case CB_3INST:
+            return a.tile_tab ? launch_gemm_t<K, CB_3INST, true>(a, xh, trellis, s) : launch_gemm_t<K, CB_3INST, false>(a, xh, trellis, s);
+        case CB_MCG:
+            return a.tile_tab ? launch_gemm_t<K, CB_MCG, true>(a, xh, trellis, s) : launch_gemm_t<K, CB_MCG, false>(a, xh, trellis, s);
+        case CB_MUL1:
+            return a.tile_tab ? launch_gemm_t<K, CB_MUL1, true>(a, xh, trellis, s) : launch_gemm_t<K, CB_MUL1, false>(a, xh, trellis, s);
+        default: return EXL3_E_CODEBOOK;
     }
-    const int grid = std::min(a.n_items, sms);
-    gemm_kernel<K, CB><<<grid, kGemmThreads, L::kSmemBytes, s>>>(a, tm_x, tm_w);
-    return check_launch();
 }
 
 }  // namespace exl3

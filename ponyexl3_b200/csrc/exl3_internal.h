@@ -116,6 +116,7 @@ struct GemvArgs {
     int xs_bytes;              // fused rotation: bytes of rotated activations per half
     int n_slots;               // fused rotation: k-block slots of rotated activations per CTA
     int stages;                // depth of the shared-memory ring
+    int early_weights;         // weights may be fetched before the previous kernel of the stream has ended
     int stage0_off;            // byte offset of the ring inside dynamic shared memory
     // output all-gather over peer memory (tensor parallel by output tile): when n_peer > 0 every
     // finished block is stored into each rank's full-width row buffer and announced on its counter
@@ -147,8 +148,6 @@ struct GemvPlan {
 };
 GemvPlan gemv_plan(int64_t ncb, int nkb, int rows, bool table, size_t partial_bytes);
 void gemv_set_tuning(int max_grid, int fuse_x_bytes);
-void gemm_set_tuning(int one_acc_rows);                      // benchmark hook, see exl3_b200_tuning.h
-void gemm_set_pairs(int on);                                 // benchmark hook, see exl3_b200_tuning.h
 
 // ---- prefill GEMM (exl3_gemm.cuh) ---------------------------------------------------------
 struct GemmArgs {
@@ -164,9 +163,8 @@ struct GemmArgs {
     int m;                    // rows (tokens)
     int t_in, t_out;          // tiles
     int tiles_m, tiles_n;
-    int n_full_tiles, n_items; // dense: whole tiles, then two half tiles per remaining tile (see gemm_tile)
-    int stages;
-    int one_acc_rows;         // tiles with at most this many rows use only the first accumulator
+    int n_items;              // output tiles (dense), or 128-column halves of table tiles
+    int stages;               // depth of the activation ring
     uint32_t cb_xor;
     // grouped launches whose output rows live on several GPUs (expert parallelism): output row r
     // (after y_row_map) is row r % rows_per_peer of y_peer[r / rows_per_peer]; when the whole grid
@@ -177,8 +175,16 @@ struct GemmArgs {
     unsigned* ctr_peer[kMaxPeers];
     unsigned* done_ctr;       // local: CTAs that have stored all their tiles
     int y_wide;               // every output row piece is 32-byte aligned: store 32 bytes at a time
+    float* ts_partials;       // partial sums of tiles shared by several CTAs
+    size_t ts_partial_bytes;  // size of that area (0: tiles are never shared)
+    unsigned* ts_ctr;         // kGemvMaxGrid arrival counters, zero between launches
+    int ts_split;             // 1: k-steps are dealt out evenly, tiles may be shared; 0: whole tiles
+    int ts_tok;               // tokens per output tile
+    int ts_x_bytes;           // bytes of one stage of the activation ring
+    int ts_box_rows;          // rows of one activation TMA box
 };
 
+size_t gemm_partial_bytes(int64_t rows);     // room for the partial sums of a dense launch on the largest grid
 int launch_gemm(const GemmArgs& a, int k, int cb, const __half* xh, const uint32_t* trellis,
                 cudaStream_t s);
 

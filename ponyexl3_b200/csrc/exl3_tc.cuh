@@ -1,7 +1,6 @@
 // Thin wrappers over the sm_100a tensor-core instructions used by the prefill GEMM:
 // tensor-memory allocation, tcgen05.mma with shared-memory descriptors, commit to an
-// mbarrier, and tensor-memory loads for the epilogue (cta_group::1; the forms for a pair of
-// CTAs are in exl3_gemm2.cuh).
+// mbarrier, and tensor-memory loads for the epilogue (cta_group::1).
 #pragma once
 #include <stdint.h>
 
@@ -102,10 +101,6 @@ __device__ __forceinline__ void tmem_ld_32cols(uint32_t taddr, float (&v)[32])
         : "memory");
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_ld_wait()
-{
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
 }  // namespace exl3

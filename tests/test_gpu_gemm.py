@@ -86,6 +86,24 @@ def test_gemm_ragged_row_counts(mod, oracle, rows):
     _check(mod, oracle, layer, x)
 
 
+@pytest.mark.parametrize("rows,inf,outf,k,cb", [
+    (17, 4096, 128, 4, 0),      # one output tile shared by many CTAs
+    (40, 2048, 384, 3, 2),      # shared tiles, tokens not a multiple of 32
+    (250, 1024, 256, 8, 0),     # K = 8: fewer tokens per tile fit the activation ring, two token tiles
+    (257, 1152, 128, 7, 1),     # one row more than a tile, a k-range that is no multiple of the ring
+    (700, 128, 640, 1, 0),      # two k-steps per tile, whole tiles
+])
+def test_gemm_tiles_shared_between_ctas(mod, oracle, rows, inf, outf, k, cb):
+    layer = _layer(mod, k, inf, outf, seed=rows, cb=cb, bias=rows % 2 == 0)
+    x = np.random.default_rng(rows).standard_normal((rows, inf)).astype(np.float16)
+    _check(mod, oracle, layer, x)
+    m = mod.EXL3Linear(layer)
+    xd = torch.from_numpy(x).cuda()
+    first = m(xd)
+    assert all(torch.equal(m(xd), first) for _ in range(3))      # whoever finishes a shared tile
+    assert mod.ops.Workspace.get(torch.device("cuda"), 1, 128).status() == 0
+
+
 def test_gemm_many_tiles_and_k_steps(mod, oracle):
     """More tiles than one wave of k-steps per stage ring, several tiles per CTA."""
     layer = _layer(mod, 4, 2048, 1280, seed=78, bias=True)
