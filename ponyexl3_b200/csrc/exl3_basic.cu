@@ -82,6 +82,17 @@ template <> __device__ __forceinline__ void load4<float>(const float* p, float (
     v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
 }
 
+// Both rotation kernels are launched as programmatic dependents: their blocks are set up while the
+// previous kernel of the stream drains.  With EXL3_FLAG_PDL (early_trigger) the next kernel, the matmul
+// that consumes `out`, may start streaming its weights right away; without the flag it may do so once
+// everything before this kernel is complete, so that weights written just before the call are seen.
+__device__ __forceinline__ void rotation_dependency(int early_trigger)
+{
+    if (early_trigger) griddep_launch_dependents();
+    griddep_wait();
+    if (!early_trigger) griddep_launch_dependents();
+}
+
 // Rows of x may be gathered (row_src) and the scale vectors chosen per output row
 // (pre_row / post_row give the row of the pre / post matrix to use), which is what the
 // sibling-group and MoE paths need; the plain rotation passes NULL for all three.
@@ -91,12 +102,9 @@ __global__ void __launch_bounds__(256)
                     const __half* __restrict__ pre, const __half* __restrict__ post,
                     __half* __restrict__ out, const int32_t* __restrict__ row_src,
                     const int32_t* __restrict__ pre_row, const int32_t* __restrict__ post_row,
-                    int wait_dependency, int out_mode, int glu)
+                    int early_trigger, int out_mode, int glu)
 {
-    // Let the next kernel of the stream (the GEMV that consumes `out`) start streaming its
-    // weights right away; it waits for this grid before it reads any activation.
-    griddep_launch_dependents();
-    if (wait_dependency) griddep_wait();
+    rotation_dependency(early_trigger);
     // 32-bit block arithmetic (the launcher refuses more than 2^31 blocks): the 64-bit divisions
     // that split a block index into (row, block of the row) cost more than the butterfly itself
     const int lane = threadIdx.x & 31;
@@ -226,10 +234,9 @@ __global__ void __launch_bounds__(256, 2)
     hadamard_mma_kernel(const T* __restrict__ x, int64_t rows, int64_t n, int64_t x_row_stride,
                         const __half* __restrict__ pre, __half* __restrict__ out,
                         const int32_t* __restrict__ row_src, const int32_t* __restrict__ pre_row,
-                        const int32_t* __restrict__ rows_dev, int wait_dependency, int glu)
+                        const int32_t* __restrict__ rows_dev, int early_trigger, int glu)
 {
-    griddep_launch_dependents();
-    if (wait_dependency || rows_dev) griddep_wait();
+    rotation_dependency(early_trigger);
     if (rows_dev) {           // the number of rows in use was left on the device by an earlier kernel
         const int64_t r = *rows_dev;
         rows = r < 0 ? 0 : (r < rows ? r : rows);
@@ -443,22 +450,22 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    const int wait = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
+    const int early = pdl ? 1 : 0;
     cudaError_t e;
     if (mma) {
         switch (x_dtype) {
             case EXL3_DT_F16:
                 e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<__half>, (const __half*)x, rows, n, x_row_stride, pre,
-                                       out, row_src, pre_row, rows_dev, wait, glu);
+                                       out, row_src, pre_row, rows_dev, early, glu);
                 break;
             case EXL3_DT_BF16:
                 e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x, rows, n,
-                                       x_row_stride, pre, out, row_src, pre_row, rows_dev, wait, glu);
+                                       x_row_stride, pre, out, row_src, pre_row, rows_dev, early, glu);
                 break;
             case EXL3_DT_F32:
                 e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<float>, (const float*)x, rows, n, x_row_stride, pre,
-                                       out, row_src, pre_row, rows_dev, wait, glu);
+                                       out, row_src, pre_row, rows_dev, early, glu);
                 break;
             default: return EXL3_E_DTYPE;
         }
@@ -467,16 +474,16 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
     switch (x_dtype) {
         case EXL3_DT_F16:
             e = cudaLaunchKernelEx(&cfg, hadamard_kernel<__half>, (const __half*)x, rows, n,
-                                   x_row_stride, pre, post, out, row_src, pre_row, post_row, wait, out_mode, glu);
+                                   x_row_stride, pre, post, out, row_src, pre_row, post_row, early, out_mode, glu);
             break;
         case EXL3_DT_BF16:
             e = cudaLaunchKernelEx(&cfg, hadamard_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x,
                                    rows, n, x_row_stride, pre, post, out, row_src, pre_row, post_row,
-                                   wait, out_mode, glu);
+                                   early, out_mode, glu);
             break;
         case EXL3_DT_F32:
             e = cudaLaunchKernelEx(&cfg, hadamard_kernel<float>, (const float*)x, rows, n,
-                                   x_row_stride, pre, post, out, row_src, pre_row, post_row, wait, out_mode, glu);
+                                   x_row_stride, pre, post, out, row_src, pre_row, post_row, early, out_mode, glu);
             break;
         default: return EXL3_E_DTYPE;
     }

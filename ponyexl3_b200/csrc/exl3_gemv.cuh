@@ -179,6 +179,9 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
     extern __shared__ __align__(1024) uint8_t smem[];
 
     EXL3_STAMP(gt_entry);
+    // Without EXL3_FLAG_PDL nothing is read, and no later kernel may start reading, before everything
+    // earlier in the stream is complete; the launch itself still overlaps the previous kernel's end.
+    if (!a.early_weights) griddep_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // The CTA is two independent halves of 16 warps; each is one "virtual CTA" of the partition.
     const int half = warp >> 4, wl = warp & 15, tidh = tid & (kHalfThreads - 1);
@@ -789,7 +792,8 @@ static int launch_gemv_t(GemvArgs a, bool pdl, cudaStream_t s)
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
+    a.early_weights = pdl || !XFUSED;   // behind the rotation kernel all earlier work is complete already
     return note_cuda(cudaLaunchKernelEx(&cfg, gemv_kernel<K, CB, NMMA, FAST, XFUSED>, a, tm_w, tm_x));
 }
 
