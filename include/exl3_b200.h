@@ -164,17 +164,32 @@ EXL3_API int exl3_gemv_blocks_counted(const void* x, int x_dtype, int64_t x_row_
                              int raw_out, void* workspace, size_t workspace_bytes, unsigned flags,
                              exl3_stream_t stream);
 
-/* Same contract for any number of rows (prefill): the packed tiles are decoded to fp16 in
- * shared memory and multiplied on the tensor cores (tcgen05.mma, fp32 accumulators in tensor
- * memory) against TMA-staged rotated activations; W is never materialised in global memory.
+/* Same contract for any number of rows (prefill): the packed tiles are decoded to fp16 into
+ * tensor memory and multiplied there (tcgen05.mma, fp32 accumulators) against TMA-staged rotated
+ * activations; W is never materialised in global memory.
  * Replaces the rows > 16 branches of EXL3Linear.__call__, ponyexl3/mlx/exl3_linear.py:137-161
  * (decode_full_mlx + matmul, ponyexl3/mlx/gemv_metal.py:630-774, and the striped path).
- * The workspace holds the rotated activations: exl3_gemm_workspace_bytes(rows, in). */
+ * The workspace holds the rotated activations and the partial sums of output tiles that several
+ * CTAs share: exl3_gemm_workspace_bytes(rows, in); without room for the latter tiles are not shared.
+ * flags: EXL3_FLAG_GLU_* as in exl3_gemv (x rows are [gate (in) | up (in)]). */
 EXL3_API size_t exl3_gemm_workspace_bytes(int64_t rows, int64_t in);
 EXL3_API int exl3_gemm(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, const uint16_t* trellis,
               int64_t t_in, int64_t t_out, int k, int cb, const uint16_t* suh, const uint16_t* svh,
               const uint16_t* bias, uint16_t* y, int64_t y_row_stride, void* workspace,
               size_t workspace_bytes, unsigned flags, exl3_stream_t stream);
+
+/* exl3_gemm for the members of a sibling group (same input, K and codebook; FusedEXL3Group,
+ * ponyexl3/mlx/exl3_fused.py:80-233) in one rotation and one GEMM launch: trellis holds the members
+ * side by side (t_in, t_out_total, 16K), suh_stack (n_members, in) and svh_cat (sum of the widths) their
+ * scales, member_out[i] the width of member i (a multiple of 128), y_members[i] the device address of its
+ * output rows with stride y_row_strides[i].  n_members <= 8; workspace exl3_gemm_workspace_bytes(rows *
+ * n_members, in). */
+EXL3_API int exl3_gemm_members(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride,
+                               const uint16_t* trellis, int64_t t_in, int64_t t_out_total, int k, int cb,
+                               const uint16_t* suh_stack, const uint16_t* svh_cat, int n_members,
+                               const int64_t* member_out, const uint64_t* y_members,
+                               const int64_t* y_row_strides, void* workspace, size_t workspace_bytes,
+                               unsigned flags, exl3_stream_t stream);
 
 /* The tensor-core GEMM over a TABLE of output tiles, for stacked MoE experts at prefill:
  * (token, slot) pairs are sorted by expert, so each expert owns a contiguous run of rows of

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256)
                     const __half* __restrict__ pre, const __half* __restrict__ post,
                     __half* __restrict__ out, const int32_t* __restrict__ row_src,
                     const int32_t* __restrict__ pre_row, const int32_t* __restrict__ post_row,
-                    int early_trigger, int out_mode, int glu)
+                    int early_trigger, int out_mode, int glu, int member_rows)
 {
     rotation_dependency(early_trigger);
     // 32-bit block arithmetic (the launcher refuses more than 2^31 blocks): the 64-bit divisions
@@ -126,7 +126,9 @@ __global__ void __launch_bounds__(256)
             const int64_t r = rq, b = ok ? i - rq * nblk : 0u;
             rr[u] = ok ? r : -1;
             cc[u] = b * 128 + lane * 4;
-            const int64_t rs = row_src ? row_src[r] : r;
+            // members of a sibling group rotate the same rows with their own signs, one after the other
+            const int64_t member = member_rows ? r / member_rows : 0;
+            const int64_t rs = row_src ? row_src[r] : r - member * member_rows;
             load4<T>(x + rs * x_row_stride + cc[u], v[u]);
             if (glu && ok) {
                 // the row holds [gate (n) | up (n)]: the input is fp16(act(gate) * up)
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
                 for (int q = 0; q < 4; q++) v[u][q] = glu_value(v[u][q], up[q], glu);
             }
-            if (pre) load4<__half>(pre + (pre_row ? (int64_t)pre_row[r] * n : 0) + cc[u], sp[u]);
+            if (pre) load4<__half>(pre + (pre_row ? (int64_t)pre_row[r] : member) * n + cc[u], sp[u]);
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(256, 2)
     hadamard_mma_kernel(const T* __restrict__ x, int64_t rows, int64_t n, int64_t x_row_stride,
                         const __half* __restrict__ pre, __half* __restrict__ out,
                         const int32_t* __restrict__ row_src, const int32_t* __restrict__ pre_row,
-                        const int32_t* __restrict__ rows_dev, int early_trigger, int glu)
+                        const int32_t* __restrict__ rows_dev, int early_trigger, int glu, int member_rows)
 {
     rotation_dependency(early_trigger);
     if (rows_dev) {           // the number of rows in use was left on the device by an earlier kernel
@@ -268,9 +270,13 @@ __global__ void __launch_bounds__(256, 2)
         const int64_t r0 = (int64_t)rb * 16 + g, r1 = r0 + 8;
         const bool ok0 = r0 < rows, ok1 = r1 < rows;
         const int64_t col = (int64_t)cb * 128 + 8 * t;
+        // (see hadamard_kernel)
+        const int64_t mb0 = member_rows && ok0 ? (uint32_t)r0 / (uint32_t)member_rows : 0;
+        const int64_t mb1 = member_rows && ok1 ? (uint32_t)r1 / (uint32_t)member_rows : 0;
         uint4 xa[4], xb[4];
         {
-            const int64_t s0 = ok0 ? (row_src ? row_src[r0] : r0) : 0, s1 = ok1 ? (row_src ? row_src[r1] : r1) : 0;
+            const int64_t s0 = ok0 ? (row_src ? row_src[r0] : r0 - mb0 * member_rows) : 0;
+            const int64_t s1 = ok1 ? (row_src ? row_src[r1] : r1 - mb1 * member_rows) : 0;
             const T* p0 = x + s0 * x_row_stride + col;
             const T* p1 = x + s1 * x_row_stride + col;
 #pragma unroll
@@ -296,8 +302,8 @@ __global__ void __launch_bounds__(256, 2)
             }
         }
         if (pre) {
-            const __half* q0 = pre + (ok0 && pre_row ? (int64_t)pre_row[r0] * n : 0) + col;
-            const __half* q1 = pre + (ok1 && pre_row ? (int64_t)pre_row[r1] * n : 0) + col;
+            const __half* q0 = pre + (ok0 && pre_row ? (int64_t)pre_row[r0] : mb0) * n + col;
+            const __half* q1 = pre + (ok1 && pre_row ? (int64_t)pre_row[r1] : mb1) * n + col;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const uint4 a = *reinterpret_cast<const uint4*>(q0 + 32 * q);
@@ -429,7 +435,7 @@ int launch_table(int cb, __half* table, cudaStream_t s)
 int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t x_row_stride,
                     const __half* pre, const __half* post, __half* out, const int32_t* row_src,
                     const int32_t* pre_row, const int32_t* post_row, bool pdl, int out_mode,
-                    cudaStream_t s, int glu, const int32_t* rows_dev)
+                    cudaStream_t s, int glu, const int32_t* rows_dev, int member_rows)
 {
     if (rows * (n >> 7) >= ((int64_t)1 << 31)) return EXL3_E_RANGE;   // the kernel counts blocks in 32 bits
     // Many rows into a plain fp16 matrix (the prefill GEMM's operand): 16-row blocks on the tensor cores.
@@ -457,15 +463,15 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
         switch (x_dtype) {
             case EXL3_DT_F16:
                 e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<__half>, (const __half*)x, rows, n, x_row_stride, pre,
-                                       out, row_src, pre_row, rows_dev, early, glu);
+                                       out, row_src, pre_row, rows_dev, early, glu, member_rows);
                 break;
             case EXL3_DT_BF16:
                 e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x, rows, n,
-                                       x_row_stride, pre, out, row_src, pre_row, rows_dev, early, glu);
+                                       x_row_stride, pre, out, row_src, pre_row, rows_dev, early, glu, member_rows);
                 break;
             case EXL3_DT_F32:
                 e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<float>, (const float*)x, rows, n, x_row_stride, pre,
-                                       out, row_src, pre_row, rows_dev, early, glu);
+                                       out, row_src, pre_row, rows_dev, early, glu, member_rows);
                 break;
             default: return EXL3_E_DTYPE;
         }
@@ -474,16 +480,16 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
     switch (x_dtype) {
         case EXL3_DT_F16:
             e = cudaLaunchKernelEx(&cfg, hadamard_kernel<__half>, (const __half*)x, rows, n,
-                                   x_row_stride, pre, post, out, row_src, pre_row, post_row, early, out_mode, glu);
+                                   x_row_stride, pre, post, out, row_src, pre_row, post_row, early, out_mode, glu, member_rows);
             break;
         case EXL3_DT_BF16:
             e = cudaLaunchKernelEx(&cfg, hadamard_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x,
                                    rows, n, x_row_stride, pre, post, out, row_src, pre_row, post_row,
-                                   early, out_mode, glu);
+                                   early, out_mode, glu, member_rows);
             break;
         case EXL3_DT_F32:
             e = cudaLaunchKernelEx(&cfg, hadamard_kernel<float>, (const float*)x, rows, n,
-                                   x_row_stride, pre, post, out, row_src, pre_row, post_row, early, out_mode, glu);
+                                   x_row_stride, pre, post, out, row_src, pre_row, post_row, early, out_mode, glu, member_rows);
             break;
         default: return EXL3_E_DTYPE;
     }

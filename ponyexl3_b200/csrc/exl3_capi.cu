@@ -492,51 +492,91 @@ size_t exl3_gemm_workspace_bytes(int64_t rows, int64_t in)
     return gemm_partial_offset(rows, in) + gemm_partial_bytes(rows);
 }
 
-int exl3_gemm(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, const uint16_t* trellis,
-              int64_t t_in, int64_t t_out, int k, int cb, const uint16_t* suh, const uint16_t* svh,
-              const uint16_t* bias, uint16_t* y, int64_t y_row_stride, void* workspace,
-              size_t workspace_bytes, unsigned flags, exl3_stream_t stream)
+// The dense GEMM: one layer, or the members of a sibling group (n_members > 1: suh and svh of all members
+// stacked, the trellises side by side, one output matrix per member).
+static int gemm_common(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, const uint16_t* trellis,
+                       int64_t t_in, int64_t t_out, int k, int cb, const uint16_t* suh, const uint16_t* svh,
+                       const uint16_t* bias, int n_members, const int64_t* member_out, const uint64_t* y,
+                       const int64_t* y_row_stride, void* workspace, size_t workspace_bytes, unsigned flags,
+                       exl3_stream_t stream)
 {
-    (void)flags;
-    if (!x || !trellis || !y) return EXL3_E_NULL;
+    if (!x || !trellis) return EXL3_E_NULL;
     if (k < 1 || k > 8) return EXL3_E_K;
     if (cb < 0 || cb > 2) return EXL3_E_CODEBOOK;
     if (t_in <= 0 || t_out <= 0 || t_in % 8 || t_out % 8) return EXL3_E_SHAPE;
     if (t_in > (1 << 24) || t_out > (1 << 24)) return EXL3_E_SHAPE;
-    if (rows < 1 || rows > (1 << 30)) return EXL3_E_ROWS;
-    const int64_t in = 16 * t_in, out = 16 * t_out;
-    if (x_row_stride < in || y_row_stride < out) return EXL3_E_SHAPE;
+    if (rows < 1 || rows * n_members > (1 << 30)) return EXL3_E_ROWS;
+    const int64_t in = 16 * t_in;
+    const int glu = glu_mode(flags);
+    if (x_row_stride < (glu ? 2 * in : in)) return EXL3_E_SHAPE;
     int rc = check_dtype_align(x, x_dtype, x_row_stride);
     if (rc) return rc;
-    if (!aligned(trellis, 16) || !aligned(y, 16) || y_row_stride % 8) return EXL3_E_ALIGN;
+    GemmArgs a = {};
+    bool wide = true;                                          // 32-byte stores in the epilogue
+    int64_t end = 0;
+    for (int i = 0; i < n_members; i++) {
+        if (!y[i]) return EXL3_E_NULL;
+        if (member_out[i] <= 0 || member_out[i] % 128 || y_row_stride[i] < member_out[i]) return EXL3_E_SHAPE;
+        if (y[i] % 16 || y_row_stride[i] % 8) return EXL3_E_ALIGN;
+        wide = wide && y_row_stride[i] % 16 == 0 && y[i] % 32 == 0;
+        end += member_out[i];
+        a.member_end[i] = (int)(end / 128);
+        a.member_y[i] = reinterpret_cast<__half*>(y[i]);
+        a.member_stride[i] = y_row_stride[i];
+    }
+    if (end != 16 * t_out) return EXL3_E_SHAPE;
+    if (!aligned(trellis, 16)) return EXL3_E_ALIGN;
     if ((suh && !aligned(suh, 8)) || (svh && !aligned(svh, 16)) || (bias && !aligned(bias, 16)))
         return EXL3_E_ALIGN;
     if (!workspace) return EXL3_E_WORKSPACE;
     if (!aligned(workspace, 256)) return EXL3_E_ALIGN;
-    const size_t part_off = gemm_partial_offset(rows, in);     // without room behind it tiles are not shared
+    const size_t part_off = gemm_partial_offset(rows * n_members, in);     // without room behind it tiles are not shared
     if (workspace_bytes < part_off) return EXL3_E_WORKSPACE;
 
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     __half* xh = reinterpret_cast<__half*>(ws + kWsScratch);
     cudaStream_t s = (cudaStream_t)stream;
-    rc = launch_hadamard(x, x_dtype, rows, in, x_row_stride, reinterpret_cast<const __half*>(suh), nullptr,
-                         xh, nullptr, nullptr, nullptr, false, HAD_OUT_F16, s);
+    rc = launch_hadamard(x, x_dtype, rows * n_members, in, x_row_stride, reinterpret_cast<const __half*>(suh), nullptr,
+                         xh, nullptr, nullptr, nullptr, false, HAD_OUT_F16, s, glu, nullptr, n_members > 1 ? (int)rows : 0);
     if (rc) return rc;
-    GemmArgs a = {};
     a.svh = reinterpret_cast<const __half*>(svh);
     a.bias = reinterpret_cast<const __half*>(bias);
-    a.y = reinterpret_cast<__half*>(y);
+    a.y = a.member_y[0];
     a.status = reinterpret_cast<int*>(ws + kWsStatus);
-    a.y_row_stride = y_row_stride;
+    a.y_row_stride = a.member_stride[0];
+    a.n_members = n_members;
     a.m = (int)rows;
-    a.xh_rows = (int)rows;
+    a.xh_rows = (int)rows * n_members;
     a.t_in = (int)t_in;
     a.t_out = (int)t_out;
     a.ts_partials = reinterpret_cast<float*>(ws + part_off);
     a.ts_partial_bytes = workspace_bytes - part_off;
     a.ts_ctr = reinterpret_cast<unsigned*>(ws + kWsSplitCtr);
-    a.y_wide = (y_row_stride % 16 == 0 && aligned(y, 32)) ? 1 : 0;   // 32-byte stores in the epilogue
+    a.y_wide = wide ? 1 : 0;
     return launch_gemm(a, k, cb, xh, reinterpret_cast<const uint32_t*>(trellis), s);
+}
+
+int exl3_gemm(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, const uint16_t* trellis,
+              int64_t t_in, int64_t t_out, int k, int cb, const uint16_t* suh, const uint16_t* svh,
+              const uint16_t* bias, uint16_t* y, int64_t y_row_stride, void* workspace,
+              size_t workspace_bytes, unsigned flags, exl3_stream_t stream)
+{
+    const int64_t out = 16 * t_out;
+    const uint64_t yp = reinterpret_cast<uint64_t>(y);
+    return gemm_common(x, x_dtype, rows, x_row_stride, trellis, t_in, t_out, k, cb, suh, svh, bias, 1, &out, &yp,
+                       &y_row_stride, workspace, workspace_bytes, flags, stream);
+}
+
+int exl3_gemm_members(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, const uint16_t* trellis,
+                      int64_t t_in, int64_t t_out_total, int k, int cb, const uint16_t* suh_stack,
+                      const uint16_t* svh_cat, int n_members, const int64_t* member_out, const uint64_t* y_members,
+                      const int64_t* y_row_strides, void* workspace, size_t workspace_bytes, unsigned flags,
+                      exl3_stream_t stream)
+{
+    if (!member_out || !y_members || !y_row_strides) return EXL3_E_NULL;
+    if (n_members < 1 || n_members > kMaxMembers) return EXL3_E_RANGE;
+    return gemm_common(x, x_dtype, rows, x_row_stride, trellis, t_in, t_out_total, k, cb, suh_stack, svh_cat, nullptr,
+                       n_members, member_out, y_members, y_row_strides, workspace, workspace_bytes, flags, stream);
 }
 
 struct TilePeers {

@@ -168,6 +168,7 @@ struct TsSeg {
     int sv_off, y_col, y_row_delta;
     int k0, k1;              // k-steps
     int tile;                // tile number (dense launches)
+    int member;              // sibling group: which member's output
     int first;               // first segment of this CTA's range
 };
 
@@ -204,7 +205,7 @@ template <bool TABLE> struct TsWalk {
                 s.m0 = p.x; s.rows = p.y - p.x;
                 s.tn0 = p.z + 8 * h; s.sv_off = p.w + 128 * h;
                 s.y_col = q.x + 128 * h; s.y_row_delta = q.z;
-                s.k0 = 0; s.k1 = nks; s.tile = item; s.first = 1;
+                s.k0 = 0; s.k1 = nks; s.tile = item; s.first = 1; s.member = 0;
                 item += gridDim.x;
                 return true;
             }
@@ -222,6 +223,13 @@ template <bool TABLE> struct TsWalk {
         s.tn0 = 8 * tn;
         s.sv_off = s.y_col = 128 * tn;
         s.y_row_delta = 0;
+        s.member = 0;
+        if (a.n_members > 1) {
+            while (tn >= a.member_end[s.member]) s.member++;
+            if (s.member) s.y_col -= 128 * a.member_end[s.member - 1];
+            s.m0 += s.member * a.m;
+            s.y_row_delta = -s.member * a.m;
+        }
         return true;
     }
 };
@@ -524,7 +532,8 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                             const int pr = orow / a.rows_per_peer;
                             yp = a.y_peer[pr] + (int64_t)(orow - pr * a.rows_per_peer) * a.y_row_stride + col0;
                         } else {
-                            yp = a.y + (int64_t)orow * a.y_row_stride + col0;
+                            yp = !TABLE && a.n_members > 1 ? a.member_y[sg.member] + (int64_t)orow * a.member_stride[sg.member] + col0
+                                                           : a.y + (int64_t)orow * a.y_row_stride + col0;
                         }
                         uint4 held = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll

@@ -66,7 +66,8 @@ constexpr int kHadamardMmaMinRows = 64;   // from here on the rotation runs on t
 int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t x_row_stride,
                     const __half* pre, const __half* post, __half* out, const int32_t* row_src,
                     const int32_t* pre_row, const int32_t* post_row, bool pdl, int out_mode,
-                    cudaStream_t s, int glu = 0, const int32_t* rows_dev = nullptr);   // glu: x rows are [gate (n) | up (n)], see glu_value
+                    cudaStream_t s, int glu = 0, const int32_t* rows_dev = nullptr,   // glu: x rows are [gate (n) | up (n)], see glu_value
+                    int member_rows = 0);   // > 0: output row r is row r % member_rows of x with row r / member_rows of pre
 
 // One logical 128-column output block of a streamed GEMV: where its weights, activations,
 // output scales and results live.  NULL descriptor table = the identity mapping of a plain
@@ -149,6 +150,8 @@ struct GemvPlan {
 GemvPlan gemv_plan(int64_t ncb, int nkb, int rows, bool table, size_t partial_bytes);
 void gemv_set_tuning(int max_grid, int fuse_x_bytes);
 
+constexpr int kMaxMembers = 8;
+
 // ---- prefill GEMM (exl3_gemm.cuh) ---------------------------------------------------------
 struct GemmArgs {
     const __half* svh;        // may be NULL
@@ -182,6 +185,12 @@ struct GemmArgs {
     int ts_tok;               // tokens per output tile
     int ts_x_bytes;           // bytes of one stage of the activation ring
     int ts_box_rows;          // rows of one activation TMA box
+    // sibling groups: member i has the column blocks [member_end[i - 1], member_end[i]) of the trellis, the
+    // rotated rows [i m, (i + 1) m) and an output matrix of its own
+    int n_members;            // 0 or 1: a plain layer
+    int member_end[kMaxMembers];
+    __half* member_y[kMaxMembers];
+    int64_t member_stride[kMaxMembers];
 };
 
 size_t gemm_partial_bytes(int64_t rows);     // room for the partial sums of a dense launch on the largest grid

@@ -317,3 +317,26 @@ def test_mlp_monolith_matches_the_three_linears(cuda, oracle, rows):
     want = oracle.linear_forward(oracle.glu(g, u, "silu"), trd, k, 0, suhd, svhd, None)
     assert y.shape == (rows, D)
     assert rel_err(y.cpu().numpy(), want) <= 2e-3
+
+
+@pytest.mark.parametrize("rows", [17, 64, 300])
+@pytest.mark.parametrize("act", ["silu", "gelu"])
+def test_group_and_mlp_prefill_equal_single_layers(cuda, rows, act):
+    """More than 16 rows: the one GEMM of a group's members against each member alone (both rotation
+    kernels, one and two token tiles), and the MLP against its linears and the activation."""
+    from ponyexl3_b200.fused import FusedEXL3Group
+    from ponyexl3_b200.linear import EXL3Linear
+    from ponyexl3_b200.mlp import EXL3MLPMonolith
+    from ponyexl3_b200.moe import glu
+
+    x = torch.from_numpy(np.random.default_rng(rows).standard_normal((rows, 512)).astype(np.float32) * 0.05).cuda().bfloat16()
+    layers = _members(4, 512, [384, 128, 640], seed=1400)
+    for o, l in zip(FusedEXL3Group(layers).forward_all(x), layers):
+        want = EXL3Linear(l)(x)
+        assert o.shape == want.shape and o.is_contiguous()
+        assert (o.float() - want.float()).norm() / want.float().norm() < 5e-4
+    gate, up = _members(4, 512, [384, 384], seed=1410)
+    down = EXL3Linear(_members(4, 384, [256], seed=1420)[0])
+    y = EXL3MLPMonolith(FusedEXL3Group([gate, up]), down, activation=act)(x)
+    want = down(glu(EXL3Linear(gate)(x), EXL3Linear(up)(x), act))
+    assert (y.float() - want.float()).norm() / want.float().norm() < 1e-3
