@@ -53,6 +53,9 @@ _PROTOTYPES = {
     "exl3_gemm": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int,
                           c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_size_t,
                           c_uint, c_void_p]),
+    "exl3_gemm_members": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int,
+                                  c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
+                                  c_uint, c_void_p]),
     "exl3_gemm_tiles": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_int64, c_int64, c_int, c_int, c_void_p, c_int64,
                                 c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_size_t, c_uint, c_void_p]),
@@ -100,6 +103,11 @@ _PROTOTYPES = {
 }
 
 _lib: ctypes.CDLL | None = None
+_host = None
+
+# Entry points the host extension calls itself (see csrc/host/exl3_host.cpp).
+_HOST_FUNCTIONS = ("exl3_workspace_bytes", "exl3_gemm_workspace_bytes", "exl3_gemv", "exl3_gemm", "exl3_gemm_members",
+                   "exl3_gemv_blocks", "exl3_gemm_tiles", "exl3_moe_decode_tables", "exl3_moe_prefill_tables")
 
 
 def use_library(path: Path) -> None:
@@ -126,6 +134,33 @@ def load() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def host():
+    """The native host path of the module calls (``_exl3_host``), bound to the loaded library; raises
+    if it has not been built, as `load` does."""
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+        import sysconfig
+
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+
+        from . import ops
+
+        path = _PKG / "lib" / ("_exl3_host" + sysconfig.get_config_var("EXT_SUFFIX"))
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: build it with `python -m ponyexl3_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_exl3_host", str(path))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_exl3_host", loader))
+        loader.exec_module(mod)
+        lib = load()
+        mod.bind({n: ctypes.cast(getattr(lib, n), c_void_p).value for n in _HOST_FUNCTIONS}, check, ops.grow_workspace)
+        for idx, ws in ops.Workspace._per_device.items():
+            mod.set_workspace(idx, ws.buf.data_ptr(), ws.nbytes)
+        _host = mod
+    return _host
 
 
 def prototypes() -> dict:

@@ -1,4 +1,5 @@
-"""In-tree build of ``libexl3b200.so`` (hand-written CUDA for sm_100a + the C ABI).
+"""In-tree build of ``libexl3b200.so`` (hand-written CUDA for sm_100a + the C ABI) and of
+``_exl3_host`` (the native host path of the module calls, a CPython extension on top of it).
 
 ``python -m ponyexl3_b200.build`` compiles every ``csrc/*.cu`` with nvcc and links
 them into ``ponyexl3_b200/lib/libexl3b200.so``.  nvcc cross-compiles, so this runs
@@ -11,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -19,6 +21,8 @@ CSRC = PKG / "csrc"
 LIBDIR = PKG / "lib"
 OBJDIR = PKG / "build"
 LIB = LIBDIR / "libexl3b200.so"
+HOST_SRC = CSRC / "host" / "exl3_host.cpp"
+HOST = LIBDIR / ("_exl3_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -83,7 +87,30 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False,
     return lib
 
 
+def build_host(force: bool = False, verbose: bool = False) -> Path:
+    """Compile the host extension against the installed PyTorch; returns its path."""
+    deps = max(p.stat().st_mtime for p in (HOST_SRC, PKG.parent / "include" / "exl3_b200.h"))
+    if not force and HOST.exists() and HOST.stat().st_mtime >= deps:
+        return HOST
+    import torch
+
+    LIBDIR.mkdir(exist_ok=True)
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent / "include"
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], cuda]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in inc), str(HOST_SRC),
+           "-o", str(HOST), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed:\n{' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
+    return HOST
+
+
 if __name__ == "__main__":
     p = build(force="--force" in sys.argv, verbose=True, ptxas_info="--ptxas" in sys.argv,
               profile="--profile" in sys.argv)
     print(p)
+    print(build_host(force="--force" in sys.argv, verbose=True))

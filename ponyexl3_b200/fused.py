@@ -5,8 +5,9 @@ Mirrors ``FusedEXL3Group`` / ``FusedEXL3Sibling`` of the reference
 out-tile axis, their ``suh`` rows stacked (each member rotates the input with its own
 signs), their ``svh`` concatenated (member widths are multiples of 128, so an output
 rotation block never straddles two members), and ``forward_all`` returns one output per
-member.  On the B200 the group is one rotation launch plus one streamed GEMV over a block
-table (``exl3_gemv_blocks``) for up to 16 rows, and per-member tensor-core GEMMs above that.
+member.  On the B200 the group is one streamed GEMV over a block table (``exl3_gemv_blocks``) for up
+to 16 rows, and one rotation launch plus one tensor-core GEMM for all members (``exl3_gemm_members``)
+above that.
 """
 
 from __future__ import annotations
@@ -14,9 +15,12 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from . import ops
+from . import _lib, ops
 from .layer import EXL3Layer, codebook_mode_from_flags, unpack_signs_or_pass
 from .linear import GEMV_MAX_ROWS, _to_dev_u16
+
+
+MAX_MEMBERS = 8         # of exl3_gemm_members
 
 
 def fusable(layers: list[EXL3Layer]) -> bool:
@@ -59,6 +63,7 @@ class FusedEXL3Group(torch.nn.Module):
         # member index of every 128-column block
         self._block_sub = np.repeat(np.arange(len(layers)), [n // 128 for n in self._out_features])
         self._offsets = np.concatenate([[0], np.cumsum(self._out_features)]).astype(np.int64)
+        self._set_spans()
         self._tables: dict[int, tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = {}
         self._cache_x: torch.Tensor | None = None
         self._cache_out: tuple[torch.Tensor, ...] | None = None
@@ -87,10 +92,15 @@ class FusedEXL3Group(torch.nn.Module):
         g._trellis, g._suh_stack, g._svh_cat = trellis.contiguous(), suh_stack.contiguous(), svh_cat
         g._block_sub = np.repeat(np.arange(len(out_features)), [n // 128 for n in out_features])
         g._offsets = np.concatenate([[0], np.cumsum(g._out_features)]).astype(np.int64)
+        g._set_spans()
         g._tables = {}
         g._cache_x = g._cache_out = None
         g.pdl = False
         return g
+
+    def _set_spans(self) -> None:
+        ends = [int(v) for v in self._offsets]
+        self._spans, self._total = list(zip(ends[:-1], ends[1:])), ends[-1]
 
     def extra_repr(self) -> str:
         return f"members={self._keys}, k={self.k}"
@@ -115,48 +125,37 @@ class FusedEXL3Group(torch.nn.Module):
             self._tables[rows] = t
         return t
 
-    @torch.no_grad()
     def forward_packed(self, x2d: torch.Tensor) -> torch.Tensor:
         """All members side by side, (rows, sum(out)) fp16, for 1..16 rows — one buffer a
         following kernel can take whole (q|k|v for the rotary step, gate|up for SwiGLU)."""
         rows = x2d.shape[0]
         if not 1 <= rows <= GEMV_MAX_ROWS:
             raise ValueError("forward_packed serves 1..16 rows")
-        blocks, row_src, suh_row = self._table(rows, x2d.device)
-        y = torch.empty((rows, int(self._offsets[-1])), dtype=torch.float16, device=x2d.device)
-        ops.gemv_blocks(x2d, xh_rows=rows * len(self._out_features), row_src=row_src,
-                        suh=self._suh_stack, suh_row=suh_row, trellis=self._trellis, k=self.k,
-                        cb=self.cb, blocks=blocks, rows=rows, svh=self._svh_cat, bias=None, y=y,
-                        pdl=self.pdl)
-        return y
+        return (_lib._host or _lib.host()).group_packed(
+            x2d, *self._native(), *self._table(rows, x2d.device), _lib.FLAG_PDL if self.pdl else 0)
 
-    @torch.no_grad()
+    def _native(self) -> tuple:
+        """What the host extension takes of the group."""
+        return (self._trellis, self.k, self.cb, self._suh_stack, self._svh_cat, len(self._out_features), self._total)
+
     def forward_all(self, x: torch.Tensor) -> tuple[torch.Tensor, ...]:
         in_shape = x.shape
         if in_shape[-1] != self.in_features:
             raise ValueError(f"expected last dim {self.in_features}, got {in_shape[-1]}")
         x2d = x.reshape(-1, self.in_features)
         rows = x2d.shape[0]
-        total = int(self._offsets[-1])
         if rows == 0:
             return tuple(torch.empty(in_shape[:-1] + (n,), dtype=torch.float16, device=x.device)
                          for n in self._out_features)
         if rows <= GEMV_MAX_ROWS:
-            blocks, row_src, suh_row = self._table(rows, x.device)
-            y = torch.empty((rows, total), dtype=torch.float16, device=x.device)
-            ops.gemv_blocks(x2d, xh_rows=rows * len(self._out_features), row_src=row_src,
-                            suh=self._suh_stack, suh_row=suh_row, trellis=self._trellis, k=self.k,
-                            cb=self.cb, blocks=blocks, rows=rows, svh=self._svh_cat, bias=None, y=y,
-                            pdl=self.pdl)
-            outs = [y[:, int(a):int(b)] for a, b in zip(self._offsets[:-1], self._offsets[1:])]
+            y = self.forward_packed(x2d)
+            outs = [y[:, a:b] for a, b in self._spans]
+        elif len(self._out_features) <= MAX_MEMBERS:
+            # prefill: one rotation and one tensor-core GEMM for all members
+            outs = (_lib._host or _lib.host()).group_prefill(x2d, *self._native(), tuple(self._out_features))
         else:
-            # prefill: one tensor-core GEMM per member on its out-tile range of the shared trellis
-            outs = []
-            for i, n in enumerate(self._out_features):
-                t0 = int(self._offsets[i]) // 16
-                tr = self._trellis[:, t0:t0 + n // 16].contiguous()
-                outs.append(ops.gemm(x2d, tr, self.k, self.cb, self._suh_stack[i],
-                                     self._svh_cat[int(self._offsets[i]):int(self._offsets[i + 1])], None))
+            outs = [ops.gemm(x2d, self._trellis[:, a // 16:b // 16].contiguous(), self.k, self.cb, self._suh_stack[i],
+                             self._svh_cat[a:b], None) for i, (a, b) in enumerate(self._spans)]
         return tuple(o.reshape(in_shape[:-1] + (n,)) for o, n in zip(outs, self._out_features))
 
     def cached(self, x: torch.Tensor) -> tuple[torch.Tensor, ...]:

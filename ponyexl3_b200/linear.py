@@ -13,7 +13,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from . import ops
+from . import _lib
 from .layer import EXL3Layer, codebook_mode_from_flags, unpack_signs_or_pass
 
 GEMV_MAX_ROWS = 16
@@ -81,23 +81,10 @@ class EXL3Linear(torch.nn.Module):
     def packed_bytes(self) -> int:
         return self.in_features * self.out_features * self.k // 8
 
-    @torch.no_grad()
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-        """`out`: optional (rows, out_features) fp16 CUDA tensor to write into (unit column stride)."""
-        in_shape = x.shape
-        if in_shape[-1] != self.in_features:
-            raise ValueError(f"expected last dim {self.in_features}, got {in_shape[-1]}")
-        x2d = x if x.ndim == 2 else x.reshape(-1, self.in_features)
-        rows = x2d.shape[0]
-        if rows == 0:
-            return torch.empty(in_shape[:-1] + (self.out_features,), dtype=torch.float16,
-                               device=x.device)
-        if out is not None and (out.shape != (rows, self.out_features) or out.dtype != torch.float16
-                                or out.stride(1) != 1):
-            raise ValueError("out must be a (rows, out_features) fp16 tensor with unit column stride")
-        if rows <= GEMV_MAX_ROWS:
-            y = ops.gemv(x2d, self._trellis, self.k, self.cb, self._suh, self._svh, self._bias,
-                         pdl=self.pdl, fast_accum=self.fast_accum, out=out)
-        else:
-            y = ops.gemm(x2d, self._trellis, self.k, self.cb, self._suh, self._svh, self._bias, out=out)
-        return y if x.ndim == 2 else y.reshape(in_shape[:-1] + (self.out_features,))
+        """`out`: optional (rows, out_features) fp16 CUDA tensor to write into (unit column stride).
+        Checks, output allocation and launch are one native call (csrc/host/exl3_host.cpp): 16 rows
+        and fewer take the streamed GEMV, more the tensor-core GEMM."""
+        return (_lib._host or _lib.host()).linear(
+            x, self._trellis, self.k, self.cb, self._suh, self._svh, self._bias,
+            (_lib.FLAG_PDL if self.pdl else 0) | (_lib.FLAG_FAST_ACCUM if self.fast_accum else 0), out)

@@ -9,18 +9,17 @@ projection, as there).
 Up to 16 rows the call is two streamed-GEMV launches: the sibling group writes ``[gate | up]``,
 and the down projection reads that buffer as it is, applying ``act(gate) * up`` while it loads
 its activations (EXL3_FLAG_GLU_*), so there is no activation kernel and no ``h`` buffer in
-between.  More rows go through the tensor-core GEMM per member, with the GLU as a separate
-kernel.
+between.  More rows take the tensor-core GEMM the same way: rotation and GEMM for gate and up together,
+then a rotation that applies the GLU while it loads, and the GEMM of the down projection.
 """
 
 from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import _lib
 from .fused import FusedEXL3Group
 from .linear import EXL3Linear
-from .moe import glu
 
 _ACTIVATIONS = ("silu", "gelu")
 
@@ -53,26 +52,19 @@ class EXL3MLPMonolith(torch.nn.Module):
     def extra_repr(self) -> str:
         return f"in={self.in_features}, hidden={self.hidden_dims}, out={self.out_features}, act={self.activation}"
 
-    @torch.no_grad()
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if x.shape[-1] != self.in_features:
             raise ValueError(f"x has {x.shape[-1]} features, the MLP expects {self.in_features}")
         lead = x.shape[:-1]
         x2d = x.reshape(-1, self.in_features)
         rows = x2d.shape[0]
-        d = self._down
+        d, g = self._down, self._group
         if rows == 0:
             return torch.empty(lead + (self.out_features,), dtype=torch.float16, device=x.device)
-        if rows <= 16:
-            self._group.pdl = self.pdl
-            gu = self._group.forward_packed(x2d)                       # (rows, 2 * hidden) = [gate | up]
-            y = ops.gemv(gu, d._trellis, d.k, d.cb, d._suh, d._svh, d._bias, pdl=self.pdl,
-                         fast_accum=d.fast_accum, glu=self.activation)
-        else:
-            g, u = self._group.forward_all(x2d)
-            if self.activation == "silu":
-                h = ops.swiglu(torch.cat([g, u], dim=1))
-            else:
-                h = glu(g, u, self.activation)
-            y = d(h)
+        pdl = _lib.FLAG_PDL if self.pdl else 0
+        glu_flag = _lib.FLAG_GLU_GELU if self.activation == "gelu" else _lib.FLAG_GLU_SILU
+        table = g._table(rows, x.device) if rows <= 16 else (None, None, None)
+        y = (_lib._host or _lib.host()).mlp(
+            x2d, *g._native(), *table, d._trellis, d.k, d.cb, d._suh, d._svh, d._bias, pdl,
+            pdl | glu_flag | (_lib.FLAG_FAST_ACCUM if d.fast_accum else 0))
         return y.reshape(lead + (self.out_features,))

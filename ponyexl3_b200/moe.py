@@ -20,7 +20,7 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import _lib, ops
 
 _ACTIVATIONS = ("silu", "gelu")
 DECODE_MAX_TOKENS = 16
@@ -68,16 +68,15 @@ class EXL3SwitchGLU(torch.nn.Module):
         self._dn_svh = dn_svh.to(torch.float16).reshape(-1).contiguous()
         self.pdl = False
 
-    # ---- decode: every (token, slot) pair is a one-row problem -------------------------------
-    def _decode(self, x2d: torch.Tensor, indices: torch.Tensor, expert_range=None) -> torch.Tensor:
+    # ---- expert parallelism, decode: every (token, slot) pair is a one-row problem ------------
+    def _decode(self, x2d: torch.Tensor, indices: torch.Tensor, expert_range) -> torch.Tensor:
         """Three launches: tables, GEMV over (pair, gate|up) blocks, GEMV over (pair, down) blocks
         with the GLU folded into its activation load (the reference's two-launch fused decode,
         ponyexl3/mlx/exl3_moe.py:345-422).  No host round trip, so the call can be captured.
 
         expert_range = (lo, hi, total): this module holds experts lo..hi-1 of `total`, `indices`
         are global; only the pairs of held experts are computed (their number stays on the device),
-        the rows of all other pairs come back as zeros."""
-        from . import _lib
+        the rows of all other pairs come back as zeros.  (All experts on one GPU: `forward`.)"""
         E, D, H = self.num_experts, self.input_dims, self.hidden_dims
         R, kk = indices.shape
         n = R * kk
@@ -96,29 +95,21 @@ class EXL3SwitchGLU(torch.nn.Module):
         counts = tab[o + 5 * n:o + 5 * n + 2]
         flags = _lib.FLAG_PDL if self.pdl else 0
         stream = torch.cuda.current_stream(dev).cuda_stream
-        if expert_range is None:
-            _lib.check(_lib.load().exl3_moe_decode_tables(
-                idx.data_ptr(), idx.element_size(), n, kk, E, D, H, blocks_gu.data_ptr(), row_src.data_ptr(),
-                suh_row.data_ptr(), blocks_dn.data_ptr(), sel.data_ptr(), flags, stream), "exl3_moe_decode_tables")
-            cnt_gu = cnt_dn = None
-            new = torch.empty
-        else:
-            lo, hi, total = expert_range
-            if hi - lo != E:
-                raise ValueError("expert_range does not match the experts held here")
-            _lib.check(_lib.load().exl3_moe_decode_tables_range(
-                idx.data_ptr(), idx.element_size(), n, kk, total, lo, hi, D, H, blocks_gu.data_ptr(),
-                row_src.data_ptr(), suh_row.data_ptr(), blocks_dn.data_ptr(), sel.data_ptr(), counts.data_ptr(),
-                flags, stream), "exl3_moe_decode_tables_range")
-            cnt_gu, cnt_dn = counts[0:1], counts[1:2]
-            new = torch.zeros
+        lo, hi, total = expert_range
+        if hi - lo != E:
+            raise ValueError("expert_range does not match the experts held here")
+        _lib.check(_lib.load().exl3_moe_decode_tables_range(
+            idx.data_ptr(), idx.element_size(), n, kk, total, lo, hi, D, H, blocks_gu.data_ptr(),
+            row_src.data_ptr(), suh_row.data_ptr(), blocks_dn.data_ptr(), sel.data_ptr(), counts.data_ptr(),
+            flags, stream), "exl3_moe_decode_tables_range")
+        cnt_gu, cnt_dn = counts[0:1], counts[1:2]
 
         ygu = torch.empty((n, 2 * H), dtype=torch.float16, device=dev)   # rows of other ranks' pairs: never read
         ops.gemv_blocks(x2d, xh_rows=2 * n, row_src=row_src, suh=self._gu_suh, suh_row=suh_row,
                         trellis=self._gu_trellis, k=self.k, cb=self.cb, blocks=blocks_gu, rows=1,
                         svh=self._gu_svh, bias=None, y=ygu, pdl=self.pdl, n_blocks_dev=cnt_gu)
         # the down launch reads [gate | up] as it is and applies the GLU while loading
-        y = new((n, D), dtype=torch.float16, device=dev)
+        y = torch.zeros((n, D), dtype=torch.float16, device=dev)
         ops.gemv_blocks(ygu, xh_rows=n, row_src=None, suh=self._dn_suh, suh_row=sel,
                         trellis=self._dn_trellis, k=self.k, cb=self.cb, blocks=blocks_dn, rows=1,
                         svh=self._dn_svh, bias=None, y=y, pdl=self.pdl, glu=self.activation,
@@ -134,8 +125,8 @@ class EXL3SwitchGLU(torch.nn.Module):
             raise ValueError("decode_range is for decode-class calls")
         return self._decode(x2d, indices, expert_range)
 
-    # ---- prefill: pairs sorted by expert, tensor-core GEMM over an expert tile table ----------
-    def _prefill(self, x2d: torch.Tensor, indices: torch.Tensor, expert_range=None, peers=None):
+    # ---- expert parallelism, prefill: pairs sorted by expert, GEMM over an expert tile table ----
+    def _prefill(self, x2d: torch.Tensor, indices: torch.Tensor, expert_range, peers) -> None:
         """Tables kernel, rotation + tile-table GEMM for gate and up, rotation (GLU applied while
         loading) + tile-table GEMM for down writing straight back into (token, slot) order: five
         launches, no host round trip.
@@ -145,7 +136,6 @@ class EXL3SwitchGLU(torch.nn.Module):
         and cover ALL tokens; only the held pairs are computed (their number stays on the device)
         and every output row is stored into the memory of the GPU that owns its token, which
         gets one arrival per GPU when the rows are complete (exl3_gemm_tiles_peers)."""
-        from . import _lib
         E, D, H = self.num_experts, self.input_dims, self.hidden_dims
         R, kk = indices.shape
         n = R * kk
@@ -164,31 +154,22 @@ class EXL3SwitchGLU(torch.nn.Module):
         suh_gu, suh_dn = tab[o + 3 * n:o + 5 * n], tab[o + 5 * n:o + 6 * n]
         counts = tab[o + 6 * n:o + 6 * n + 2]
         stream = torch.cuda.current_stream(dev).cuda_stream
-        if expert_range is None:
-            _lib.check(_lib.load().exl3_moe_prefill_tables(
-                idx.data_ptr(), idx.element_size(), n, kk, E, D, H, order.data_ptr(), row_src.data_ptr(),
-                suh_gu.data_ptr(), suh_dn.data_ptr(), tiles_gu.data_ptr(), tiles_dn.data_ptr(), 0, stream),
-                "exl3_moe_prefill_tables")
-            rows_gu = rows_dn = None
-        else:
-            lo, hi, total = expert_range
-            if hi - lo != E:
-                raise ValueError("expert_range does not match the experts held here")
-            _lib.check(_lib.load().exl3_moe_prefill_tables_range(
-                idx.data_ptr(), idx.element_size(), n, kk, total, lo, hi, D, H, order.data_ptr(), row_src.data_ptr(),
-                suh_gu.data_ptr(), suh_dn.data_ptr(), tiles_gu.data_ptr(), tiles_dn.data_ptr(), counts.data_ptr(),
-                0, stream), "exl3_moe_prefill_tables_range")
-            rows_gu, rows_dn = counts[0:1], counts[1:2]
+        lo, hi, total = expert_range
+        if hi - lo != E:
+            raise ValueError("expert_range does not match the experts held here")
+        _lib.check(_lib.load().exl3_moe_prefill_tables_range(
+            idx.data_ptr(), idx.element_size(), n, kk, total, lo, hi, D, H, order.data_ptr(), row_src.data_ptr(),
+            suh_gu.data_ptr(), suh_dn.data_ptr(), tiles_gu.data_ptr(), tiles_dn.data_ptr(), counts.data_ptr(),
+            0, stream), "exl3_moe_prefill_tables_range")
+        rows_gu, rows_dn = counts[0:1], counts[1:2]
         ygu = torch.empty((n, 2 * H), dtype=torch.float16, device=dev)
         ops.gemm_tiles(x2d, xh_rows=2 * n, row_src=row_src, suh=self._gu_suh, suh_row=suh_gu,
                        trellis=self._gu_trellis, k=self.k, cb=self.cb, tiles=tiles_gu, svh=self._gu_svh, y=ygu,
                        xh_rows_dev=rows_gu)
         # the down launch reads [gate | up] as it is and applies the GLU while it rotates the rows
-        out = None if peers is not None else torch.empty((n, D), dtype=torch.float16, device=dev)
         ops.gemm_tiles(ygu, xh_rows=n, row_src=None, suh=self._dn_suh, suh_row=suh_dn, trellis=self._dn_trellis,
-                       k=self.k, cb=self.cb, tiles=tiles_dn, svh=self._dn_svh, y=out, y_row_map=order,
+                       k=self.k, cb=self.cb, tiles=tiles_dn, svh=self._dn_svh, y=None, y_row_map=order,
                        glu=self.activation, xh_rows_dev=rows_dn, peers=peers)
-        return None if out is None else out.view(R, kk, D)
 
     @torch.no_grad()
     def prefill_range(self, x2d: torch.Tensor, indices: torch.Tensor, expert_range, peers) -> None:
@@ -196,7 +177,6 @@ class EXL3SwitchGLU(torch.nn.Module):
         tokens; the outputs land in the owners' buffers named by `peers`."""
         self._prefill(x2d, indices, expert_range, peers)
 
-    @torch.no_grad()
     def forward(self, x: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
         if indices.ndim != 3:
             raise ValueError("indices must be (B, S, k)")
@@ -204,7 +184,11 @@ class EXL3SwitchGLU(torch.nn.Module):
         R = B * S
         x2d = x.reshape(R, self.input_dims)
         idx = indices.reshape(R, kk)
-        y = self._decode(x2d, idx) if R <= DECODE_MAX_TOKENS else self._prefill(x2d, idx)
+        y = (_lib._host or _lib.host()).switch_glu(
+            x2d, idx, self._gu_trellis, self._gu_suh, self._gu_svh, self._dn_trellis, self._dn_suh, self._dn_svh,
+            self.num_experts, self.hidden_dims, self.k, self.cb,
+            _lib.FLAG_GLU_GELU if self.activation == "gelu" else _lib.FLAG_GLU_SILU, _lib.FLAG_PDL if self.pdl else 0,
+            R <= DECODE_MAX_TOKENS)
         return y.reshape(B, S, kk, self.input_dims)
 
 

@@ -64,6 +64,8 @@ class Workspace:
             floor = int(_lib.load().exl3_workspace_bytes(16, 32768))
             ws = Workspace(torch.device("cuda", idx), max(int(nbytes), floor, ws.nbytes if ws else 0))
             cls._per_device[idx] = ws
+            if _lib._host is not None:
+                _lib._host.set_workspace(idx, ws.buf.data_ptr(), ws.nbytes)
         return ws
 
     _need: dict[tuple[int, int], int] = {}
@@ -98,6 +100,12 @@ class Workspace:
             if old is not self:
                 st |= old._status_one()
         return st
+
+
+def grow_workspace(device_index: int, nbytes: int) -> None:
+    """Called by the host extension when a device's workspace is missing or too small."""
+    ws = Workspace.get_bytes(torch.device("cuda", device_index), nbytes)
+    _lib.host().set_workspace(device_index, ws.buf.data_ptr(), ws.nbytes)
 
 
 def unpack_trellis(packed: torch.Tensor, k: int) -> torch.Tensor:
