@@ -116,8 +116,10 @@ struct MoePrefillArgs {
 
 constexpr int kMoeMaxExperts = 1024;
 
-// One CTA: shared-memory histogram, scan, scatter.  32 K pairs take a few microseconds; the
-// tables are tiny next to the GEMMs they drive.
+// Every CTA counts all pairs per expert (and those in front of its own share of the pairs) in shared memory,
+// scans the counts, and then places its share of the pairs and writes its share of the tables: the
+// counting is cheap to repeat, and no CTA waits for another.  One CTA alone took 133 us for 32,768 pairs
+// over 256 experts, nearly all of it the latency of its scattered stores; 32 take about 8.
 //
 // Row layout.  The held pairs are sorted by expert; expert e owns sorted positions
 // [seg, seg + cnt).  The rotated rows of the gate/up launch keep an expert's rows together —
@@ -128,9 +130,9 @@ __global__ void __launch_bounds__(1024) moe_prefill_tables_kernel(const MoePrefi
 {
     griddep_launch_dependents();
     griddep_wait();
-    __shared__ int count[kMoeMaxExperts], seg[kMoeMaxExperts], blk0[kMoeMaxExperts], cursor[kMoeMaxExperts];
-    __shared__ int total_blocks;
-    const int tid = threadIdx.x;
+    __shared__ int count[kMoeMaxExperts], before[kMoeMaxExperts], seg[kMoeMaxExperts], blk0[kMoeMaxExperts];
+    __shared__ int warp_rows[32], warp_blocks[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int E_here = a.e_hi - a.e_lo;
     auto expert = [&](int s) -> int {       // local index of the pair's expert, -1: not held here
         const long long e = a.idx64 ? static_cast<const long long*>(a.indices)[s]
@@ -138,32 +140,46 @@ __global__ void __launch_bounds__(1024) moe_prefill_tables_kernel(const MoePrefi
         const int ec = (int)(e < 0 ? 0 : (e >= a.E ? a.E - 1 : e));      // a bad index must not leave the tensors
         return ec >= a.e_lo && ec < a.e_hi ? ec - a.e_lo : -1;
     };
-    for (int e = tid; e < E_here; e += blockDim.x) { count[e] = 0; cursor[e] = 0; }
+    count[tid] = before[tid] = 0;            // kMoeMaxExperts = threads
     __syncthreads();
-    for (int s = tid; s < a.n; s += blockDim.x) {
+    const int s0 = (int)((int64_t)a.n * blockIdx.x / gridDim.x), s1 = (int)((int64_t)a.n * (blockIdx.x + 1) / gridDim.x);
+#pragma unroll 8
+    for (int s = tid; s < a.n; s += 1024) {
         const int e = expert(s);
-        if (e >= 0) atomicAdd(&count[e], 1);
-    }
-    __syncthreads();
-    if (tid == 0) {                       // E <= 1024: a serial scan is a microsecond
-        int rows = 0, blocks = 0;
-        for (int e = 0; e < E_here; e++) {
-            seg[e] = rows;
-            blk0[e] = blocks;
-            rows += count[e];
-            blocks += (count[e] + 255) >> 8;
-        }
-        total_blocks = blocks;
-        if (a.counts) {
-            a.counts[0] = 2 * rows;
-            a.counts[1] = rows;
+        if (e >= 0) {
+            atomicAdd(&count[e], 1);
+            if (s < s0) atomicAdd(&before[e], 1);
         }
     }
     __syncthreads();
-    for (int s = tid; s < a.n; s += blockDim.x) {
+    // exclusive scans of rows and row tiles over the experts, one expert per thread
+    const int rows = count[tid], blocks = (rows + 255) >> 8;
+    int r = rows, bl = blocks;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int pr = __shfl_up_sync(0xFFFFFFFFu, r, d), pb = __shfl_up_sync(0xFFFFFFFFu, bl, d);
+        if (lane >= d) { r += pr; bl += pb; }
+    }
+    if (lane == 31) { warp_rows[warp] = r; warp_blocks[warp] = bl; }
+    __syncthreads();
+    int r0 = 0, b0 = 0, total_rows = 0, total_blocks = 0;
+#pragma unroll
+    for (int w = 0; w < 32; w++) {
+        if (w < warp) { r0 += warp_rows[w]; b0 += warp_blocks[w]; }
+        total_rows += warp_rows[w];
+        total_blocks += warp_blocks[w];
+    }
+    seg[tid] = r0 + r - rows;
+    blk0[tid] = b0 + bl - blocks;
+    if (a.counts && blockIdx.x == 0 && tid == 0) {
+        a.counts[0] = 2 * total_rows;
+        a.counts[1] = total_rows;
+    }
+    __syncthreads();
+    for (int s = s0 + tid; s < s1; s += 1024) {
         const int e = expert(s);
         if (e < 0) continue;
-        const int i = atomicAdd(&cursor[e], 1);
+        const int i = atomicAdd(&before[e], 1);
         const int pos = seg[e] + i;
         a.order[pos] = s;
         const int tok = s / a.kk;
@@ -175,7 +191,7 @@ __global__ void __launch_bounds__(1024) moe_prefill_tables_kernel(const MoePrefi
         a.suh_row_dn[pos] = e;
     }
     // tile tables: slot = row tile of one expert; every slot x every 256-column tile of the projection
-    const int ct_h = (a.H + 255) / 256, ct_d = (a.D + 255) / 256;
+    const int ct_h = (a.H + 255) / 256, ct_d = (a.D + 255) / 256, per_slot = 2 * ct_h + ct_d;
     auto put = [&](int32_t* tab, int idx, int row0, int row_end, int tn0, int sv, int ycol, int ncols, int shift) {
         int4 u, v;
         u.x = row0 < row_end ? row0 + shift : 0;
@@ -185,26 +201,36 @@ __global__ void __launch_bounds__(1024) moe_prefill_tables_kernel(const MoePrefi
         reinterpret_cast<int4*>(tab)[2 * idx] = u;
         reinterpret_cast<int4*>(tab)[2 * idx + 1] = v;
     };
-    auto emit = [&](int slot, int e, int row0, int row_end, int gate_shift, int up_shift) {
-        for (int j = 0; j < ct_h; j++) {
-            const int nc = min(a.H - 256 * j, 256);
-            put(a.tiles_gu, slot * ct_h + j, row0, row_end, e * (a.H / 16) + 16 * j, e * 2 * a.H + 256 * j, 256 * j, nc,
-                gate_shift);
-            put(a.tiles_gu, (a.slots + slot) * ct_h + j, row0, row_end, (E_here + e) * (a.H / 16) + 16 * j,
-                e * 2 * a.H + a.H + 256 * j, a.H + 256 * j, nc, up_shift);
+    for (int i = blockIdx.x * 1024 + tid; i < a.slots * per_slot; i += gridDim.x * 1024) {
+        const int slot = i / per_slot;
+        int j = i - slot * per_slot;
+        int e = 0, row0 = 0, row_end = 0, sg = 0, cnt = 0;       // unused slots: no rows
+        if (slot < total_blocks) {
+            int lo = 0, hi = E_here - 1;                          // the last expert whose first slot is not behind this one ...
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (blk0[mid] <= slot) lo = mid;
+                else hi = mid - 1;
+            }
+            e = lo;                                               // ... has rows: later ones would start at the next slot
+            sg = seg[e];
+            cnt = count[e];
+            row0 = sg + 256 * (slot - blk0[e]);
+            row_end = min(row0 + 256, sg + cnt);
         }
-        for (int j = 0; j < ct_d; j++)
+        if (j < ct_h) {
+            put(a.tiles_gu, slot * ct_h + j, row0, row_end, e * (a.H / 16) + 16 * j, e * 2 * a.H + 256 * j, 256 * j,
+                min(a.H - 256 * j, 256), sg);
+        } else if (j < 2 * ct_h) {
+            j -= ct_h;
+            put(a.tiles_gu, (a.slots + slot) * ct_h + j, row0, row_end, (E_here + e) * (a.H / 16) + 16 * j,
+                e * 2 * a.H + a.H + 256 * j, a.H + 256 * j, min(a.H - 256 * j, 256), sg + cnt);
+        } else {
+            j -= 2 * ct_h;
             put(a.tiles_dn, slot * ct_d + j, row0, row_end, e * (a.D / 16) + 16 * j, e * a.D + 256 * j, 256 * j,
                 min(a.D - 256 * j, 256), 0);
-    };
-    for (int e = tid; e < E_here; e += blockDim.x) {
-        const int nb = (count[e] + 255) >> 8;
-        for (int b = 0; b < nb; b++) {
-            const int row0 = seg[e] + 256 * b;
-            emit(blk0[e] + b, e, row0, min(row0 + 256, seg[e] + count[e]), seg[e], seg[e] + count[e]);
         }
     }
-    for (int slot = total_blocks + tid; slot < a.slots; slot += blockDim.x) emit(slot, 0, 0, 0, 0, 0);   // unused
 }
 
 }  // namespace exl3
@@ -278,7 +304,7 @@ static int moe_prefill_tables_impl(const void* indices, int index_bytes, int n_p
     a.order = order; a.row_src_gu = row_src_gu; a.suh_row_gu = suh_row_gu; a.suh_row_dn = suh_row_dn;
     a.tiles_gu = tiles_gu; a.tiles_dn = tiles_dn;
     a.counts = counts;
-    return launch_kernel(moe_prefill_tables_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream,
+    return launch_kernel(moe_prefill_tables_kernel, dim3((unsigned)std::max(1, std::min(32, n_pairs / 512))), dim3(1024), 0, (cudaStream_t)stream,
                          (flags & EXL3_FLAG_PDL) != 0, a);
 }
 
