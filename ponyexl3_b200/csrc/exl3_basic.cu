@@ -183,23 +183,19 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- the rotation of many rows, on the tensor cores ---------------------------------------------
-// had128(x * suh) for blocks of 16 rows x 128 columns as mma.sync m16n8k16 products with the
-// +-1 Sylvester matrix H[k][n] = (-1)^popcount(k & n): the warp-shuffle butterfly above costs
-// about 130 instructions per row and 128-block and made the prefill GEMM's input rotation
-// instruction-bound at a quarter of the memory bandwidth; here a row and block costs about 40.
-// fp16 inputs times +-1 are exact and the sums are fp32, as in the butterfly; only the order of
-// the fp32 additions differs.
+// had128(x * suh) for blocks of 16 rows x 128 columns.  H128 = H8 (x) H16: the 16-point transform over four
+// of the seven column bits is a product with the +-1 matrix H16 (mma.sync m16n8k16, 16 of them per block),
+// the 8-point one over the other three is butterflies between the eight accumulator groups, two values per
+// instruction.  fp16 inputs times +-1 are exact and the sums are fp32, as in the butterfly kernel; only the
+// order of the fp32 additions differs.  As one 128-point product (128 MMAs per block) the kernel was bound
+// by the rate of mma.sync: 42 us for 8192 x 5120 and 138 us for 65,536 x 2048.
 //
-// A lane loads 16 contiguous bytes (8 columns) of rows g and g + 8 per quarter of the block.
-// The MMA's k index is a free bijection as long as A and B agree: k-step (q, s) takes columns
-// 32 q + 8 t + 4 s + {0, 1} and + {2, 3} of lane t as its k = 2t, 2t+1 and 2t+8, 2t+9.  The
-// matching B fragment is H at those columns against output column n = 8 nt + g: its sign splits
-// into a part that depends on the column's low three bits and g, a part parity(t & nt) that
-// depends on the lane and the low two bits of nt (together sixteen constant registers per lane),
-// and a part parity(q & (nt >> 2)) that is known at compile time and picks one of two
-// accumulators, subtracted at the end: no sign arithmetic is left inside the loop.
-constexpr int kHadTileRow = 272;                 // 256 bytes of a row + 16: the fragment stores hit 32 banks
-constexpr int kHadTileBytes = 16 * kHadTileRow;
+// A lane loads 16 contiguous bytes (8 columns) of rows g and g + 8 per quarter of the block: column
+// 32 q + 8 t + 4 s + c, c = 0..3.  The MMA's k index is a free bijection as long as A and B agree: group
+// (q, s) takes its sixteen columns as k = 2 t + (c & 1) + 8 (c >> 1), so the four bits of k are the column
+// bits 0 (c), 3, 4 (t) and 1 (c); the bits of n are given the same meaning, which makes B the plain H16 for
+// every group and leaves a lane, after the butterflies over q and s, with the same 8 contiguous columns
+// per quarter that it loaded: stores are as wide as the loads.
 template <typename T> struct Load8;
 template <> struct Load8<__half> {
     static __device__ __forceinline__ uint4 at(const __half* p) { return *reinterpret_cast<const uint4*>(p); }
@@ -243,24 +239,16 @@ __global__ void __launch_bounds__(256, 2)
         const int64_t r = *rows_dev;
         rows = r < 0 ? 0 : (r < rows ? r : rows);
     }
-    __shared__ __align__(16) uint8_t stile[8 * kHadTileBytes];
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // B fragments, constant per lane: pt[nl][s][j] holds H at columns 4 s + 2 j + {0, 1} of the
-    // lane's 8-column group against output column 8 (4 nh + nl) + g, without the sign of the
-    // quarter (see the loop): the column's low bits meet g, the lane's t meets nl.
-    uint32_t pt[4][2][2];
+    // B fragments of H16[k][n] = (-1)^popcount(k & n), constant per lane: n = 8 nt + g, k = 2 t + {0, 1} (+ 8)
+    uint32_t hb[2][2];
 #pragma unroll
-    for (int nl = 0; nl < 4; nl++) {
-        const uint32_t flip = (__popc(t & nl) & 1) ? 0x80008000u : 0u;
+    for (int nt = 0; nt < 2; nt++)
 #pragma unroll
-        for (int s = 0; s < 2; s++)
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const uint32_t lo = (__popc((4 * s + 2 * j) & g) & 1) ? 0xBC00u : 0x3C00u;
-                const uint32_t hi = (__popc((4 * s + 2 * j + 1) & g) & 1) ? 0xBC00u : 0x3C00u;
-                pt[nl][s][j] = (lo | (hi << 16)) ^ flip;
-            }
-    }
+        for (int j = 0; j < 2; j++) {
+            const int n16 = 8 * nt + g, k = 2 * t + 8 * j;
+            hb[nt][j] = 0x3C003C00u | ((__popc(n16 & k) & 1) ? 0x8000u : 0u) | ((__popc(n16 & (k + 1)) & 1) ? 0x80000000u : 0u);
+        }
     const uint32_t nblk = (uint32_t)(n >> 7);
     const uint32_t total = (uint32_t)((rows + 15) >> 4) * nblk;
     const uint32_t warp0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -318,44 +306,47 @@ __global__ void __launch_bounds__(256, 2)
                 xb[q].w = h2_as_u32(__hmul2(u32_as_h2(xb[q].w), u32_as_h2(b.w)));
             }
         }
-        // The accumulator fragments (4 bytes per lane, row and 8-column group) go through a padded
-        // tile in shared memory so that every lane stores 16 contiguous bytes: 8 instead of 32
-        // stores, and whole 32-byte sectors.
-        uint8_t* tile = stile + (threadIdx.x >> 5) * kHadTileBytes;
+        // c[2 q + s][nt]: columns 32 q' + 8 t + 4 s' + 2 nt + {0, 1} of rows g (first pair) and g + 8, for the
+        // 16-point transform of group (q, s); the butterflies turn (q, s) into (q', s')
+        uint64_t c[8][2][2];
 #pragma unroll
-        for (int nh = 0; nh < 4; nh++)
+        for (int q = 0; q < 4; q++)
 #pragma unroll
-            for (int nl = 0; nl < 4; nl++) {
-                // output columns 8 nt + g, nt = 4 nh + nl: quarter q enters with the sign
-                // parity(q & nh), known at compile time, so it picks one of two accumulators
-                float cp[4] = {0.f, 0.f, 0.f, 0.f}, cm[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int s = 0; s < 2; s++) {
+                const uint32_t af[4] = {s ? xa[q].z : xa[q].x, s ? xb[q].z : xb[q].x, s ? xa[q].w : xa[q].y, s ? xb[q].w : xb[q].y};
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const uint32_t a0[4] = {xa[q].x, xb[q].x, xa[q].y, xb[q].y};
-                    const uint32_t a1[4] = {xa[q].z, xb[q].z, xa[q].w, xb[q].w};
-                    if (((q & nh) == 1) || ((q & nh) == 2)) {       // odd number of common bits
-                        mma_16816(cm, a0, pt[nl][0][0], pt[nl][0][1]);
-                        mma_16816(cm, a1, pt[nl][1][0], pt[nl][1][1]);
-                    } else {
-                        mma_16816(cp, a0, pt[nl][0][0], pt[nl][0][1]);
-                        mma_16816(cp, a1, pt[nl][1][0], pt[nl][1][1]);
-                    }
+                for (int nt = 0; nt < 2; nt++) {
+                    float d[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma_16816(d, af, hb[nt][0], hb[nt][1]);
+                    c[2 * q + s][nt][0] = f32x2(d[0], d[1]);
+                    c[2 * q + s][nt][1] = f32x2(d[2], d[3]);
                 }
-                const int nt = 4 * nh + nl;
-                *reinterpret_cast<__half2*>(tile + g * kHadTileRow + 16 * nt + 4 * t) =
-                    __floats2half2_rn((cp[0] - cm[0]) * EXL3_HAD_SCALE, (cp[1] - cm[1]) * EXL3_HAD_SCALE);
-                *reinterpret_cast<__half2*>(tile + (g + 8) * kHadTileRow + 16 * nt + 4 * t) =
-                    __floats2half2_rn((cp[2] - cm[2]) * EXL3_HAD_SCALE, (cp[3] - cm[3]) * EXL3_HAD_SCALE);
             }
-        __syncwarp();
+        const uint64_t minus = f32x2(-1.f, -1.f), scale = f32x2(EXL3_HAD_SCALE, EXL3_HAD_SCALE);
 #pragma unroll
-        for (int i = 0; i < 8; i++) {          // 16 rows x 16 chunks of 16 bytes, two rows per turn
-            const int rr = 2 * i + (lane >> 4), ch = lane & 15;
-            const int64_t r = (int64_t)rb * 16 + rr;
-            const uint4 v = *reinterpret_cast<const uint4*>(tile + rr * kHadTileRow + 16 * ch);
-            if (r < rows) *reinterpret_cast<uint4*>(out + r * n + (int64_t)cb * 128 + 8 * ch) = v;
-        }
-        __syncwarp();
+        for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (i & h) continue;
+#pragma unroll
+                for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        const uint64_t u = c[i][nt][r], v = c[i + h][nt][r];
+                        c[i][nt][r] = add_f32x2(u, v);
+                        c[i + h][nt][r] = fma_f32x2(v, minus, u);
+                    }
+            }
+        auto put = [&](int64_t row, int r) {
+            __half* o = out + row * n + col;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                *reinterpret_cast<uint4*>(o + 32 * q) =
+                    make_uint4(f16_pair(mul_f32x2(c[2 * q][0][r], scale)), f16_pair(mul_f32x2(c[2 * q][1][r], scale)),
+                               f16_pair(mul_f32x2(c[2 * q + 1][0][r], scale)), f16_pair(mul_f32x2(c[2 * q + 1][1][r], scale)));
+        };
+        if (ok0) put(r0, 0);
+        if (ok1) put(r1, 1);
     }
 }
 

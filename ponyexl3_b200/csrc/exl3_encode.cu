@@ -186,23 +186,6 @@ __device__ __forceinline__ int64_t next_tile(EncodeShared& sh, const EncodeArgs&
     return tile;
 }
 
-__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi)
-{
-    return (uint64_t)__float_as_uint(lo) | ((uint64_t)__float_as_uint(hi) << 32);
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // (k & ~(J - 1)) | j as one three-input operation (written in C, ptxas made two of it).
 template <int J> __device__ __forceinline__ uint32_t key_with_index(uint32_t k, uint32_t j)
 {
@@ -306,7 +289,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                     if (low < 1e29f) off += (double)low * (1.0 - 2.4e-7);
                 }
                 if (tid == 0) sh.smin[(t + 2) % 3] = 0x7F800000u;
-                const uint64_t nw = pack_f32x2(-w, -w);
+                const uint64_t nw = f32x2(-w, -w);
                 uint32_t low_new = 0x7F800000u;
 #pragma unroll
                 for (int g = 0; g < G; g++) {
@@ -318,7 +301,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
 #pragma unroll
                         for (int q = 0; q < JC / 2; q++) {
                             const uint32_t j = j_first + c * JC + 2 * q;
-                            mf2[q] = pack_f32x2(mfc[pred_slot(h, hs, j, rot)], mfc[pred_slot(h, hs, j + 1, rot)]);
+                            mf2[q] = f32x2(mfc[pred_slot(h, hs, j, rot)], mfc[pred_slot(h, hs, j + 1, rot)]);
                         }
 #pragma unroll
                         for (int i = 0; i < L; i++) {
@@ -328,7 +311,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                                 uint32_t pair = cbr[g * L + i][c * (JC / 2) + q];
                                 asm volatile("" : "+r"(pair));   // converted here: hoisted, 128 floats spill
                                 const float2 cf = __half22float2(u32_as_h2(pair));
-                                const uint64_t d = add_f32x2(pack_f32x2(cf.x, cf.y), nw);
+                                const uint64_t d = add_f32x2(f32x2(cf.x, cf.y), nw);
                                 const uint64_t k2 = fma_f32x2(d, d, mf2[q]);
                                 const uint32_t j = c * JC + 2 * q;
                                 key[2 * q] = key_with_index<J>((uint32_t)k2, j);
