@@ -202,6 +202,8 @@ EXL3_API int exl3_gemm_members(const void* x, int x_dtype, int64_t rows, int64_t
  * had(x[row_src[i]] * suh[suh_row[i]]) as in exl3_gemv_blocks.  y_row_map (may be NULL): the
  * y row that computed row r + y_row_delta is stored to — the last projection of a MoE call
  * writes straight back into (token, slot) order instead of sorted order.
+ * flags >> 16 (optional): average rows of the tiles in use, which sizes the stages of the activation
+ * ring; any value gives the same results.
  * Replaces the segmented trellis GEMM of the reference, inner_mm_seg_mlx with its expert block
  * table, ponyexl3/mlx/gemv_metal.py:1519-1741 and ponyexl3/mlx/exl3_moe.py:79-99,685-768. */
 EXL3_API int exl3_gemm_tiles(const void* x, int x_dtype, int64_t x_row_stride, int64_t xh_rows,

@@ -632,6 +632,7 @@ static int gemm_tiles_impl(const void* x, int x_dtype, int64_t x_row_stride, int
     a.tile_tab = tiles;
     a.y_row_map = y_row_map;
     a.n_tiles_tab = (int)n_tiles;
+    a.rows_hint = (int)(flags >> 16);
     a.xh_rows = (int)xh_rows;
     a.m = (int)xh_rows;
     a.t_in = (int)t_in;

@@ -13,12 +13,12 @@ EXL3_DECL(1) EXL3_DECL(2) EXL3_DECL(3) EXL3_DECL(4) EXL3_DECL(5) EXL3_DECL(6) EX
 
 // How many CTAs a dense launch of `tiles` output tiles of nks k-steps gets, and whether they share tiles.
 // Cost in k-steps of the slowest CTA: its k-steps, and for each of its segments the hand-over and the
-// epilogue, measured at about ten k-steps.  Whole tiles are the case of every segment being one; for
-// shared tiles a count that lets ranges end on tile boundaries saves a segment per CTA, so all counts
-// down to half of the SMs are looked at.  The choice is remembered per shape.
+// epilogue, which the decode warps do themselves.  For shared tiles a count that lets ranges end on tile
+// boundaries saves a segment per CTA, so all counts down to half of the SMs are looked at.  The choice is
+// remembered per shape.
 int ts_plan(int64_t tiles, int nks, int sms, int64_t rows, size_t partial_bytes, int* split)
 {
-    constexpr double kSegment = 10.0;
+    constexpr double kWhole = 6.0, kShared = 10.0;
     struct Memo { int64_t tiles; int nks, sms, room, grid, split; };
     static thread_local Memo memo[32] = {};
     static thread_local int memo_next = 0;
@@ -31,7 +31,7 @@ int ts_plan(int64_t tiles, int nks, int sms, int64_t rows, size_t partial_bytes,
         }
     const int whole = (int)std::min<int64_t>(tiles, sms);
     int best = whole, best_split = 0;
-    double best_cost = (double)((tiles + whole - 1) / whole) * (nks + kSegment);
+    double best_cost = (double)((tiles + whole - 1) / whole) * (nks + kWhole);
     const int64_t units = tiles * nks;
     if (room && tiles < 64 * sms && units >= 4) {
         const int most = (int)std::min<int64_t>(sms, units / 4);
@@ -41,7 +41,11 @@ int ts_plan(int64_t tiles, int nks, int sms, int64_t rows, size_t partial_bytes,
                 int64_t u = units * c / g;
                 const int64_t u1 = units * (c + 1) / g;
                 double t = (double)(u1 - u);
-                for (; u < u1; u = (u / nks + 1) * nks) t += kSegment;
+                while (u < u1) {
+                    const int64_t end = std::min(u1, (u / nks + 1) * nks);
+                    t += end - u == nks ? kWhole : kShared;
+                    u = end;
+                }
                 worst = std::max(worst, t);
             }
             if (worst < best_cost - 1e-9) { best_cost = worst; best = g; best_split = 1; }

@@ -31,6 +31,7 @@
 // named barriers still meet) and the tensor memory is freed at the end.
 #pragma once
 #include <algorithm>
+#include <cmath>
 
 #include "exl3_internal.h"
 #include "exl3_tc.cuh"
@@ -38,10 +39,15 @@
 
 namespace exl3 {
 
-constexpr int kTsThreads = 640;
 constexpr int kTsDecodeWarps = 16, kTsFirstDecodeWarp = 4, kTsSets = 4;
+constexpr int kTsThreads = 32 * (kTsFirstDecodeWarp + kTsDecodeWarps);
 constexpr int kTsOuts = 128, kTsMaxTok = 256, kTsStepTiles = 4;      // k-step: 4 tile rows
-constexpr int kTsAStages = 8, kTsACol0 = 256;       // tensor memory: D in columns 0..255, A stages behind it
+constexpr int kTsStages = 8;                        // k-steps in flight: stages of ring w and of the weights in tensor memory
+// Tensor memory, 512 columns: two accumulators of up to 128 tokens (a tile's MMAs go on while the one before
+// is finished) or one of up to 256, then the stages of weights.  With four stages instead of eight, and the
+// columns given to larger double accumulators, every shape was slower: a set then waits for the MMAs of its
+// own k-step before it can decode the next.
+constexpr int kTsACol0 = 256;
 constexpr int kTsMaxXStages = 8;
 constexpr int kTsCtrlBytes = 1024;
 constexpr int kTsHBytes = 128 * 128 * 2, kTsYBytes = 128 * 128 * 2;
@@ -51,7 +57,7 @@ constexpr int kTsSmemBytes = 227 * 1024;
 template <int K> struct TsLayout {
     static constexpr int kTileWords = 8 * K;
     static constexpr int kWBytes = 32 * kTileWords * 4;                 // 8 x 4 packed tiles: K KiB
-    static constexpr int kXOff = kTsWOff + kTsAStages * kWBytes;
+    static constexpr int kXOff = kTsWOff + kTsStages * kWBytes;
     static constexpr int kXRoom = kTsSmemBytes - kXOff;
     // tokens per tile of a dense launch: at least four stages of activations have to fit
     static constexpr int kTok = kXRoom / 512 >= kTsMaxTok ? kTsMaxTok : kXRoom / 512 / 16 * 16;
@@ -177,10 +183,15 @@ template <bool TABLE> struct TsWalk {
     // the same value in every lane already; the broadcast tells the compiler
     static __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
     int64_t u, u1, u0;
-    int item;
+    // tables: a warp looks at 32 of its CTA's items at a time, one per lane, and takes those in use in turn
+    int item;                 // first item not looked at yet
+    uint32_t found;           // items in use among those looked at last
+    int4 p, q;                // this lane's
+    int it;
     __device__ __forceinline__ void start(const GemmArgs& a)
     {
         item = (int)blockIdx.x;
+        found = 0;
         const int64_t g = gridDim.x, c = blockIdx.x, nks = a.t_in >> 2;
         if (a.ts_split) {
             u0 = a.n_items * nks * c / g;
@@ -195,21 +206,40 @@ template <bool TABLE> struct TsWalk {
     {
         const int nks = a.t_in >> 2;
         if (TABLE) {
-            for (; item < a.n_items; item += gridDim.x) {
-                const int h = item & 1;
-                int4 p = reinterpret_cast<const int4*>(a.tile_tab)[item & ~1];
-                int4 q = reinterpret_cast<const int4*>(a.tile_tab)[item | 1];
-                p.x = uniform(p.x); p.y = uniform(p.y); p.z = uniform(p.z); p.w = uniform(p.w);
-                q.x = uniform(q.x); q.y = uniform(q.y); q.z = uniform(q.z);
-                if (p.x >= p.y || 128 * h >= q.y) continue;
-                s.m0 = p.x; s.rows = p.y - p.x;
-                s.tn0 = p.z + 8 * h; s.sv_off = p.w + 128 * h;
-                s.y_col = q.x + 128 * h; s.y_row_delta = q.z;
-                s.k0 = 0; s.k1 = nks; s.tile = item; s.first = 1; s.member = 0;
-                item += gridDim.x;
-                return true;
+            // Items: column halves of the table's tiles, then once more for the second part of tiles with more
+            // rows than ts_tok (parts of equal size).
+            while (!found) {
+                if (item >= a.n_items) return false;
+                it = item + (int)(threadIdx.x & 31) * (int)gridDim.x;
+                const int per_part = 2 * a.n_tiles_tab, part = it / per_part, e = it - part * per_part, h = e & 1;
+                bool used = it < a.n_items;
+                if (used) {
+                    p = reinterpret_cast<const int4*>(a.tile_tab)[e & ~1];
+                    q = reinterpret_cast<const int4*>(a.tile_tab)[e | 1];
+                    const int rows = p.y - p.x, parts = (rows + a.ts_tok - 1) / a.ts_tok;
+                    used = rows > 0 && 128 * h < q.y && part < parts;
+                    if (used) {
+                        const int size = ((rows + parts - 1) / parts + 15) & ~15;
+                        p.x += part * size;
+                        p.y = min(size, p.y - p.x);                // now: rows of the part
+                        used = p.y > 0;
+                        p.z += 8 * h; p.w += 128 * h; q.x += 128 * h;
+                    }
+                }
+                found = __ballot_sync(0xFFFFFFFFu, used);
+                item += 32 * (int)gridDim.x;
             }
-            return false;
+            const int l = __ffs(found) - 1;
+            found &= found - 1;
+            s.m0 = __shfl_sync(0xFFFFFFFFu, p.x, l);
+            s.rows = __shfl_sync(0xFFFFFFFFu, p.y, l);
+            s.tn0 = __shfl_sync(0xFFFFFFFFu, p.z, l);
+            s.sv_off = __shfl_sync(0xFFFFFFFFu, p.w, l);
+            s.y_col = __shfl_sync(0xFFFFFFFFu, q.x, l);
+            s.y_row_delta = __shfl_sync(0xFFFFFFFFu, q.z, l);
+            s.tile = __shfl_sync(0xFFFFFFFFu, it, l);
+            s.k0 = 0; s.k1 = nks; s.first = 1; s.member = 0;
+            return true;
         }
         if (u >= u1) return false;
         s.first = u == u0;
@@ -234,19 +264,19 @@ template <bool TABLE> struct TsWalk {
     }
 };
 
-template <int K, int CB, bool TABLE>
+template <int K, int CB, bool TABLE, bool AHEAD>
 __global__ void __launch_bounds__(kTsThreads, 1)
     gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w)
 {
     using L = TsLayout<K>;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* w_full = reinterpret_cast<uint64_t*>(smem);      // packed tiles landed                      [8]
-    uint64_t* w_empty = w_full + kTsAStages;                   // ... read by the set's four warps          [8]
-    uint64_t* full = w_empty + kTsAStages;                     // weights decoded AND activations landed    [8]
-    uint64_t* empty = full + kTsAStages;                       // the k-step's MMAs are done                [8]
-    uint64_t* d_full = empty + kTsAStages;                   // the segment's sums are complete
-    uint64_t* d_empty = d_full + 1;                            // ... and drained
-    uint64_t* h_full = d_empty + 1;                            // the rotated tile is complete
+    uint64_t* w_empty = w_full + kTsStages;                   // ... read by the set's four warps          [8]
+    uint64_t* full = w_empty + kTsStages;                     // weights decoded AND activations landed    [8]
+    uint64_t* empty = full + kTsStages;                       // the k-step's MMAs are done                [8]
+    uint64_t* d_full = empty + kTsStages;                      // a segment's sums are complete             [2]
+    uint64_t* d_empty = d_full + 2;                            // ... and drained                          [2]
+    uint64_t* h_full = d_empty + 2;                            // the rotated tile is complete
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(h_full + 1);
     volatile int* handoff = reinterpret_cast<volatile int*>(tmem_slot + 2);
     const TsWait wait{reinterpret_cast<volatile int*>(tmem_slot + 1), a.status};
@@ -263,14 +293,16 @@ __global__ void __launch_bounds__(kTsThreads, 1)
 
     if (tid == 0) {
         *wait.abort_word = 0;
-        for (int s = 0; s < kTsAStages; s++) {
+        for (int s = 0; s < kTsStages; s++) {
             mbar_init(smem_u32(&w_full[s]), 1);
             mbar_init(smem_u32(&w_empty[s]), 4);
             mbar_init(smem_u32(&full[s]), 5);                  // a set's four warps and the activations' copy
             mbar_init(smem_u32(&empty[s]), 1);
         }
-        mbar_init(smem_u32(d_full), 1);
-        mbar_init(smem_u32(d_empty), kTsDecodeWarps);
+        for (int s = 0; s < 2; s++) {
+            mbar_init(smem_u32(&d_full[s]), 1);
+            mbar_init(smem_u32(&d_empty[s]), kTsDecodeWarps);
+        }
         mbar_init(smem_u32(h_full), 1);
         mbar_fence_init();
     }
@@ -299,7 +331,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                     mbar_arrive_expect_tx(bar, L::kWBytes);
                     tma_load_3d(smem_u32(w_ring) + s * L::kWBytes, &tm_w, 0, sg.tn0, kTsStepTiles * ks, bar);
                 }
-                if (++s == kTsAStages) { s = 0; parity ^= 1u; }
+                if (++s == kTsStages) { s = 0; parity ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -315,9 +347,9 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             const int boxes = (sg.rows + box_rows - 1) / box_rows;
             for (int ks = sg.k0; ks < sg.k1; ks++, v++) {
                 const int u = v - nx;
-                if (u >= 0) wait(&empty[u & (kTsAStages - 1)], (uint32_t)(u / kTsAStages) & 1u);
+                if (u >= 0) wait(&empty[u & (kTsStages - 1)], (uint32_t)(u / kTsStages) & 1u);
                 if (leader) {
-                    const uint32_t bar = smem_u32(&full[v & (kTsAStages - 1)]);
+                    const uint32_t bar = smem_u32(&full[v & (kTsStages - 1)]);
                     const uint32_t dst = smem_u32(x_ring) + (uint32_t)(s * x_bytes);
                     mbar_arrive_expect_tx(bar, (uint32_t)(boxes * box_bytes));
                     tma_load_2d(dst, &tm_x, ks * 64, sg.m0, bar);
@@ -331,37 +363,38 @@ __global__ void __launch_bounds__(kTsThreads, 1)
         // -------------------------------------------------------------------- MMA issuer ----
         const bool leader = elect_one();
         if (TABLE) griddep_wait();
-        int xs = 0, as = 0;
-        uint32_t parity = 0, dpar = 1;
+        int xs = 0, as = 0, db = 0, v = 0;
+        uint32_t dpar = 1;
         const uint32_t x0 = smem_u32(x_ring);
         while (walk.next(a, sg)) {
-            wait(d_empty, dpar);
-            dpar ^= 1u;
+            wait(&d_empty[db], dpar);
             tc_fence_after_sync();
+            const uint32_t d_tmem = tmem_base + (uint32_t)(128 * db);
             const uint32_t idesc = mma_idesc_f16(128, (sg.rows + 15) & ~15);
             uint32_t accum = 0;
-            for (int ks = sg.k0; ks < sg.k1; ks++) {
+            for (int ks = sg.k0; ks < sg.k1; ks++, v++) {
                 const uint32_t at = tmem_base + kTsACol0 + 32 * as;
                 const uint64_t xd = smem_desc_sw128(x0 + (uint32_t)(xs * x_bytes));
-                wait(&full[as], parity);
+                wait(&full[v & (kTsStages - 1)], (uint32_t)(v / kTsStages) & 1u);
                 tc_fence_after_sync();
                 if (leader) {                                  // 16 k = 8 columns of A, 32 bytes of B
-                    tc_mma_f16_ts(tmem_base, at, xd, idesc, accum);
-                    tc_mma_f16_ts(tmem_base, at + 8, xd + 2, idesc, 1u);
-                    tc_mma_f16_ts(tmem_base, at + 16, xd + 4, idesc, 1u);
-                    tc_mma_f16_ts(tmem_base, at + 24, xd + 6, idesc, 1u);
-                    tc_commit(smem_u32(&empty[as]));
+                    tc_mma_f16_ts(d_tmem, at, xd, idesc, accum);
+                    tc_mma_f16_ts(d_tmem, at + 8, xd + 2, idesc, 1u);
+                    tc_mma_f16_ts(d_tmem, at + 16, xd + 4, idesc, 1u);
+                    tc_mma_f16_ts(d_tmem, at + 24, xd + 6, idesc, 1u);
+                    tc_commit(smem_u32(&empty[v & (kTsStages - 1)]));
                 }
                 accum = 1u;
                 if (++xs == nx) xs = 0;
-                if (++as == kTsAStages) { as = 0; parity ^= 1u; }
+                if (++as == kTsStages) as = 0;
             }
-            if (leader) tc_commit(smem_u32(d_full));
+            if (leader) tc_commit(smem_u32(&d_full[db]));
+            if (++db == a.ts_dbuf) { db = 0; dpar ^= 1u; }
         }
     } else if (warp >= kTsFirstDecodeWarp) {
-        // -------------------------------------------------------- decode, then finish ----
-        const int dt = tid - 32 * kTsFirstDecodeWarp;
+        // ------------------------------------------------- decode, and finish the tiles ----
         const int q = warp & 3, set = (warp - kTsFirstDecodeWarp) >> 2;
+        const int dt = tid - 32 * kTsFirstDecodeWarp;
         const int prev_word = (lane + 31) & 31;
         const uint32_t xc = a.cb_xor;
         const int nks = a.t_in >> 2;
@@ -383,15 +416,25 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             }
         }
         if (TABLE) griddep_wait();
-        int kc = 0;                                                // k-steps of this CTA so far
+        // A set decodes its k-steps in order, whatever tiles they belong to.  With AHEAD the warps decode up to
+        // eight k-steps of the next tile before they finish one, so that the tensor core has work in the meantime
+        // (SwitchGLU of 4096 tokens 546 -> 524 us); a CTA with hardly more than one tile is 1 us quicker without.
+        int kc = 0, v = set;                                       // end of the current tile's k-steps; next one of this set
+        int db = 0;
         uint32_t dpar = 0, hpar = 0;
-        while (walk.next(a, sg)) {
+        TsSeg nx_sg;
+        bool more = walk.next(a, nx_sg);
+        while (more) {
+            sg = nx_sg;
+            more = walk.next(a, nx_sg);
             const int n_steps = sg.k1 - sg.k0;
-            for (int v = kc + ((set - kc) & 3); v < kc + n_steps; v += kTsSets) {
+            kc += n_steps;
+            const int v_end = kc + (AHEAD && more ? min(kTsStages, nx_sg.k1 - nx_sg.k0) : 0);
+            for (; v < v_end; v += kTsSets) {
                 // Eight stages, four sets: a stage of ring w always belongs to the same set.  (With another number a
                 // set could look at a barrier two phases early and read a stale parity.)
-                const int st = v & (kTsAStages - 1);
-                const uint32_t parity = (uint32_t)(v / kTsAStages) & 1u;
+                const int st = v & (kTsStages - 1);
+                const uint32_t parity = (uint32_t)(v / kTsStages) & 1u;
                 wait(&w_full[st], parity);
                 // tile columns 2q, 2q + 1 of all four tile rows: words first, so that the slot can be refilled
                 const uint32_t* wt = reinterpret_cast<const uint32_t*>(w_ring + st * L::kWBytes) + 2 * q * L::kTileWords;
@@ -436,25 +479,38 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&full[st]));
             }
-            kc += n_steps;
 
-            // ---- the segment's sums are complete ----
-            wait(d_full, dpar);
-            dpar ^= 1u;
-            tc_fence_after_sync();
-            const uint32_t lane_base = tmem_base + ((uint32_t)(32 * q) << 16);
+            // ---- finish the tile: what it needs from global memory first ----
             const int out = 32 * q + lane;                         // this thread's column of the tile
             const int n16 = (sg.rows + 15) >> 4;
+            if (a.svh) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.svh + sg.sv_off + 32 * set));
+            auto out_row = [&](int tg) {                           // output row of this thread's token
+                const int row = 128 * tg + out, grow = sg.m0 + row + sg.y_row_delta;
+                return a.y_row_map && row < sg.rows ? a.y_row_map[grow] : grow;
+            };
+            int orow = out_row(0);
+            wait(&d_full[db], dpar);
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem_base + (uint32_t)(128 * db);
+            const uint32_t lane_base = d_tmem + ((uint32_t)(32 * q) << 16);
             const size_t slot_floats = (size_t)kTsOuts * a.ts_tok;
+            bool held = true;
+            auto release_d = [&]() {                               // the next tile's MMAs may go into this D
+                if (!held) return;
+                held = false;
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&d_empty[db]));
+            };
             bool finish = true;
             int c_first = 0, n_contrib = 1, slot_first = 0;
             if (n_steps != nks) {
                 float* part = a.ts_partials + (size_t)(2 * blockIdx.x + (sg.first ? 0 : 1)) * slot_floats + out;
                 for (int ch = set; ch < n16; ch += kTsSets) {
-                    float v[16];
-                    tmem_ld_16cols(lane_base + 16 * ch, v);
+                    float f[16];
+                    tmem_ld_16cols(lane_base + 16 * ch, f);
 #pragma unroll
-                    for (int i = 0; i < 16; i++) __stcg(part + (16 * ch + i) * kTsOuts, v[i]);
+                    for (int i = 0; i < 16; i++) __stcg(part + (16 * ch + i) * kTsOuts, f[i]);
                 }
                 named_bar_sync(1, 512);
                 if (dt == 0) {
@@ -477,26 +533,28 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                 slot_first = handoff[3];
             }
             if (finish) {
-                for (int tg = 0; 128 * tg < sg.rows; tg++) {
-                    const int ch1 = min(8 * tg + 8, n16);
-                    for (int ch = 8 * tg + set; ch < ch1; ch += kTsSets) {
-                        float v[16];
+                // The rotated half goes over D's first 128 columns, which have been read by then.
+#pragma unroll 1
+                for (int tg = 0; 128 * tg < sg.rows; tg++) {       // 128 tokens at a time
+#pragma unroll 1
+                    for (int ch = 8 * tg + set; ch < min(8 * tg + 8, n16); ch += kTsSets) {
+                        float f[16];
                         if (n_steps == nks) {
-                            tmem_ld_16cols(lane_base + 16 * ch, v);
+                            tmem_ld_16cols(lane_base + 16 * ch, f);
                         } else {
 #pragma unroll
-                            for (int i = 0; i < 16; i++) v[i] = 0.f;
+                            for (int i = 0; i < 16; i++) f[i] = 0.f;
 #pragma unroll 2
                             for (int j = 0; j < n_contrib; j++) {  // in CTA order
                                 const float* p = a.ts_partials + (size_t)(2 * (c_first + j) + (j == 0 ? slot_first : 0)) * slot_floats +
                                                  out + (size_t)(16 * ch) * kTsOuts;
 #pragma unroll
-                                for (int i = 0; i < 16; i++) v[i] += __ldcg(p + i * kTsOuts);
+                                for (int i = 0; i < 16; i++) f[i] += __ldcg(p + i * kTsOuts);
                             }
                         }
                         uint32_t hv[8];
 #pragma unroll
-                        for (int i = 0; i < 8; i++) hv[i] = h2_as_u32(__floats2half2_rn(v[2 * i], v[2 * i + 1]));
+                        for (int i = 0; i < 8; i++) hv[i] = h2_as_u32(__floats2half2_rn(f[2 * i], f[2 * i + 1]));
                         const int c16 = ch & 7;                    // 16 tokens = two 16-byte pieces of a 64-token row
                         uint8_t* row = y_buf + (c16 >> 2) * 16384 + out * 128;
                         const int piece = 2 * (c16 & 3), sw = out & 7;
@@ -506,27 +564,26 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                     fence_proxy_async_smem();
                     tc_fence_before_sync();
                     named_bar_sync(1, 512);
-                    if (dt == 0) {
+                    if (warp == kTsFirstDecodeWarp) {
                         tc_fence_after_sync();
-                        const uint32_t ya = smem_u32(y_buf), hb = smem_u32(h_mat);
+                        const uint64_t yd = smem_desc_mn_sw128(smem_u32(y_buf)), hd = smem_desc_sw128(smem_u32(h_mat));
+                        if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < 8; kk++)
-                            tc_mma_f16(tmem_base + 128 * tg, smem_desc_mn_sw128(ya + kk * 2048),
-                                       smem_desc_sw128(hb + (kk >> 2) * 16384 + (kk & 3) * 32),
-                                       mma_idesc_f16(128, 128) | kIdescMajorA, kk > 0 ? 1u : 0u);
-                        tc_commit(smem_u32(h_full));
+                            for (int kk = 0; kk < 8; kk++)
+                                tc_mma_f16(d_tmem, yd + 128 * kk, hd + (kk >> 2) * 1024 + (kk & 3) * 2,
+                                           mma_idesc_f16(128, 128) | kIdescMajorA, kk > 0 ? 1u : 0u);
+                            tc_commit(smem_u32(h_full));
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
                     wait(h_full, hpar);
                     hpar ^= 1u;
                     tc_fence_after_sync();
-                    float v[32];
-                    tmem_ld_32cols(lane_base + 128 * tg + 32 * set, v);
-                    const int row = 128 * tg + 32 * q + lane;      // lane = token now
-                    if (row < sg.rows) {
-                        const int grow = sg.m0 + row + sg.y_row_delta;
-                        const int orow = a.y_row_map ? a.y_row_map[grow] : grow;
-                        const int col0 = sg.y_col + 32 * set, sv0 = sg.sv_off + 32 * set;
+                    float f[32];
+                    tmem_ld_32cols(lane_base + 32 * set, f);
+                    if (128 * tg + 128 >= sg.rows) release_d();    // the last reads of D
+                    if (128 * tg + out < sg.rows) {                // lane = token now
+                        const int col0 = sg.y_col + 32 * set;
                         __half* yp;
                         if (a.n_peer > 0) {      // the row belongs to the GPU that holds its token
                             const int pr = orow / a.rows_per_peer;
@@ -535,48 +592,42 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                             yp = !TABLE && a.n_members > 1 ? a.member_y[sg.member] + (int64_t)orow * a.member_stride[sg.member] + col0
                                                            : a.y + (int64_t)orow * a.y_row_stride + col0;
                         }
-                        uint4 held = make_uint4(0u, 0u, 0u, 0u);
+                        const uint64_t scale = f32x2(EXL3_HAD_SCALE, EXL3_HAD_SCALE);
+                        uint4 held16 = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
                         for (int c = 0; c < 4; c++) {
-                            float o[8];
+                            const uint4 sv = a.svh ? *reinterpret_cast<const uint4*>(a.svh + sg.sv_off + 32 * set + 8 * c)
+                                                   : make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
+                            const uint32_t sw4[4] = {sv.x, sv.y, sv.z, sv.w};
+                            uint32_t h[4];
 #pragma unroll
-                            for (int i = 0; i < 8; i++) o[i] = v[8 * c + i] * EXL3_HAD_SCALE;
-                            if (a.svh) {
-                                const uint4 sv = *reinterpret_cast<const uint4*>(a.svh + sv0 + 8 * c);
-                                const uint32_t sw[4] = {sv.x, sv.y, sv.z, sv.w};
-#pragma unroll
-                                for (int i = 0; i < 4; i++) {
-                                    const float2 f = __half22float2(u32_as_h2(sw[i]));
-                                    o[2 * i] *= f.x;
-                                    o[2 * i + 1] *= f.y;
-                                }
+                            for (int i = 0; i < 4; i++) {
+                                const float2 w2 = __half22float2(u32_as_h2(sw4[i]));
+                                h[i] = f16_pair(mul_f32x2(mul_f32x2(f32x2(f[8 * c + 2 * i], f[8 * c + 2 * i + 1]), scale), f32x2(w2.x, w2.y)));
                             }
-                            __half2 h[4];
-#pragma unroll
-                            for (int i = 0; i < 4; i++) h[i] = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
                             if (a.bias) {
-                                const uint4 bv = *reinterpret_cast<const uint4*>(a.bias + sv0 + 8 * c);
+                                const uint4 bv = *reinterpret_cast<const uint4*>(a.bias + sg.sv_off + 32 * set + 8 * c);
                                 const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
-                                for (int i = 0; i < 4; i++) h[i] = __hadd2(h[i], u32_as_h2(bw[i]));
+                                for (int i = 0; i < 4; i++) h[i] = h2_as_u32(__hadd2(u32_as_h2(h[i]), u32_as_h2(bw[i])));
                             }
-                            const uint4 ov = make_uint4(h2_as_u32(h[0]), h2_as_u32(h[1]), h2_as_u32(h[2]), h2_as_u32(h[3]));
+                            const uint4 ov = make_uint4(h[0], h[1], h[2], h[3]);
                             if (!a.y_wide) {
                                 *reinterpret_cast<uint4*>(yp + 8 * c) = ov;
                             } else if (c & 1) {
-                                st_global_256(yp + 8 * (c - 1), held, ov);   // whole sectors, also into another GPU
+                                st_global_256(yp + 8 * (c - 1), held16, ov);   // whole sectors, also into another GPU
                             } else {
-                                held = ov;
+                                held16 = ov;
                             }
                         }
                     }
+                    if (128 * tg + 128 < sg.rows) orow = out_row(1);
                 }
             }
-            tc_fence_before_sync();
-            // handoff and y_buf are read by all warps before any of them comes here again: the next use is
-            // behind the named barrier of the next shared tile
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(d_empty));
+            release_d();
+            // (handoff and y_buf are read by all warps before any of them comes here again: the next use is
+            // behind the named barrier of the next tile)
+            if (++db == a.ts_dbuf) { db = 0; dpar ^= 1u; }
         }
     }
     __syncwarp();
@@ -622,8 +673,9 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxDevices) return EXL3_E_UNSUPPORTED;
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             kTsSmemBytes);
+        cudaError_t e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
+        if (e == cudaSuccess && !TABLE)
+            e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
         if (e != cudaSuccess) return note_cuda(e);
         attr_set[dev] = true;
     }
@@ -632,10 +684,18 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
     int grid;
     a.ts_split = 0;
     if (TABLE) {
+        // Rows of a tile: what nearly all tiles need if the caller says how many rows a tile has on average
+        // (the activation ring is as deep as its stages are small), the table's 256 if not.
         a.ts_tok = kTsMaxTok;
         a.ts_box_rows = 64;
-        a.n_items = 2 * a.n_tiles_tab;
-        grid = std::min(a.n_items, sms);
+        if (a.rows_hint > 0 && a.rows_hint < 200) {
+            const double most = a.rows_hint + 2.5 * std::sqrt((double)a.rows_hint);
+            a.ts_tok = std::max(128, std::min(kTsMaxTok, ((int)most + 31) / 32 * 32));
+            a.ts_box_rows = 32;
+        }
+        a.n_items = 2 * a.n_tiles_tab * (a.ts_tok < kTsMaxTok ? 2 : 1);
+        // an odd stride: which items are in use repeats with a period of 2 or 4
+        grid = std::min(a.n_items, (sms - 1) | 1);
     } else {
         a.tiles_m = (a.m + L::kTok - 1) / L::kTok;
         a.ts_tok = ((a.m + a.tiles_m - 1) / a.tiles_m + 15) / 16 * 16;
@@ -646,7 +706,8 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
         grid = ts_plan(a.n_items, nks, sms, a.m, a.ts_partial_bytes, &a.ts_split);
     }
     a.ts_x_bytes = (a.ts_tok + a.ts_box_rows - 1) / a.ts_box_rows * a.ts_box_rows * 128;
-    a.stages = std::min(kTsMaxXStages, L::kXRoom / a.ts_x_bytes);
+    a.stages = std::min(kTsStages, L::kXRoom / a.ts_x_bytes);
+    a.ts_dbuf = a.ts_tok <= 128 ? 2 : 1;
     CUtensorMap tm_x, tm_w;
     {
         const uint64_t in = (uint64_t)a.t_in * 16;
@@ -663,7 +724,8 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
                              CU_TENSOR_MAP_SWIZZLE_NONE);
         if (rc) return rc;
     }
-    return launch_kernel(gemm_kernel<K, CB, TABLE>, dim3((unsigned)grid), dim3(kTsThreads), kTsSmemBytes, s, true, a, tm_x, tm_w);
+    const auto kernel = TABLE || a.n_items >= 2 * grid ? gemm_kernel<K, CB, TABLE, true> : gemm_kernel<K, CB, TABLE, TABLE>;
+    return launch_kernel(kernel, dim3((unsigned)grid), dim3(kTsThreads), kTsSmemBytes, s, true, a, tm_x, tm_w);
 }
 
 template <int K>

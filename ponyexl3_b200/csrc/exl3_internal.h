@@ -162,6 +162,7 @@ struct GemmArgs {
     const int32_t* tile_tab;  // grouped launches: device table of 8 ints per tile, else NULL
     const int32_t* y_row_map; // grouped launches: output row of every computed row, or NULL (identity)
     int n_tiles_tab;          // slots in tile_tab
+    int rows_hint;            // average rows of the tiles in use, 0: unknown
     int xh_rows;              // rows of the rotated-activation matrix
     int m;                    // rows (tokens)
     int t_in, t_out;          // tiles
@@ -185,6 +186,7 @@ struct GemmArgs {
     int ts_tok;               // tokens per output tile
     int ts_x_bytes;           // bytes of one stage of the activation ring
     int ts_box_rows;          // rows of one activation TMA box
+    int ts_dbuf;              // accumulators in tensor memory
     // sibling groups: member i has the column blocks [member_end[i - 1], member_end[i]) of the trellis, the
     // rotated rows [i m, (i + 1) m) and an output matrix of its own
     int n_members;            // 0 or 1: a plain layer

@@ -13,6 +13,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <algorithm>
 #include <string>
 
 #include "../../../include/exl3_b200.h"
@@ -372,13 +373,14 @@ PyObject* switch_glu(PyObject* const* arg)
                 *suh_dn = suh_gu + 2 * n;
         check(api.exl3_moe_prefill_tables(idx.data_ptr(), bytes, (int)n, (int)kk, (int)E, D, H, order, row_src, suh_gu, suh_dn,
                                           tiles_gu, tiles_dn, 0, es), "exl3_moe_prefill_tables");
+        const unsigned hint = (unsigned)std::min<int64_t>(n / E, 0xFFFF) << 16;      // rows of an expert
         Workspace ws = workspace(dev, api.exl3_gemm_workspace_bytes(2 * n, D));
         check(api.exl3_gemm_tiles(r.t.data_ptr(), r.dtype, r.stride, 2 * n, row_src, gu_suh, suh_gu, gu.trellis, gu.t_in,
-                                  gu.t_out, k, cb, tiles_gu, n_gu, gu_svh, u16(ygu), 2 * H, nullptr, ws.ptr, ws.bytes, 0, es),
+                                  gu.t_out, k, cb, tiles_gu, n_gu, gu_svh, u16(ygu), 2 * H, nullptr, ws.ptr, ws.bytes, hint, es),
               "exl3_gemm_tiles");
         ws = workspace(dev, api.exl3_gemm_workspace_bytes(n, H));
         check(api.exl3_gemm_tiles(ygu.data_ptr(), EXL3_DT_F16, 2 * H, n, nullptr, dn_suh, suh_dn, dn.trellis, dn.t_in, dn.t_out,
-                                  k, cb, tiles_dn, n_dn, dn_svh, u16(y), D, order, ws.ptr, ws.bytes, glu, es), "exl3_gemm_tiles");
+                                  k, cb, tiles_dn, n_dn, dn_svh, u16(y), D, order, ws.ptr, ws.bytes, glu | hint, es), "exl3_gemm_tiles");
     }
     return THPVariable_Wrap(std::move(y));
 }
