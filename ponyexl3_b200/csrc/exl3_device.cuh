@@ -186,6 +186,9 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
         : "memory");
 }
 
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];\n" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+
 // Programmatic dependent launch: let the next kernel of the stream start its
 // independent prologue / wait until the kernels this one depends on have finished.
 __device__ __forceinline__ void griddep_launch_dependents()

@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             // ---- finish the tile: what it needs from global memory first ----
             const int out = 32 * q + lane;                         // this thread's column of the tile
             const int n16 = (sg.rows + 15) >> 4;
-            if (a.svh) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.svh + sg.sv_off + 32 * set));
+            if (a.svh) prefetch_l1(a.svh + sg.sv_off + 32 * set);
             auto out_row = [&](int tg) {                           // output row of this thread's token
                 const int row = 128 * tg + out, grow = sg.m0 + row + sg.y_row_delta;
                 return a.y_row_map && row < sg.rows ? a.y_row_map[grow] : grow;

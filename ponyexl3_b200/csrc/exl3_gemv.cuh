@@ -180,9 +180,6 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
     extern __shared__ __align__(1024) uint8_t smem[];
 
     EXL3_STAMP(gt_entry);
-    // Without EXL3_FLAG_PDL nothing is read, and no later kernel may start reading, before everything
-    // earlier in the stream is complete; the launch itself still overlaps the previous kernel's end.
-    if (!a.early_weights) griddep_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // The CTA is two independent halves of 16 warps; each is one "virtual CTA" of the partition.
     const int half = warp >> 4, wl = warp & 15, tidh = tid & (kHalfThreads - 1);
@@ -237,6 +234,21 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
         done_cnt[tidh] = 0;
         issued[tidh] = -1;
         mbar_fence_init();
+    }
+    if (!a.early_weights) {
+        // Without EXL3_FLAG_PDL nothing is read, and no later kernel may start reading, before everything
+        // earlier in the stream is complete; the set-up above still overlaps the previous kernel's end, and
+        // so do hints that bring the range's weights and signs into L2, where a late write would find them.
+        if (!a.blocks && !a.ncb_dev) {
+            if (wl == 1 && lane < min(nitems, ns)) {
+                const int kq = kb0 + lane, dq = kq / nkb;
+                tma_prefetch_l2_3d(&tm_w, 0, 8 * (cb0 + dq), 8 * (kq - dq * nkb));
+            }
+            if (XFUSED && wl == 2 && a.suh)
+                for (int i = lane; i < 2 * min(nitems, nkb); i += 32)
+                    prefetch_l2(a.suh + (size_t)((kb0 + (i >> 1)) % nkb) * 128 + 64 * (i & 1));
+        }
+        griddep_wait();
     }
     __syncthreads();
     griddep_launch_dependents();
@@ -451,6 +463,15 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
 #endif
     }
     EXL3_STAMP(gt_loop);
+    // Block tables: the output scales lie where the table says, two dependent loads that would be waited for
+    // when the last segment is handed over (SwitchGLU of 16 tokens: 2 us of 134).
+    if (a.blocks && wl == kHalfWarps - 1 && a.svh && !a.raw_out) {
+        const int nblk = (kb0 + nitems - 1) / nkb + 1;
+        for (int i = lane; i < 2 * nblk; i += 32) {
+            const int off = a.blocks[cb0 + (i >> 1)].sv_off;
+            if (off >= 0) prefetch_l1(a.svh + off + 64 * (i & 1));
+        }
+    }
 
     float acc[2][NMMA][4];
 #pragma unroll
