@@ -180,9 +180,11 @@ struct TsSeg {
 
 // The segments of one CTA, the same sequence for every role.
 template <bool TABLE> struct TsWalk {
-    // the same value in every lane already; the broadcast tells the compiler
-    static __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
-    int64_t u, u1, u0;
+    // The same value in every lane already; the reduction tells the compiler, because its result is a uniform
+    // register.  (Behind a shuffle or a 64-bit division all of the issuing warps' loop control and descriptors
+    // lived in ordinary registers and were moved over for every instruction: 5 to 9 % of the kernel.)
+    static __device__ __forceinline__ int uniform(int v) { return __reduce_max_sync(0xFFFFFFFFu, v); }
+    int u, u1, u0;
     // tables: a warp looks at 32 of its CTA's items at a time, one per lane, and takes those in use in turn
     int item;                 // first item not looked at yet
     uint32_t found;           // items in use among those looked at last
@@ -194,11 +196,11 @@ template <bool TABLE> struct TsWalk {
         found = 0;
         const int64_t g = gridDim.x, c = blockIdx.x, nks = a.t_in >> 2;
         if (a.ts_split) {
-            u0 = a.n_items * nks * c / g;
-            u1 = a.n_items * nks * (c + 1) / g;
+            u0 = uniform((int)(a.n_items * nks * c / g));
+            u1 = uniform((int)(a.n_items * nks * (c + 1) / g));
         } else {
-            u0 = a.n_items * c / g * nks;
-            u1 = a.n_items * (c + 1) / g * nks;
+            u0 = uniform((int)(a.n_items * c / g * nks));
+            u1 = uniform((int)(a.n_items * (c + 1) / g * nks));
         }
         u = u0;
     }
@@ -243,9 +245,9 @@ template <bool TABLE> struct TsWalk {
         }
         if (u >= u1) return false;
         s.first = u == u0;
-        s.tile = uniform((int)(u / nks));
-        s.k0 = uniform((int)(u - (int64_t)s.tile * nks));
-        s.k1 = uniform((int)min((int64_t)nks, s.k0 + (u1 - u)));
+        s.tile = uniform(u / nks);
+        s.k0 = u - s.tile * nks;
+        s.k1 = min(nks, s.k0 + (u1 - u));
         u += s.k1 - s.k0;
         const int tn = uniform(s.tile / a.tiles_m), tm = s.tile - tn * a.tiles_m;
         s.m0 = tm * a.ts_tok;
@@ -436,7 +438,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                 const int st = v & (kTsStages - 1);
                 const uint32_t parity = (uint32_t)(v / kTsStages) & 1u;
                 wait(&w_full[st], parity);
-                // tile columns 2q, 2q + 1 of all four tile rows: words first, so that the slot can be refilled
+                // tile columns 2q, 2q + 1 of all four tile rows
                 const uint32_t* wt = reinterpret_cast<const uint32_t*>(w_ring + st * L::kWBytes) + 2 * q * L::kTileWords;
                 uint32_t pw[2][4][K == 4 ? 4 : 3];
 #pragma unroll
@@ -455,8 +457,6 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                             pw[h][tk][2] = LaneWords<K>::kThree ? tw[lw.i2] : 0u;
                         }
                     }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&w_empty[st]));
                 wait(&empty[st], parity ^ 1u);
                 tc_fence_after_sync();
 #pragma unroll
@@ -474,6 +474,11 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                     }
                     tmem_st_16x32cols(tmem_base + ((uint32_t)(32 * q + 16 * h) << 16) + kTsACol0 + 32 * st, frag);
                 }
+                // Only now is it certain that the packed words have been read: the stores above depend on them.  (With
+                // the slot given back before the wait for `empty`, some loads were found to take place after it, and
+                // to see the words of eight k-steps later.)
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&w_empty[st]));
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -703,6 +708,7 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
         a.ts_box_rows = a.ts_tok;
         a.tiles_n = a.t_out / 8;
         a.n_items = a.tiles_m * a.tiles_n;
+        if ((int64_t)a.n_items * nks >= ((int64_t)1 << 31)) return EXL3_E_SHAPE;   // (k-steps are counted in 32 bits)
         grid = ts_plan(a.n_items, nks, sms, a.m, a.ts_partial_bytes, &a.ts_split);
     }
     a.ts_x_bytes = (a.ts_tok + a.ts_box_rows - 1) / a.ts_box_rows * a.ts_box_rows * 128;

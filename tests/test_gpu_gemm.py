@@ -104,6 +104,17 @@ def test_gemm_tiles_shared_between_ctas(mod, oracle, rows, inf, outf, k, cb):
     assert mod.ops.Workspace.get(torch.device("cuda"), 1, 128).status() == 0
 
 
+def test_gemm_of_many_tiles_per_cta_equals_small_calls(mod):
+    """Every CTA has several tiles and decodes ahead of the one it finishes: the same rows in calls of 128
+    (one tile per CTA) and all at once, several times over."""
+    m = mod.EXL3Linear(_layer(mod, 4, 5120, 5120, seed=81))
+    x = torch.from_numpy(np.random.default_rng(8).standard_normal((2048, 5120)).astype(np.float16)).cuda()
+    want = torch.cat([m(x[i:i + 128]) for i in range(0, 2048, 128)]).float()
+    for _ in range(6):
+        y = m(x).float()
+        assert (y - want).abs().max() < 0.02 * want.abs().mean() and (y - want).norm() / want.norm() < 5e-4
+
+
 def test_gemm_many_tiles_and_k_steps(mod, oracle):
     """More tiles than one wave of k-steps per stage ring, several tiles per CTA."""
     layer = _layer(mod, 4, 2048, 1280, seed=78, bias=True)
