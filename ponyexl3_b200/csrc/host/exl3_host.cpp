@@ -21,7 +21,8 @@
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr int kGemvMaxRows = 16;
+constexpr int kGemvMaxRows = 16;      // what the streamed GEMV can do
+constexpr int kMaxMembers = 8;        // of exl3_gemm_members
 
 #define EXL3_FN(name) decltype(&::name) name = nullptr
 struct Api {
@@ -164,6 +165,18 @@ void gemm(const Rows& x, int64_t rows, const Weights& w, int k, int cb, const ui
                         y_stride, ws.ptr, ws.bytes, 0, (exl3_stream_t)s), "exl3_gemm");
 }
 
+// GEMV or GEMM.  Nine to sixteen rows take a second MMA and a rotation kernel in the GEMV, and the GEMM is as
+// quick or quicker: us at 16 rows, GEMV / GEMM, K = 4: 4096 x 4096 16.8 / 15.1, 5120 x 17408 38.5 / 34.0,
+// 17408 x 5120 39.1 / 38.3, 512 x 512 9.5 / 8.9 (at 8 rows 12.7 / 14.6, 32.0 / 32.5, 33.7 / 37.9, 6.9 / 8.8);
+// the other way round only for long inputs at K = 2 and 3, by up to 4 %.  The GEMM asks for 16-byte
+// alignment where the GEMV takes 8.
+bool use_gemv(int64_t rows, const uint16_t* svh, const uint16_t* bias, const uint16_t* y, int64_t y_stride)
+{
+    if (rows <= kGemvMaxRows / 2 || rows > kGemvMaxRows) return rows <= kGemvMaxRows;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(svh) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(y);
+    return bits % 16 != 0 || y_stride % 8 != 0;
+}
+
 uint16_t* u16(const at::Tensor& t) { return static_cast<uint16_t*>(t.data_ptr()); }
 
 // ---- linear(x, trellis, k, cb, suh, svh, bias, flags, out) ---------------------------------------------------
@@ -197,7 +210,7 @@ PyObject* linear(PyObject* const* arg)
     const uint16_t* suh = ptr_or_null<uint16_t>(arg[4], "suh");
     const uint16_t* svh = ptr_or_null<uint16_t>(arg[5], "svh");
     const uint16_t* bias = ptr_or_null<uint16_t>(arg[6], "bias");
-    if (rows <= kGemvMaxRows)
+    if (use_gemv(rows, svh, bias, u16(y), y_stride))
         gemv(r, rows, w, k, cb, suh, svh, bias, u16(y), y_stride, (unsigned)integer(arg[7]), dev, s);
     else
         gemm(r, rows, w, k, cb, suh, svh, bias, u16(y), y_stride, dev, s);
@@ -247,7 +260,22 @@ void group_gemm(const Rows& x, int64_t rows, const Group& g, const int64_t* widt
           "exl3_gemm_members");
 }
 
-// group_packed(x2d, group..., blocks, row_src, suh_row, flags) -> (rows, total), rows <= 16
+// All members side by side in one (rows, total) matrix.
+void group_gemm_packed(const Rows& x, const Group& g, PyObject* width_tuple, const at::Tensor& y, int dev, cudaStream_t s)
+{
+    c10::SmallVector<int64_t, 4> widths, strides;
+    c10::SmallVector<uint64_t, 4> ptrs;
+    uint64_t at = reinterpret_cast<uint64_t>(y.data_ptr());
+    for (int64_t i = 0; i < g.members; i++) {
+        widths.push_back(integer(PyTuple_GET_ITEM(width_tuple, i)));
+        strides.push_back(g.total);
+        ptrs.push_back(at);
+        at += 2 * (uint64_t)widths.back();
+    }
+    group_gemm(x, x.rows, g, widths.data(), ptrs.data(), strides.data(), dev, s);
+}
+
+// group_packed(x2d, group..., blocks, row_src, suh_row, flags, widths) -> (rows, total), rows <= 16
 PyObject* group_packed(PyObject* const* arg)
 {
     const at::Tensor& x = cuda_tensor(arg[0], "x");
@@ -259,8 +287,11 @@ PyObject* group_packed(PyObject* const* arg)
     const c10::cuda::CUDAGuard guard(x.device());
     const int dev = x.device().index();
     at::Tensor y = empty_half({r.rows, g.total}, x.device());
-    group_gemv(r, r.rows, g, arg[8], arg[9], arg[10], y, (unsigned)integer(arg[11]), dev,
-               c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+    const cudaStream_t s = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+    if (g.members > kMaxMembers || use_gemv(r.rows, g.svh, nullptr, u16(y), g.total))
+        group_gemv(r, r.rows, g, arg[8], arg[9], arg[10], y, (unsigned)integer(arg[11]), dev, s);
+    else
+        group_gemm_packed(r, g, arg[12], y, dev, s);
     return THPVariable_Wrap(std::move(y));
 }
 
@@ -307,7 +338,7 @@ PyObject* mlp(PyObject* const* arg)
     const at::Tensor gu = empty_half({r.rows, g.total}, x.device());
     at::Tensor y = empty_half({r.rows, 16 * d.t_out}, x.device());
     const Rows h{gu, r.rows, g.total, EXL3_DT_F16};
-    if (r.rows <= kGemvMaxRows) {
+    if (use_gemv(r.rows, svh, bias, g.svh, 0)) {
         group_gemv(r, r.rows, g, arg[8], arg[9], arg[10], gu, gflags, dev, s);
         gemv(h, r.rows, d, dk, dcb, suh, svh, bias, u16(y), 16 * d.t_out, dflags, dev, s);
     } else {
@@ -443,7 +474,7 @@ PyMethodDef methods[] = {
     EXL3_METHOD(bind, 3),
     EXL3_METHOD(set_workspace, 3),
     EXL3_METHOD(linear, 9),
-    EXL3_METHOD(group_packed, 12),
+    EXL3_METHOD(group_packed, 13),
     EXL3_METHOD(group_prefill, 9),
     EXL3_METHOD(mlp, 19),
     EXL3_METHOD(switch_glu, 15),

@@ -132,7 +132,8 @@ class FusedEXL3Group(torch.nn.Module):
         if not 1 <= rows <= GEMV_MAX_ROWS:
             raise ValueError("forward_packed serves 1..16 rows")
         return (_lib._host or _lib.host()).group_packed(
-            x2d, *self._native(), *self._table(rows, x2d.device), _lib.FLAG_PDL if self.pdl else 0)
+            x2d, *self._native(), *self._table(rows, x2d.device), _lib.FLAG_PDL if self.pdl else 0,
+            tuple(self._out_features))
 
     def _native(self) -> tuple:
         """What the host extension takes of the group."""

@@ -5,7 +5,8 @@ Same construction and call contract as the reference's ``EXL3Linear``
 ``x[..., in]`` (fp16 / bf16 / fp32), returns fp16 ``[..., out]`` with the leading
 shape preserved, optional fp16 bias, no autograd, and the packed trellis kept out
 of the parameter tree.  Routing by row count replaces the reference's ladder:
-rows <= 16 take the streamed GEMV; larger batches take the tensor-core prefill GEMM.
+rows <= 8 take the streamed GEMV (16 where the tensors are not 16-byte aligned); larger batches
+take the tensor-core prefill GEMM.
 """
 
 from __future__ import annotations
@@ -83,7 +84,7 @@ class EXL3Linear(torch.nn.Module):
 
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """`out`: optional (rows, out_features) fp16 CUDA tensor to write into (unit column stride).
-        Checks, output allocation and launch are one native call (csrc/host/exl3_host.cpp): 16 rows
+        Checks, output allocation and launch are one native call (csrc/host/exl3_host.cpp): 8 rows
         and fewer take the streamed GEMV, more the tensor-core GEMM."""
         return (_lib._host or _lib.host()).linear(
             x, self._trellis, self.k, self.cb, self._suh, self._svh, self._bias,
