@@ -41,13 +41,24 @@ namespace exl3 {
 
 constexpr int kTsDecodeWarps = 16, kTsFirstDecodeWarp = 4, kTsSets = 4;
 constexpr int kTsThreads = 32 * (kTsFirstDecodeWarp + kTsDecodeWarps);
-constexpr int kTsOuts = 128, kTsMaxTok = 256, kTsStepTiles = 4;      // k-step: 4 tile rows
-constexpr int kTsStages = 8;                        // k-steps in flight: stages of ring w and of the weights in tensor memory
-// Tensor memory, 512 columns: two accumulators of up to 128 tokens (a tile's MMAs go on while the one before
-// is finished) or one of up to 256, then the stages of weights.  With four stages instead of eight, and the
-// columns given to larger double accumulators, every shape was slower: a set then waits for the MMAs of its
-// own k-step before it can decode the next.
-constexpr int kTsACol0 = 256;
+constexpr int kTsOuts = 128, kTsStepTiles = 4;      // k-step: 4 tile rows
+constexpr int kTsMaxTok = 256, kTsWideTok = 384;    // tokens of a tile; of a wide one
+constexpr int kTsStages = 8;                        // barriers of the k-steps in flight
+// Three forms of the kernel.
+//   PLAIN  for CTAs with hardly more than one tile.
+//   AHEAD  decodes k-steps of the next tile before it finishes one.
+//   WIDE   AHEAD with up to 384 tokens a tile: the weights are decoded once for all of them, and decoding
+//          is what bounds the kernel.
+// Tensor memory, 512 columns: PLAIN and AHEAD have two accumulators of up to 128 tokens (a tile's MMAs go on
+// while the one before is finished) or one of up to 256, and eight stages of weights; WIDE has one of 384 and
+// four stages.  (Four stages with 256 tokens were slower for every shape: a set of decode warps then waits for
+// the MMAs of its own k-step before it can decode the next.)
+enum : int { TS_PLAIN = 0, TS_AHEAD = 1, TS_WIDE = 2 };
+template <int MODE> struct TsForm {
+    static constexpr bool kAhead = MODE != TS_PLAIN, kWide = MODE == TS_WIDE;
+    static constexpr int kStages = kWide ? 4 : 8;   // stages of ring w and of the weights in tensor memory
+    static constexpr int kACol0 = kWide ? 384 : 256;
+};
 constexpr int kTsMaxXStages = 8;
 constexpr int kTsCtrlBytes = 1024;
 constexpr int kTsHBytes = 128 * 128 * 2, kTsYBytes = 128 * 128 * 2;
@@ -57,10 +68,13 @@ constexpr int kTsSmemBytes = 227 * 1024;
 template <int K> struct TsLayout {
     static constexpr int kTileWords = 8 * K;
     static constexpr int kWBytes = 32 * kTileWords * 4;                 // 8 x 4 packed tiles: K KiB
-    static constexpr int kXOff = kTsWOff + kTsStages * kWBytes;
-    static constexpr int kXRoom = kTsSmemBytes - kXOff;
-    // tokens per tile of a dense launch: at least four stages of activations have to fit
-    static constexpr int kTok = kXRoom / 512 >= kTsMaxTok ? kTsMaxTok : kXRoom / 512 / 16 * 16;
+    template <int MODE> static constexpr int xoff() { return kTsWOff + TsForm<MODE>::kStages * kWBytes; }
+    template <int MODE> static constexpr int xroom() { return kTsSmemBytes - xoff<MODE>(); }
+    // tokens per tile of a dense launch: at least four stages of activations have to fit, three wide ones
+    static constexpr int kTok = std::min(kTsMaxTok, kTsSmemBytes - kTsWOff - 8 * kWBytes >= 512 * kTsMaxTok
+                                                        ? kTsMaxTok
+                                                        : (kTsSmemBytes - kTsWOff - 8 * kWBytes) / 512 / 16 * 16);
+    static constexpr int kTokWide = std::min(kTsWideTok, (kTsSmemBytes - kTsWOff - 4 * kWBytes) / 384 / 16 * 16);
 };
 
 // Bounded wait.  It has no result, so that the code behind it stays warp-uniform for the compiler; a
@@ -266,11 +280,13 @@ template <bool TABLE> struct TsWalk {
     }
 };
 
-template <int K, int CB, bool TABLE, bool AHEAD>
+template <int K, int CB, bool TABLE, int MODE>
 __global__ void __launch_bounds__(kTsThreads, 1)
     gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w)
 {
     using L = TsLayout<K>;
+    using F = TsForm<MODE>;
+    constexpr int NS = F::kStages;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* w_full = reinterpret_cast<uint64_t*>(smem);      // packed tiles landed                      [8]
     uint64_t* w_empty = w_full + kTsStages;                   // ... read by the set's four warps          [8]
@@ -285,7 +301,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
     uint8_t* h_mat = smem + kTsHOff;
     uint8_t* y_buf = smem + kTsYOff;
     uint8_t* w_ring = smem + kTsWOff;
-    uint8_t* x_ring = smem + L::kXOff;
+    uint8_t* x_ring = smem + L::template xoff<MODE>();
 
     const int tid = threadIdx.x, warp = TsWalk<TABLE>::uniform(tid >> 5), lane = tid & 31;
     const int nx = a.stages, x_bytes = a.ts_x_bytes;           // depth and stage size of ring x
@@ -333,7 +349,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                     mbar_arrive_expect_tx(bar, L::kWBytes);
                     tma_load_3d(smem_u32(w_ring) + s * L::kWBytes, &tm_w, 0, sg.tn0, kTsStepTiles * ks, bar);
                 }
-                if (++s == kTsStages) { s = 0; parity ^= 1u; }
+                if (++s == NS) { s = 0; parity ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -372,10 +388,12 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             wait(&d_empty[db], dpar);
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem_base + (uint32_t)(128 * db);
-            const uint32_t idesc = mma_idesc_f16(128, (sg.rows + 15) & ~15);
+            // (an MMA takes at most 256 tokens: a wide tile is two halves)
+            const int n16 = (sg.rows + 15) & ~15, n0 = F::kWide ? ((n16 >> 1) + 15) & ~15 : n16, n1 = n16 - n0;
+            const uint32_t idesc = mma_idesc_f16(128, n0), idesc1 = mma_idesc_f16(128, n1);
             uint32_t accum = 0;
             for (int ks = sg.k0; ks < sg.k1; ks++, v++) {
-                const uint32_t at = tmem_base + kTsACol0 + 32 * as;
+                const uint32_t at = tmem_base + F::kACol0 + 32 * as;
                 const uint64_t xd = smem_desc_sw128(x0 + (uint32_t)(xs * x_bytes));
                 wait(&full[v & (kTsStages - 1)], (uint32_t)(v / kTsStages) & 1u);
                 tc_fence_after_sync();
@@ -384,11 +402,18 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                     tc_mma_f16_ts(d_tmem, at + 8, xd + 2, idesc, 1u);
                     tc_mma_f16_ts(d_tmem, at + 16, xd + 4, idesc, 1u);
                     tc_mma_f16_ts(d_tmem, at + 24, xd + 6, idesc, 1u);
+                    if (F::kWide && n1 > 0) {
+                        const uint64_t xe = xd + (uint64_t)(8 * n0);           // n0 rows of 128 bytes further
+                        tc_mma_f16_ts(d_tmem + n0, at, xe, idesc1, accum);
+                        tc_mma_f16_ts(d_tmem + n0, at + 8, xe + 2, idesc1, 1u);
+                        tc_mma_f16_ts(d_tmem + n0, at + 16, xe + 4, idesc1, 1u);
+                        tc_mma_f16_ts(d_tmem + n0, at + 24, xe + 6, idesc1, 1u);
+                    }
                     tc_commit(smem_u32(&empty[v & (kTsStages - 1)]));
                 }
                 accum = 1u;
                 if (++xs == nx) xs = 0;
-                if (++as == kTsStages) as = 0;
+                if (++as == NS) as = 0;
             }
             if (leader) tc_commit(smem_u32(&d_full[db]));
             if (++db == a.ts_dbuf) { db = 0; dpar ^= 1u; }
@@ -418,9 +443,10 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             }
         }
         if (TABLE) griddep_wait();
-        // A set decodes its k-steps in order, whatever tiles they belong to.  With AHEAD the warps decode up to
-        // eight k-steps of the next tile before they finish one, so that the tensor core has work in the meantime
-        // (SwitchGLU of 4096 tokens 546 -> 524 us); a CTA with hardly more than one tile is 1 us quicker without.
+        // A set decodes its k-steps in order, whatever tiles they belong to.  With AHEAD the warps decode as many
+        // k-steps of the next tile as there are stages before they finish one, so that the tensor core has work
+        // in the meantime (SwitchGLU of 4096 tokens 546 -> 524 us); a CTA with hardly more than one tile is 1 us
+        // quicker without.
         int kc = 0, v = set;                                       // end of the current tile's k-steps; next one of this set
         int db = 0;
         uint32_t dpar = 0, hpar = 0;
@@ -431,13 +457,12 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             more = walk.next(a, nx_sg);
             const int n_steps = sg.k1 - sg.k0;
             kc += n_steps;
-            const int v_end = kc + (AHEAD && more ? min(kTsStages, nx_sg.k1 - nx_sg.k0) : 0);
+            const int v_end = kc + (F::kAhead && more ? min(NS, nx_sg.k1 - nx_sg.k0) : 0);
             for (; v < v_end; v += kTsSets) {
-                // Eight stages, four sets: a stage of ring w always belongs to the same set.  (With another number a
+                // Four or eight stages, four sets: a stage always belongs to the same set.  (With another number a
                 // set could look at a barrier two phases early and read a stale parity.)
-                const int st = v & (kTsStages - 1);
-                const uint32_t parity = (uint32_t)(v / kTsStages) & 1u;
-                wait(&w_full[st], parity);
+                const int st = v & (NS - 1), vb = v - NS;      // vb: the k-step that had the stage before
+                wait(&w_full[st], (uint32_t)(v / NS) & 1u);
                 // tile columns 2q, 2q + 1 of all four tile rows
                 const uint32_t* wt = reinterpret_cast<const uint32_t*>(w_ring + st * L::kWBytes) + 2 * q * L::kTileWords;
                 uint32_t pw[2][4][K == 4 ? 4 : 3];
@@ -457,7 +482,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                             pw[h][tk][2] = LaneWords<K>::kThree ? tw[lw.i2] : 0u;
                         }
                     }
-                wait(&empty[st], parity ^ 1u);
+                if (vb >= 0) wait(&empty[vb & (kTsStages - 1)], (uint32_t)(vb / kTsStages) & 1u);
                 tc_fence_after_sync();
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
@@ -472,7 +497,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                         frag[4 * tk + 2] = decode_pair_rt<CB>(cw[2], cw[3], xc);
                         frag[4 * tk + 3] = decode_pair_rt<CB>(cw[6], cw[7], xc);
                     }
-                    tmem_st_16x32cols(tmem_base + ((uint32_t)(32 * q + 16 * h) << 16) + kTsACol0 + 32 * st, frag);
+                    tmem_st_16x32cols(tmem_base + ((uint32_t)(32 * q + 16 * h) << 16) + F::kACol0 + 32 * st, frag);
                 }
                 // Only now is it certain that the packed words have been read: the stores above depend on them.  (With
                 // the slot given back before the wait for `empty`, some loads were found to take place after it, and
@@ -482,7 +507,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&full[st]));
+                if (lane == 0) mbar_arrive(smem_u32(&full[v & (kTsStages - 1)]));
             }
 
             // ---- finish the tile: what it needs from global memory first ----
@@ -626,7 +651,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                             }
                         }
                     }
-                    if (128 * tg + 128 < sg.rows) orow = out_row(1);
+                    if (128 * tg + 128 < sg.rows) orow = out_row(tg + 1);
                 }
             }
             release_d();
@@ -660,14 +685,15 @@ __global__ void __launch_bounds__(kTsThreads, 1)
 // ---- host side ----------------------------------------------------------------------------------
 
 // Bytes of partial sums a dense launch may use: two slots of 128 columns x (tokens of a tile) per CTA.
-inline size_t gemm_tile_partial_bytes(int64_t rows, int ctas)
-{
-    const int64_t tiles = (rows + kTsMaxTok - 1) / kTsMaxTok;
-    const int64_t tok = ((rows + tiles - 1) / tiles + 15) / 16 * 16;
-    return (size_t)ctas * 2 * kTsOuts * (size_t)tok * sizeof(float);
-}
+inline size_t gemm_tile_partial_bytes(int tok, int ctas) { return (size_t)ctas * 2 * kTsOuts * (size_t)tok * sizeof(float); }
 
-int ts_plan(int64_t tiles, int nks, int sms, int64_t rows, size_t partial_bytes, int* split);   // exl3_gemm.cu
+// The launch plan of a dense GEMM (exl3_gemm.cu).
+struct TsPlan {
+    int tok, tiles_m;        // tokens per output tile, tiles of tokens
+    int grid, split;         // CTAs; whether they share tiles
+    int wide;
+};
+TsPlan ts_plan(int64_t rows, int64_t tiles_n, int nks, int sms, size_t partial_bytes, int tok, int tok_wide);
 
 template <int K, int CB, bool TABLE>
 static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, cudaStream_t s)
@@ -678,15 +704,17 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxDevices) return EXL3_E_UNSUPPORTED;
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
+        cudaError_t e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, TS_AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
         if (e == cudaSuccess && !TABLE)
-            e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
+            e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, TABLE ? TS_AHEAD : TS_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
+        if (e == cudaSuccess && !TABLE)
+            e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, TABLE ? TS_AHEAD : TS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
         if (e != cudaSuccess) return note_cuda(e);
         attr_set[dev] = true;
     }
     a.cb_xor = 0x3B603B60u;
     const int sms = device_sm_count(), nks = a.t_in / kTsStepTiles;
-    int grid;
+    int grid, mode = TS_AHEAD;
     a.ts_split = 0;
     if (TABLE) {
         // Rows of a tile: what nearly all tiles need if the caller says how many rows a tile has on average
@@ -702,17 +730,19 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
         // an odd stride: which items are in use repeats with a period of 2 or 4
         grid = std::min(a.n_items, (sms - 1) | 1);
     } else {
-        a.tiles_m = (a.m + L::kTok - 1) / L::kTok;
-        a.ts_tok = ((a.m + a.tiles_m - 1) / a.tiles_m + 15) / 16 * 16;
-        a.tiles_m = (a.m + a.ts_tok - 1) / a.ts_tok;
-        a.ts_box_rows = a.ts_tok;
         a.tiles_n = a.t_out / 8;
+        const TsPlan plan = ts_plan(a.m, a.tiles_n, nks, sms, a.ts_partial_bytes, L::kTok, L::kTokWide);
+        a.ts_tok = plan.tok;
+        a.tiles_m = plan.tiles_m;
         a.n_items = a.tiles_m * a.tiles_n;
         if ((int64_t)a.n_items * nks >= ((int64_t)1 << 31)) return EXL3_E_SHAPE;   // (k-steps are counted in 32 bits)
-        grid = ts_plan(a.n_items, nks, sms, a.m, a.ts_partial_bytes, &a.ts_split);
+        a.ts_box_rows = a.ts_tok > 256 ? a.ts_tok / 2 : a.ts_tok;                  // (a box has at most 256 rows)
+        a.ts_split = plan.split;
+        grid = plan.grid;
+        mode = plan.wide ? TS_WIDE : a.n_items >= 2 * grid ? TS_AHEAD : TS_PLAIN;
     }
     a.ts_x_bytes = (a.ts_tok + a.ts_box_rows - 1) / a.ts_box_rows * a.ts_box_rows * 128;
-    a.stages = std::min(kTsStages, L::kXRoom / a.ts_x_bytes);
+    a.stages = std::min(kTsStages, (mode == TS_WIDE ? L::template xroom<TS_WIDE>() : L::template xroom<TS_AHEAD>()) / a.ts_x_bytes);
     a.ts_dbuf = a.ts_tok <= 128 ? 2 : 1;
     CUtensorMap tm_x, tm_w;
     {
@@ -730,7 +760,9 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
                              CU_TENSOR_MAP_SWIZZLE_NONE);
         if (rc) return rc;
     }
-    const auto kernel = TABLE || a.n_items >= 2 * grid ? gemm_kernel<K, CB, TABLE, true> : gemm_kernel<K, CB, TABLE, TABLE>;
+    const auto kernel = TABLE || mode == TS_AHEAD ? gemm_kernel<K, CB, TABLE, TS_AHEAD>
+                        : mode == TS_WIDE         ? gemm_kernel<K, CB, TABLE, TABLE ? TS_AHEAD : TS_WIDE>
+                                                  : gemm_kernel<K, CB, TABLE, TABLE ? TS_AHEAD : TS_PLAIN>;
     return launch_kernel(kernel, dim3((unsigned)grid), dim3(kTsThreads), kTsSmemBytes, s, true, a, tm_x, tm_w);
 }
 

@@ -92,6 +92,11 @@ def test_gemm_ragged_row_counts(mod, oracle, rows):
     (250, 1024, 256, 8, 0),     # K = 8: fewer tokens per tile fit the activation ring, two token tiles
     (257, 1152, 128, 7, 1),     # one row more than a tile, a k-range that is no multiple of the ring
     (700, 128, 640, 1, 0),      # two k-steps per tile, whole tiles
+    (272, 512, 128, 4, 0),      # the smallest wide tile, halves of 144 and 128 tokens
+    (384, 640, 256, 3, 0),      # the largest wide tile
+    (336, 1024, 128, 8, 2),     # ... at K = 8
+    (400, 512, 256, 5, 1),      # two tiles, the second a few tokens short
+    (1537, 256, 384, 6, 0),     # a last tile of few tokens
 ])
 def test_gemm_tiles_shared_between_ctas(mod, oracle, rows, inf, outf, k, cb):
     layer = _layer(mod, k, inf, outf, seed=rows, cb=cb, bias=rows % 2 == 0)
