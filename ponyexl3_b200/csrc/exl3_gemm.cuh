@@ -143,6 +143,14 @@ __device__ __forceinline__ void tmem_ld_16cols(uint32_t taddr, float (&v)[16])
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// 16 bytes that no earlier kernel of the stream writes; volatile, so that the load stays where it is written.
+__device__ __forceinline__ uint4 ldg_nc_128(const __half* p)
+{
+    uint4 v;
+    asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // One 32-byte store (sm_100: 256-bit vector stores); p must be 32-byte aligned.
 __device__ __forceinline__ void st_global_256(void* p, const uint4& a, const uint4& b)
 {
@@ -513,12 +521,19 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             // ---- finish the tile: what it needs from global memory first ----
             const int out = 32 * q + lane;                         // this thread's column of the tile
             const int n16 = (sg.rows + 15) >> 4;
-            if (a.svh) prefetch_l1(a.svh + sg.sv_off + 32 * set);
             auto out_row = [&](int tg) {                           // output row of this thread's token
                 const int row = 128 * tg + out, grow = sg.m0 + row + sg.y_row_delta;
                 return a.y_row_map && row < sg.rows ? a.y_row_map[grow] : grow;
             };
             int orow = out_row(0);
+            // a shared tile's first and last contributor (64-bit divisions, done behind the last MMAs)
+            int cf = 0, cl = 0, slot_first = 0;
+            if (n_steps != nks && dt == 0) {
+                const int64_t U = (int64_t)a.n_items * nks, G = gridDim.x, f = (int64_t)sg.tile * nks;
+                cf = (int)(((f + 1) * G - 1) / U);
+                cl = (int)(((f + nks) * G - 1) / U);
+                slot_first = U * cf / G == f ? 0 : 1;
+            }
             wait(&d_full[db], dpar);
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem_base + (uint32_t)(128 * db);
@@ -533,28 +548,27 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                 if (lane == 0) mbar_arrive(smem_u32(&d_empty[db]));
             };
             bool finish = true;
-            int c_first = 0, n_contrib = 1, slot_first = 0;
+            int c_first = 0, n_contrib = 1;
             if (n_steps != nks) {
-                float* part = a.ts_partials + (size_t)(2 * blockIdx.x + (sg.first ? 0 : 1)) * slot_floats + out;
+                float4* part = reinterpret_cast<float4*>(a.ts_partials + (size_t)(2 * blockIdx.x + (sg.first ? 0 : 1)) * slot_floats) + out;
                 for (int ch = set; ch < n16; ch += kTsSets) {
                     float f[16];
                     tmem_ld_16cols(lane_base + 16 * ch, f);
 #pragma unroll
-                    for (int i = 0; i < 16; i++) __stcg(part + (16 * ch + i) * kTsOuts, f[i]);
+                    for (int i = 0; i < 4; i++)
+                        __stcg(part + (4 * ch + i) * kTsOuts, make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]));
                 }
                 named_bar_sync(1, 512);
                 if (dt == 0) {
                     // as in the streamed GEMV: the barrier orders the CTA's stores before this release, the
                     // count wraps to zero with the last arrival and is an acquire for the reads below
-                    const int64_t U = (int64_t)a.n_items * nks, G = gridDim.x, f = (int64_t)sg.tile * nks;
-                    const int cf = (int)(((f + 1) * G - 1) / U), cl = (int)(((f + nks) * G - 1) / U);
                     unsigned old;
                     asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;"
                                  : "=r"(old) : "l"(a.ts_ctr + cf), "r"((unsigned)(cl - cf)) : "memory");
                     handoff[0] = old == (unsigned)(cl - cf) ? 1 : 0;
                     handoff[1] = cf;
                     handoff[2] = cl - cf + 1;
-                    handoff[3] = U * cf / G == f ? 0 : 1;
+                    handoff[3] = slot_first;
                 }
                 named_bar_sync(1, 512);
                 finish = handoff[0] != 0;
@@ -566,30 +580,52 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                 // The rotated half goes over D's first 128 columns, which have been read by then.
 #pragma unroll 1
                 for (int tg = 0; 128 * tg < sg.rows; tg++) {       // 128 tokens at a time
+                    if (n_steps == nks) {
 #pragma unroll 1
-                    for (int ch = 8 * tg + set; ch < min(8 * tg + 8, n16); ch += kTsSets) {
-                        float f[16];
-                        if (n_steps == nks) {
+                        for (int ch = 8 * tg + set; ch < min(8 * tg + 8, n16); ch += kTsSets) {
+                            float f[16];
                             tmem_ld_16cols(lane_base + 16 * ch, f);
-                        } else {
+                            uint32_t hv[8];
 #pragma unroll
-                            for (int i = 0; i < 16; i++) f[i] = 0.f;
-#pragma unroll 2
-                            for (int j = 0; j < n_contrib; j++) {  // in CTA order
-                                const float* p = a.ts_partials + (size_t)(2 * (c_first + j) + (j == 0 ? slot_first : 0)) * slot_floats +
-                                                 out + (size_t)(16 * ch) * kTsOuts;
-#pragma unroll
-                                for (int i = 0; i < 16; i++) f[i] += __ldcg(p + i * kTsOuts);
-                            }
+                            for (int i = 0; i < 8; i++) hv[i] = h2_as_u32(__floats2half2_rn(f[2 * i], f[2 * i + 1]));
+                            const int c16 = ch & 7;                // 16 tokens = two 16-byte pieces of a 64-token row
+                            uint8_t* row = y_buf + (c16 >> 2) * 16384 + out * 128;
+                            const int piece = 2 * (c16 & 3), sw = out & 7;
+                            *reinterpret_cast<uint4*>(row + ((piece ^ sw) << 4)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+                            *reinterpret_cast<uint4*>(row + (((piece + 1) ^ sw) << 4)) = make_uint4(hv[4], hv[5], hv[6], hv[7]);
                         }
-                        uint32_t hv[8];
+                    } else {
+                        // The contributors' sums, added in CTA order: eight tokens at a time, the slots of four CTAs
+                        // in flight at once.  (The round trips to L2 are what this costs.)
+#pragma unroll 1
+                        for (int u8 = 16 * tg + set; u8 < min(16 * tg + 16, 2 * n16); u8 += kTsSets) {
+                            float f[8];
 #pragma unroll
-                        for (int i = 0; i < 8; i++) hv[i] = h2_as_u32(__floats2half2_rn(f[2 * i], f[2 * i + 1]));
-                        const int c16 = ch & 7;                    // 16 tokens = two 16-byte pieces of a 64-token row
-                        uint8_t* row = y_buf + (c16 >> 2) * 16384 + out * 128;
-                        const int piece = 2 * (c16 & 3), sw = out & 7;
-                        *reinterpret_cast<uint4*>(row + ((piece ^ sw) << 4)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
-                        *reinterpret_cast<uint4*>(row + (((piece + 1) ^ sw) << 4)) = make_uint4(hv[4], hv[5], hv[6], hv[7]);
+                            for (int i = 0; i < 8; i++) f[i] = 0.f;
+#pragma unroll 1
+                            for (int j0 = 0; j0 < n_contrib; j0 += 4) {
+                                float4 p[4][2];
+#pragma unroll
+                                for (int j = 0; j < 4; j++) {
+                                    const bool in = j0 + j < n_contrib;
+                                    const int c = in ? 2 * (c_first + j0 + j) + (j0 + j == 0 ? slot_first : 0) : 0;
+                                    const float4* q4 = reinterpret_cast<const float4*>(a.ts_partials + (size_t)c * slot_floats) + out + 2 * u8 * kTsOuts;
+                                    p[j][0] = p[j][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                                    if (in) { p[j][0] = __ldcg(q4); p[j][1] = __ldcg(q4 + kTsOuts); }
+                                }
+#pragma unroll
+                                for (int j = 0; j < 4; j++) {
+                                    f[0] += p[j][0].x; f[1] += p[j][0].y; f[2] += p[j][0].z; f[3] += p[j][0].w;
+                                    f[4] += p[j][1].x; f[5] += p[j][1].y; f[6] += p[j][1].z; f[7] += p[j][1].w;
+                                }
+                            }
+                            uint32_t hv[4];
+#pragma unroll
+                            for (int i = 0; i < 4; i++) hv[i] = h2_as_u32(__floats2half2_rn(f[2 * i], f[2 * i + 1]));
+                            const int c8 = u8 & 15;                // 8 tokens = one 16-byte piece of a 64-token row
+                            *reinterpret_cast<uint4*>(y_buf + (c8 >> 3) * 16384 + out * 128 + (((c8 & 7) ^ (out & 7)) << 4)) =
+                                make_uint4(hv[0], hv[1], hv[2], hv[3]);
+                        }
                     }
                     fence_proxy_async_smem();
                     tc_fence_before_sync();
@@ -606,15 +642,11 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                         }
                         __syncwarp();
                     }
-                    wait(h_full, hpar);
-                    hpar ^= 1u;
-                    tc_fence_after_sync();
-                    float f[32];
-                    tmem_ld_32cols(lane_base + 32 * set, f);
-                    if (128 * tg + 128 >= sg.rows) release_d();    // the last reads of D
-                    if (128 * tg + out < sg.rows) {                // lane = token now
+                    const bool used = 128 * tg + out < sg.rows;    // lane = token now
+                    __half* yp = nullptr;
+                    auto address = [&]() {
+                        if (!used) return;
                         const int col0 = sg.y_col + 32 * set;
-                        __half* yp;
                         if (a.n_peer > 0) {      // the row belongs to the GPU that holds its token
                             const int pr = orow / a.rows_per_peer;
                             yp = a.y_peer[pr] + (int64_t)(orow - pr * a.rows_per_peer) * a.y_row_stride + col0;
@@ -622,13 +654,30 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                             yp = !TABLE && a.n_members > 1 ? a.member_y[sg.member] + (int64_t)orow * a.member_stride[sg.member] + col0
                                                            : a.y + (int64_t)orow * a.y_row_stride + col0;
                         }
+                    };
+                    // (behind the product; a table's launches are quicker with it after: 290 against 280 us as below)
+                    if (!TABLE) address();
+                    // The output scales are fetched behind the product: between the stores below, which might alias
+                    // them, the loads would be made and waited for one after the other, and a prefetch into L1 does
+                    // not help (SwitchGLU of 200 tokens 298 -> 284 us).
+                    uint4 sv[4];
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        sv[c] = a.svh ? ldg_nc_128(a.svh + sg.sv_off + 32 * set + 8 * c)
+                                      : make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
+                    wait(h_full, hpar);
+                    hpar ^= 1u;
+                    tc_fence_after_sync();
+                    float f[32];
+                    tmem_ld_32cols(lane_base + 32 * set, f);
+                    if (128 * tg + 128 >= sg.rows) release_d();    // the last reads of D
+                    if (TABLE) address();
+                    if (used) {
                         const uint64_t scale = f32x2(EXL3_HAD_SCALE, EXL3_HAD_SCALE);
                         uint4 held16 = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
                         for (int c = 0; c < 4; c++) {
-                            const uint4 sv = a.svh ? *reinterpret_cast<const uint4*>(a.svh + sg.sv_off + 32 * set + 8 * c)
-                                                   : make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
-                            const uint32_t sw4[4] = {sv.x, sv.y, sv.z, sv.w};
+                            const uint32_t sw4[4] = {sv[c].x, sv[c].y, sv[c].z, sv[c].w};
                             uint32_t h[4];
 #pragma unroll
                             for (int i = 0; i < 4; i++) {
@@ -636,7 +685,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                                 h[i] = f16_pair(mul_f32x2(mul_f32x2(f32x2(f[8 * c + 2 * i], f[8 * c + 2 * i + 1]), scale), f32x2(w2.x, w2.y)));
                             }
                             if (a.bias) {
-                                const uint4 bv = *reinterpret_cast<const uint4*>(a.bias + sg.sv_off + 32 * set + 8 * c);
+                                const uint4 bv = __ldg(reinterpret_cast<const uint4*>(a.bias + sg.sv_off + 32 * set + 8 * c));
                                 const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
                                 for (int i = 0; i < 4; i++) h[i] = h2_as_u32(__hadd2(u32_as_h2(h[i]), u32_as_h2(bw[i])));
