@@ -15,56 +15,85 @@ namespace exl3 {
 
 // ------------------------------------------------------------------ residual + RMSNorm ----
 // x <- fp16(x + delta) (delta may be NULL), h <- fp16(x * rsqrt(mean(x^2) + eps) * w).
-// One CTA per row, eight elements per thread and turn.
-__global__ void __launch_bounds__(256) add_rmsnorm_kernel(__half* x, const __half* delta, const __half* w,
-                                                          __half* h, int n, int64_t x_stride,
-                                                          int64_t d_stride, int64_t h_stride, float eps)
+// One CTA per row, eight elements per thread and turn.  A row is a handful of dependent round trips to L2, so
+// there are as many threads as the row has pieces (up to 1024), the first two turns' values stay in registers
+// between the two passes, and the weights are fetched before the sum is known; under EXL3_FLAG_PDL even before
+// the previous kernel has ended.
+constexpr int kNormTurns = 2;
+__global__ void __launch_bounds__(1024) add_rmsnorm_kernel(__half* x, const __half* delta, const __half* w,
+                                                           __half* h, int n, int64_t x_stride,
+                                                           int64_t d_stride, int64_t h_stride, float eps, int early)
 {
     griddep_launch_dependents();
-    griddep_wait();
-    __shared__ float red[8];
+    if (!early) griddep_wait();
+    __shared__ float red[32];
     __half* xr = x + (int64_t)blockIdx.x * x_stride;
     const __half* dr = delta ? delta + (int64_t)blockIdx.x * d_stride : nullptr;
-    float ss = 0.f;
-    for (int i = threadIdx.x * 8; i < n; i += 256 * 8) {
-        uint4 v = *reinterpret_cast<const uint4*>(xr + i);
-        __half2* hv = reinterpret_cast<__half2*>(&v);
-        if (dr) {
-            const uint4 d = *reinterpret_cast<const uint4*>(dr + i);
-            const __half2* hd = reinterpret_cast<const __half2*>(&d);
+    const int first = threadIdx.x * 8, step = blockDim.x * 8;
+    uint4 v[kNormTurns], g[kNormTurns], d[kNormTurns];
 #pragma unroll
-            for (int q = 0; q < 4; q++) hv[q] = __hadd2(hv[q], hd[q]);
-            *reinterpret_cast<uint4*>(xr + i) = v;
+    for (int q = 0; q < kNormTurns; q++) {
+        const int i = first + q * step;
+        v[q] = g[q] = d[q] = make_uint4(0u, 0u, 0u, 0u);
+        if (i < n) g[q] = *reinterpret_cast<const uint4*>(w + i);
+    }
+    if (early) griddep_wait();
+#pragma unroll
+    for (int q = 0; q < kNormTurns; q++) {
+        const int i = first + q * step;
+        if (i < n) {
+            v[q] = *reinterpret_cast<const uint4*>(xr + i);
+            if (dr) d[q] = *reinterpret_cast<const uint4*>(dr + i);
+        }
+    }
+    float ss = 0.f;
+    auto add = [&](uint4& a, const uint4& b, int i) {      // a += b, stored; its squares counted
+        __half2* ha = reinterpret_cast<__half2*>(&a);
+        const __half2* hb = reinterpret_cast<const __half2*>(&b);
+        if (dr) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) ha[q] = __hadd2(ha[q], hb[q]);
+            *reinterpret_cast<uint4*>(xr + i) = a;
         }
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            const float2 f = __half22float2(hv[q]);
+            const float2 f = __half22float2(ha[q]);
             ss += f.x * f.x + f.y * f.y;
         }
+    };
+#pragma unroll
+    for (int q = 0; q < kNormTurns; q++)
+        if (first + q * step < n) add(v[q], d[q], first + q * step);
+    for (int i = first + kNormTurns * step; i < n; i += step) {
+        uint4 a = *reinterpret_cast<const uint4*>(xr + i);
+        add(a, dr ? *reinterpret_cast<const uint4*>(dr + i) : a, i);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
     __syncthreads();
-    float tot = 0.f;
+    float tot = (threadIdx.x & 31) < (blockDim.x >> 5) ? red[threadIdx.x & 31] : 0.f;
 #pragma unroll
-    for (int q = 0; q < 8; q++) tot += red[q];
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
     const float rstd = rsqrtf(tot / (float)n + eps);
     __half* hr = h + (int64_t)blockIdx.x * h_stride;
-    for (int i = threadIdx.x * 8; i < n; i += 256 * 8) {
-        const uint4 v = *reinterpret_cast<const uint4*>(xr + i);   // own writes: same thread, same address
-        const uint4 g = *reinterpret_cast<const uint4*>(w + i);
-        const __half2* hv = reinterpret_cast<const __half2*>(&v);
-        const __half2* hg = reinterpret_cast<const __half2*>(&g);
+    auto norm = [&](const uint4& a, const uint4& b, int i) {
+        const __half2* ha = reinterpret_cast<const __half2*>(&a);
+        const __half2* hb = reinterpret_cast<const __half2*>(&b);
         uint4 o;
         __half2* ho = reinterpret_cast<__half2*>(&o);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            const float2 f = __half22float2(hv[q]), gg = __half22float2(hg[q]);
+            const float2 f = __half22float2(ha[q]), gg = __half22float2(hb[q]);
             ho[q] = __floats2half2_rn(f.x * rstd * gg.x, f.y * rstd * gg.y);
         }
         *reinterpret_cast<uint4*>(hr + i) = o;
-    }
+    };
+#pragma unroll
+    for (int q = 0; q < kNormTurns; q++)
+        if (first + q * step < n) norm(v[q], g[q], first + q * step);
+    for (int i = first + kNormTurns * step; i < n; i += step)     // own writes: same thread, same address
+        norm(*reinterpret_cast<const uint4*>(xr + i), *reinterpret_cast<const uint4*>(w + i), i);
 }
 
 // ------------------------------------------------------------- RoPE + KV-cache append ----
@@ -164,9 +193,14 @@ struct AttnArgs {
     float scale_log2;         // log2(e) / sqrt(128)
 };
 
-template <int NW>   // warps = 16-row query tiles
-__global__ void __launch_bounds__(NW * 32) attn_partial_kernel(const AttnArgs a)
+// NW 16-row query tiles, and for few of them WK warps per tile that take a share of each tile's keys: one warp
+// per CTA was bound by its own chain of products and exponentials (33 x 8 CTAs, 8192 keys: 11.8 us against
+// KATTNUS with four).  Every warp has its own running maximum, sum and output; they are merged at the end by
+// the rule of the combine kernel.
+template <int NW, int WK>
+__global__ void __launch_bounds__(NW * WK * 32) attn_partial_kernel(const AttnArgs a)
 {
+    constexpr int kThreads = NW * WK * 32, NT = 8 / WK, K2 = 4 / WK;   // 8-key and 16-key pieces of a warp
     extern __shared__ __align__(128) uint8_t smem[];
     griddep_launch_dependents();
     griddep_wait();
@@ -184,7 +218,7 @@ __global__ void __launch_bounds__(NW * 32) attn_partial_kernel(const AttnArgs a)
 
     auto load_tile = [&](int ti, int buf) {
         const int key0 = p0 + ti * kAttnTile;
-        for (int c = tid; c < kAttnTile * 16; c += NW * 32) {        // 16-byte pieces: 16 per row
+        for (int c = tid; c < kAttnTile * 16; c += kThreads) {        // 16-byte pieces: 16 per row
             const int row = c >> 4, piece = c & 15;
             const int key = key0 + row;
             const bool ok = key < p1;
@@ -198,7 +232,7 @@ __global__ void __launch_bounds__(NW * 32) attn_partial_kernel(const AttnArgs a)
     if (ntiles > 0) load_tile(0, 0);
 
     // query fragments of this warp's 16 rows (rows m0 + g and m0 + g + 8), all 8 k-steps
-    const int m0 = warp * 16;
+    const int m0 = warp % NW * 16, wk = warp / NW;
     uint32_t qf[8][4];
     int lim[2];                                          // last visible key of the two rows
 #pragma unroll
@@ -233,13 +267,13 @@ __global__ void __launch_bounds__(NW * 32) attn_partial_kernel(const AttnArgs a)
         const __half* ks_ = reinterpret_cast<const __half*>(smem + buf * kAttnTileBytes);
         const int key0 = p0 + ti * kAttnTile;
 
-        // S = Q K^T for 64 keys: 8 key tiles x 8 k-steps
-        float s[8][4];
+        // S = Q K^T for this warp's keys: 8-key pieces x 8 k-steps
+        float s[NT][4];
 #pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
+        for (int nt = 0; nt < NT; nt++) {
 #pragma unroll
             for (int q = 0; q < 4; q++) s[nt][q] = 0.f;
-            const __half* kr = ks_ + (nt * 8 + g) * kAttnLd + 2 * t;
+            const __half* kr = ks_ + ((wk * NT + nt) * 8 + g) * kAttnLd + 2 * t;
 #pragma unroll
             for (int ks = 0; ks < 8; ks++) {
                 const uint32_t b0 = *reinterpret_cast<const uint32_t*>(kr + ks * 16);
@@ -250,10 +284,10 @@ __global__ void __launch_bounds__(NW * 32) attn_partial_kernel(const AttnArgs a)
         // scale, mask (keys past a row's own position, and the zero-filled tail), running max
         float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-        for (int nt = 0; nt < 8; nt++)
+        for (int nt = 0; nt < NT; nt++)
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const int key = key0 + nt * 8 + 2 * t + (q & 1);
+                const int key = key0 + (wk * NT + nt) * 8 + 2 * t + (q & 1);
                 const int h = q >> 1;
                 const float v = (key <= lim[h] && key < p1) ? s[nt][q] * a.scale_log2 : -INFINITY;
                 s[nt][q] = v;
@@ -275,10 +309,10 @@ __global__ void __launch_bounds__(NW * 32) attn_partial_kernel(const AttnArgs a)
             o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
             o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
         }
-        // P = exp2(S - m), as A fragments of the 4 k-steps of P V
-        uint32_t pa[4][4];
+        // P = exp2(S - m), as A fragments of the k-steps of P V
+        uint32_t pa[K2][4];
 #pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
+        for (int nt = 0; nt < NT; nt++) {
             float p[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -288,15 +322,15 @@ __global__ void __launch_bounds__(NW * 32) attn_partial_kernel(const AttnArgs a)
             pa[nt >> 1][(nt & 1) * 2 + 0] = pack_h2(p[0], p[1]);
             pa[nt >> 1][(nt & 1) * 2 + 1] = pack_h2(p[2], p[3]);
         }
-        // O += P V: 16 feature tiles x 4 k-steps, V fragments through transposing ldmatrix
+        // O += P V: 16 feature tiles x 16-key k-steps, V fragments through transposing ldmatrix
         const uint32_t vs_ = s_v + buf * kAttnTileBytes;
         const int lrow_ = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 8;
 #pragma unroll
-        for (int k2 = 0; k2 < 4; k2++)
+        for (int k2 = 0; k2 < K2; k2++)
 #pragma unroll
             for (int dp = 0; dp < 8; dp++) {          // two feature tiles per ldmatrix.x4
                 uint32_t b[4];
-                ldmatrix_x4_trans(vs_ + (uint32_t)(((k2 * 16 + lrow_) * kAttnLd + dp * 16 + lcol) * 2), b);
+                ldmatrix_x4_trans(vs_ + (uint32_t)((((wk * K2 + k2) * 16 + lrow_) * kAttnLd + dp * 16 + lcol) * 2), b);
                 mma_16816(o[2 * dp], pa[k2], b[0], b[1]);
                 mma_16816(o[2 * dp + 1], pa[k2], b[2], b[3]);
             }
@@ -308,6 +342,45 @@ __global__ void __launch_bounds__(NW * 32) attn_partial_kernel(const AttnArgs a)
     for (int h = 0; h < 2; h++) {
         lrow[h] += __shfl_xor_sync(0xffffffffu, lrow[h], 1);
         lrow[h] += __shfl_xor_sync(0xffffffffu, lrow[h], 2);
+    }
+    if constexpr (WK > 1) {
+        // the warps of a query tile leave theirs in shared memory (behind the loop's last barrier) and share the merge
+        constexpr int kLd = 132;
+        float* so = reinterpret_cast<float*>(smem);                  // [WK][16 NW][kLd]
+        float* sm = so + WK * 16 * NW * kLd;                         // [WK][16 NW][2]
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int m = m0 + g + 8 * h;
+            float* p = so + (wk * 16 * NW + m) * kLd + 2 * t;
+#pragma unroll
+            for (int i = 0; i < 16; i++) *reinterpret_cast<float2*>(p + i * 8) = make_float2(o[i][2 * h], o[i][2 * h + 1]);
+            if (t == 0) {
+                sm[(wk * 16 * NW + m) * 2] = mrow[h];
+                sm[(wk * 16 * NW + m) * 2 + 1] = lrow[h];
+            }
+        }
+        __syncthreads();
+        for (int i = tid; i < M * 32; i += kThreads) {
+            const int m = i >> 5, d4 = 4 * (i & 31);
+            float mx = -INFINITY, l = 0.f;
+#pragma unroll
+            for (int q = 0; q < WK; q++) mx = fmaxf(mx, sm[(q * 16 * NW + m) * 2]);
+            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < WK; q++) {
+                const float mq = sm[(q * 16 * NW + m) * 2], f = mq == -INFINITY ? 0.f : exp2f(mq - mx);
+                const float4 v = *reinterpret_cast<const float4*>(so + (q * 16 * NW + m) * kLd + d4);
+                r.x += f * v.x; r.y += f * v.y; r.z += f * v.z; r.w += f * v.w;
+                l += f * sm[(q * 16 * NW + m) * 2 + 1];
+            }
+            const int64_t row = ((int64_t)kvh * a.nsplit + split) * M + m;
+            *reinterpret_cast<float4*>(a.part_o + row * 128 + d4) = r;
+            if (d4 == 0) {
+                a.part_ml[row * 2] = mx;
+                a.part_ml[row * 2 + 1] = l;
+            }
+        }
+        return;
     }
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -380,20 +453,21 @@ __global__ void __launch_bounds__(32 * kCombineMaxLanes) attn_combine_kernel(con
     }
 }
 
-template <int NW> static int launch_attn_partial(const AttnArgs& a, cudaStream_t s, bool pdl)
+template <int NW, int WK> static int launch_attn_partial(const AttnArgs& a, cudaStream_t s, bool pdl)
 {
-    const size_t smem = 2 * (size_t)a.nbuf * kAttnTileBytes;
+    const size_t merge = WK > 1 ? (size_t)WK * 16 * NW * (132 + 2) * sizeof(float) : 0;
+    const size_t smem = std::max(2 * (size_t)a.nbuf * kAttnTileBytes, merge);
     static bool set[kMaxDevices] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxDevices) return EXL3_E_UNSUPPORTED;
     if (!set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(attn_partial_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(attn_partial_kernel<NW, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              4 * kAttnTileBytes);
         if (e != cudaSuccess) return note_cuda(e);
         set[dev] = true;
     }
-    return launch_kernel(attn_partial_kernel<NW>, dim3((unsigned)a.nsplit, (unsigned)a.hkv), dim3(NW * 32), smem, s,
+    return launch_kernel(attn_partial_kernel<NW, WK>, dim3((unsigned)a.nsplit, (unsigned)a.hkv), dim3(NW * WK * 32), smem, s,
                          pdl, a);
 }
 
@@ -424,10 +498,12 @@ extern "C" int exl3_add_rmsnorm(uint16_t* x, const uint16_t* delta, const uint16
     if (rows < 1 || n < 8 || n % 8) return EXL3_E_SHAPE;
     if (x_row_stride % 8 || h_row_stride % 8 || (delta && delta_row_stride % 8)) return EXL3_E_ALIGN;
     if (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)h | (uintptr_t)delta) & 15) return EXL3_E_ALIGN;
-    return launch_kernel(add_rmsnorm_kernel, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream,
-                         (flags & EXL3_FLAG_PDL) != 0, reinterpret_cast<__half*>(x),
+    const bool pdl = (flags & EXL3_FLAG_PDL) != 0;
+    const unsigned threads = (unsigned)std::min<int64_t>(1024, (n / 8 + 31) / 32 * 32);
+    return launch_kernel(add_rmsnorm_kernel, dim3((unsigned)rows), dim3(threads), 0, (cudaStream_t)stream,
+                         pdl, reinterpret_cast<__half*>(x),
                          reinterpret_cast<const __half*>(delta), reinterpret_cast<const __half*>(weight),
-                         reinterpret_cast<__half*>(h), (int)n, x_row_stride, delta_row_stride, h_row_stride, eps);
+                         reinterpret_cast<__half*>(h), (int)n, x_row_stride, delta_row_stride, h_row_stride, eps, pdl ? 1 : 0);
 }
 
 extern "C" int exl3_rope_append(const uint16_t* qkv, int64_t qkv_row_stride, const uint16_t* cos_table,
@@ -497,14 +573,14 @@ extern "C" int exl3_attn_decode(const uint16_t* q, const uint16_t* k_cache, cons
     const bool pdl = (flags & EXL3_FLAG_PDL) != 0;
     int rc;
     switch ((m + 15) / 16) {
-        case 1: rc = launch_attn_partial<1>(a, s, pdl); break;
-        case 2: rc = launch_attn_partial<2>(a, s, pdl); break;
-        case 3: rc = launch_attn_partial<3>(a, s, pdl); break;
-        case 4: rc = launch_attn_partial<4>(a, s, pdl); break;
-        case 5: rc = launch_attn_partial<5>(a, s, pdl); break;
-        case 6: rc = launch_attn_partial<6>(a, s, pdl); break;
-        case 7: rc = launch_attn_partial<7>(a, s, pdl); break;
-        default: rc = launch_attn_partial<8>(a, s, pdl); break;
+        case 1: rc = launch_attn_partial<1, 4>(a, s, pdl); break;
+        case 2: rc = launch_attn_partial<2, 2>(a, s, pdl); break;
+        case 3: rc = launch_attn_partial<3, 1>(a, s, pdl); break;
+        case 4: rc = launch_attn_partial<4, 1>(a, s, pdl); break;
+        case 5: rc = launch_attn_partial<5, 1>(a, s, pdl); break;
+        case 6: rc = launch_attn_partial<6, 1>(a, s, pdl); break;
+        case 7: rc = launch_attn_partial<7, 1>(a, s, pdl); break;
+        default: rc = launch_attn_partial<8, 1>(a, s, pdl); break;
     }
     if (rc) return rc;
     const int lanes = std::min(kCombineMaxLanes, std::max(4, (a.nsplit + 3) / 4));
