@@ -273,19 +273,19 @@ __global__ void __launch_bounds__(256, 2)
                 xb[q] = ok1 ? Load8<T>::at(p1 + 32 * q) : make_uint4(0u, 0u, 0u, 0u);
             }
             if (glu) {
-                // the row holds [gate (n) | up (n)]: the input is fp16(act(gate) * up)
+                // the row holds [gate (n) | up (n)]: the input is fp16(act(gate) * up); all loads in flight first
+                uint4 ua[4], ub[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    if (ok0) {
-                        const uint4 u = Load8<T>::at(p0 + n + 32 * q);
-                        xa[q] = make_uint4(glu_pair(xa[q].x, u.x, glu), glu_pair(xa[q].y, u.y, glu),
-                                           glu_pair(xa[q].z, u.z, glu), glu_pair(xa[q].w, u.w, glu));
-                    }
-                    if (ok1) {
-                        const uint4 u = Load8<T>::at(p1 + n + 32 * q);
-                        xb[q] = make_uint4(glu_pair(xb[q].x, u.x, glu), glu_pair(xb[q].y, u.y, glu),
-                                           glu_pair(xb[q].z, u.z, glu), glu_pair(xb[q].w, u.w, glu));
-                    }
+                    ua[q] = ok0 ? Load8<T>::at(p0 + n + 32 * q) : make_uint4(0u, 0u, 0u, 0u);
+                    ub[q] = ok1 ? Load8<T>::at(p1 + n + 32 * q) : make_uint4(0u, 0u, 0u, 0u);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    xa[q] = make_uint4(glu_pair(xa[q].x, ua[q].x, glu), glu_pair(xa[q].y, ua[q].y, glu),
+                                       glu_pair(xa[q].z, ua[q].z, glu), glu_pair(xa[q].w, ua[q].w, glu));
+                    xb[q] = make_uint4(glu_pair(xb[q].x, ub[q].x, glu), glu_pair(xb[q].y, ub[q].y, glu),
+                                       glu_pair(xb[q].z, ub[q].z, glu), glu_pair(xb[q].w, ub[q].w, glu));
                 }
             }
         }

@@ -118,11 +118,24 @@ __device__ __forceinline__ void had128_warp(float (&v)[4], int lane)
 // act(g) * u in fp32 (the caller rounds to fp16): mode 1 = SiLU, 2 = tanh-GELU, the two
 // activations of the reference's SwitchGLU (ponyexl3/mlx/exl3_moe.py:62-75).
 enum : int { GLU_NONE = 0, GLU_SILU = 1, GLU_GELU = 2 };
+// g / (1 + exp(-g)).  The division is a product with the approximate reciprocal and one correction by the
+// residual (Markstein, IBM J. Res. Dev. 34, 1990), without the branch for operands that do not occur here;
+// the exponent is clamped where the quotient is far below fp16.  The plain division kept a rotation from
+// overlapping the elements of a row: SwitchGLU of 4096 tokens 507 -> 499 us, MLP of 300 rows
+// 167 -> 162.  Every fp16 g gives the same float as the division where the result is above 1e-30.
+__device__ __forceinline__ float silu(float g)
+{
+    const float d = 1.f + __expf(fminf(-g, 80.f));
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = g * r;
+    return d == 1.f ? g : __fmaf_rn(__fmaf_rn(-q, d, g), r, q);   // (also for an infinite g)
+}
 __device__ __forceinline__ float glu_value(float g, float u, int mode)
 {
     if (mode == GLU_GELU)
         return 0.5f * g * (1.f + tanhf(0.797884560803f * (g + 0.044715f * g * g * g))) * u;
-    return g / (1.f + __expf(-g)) * u;
+    return silu(g) * u;
 }
 
 // ---- shared-memory barriers and bulk copies ------------------------------------------------

@@ -194,8 +194,8 @@ struct AttnArgs {
 };
 
 // NW 16-row query tiles, and for few of them WK warps per tile that take a share of each tile's keys: one warp
-// per CTA was bound by its own chain of products and exponentials (33 x 8 CTAs, 8192 keys: 11.8 us against
-// KATTNUS with four).  Every warp has its own running maximum, sum and output; they are merged at the end by
+// per CTA was bound by its own chain of products and exponentials (33 x 8 CTAs, 8192 keys: 11.8 us, 10.4
+// with four).  Every warp has its own running maximum, sum and output; they are merged at the end by
 // the rule of the combine kernel.
 template <int NW, int WK>
 __global__ void __launch_bounds__(NW * WK * 32) attn_partial_kernel(const AttnArgs a)
