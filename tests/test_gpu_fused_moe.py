@@ -194,6 +194,28 @@ def test_config4_4096_tokens_sampled(cuda, oracle):
     assert rel_err(y[toks, slots], want) <= 2e-3
 
 
+@pytest.mark.parametrize("k", [1, 4, 8])
+@pytest.mark.parametrize("tokens,width", [(16, 2048), (16, 1920), (15, 2048)])
+def test_decode_with_the_longest_ranges_rotates_in_the_kernel(cuda, k, tokens, width):
+    """128 pairs give a GEMV half up to 56 rotated blocks, the most that are rotated inside the kernel: the same
+    bits as with a rotation kernel of its own in front of it."""
+    import torch
+    from ponyexl3_b200 import _lib
+
+    w = _experts(16, width, 512, k, seed=60 + k)
+    m = _switch(w, k, 0)
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = (torch.randn((1, tokens, width), device="cuda", generator=g) * 0.02).half()
+    idx = torch.topk(torch.randn((1, tokens, 16), device="cuda", generator=g), 8, dim=-1).indices
+    got = m(x, idx).clone()
+    _lib.load().exl3_tune_gemv(0, 0)
+    try:
+        want = m(x, idx).clone()
+    finally:
+        _lib.load().exl3_tune_gemv(0, 28 * 1024)
+    assert torch.isfinite(got).all() and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("world", [2, 3, 8])
 @pytest.mark.parametrize("tokens", [1, 5, 16])
 def test_decode_over_an_expert_range_sums_to_the_full_switch(cuda, oracle, world, tokens):
