@@ -318,6 +318,44 @@ def test_glu_folded_into_the_down_projection(cuda, oracle, act, rows):
     assert ops.Workspace.get(torch.device("cuda"), 1, 128).status() == 0
 
 
+def test_glu_on_load_equals_the_division_for_every_fp16_gate(cuda):
+    """The quotient without a division inside the rotations against the activation kernel, which divides: the
+    same bits for every finite fp16 gate.  Powers of two as `up` bring the products to unit size, which is exact."""
+    from ponyexl3_b200 import ops
+
+    H, k = 8192, 4
+    tr, suh, svh, _ = synthetic_layer(k, H, 128, seed=710)
+    t = lambda a: torch.from_numpy(a).cuda()
+    g = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.float16).cuda()
+    g = torch.where(g.isfinite(), g, torch.zeros_like(g))[torch.randperm(65536, generator=torch.Generator().manual_seed(1)).cuda()]
+    size = (g.float() / (1 + torch.exp(-g.float()))).abs().clamp(2.0**-15, 2.0**14)
+    up = torch.exp2(-torch.floor(torch.log2(size))).half()
+    for rows in (8, 16):                                  # rotated inside the GEMV, and by the rotation kernel
+        gu = torch.cat([g.view(8, H), up.view(8, H)], 1).repeat(rows // 8, 1)
+        y = ops.gemv(gu, t(tr.view(np.int16)), k, 0, t(suh), t(svh), None, glu="silu")
+        want = ops.gemv(ops.swiglu(gu), t(tr.view(np.int16)), k, 0, t(suh), t(svh), None)
+        assert torch.isfinite(want).all() and torch.equal(y, want)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("rows", [1, 12])
+def test_glu_of_gates_beyond_the_range_of_fp16(cuda, dtype, rows):
+    """Gates of bf16 and fp32 rows are not rounded to fp16 first: hugely negative ones give 0, in the rotation
+    inside the GEMV and in the rotation kernel.  The same layer on the GLU's result computed outside: a gate whose
+    exponential differs in the last bit flips one fp16 rounding of h, so the bound is that of a linear."""
+    from ponyexl3_b200 import ops
+
+    H, k = 512, 4
+    tr, suh, svh, _ = synthetic_layer(k, H, 128, seed=720)
+    t = lambda a: torch.from_numpy(a).cuda()
+    gu = torch.from_numpy(np.random.default_rng(rows).standard_normal((rows, 2 * H)).astype(np.float32)).cuda().to(getattr(torch, dtype))
+    gu[:, :32] = torch.tensor([-1e38, -3e34, -1e5, -95.0], device="cuda").repeat(8).to(gu.dtype)
+    h = (gu[:, :H].float() / (1 + torch.exp(-gu[:, :H].float())) * gu[:, H:].float()).half()
+    y = ops.gemv(gu, t(tr.view(np.int16)), k, 0, t(suh), t(svh), None, glu="silu")
+    want = ops.gemv(h, t(tr.view(np.int16)), k, 0, t(suh), t(svh), None)
+    assert (y.float() - want.float()).norm() / want.float().norm() < 1e-3
+
+
 @pytest.mark.parametrize("rows", [1, 5, 16, 40])
 def test_mlp_monolith_matches_the_three_linears(cuda, oracle, rows):
     """gate|up -> SiLU-GLU -> down as one module (the reference's EXL3MLPMonolith): equals the
