@@ -17,15 +17,17 @@ namespace exl3 {
 // x <- fp16(x + delta) (delta may be NULL), h <- fp16(x * rsqrt(mean(x^2) + eps) * w).
 // One CTA per row, eight elements per thread and turn.  A row is a handful of dependent round trips to L2, so
 // there are as many threads as the row has pieces (up to 1024), the first two turns' values stay in registers
-// between the two passes, and the weights are fetched before the sum is known; under EXL3_FLAG_PDL even before
-// the previous kernel has ended.
+// between the two passes, and the weights are fetched before the sum is known.  Nothing is read before the
+// previous kernel has ended, which may have written any of it; a hint brings the weights into L2 by then.
 constexpr int kNormTurns = 2;
 __global__ void __launch_bounds__(1024) add_rmsnorm_kernel(__half* x, const __half* delta, const __half* w,
                                                            __half* h, int n, int64_t x_stride,
-                                                           int64_t d_stride, int64_t h_stride, float eps, int early)
+                                                           int64_t d_stride, int64_t h_stride, float eps)
 {
     griddep_launch_dependents();
-    if (!early) griddep_wait();
+    if ((threadIdx.x & 7) == 0)                            // eight threads read a 128-byte line
+        for (int i = threadIdx.x * 8; i < n; i += blockDim.x * 8) prefetch_l2(w + i);
+    griddep_wait();
     __shared__ float red[32];
     __half* xr = x + (int64_t)blockIdx.x * x_stride;
     const __half* dr = delta ? delta + (int64_t)blockIdx.x * d_stride : nullptr;
@@ -35,15 +37,10 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_kernel(__half* x, const __ha
     for (int q = 0; q < kNormTurns; q++) {
         const int i = first + q * step;
         v[q] = g[q] = d[q] = make_uint4(0u, 0u, 0u, 0u);
-        if (i < n) g[q] = *reinterpret_cast<const uint4*>(w + i);
-    }
-    if (early) griddep_wait();
-#pragma unroll
-    for (int q = 0; q < kNormTurns; q++) {
-        const int i = first + q * step;
         if (i < n) {
             v[q] = *reinterpret_cast<const uint4*>(xr + i);
             if (dr) d[q] = *reinterpret_cast<const uint4*>(dr + i);
+            g[q] = *reinterpret_cast<const uint4*>(w + i);
         }
     }
     float ss = 0.f;
@@ -498,12 +495,11 @@ extern "C" int exl3_add_rmsnorm(uint16_t* x, const uint16_t* delta, const uint16
     if (rows < 1 || n < 8 || n % 8) return EXL3_E_SHAPE;
     if (x_row_stride % 8 || h_row_stride % 8 || (delta && delta_row_stride % 8)) return EXL3_E_ALIGN;
     if (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)h | (uintptr_t)delta) & 15) return EXL3_E_ALIGN;
-    const bool pdl = (flags & EXL3_FLAG_PDL) != 0;
     const unsigned threads = (unsigned)std::min<int64_t>(1024, (n / 8 + 31) / 32 * 32);
     return launch_kernel(add_rmsnorm_kernel, dim3((unsigned)rows), dim3(threads), 0, (cudaStream_t)stream,
-                         pdl, reinterpret_cast<__half*>(x),
+                         (flags & EXL3_FLAG_PDL) != 0, reinterpret_cast<__half*>(x),
                          reinterpret_cast<const __half*>(delta), reinterpret_cast<const __half*>(weight),
-                         reinterpret_cast<__half*>(h), (int)n, x_row_stride, delta_row_stride, h_row_stride, eps, pdl ? 1 : 0);
+                         reinterpret_cast<__half*>(h), (int)n, x_row_stride, delta_row_stride, h_row_stride, eps);
 }
 
 extern "C" int exl3_rope_append(const uint16_t* qkv, int64_t qkv_row_stride, const uint16_t* cos_table,

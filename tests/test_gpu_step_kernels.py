@@ -33,6 +33,27 @@ def test_add_rmsnorm(ops, rows, n, with_delta):
     assert _rel(h, want_h) < 1e-3
 
 
+def test_add_rmsnorm_waits_for_a_weight_written_by_the_kernel_before(ops):
+    """With a programmatic launch the norm starts while its predecessor runs; every operand, the weight among
+    them, may be that kernel's output.  The predecessor is a GEMM of one CTA, which lets its successor start at once
+    and stores last; a spin kernel in front of both has them queued together."""
+    from ponyexl3_b200 import EXL3Linear
+    g = torch.Generator(device="cuda").manual_seed(6)
+    m = EXL3Linear.from_device_tensors(
+        trellis=torch.randint(-32768, 32768, (8, 8, 64), dtype=torch.int16, device="cuda", generator=g), k=4, cb=0,
+        suh=torch.ones(128, device="cuda").half(), svh=torch.ones(128, device="cuda").half())
+    rows = torch.randn((256, 128), device="cuda", generator=g).half()
+    x = torch.randn((1, 128), device="cuda", generator=g).half()
+    buf = torch.empty((256, 128), dtype=torch.float16, device="cuda")
+    m(rows, out=buf)
+    want = ops.add_rmsnorm(x, None, buf[255].clone(), 1e-6)
+    for _ in range(10):
+        buf.zero_()
+        torch.cuda._sleep(1000000)
+        m(rows, out=buf)
+        assert torch.equal(ops.add_rmsnorm(x, None, buf[255], 1e-6, pdl=True), want)
+
+
 @pytest.mark.parametrize("rows,hq,hkv", [(1, 40, 8), (16, 40, 8), (3, 5, 1)])
 def test_rope_append(ops, rows, hq, hkv):
     g = torch.Generator(device="cuda").manual_seed(2)
