@@ -273,6 +273,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
             if (tid == 0) sh.smin[1] = 0x7F800000u;
             __syncthreads();
             double off = 0.0;                            // lower bound of every m_t[b]
+            bool tame = true;                            // all weights so far are small against the 1e30 of the unreachable
             for (int t = 0; t < 255; t++) {
                 const int cur = E::kInPlace ? 0 : (t & 1), nxt = E::kInPlace ? 0 : cur ^ 1;
                 const int rot = E::kInPlace ? (K * t) % LB : 0;
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                 double* mdn = md0 + nxt * NB;
                 float* mfn = mf0 + nxt * NB;
                 const float w = sh.w[t];
-                const bool tame = fabsf(w) < 1e6f;
+                tame = tame && fabsf(w) < 1e6f;
                 // costs in mfc are relative to the bound of the step before
                 const float near = (float)off * 9.3e-10f;   // 2^-30: closer than this, float64 roundings decide
                 if (t > 0) {
