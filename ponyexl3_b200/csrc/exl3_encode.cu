@@ -186,6 +186,14 @@ __device__ __forceinline__ int64_t next_tile(EncodeShared& sh, const EncodeArgs&
     return tile;
 }
 
+// The larger one; NaN if either is (a NaN weight makes all costs NaN, and then index 0 wins everywhere).
+__device__ __forceinline__ float fmax_nan(float a, float b)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // (k & ~(J - 1)) | j as one three-input operation (written in C, ptxas made two of it).
 template <int J> __device__ __forceinline__ uint32_t key_with_index(uint32_t k, uint32_t j)
 {
@@ -379,7 +387,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                             const uint32_t b = (h << K) | (l0 + i);
                             // in place, base b' = (h << K) | l of the next step takes the address of h | l << (LB - K)
                             const uint32_t at = E::kInPlace ? slot(h | (i << (LB - K)), rot) : slot(b, 0);
-                            const float rel = fmaxf((float)(val[i] - off), 0.f);
+                            const float rel = fmax_nan((float)(val[i] - off), 0.f);
                             mdn[at] = val[i];
                             mfn[at] = rel;
                             low_new = min(low_new, __float_as_uint(rel));

@@ -70,17 +70,18 @@ def test_encoder_where_fp32_keys_cannot_decide(ops, oracle, k, cb):
 
 @pytest.mark.parametrize("k,cb", [(1, 0), (2, 0), (3, 1), (4, 0), (5, 1), (6, 2), (7, 0), (8, 2)])
 def test_encoder_of_weights_without_measure(ops, oracle, k, cb):
-    """Squared errors of the size of the 1e30 that marks unreachable states and beyond the range of fp32, and
-    infinite weights, at the start, in the middle and at the end of a tile: the states of the oracle's search."""
+    """Squared errors of the size of the 1e30 that marks unreachable states and beyond the range of fp32, infinite
+    weights and NaN, each at the start, in the middle and at the end of a tile: the states of the oracle's search."""
     rng = np.random.default_rng(60 + k)
     w = rng.standard_normal((8, 256)).astype(np.float32)
     w[0, 5] = 1e16
-    w[1, 100] = -1e18
+    w[1, 100] = np.nan
     w[2, 30] = np.inf
     w[3, 7] = -3e37
     w[4, [3, 200]] = 2e15, 5e15
     w[5, [0, 255]] = 4e17, 1e16
-    w[6, [0, 128]] = 3e15, -np.inf
+    w[6, [0, 128]] = np.nan, -np.inf
+    w[7, 255] = np.nan
     states, _ = ops.quantize_tiles(torch.from_numpy(w).cuda(), k, cb)
     for t in range(8):
         want, _ = oracle.quantize_tile(w[t], k, cb)
