@@ -2,6 +2,8 @@
 // bit-exact test target), the codebook table, and the stand-alone Hadamard-128
 // rotation.  All are HBM-trivial; the matmul kernels reuse the same device
 // functions, so a bit-exact decode here proves the arithmetic they run.
+#include <type_traits>
+
 #include "exl3_internal.h"
 
 namespace exl3 {
@@ -196,6 +198,11 @@ __global__ void __launch_bounds__(256)
 // bits 0 (c), 3, 4 (t) and 1 (c); the bits of n are given the same meaning, which makes B the plain H16 for
 // every group and leaves a lane, after the butterflies over q and s, with the same 8 contiguous columns
 // per quarter that it loaded: stores are as wide as the loads.
+//
+// x * pre is rounded to fp16, which is exact for +-1 only.  With SPLIT it is two fp16 parts and two products: for
+// the rows of a sibling group that one by one would be few enough for the butterfly kernel, which does not round
+// it (multipliers of 0.5 to 1.5, 40 rows: 5.0e-4 off the oracle without, 7e-5 with it).  A group of 5120 + 2 x 1024
+// columns and 24 to 63 rows takes 19.4 .. 21.0 us without, 19.6 .. 21.2 with it, 23.1 .. 27.2 by the butterfly kernel.
 template <typename T> struct Load8;
 template <> struct Load8<__half> {
     static __device__ __forceinline__ uint4 at(const __half* p) { return *reinterpret_cast<const uint4*>(p); }
@@ -227,7 +234,15 @@ __device__ __forceinline__ uint32_t glu_pair(uint32_t gate, uint32_t up, int glu
     return h2_as_u32(__floats2half2_rn(glu_value(gf.x, uf.x, glu), glu_value(gf.y, uf.y, glu)));
 }
 
-template <typename T>
+// x * p as the rounded product (in place of x) and what that leaves out, exact but for what is below 2^-24.
+__device__ __forceinline__ void split_product(uint32_t& x, uint32_t p, uint32_t& rest)
+{
+    const __half2 x2 = u32_as_h2(x), p2 = u32_as_h2(p), h = __hmul2_rn(x2, p2);
+    x = h2_as_u32(h);
+    rest = h2_as_u32(__hfma2(x2, p2, __hneg2(h)));
+}
+
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(256, 2)
     hadamard_mma_kernel(const T* __restrict__ x, int64_t rows, int64_t n, int64_t x_row_stride,
                         const __half* __restrict__ pre, __half* __restrict__ out,
@@ -289,6 +304,10 @@ __global__ void __launch_bounds__(256, 2)
                 }
             }
         }
+        uint4 la[4], lb[4];                                  // SPLIT: the second parts
+        if (SPLIT && !pre)
+#pragma unroll
+            for (int q = 0; q < 4; q++) la[q] = lb[q] = make_uint4(0u, 0u, 0u, 0u);
         if (pre) {
             const __half* q0 = pre + (ok0 && pre_row ? (int64_t)pre_row[r0] : mb0) * n + col;
             const __half* q1 = pre + (ok1 && pre_row ? (int64_t)pre_row[r1] : mb1) * n + col;
@@ -296,6 +315,13 @@ __global__ void __launch_bounds__(256, 2)
             for (int q = 0; q < 4; q++) {
                 const uint4 a = *reinterpret_cast<const uint4*>(q0 + 32 * q);
                 const uint4 b = *reinterpret_cast<const uint4*>(q1 + 32 * q);
+                if constexpr (SPLIT) {
+                    split_product(xa[q].x, a.x, la[q].x); split_product(xa[q].y, a.y, la[q].y);
+                    split_product(xa[q].z, a.z, la[q].z); split_product(xa[q].w, a.w, la[q].w);
+                    split_product(xb[q].x, b.x, lb[q].x); split_product(xb[q].y, b.y, lb[q].y);
+                    split_product(xb[q].z, b.z, lb[q].z); split_product(xb[q].w, b.w, lb[q].w);
+                    continue;
+                }
                 xa[q].x = h2_as_u32(__hmul2(u32_as_h2(xa[q].x), u32_as_h2(a.x)));
                 xa[q].y = h2_as_u32(__hmul2(u32_as_h2(xa[q].y), u32_as_h2(a.y)));
                 xa[q].z = h2_as_u32(__hmul2(u32_as_h2(xa[q].z), u32_as_h2(a.z)));
@@ -318,6 +344,10 @@ __global__ void __launch_bounds__(256, 2)
                 for (int nt = 0; nt < 2; nt++) {
                     float d[4] = {0.f, 0.f, 0.f, 0.f};
                     mma_16816(d, af, hb[nt][0], hb[nt][1]);
+                    if constexpr (SPLIT) {
+                        const uint32_t lf[4] = {s ? la[q].z : la[q].x, s ? lb[q].z : lb[q].x, s ? la[q].w : la[q].y, s ? lb[q].w : lb[q].y};
+                        mma_16816(d, lf, hb[nt][0], hb[nt][1]);
+                    }
                     c[2 * q + s][nt][0] = f32x2(d[0], d[1]);
                     c[2 * q + s][nt][1] = f32x2(d[2], d[3]);
                 }
@@ -451,19 +481,16 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
     const int early = pdl ? 1 : 0;
     cudaError_t e;
     if (mma) {
+        const bool split = member_rows > 0 && member_rows < kHadamardMmaMinRows;
+        auto launch = [&](auto* xt) {
+            using T = std::remove_const_t<std::remove_pointer_t<decltype(xt)>>;
+            return cudaLaunchKernelEx(&cfg, split ? hadamard_mma_kernel<T, true> : hadamard_mma_kernel<T, false>, xt, rows, n,
+                                      x_row_stride, pre, out, row_src, pre_row, rows_dev, early, glu, member_rows);
+        };
         switch (x_dtype) {
-            case EXL3_DT_F16:
-                e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<__half>, (const __half*)x, rows, n, x_row_stride, pre,
-                                       out, row_src, pre_row, rows_dev, early, glu, member_rows);
-                break;
-            case EXL3_DT_BF16:
-                e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x, rows, n,
-                                       x_row_stride, pre, out, row_src, pre_row, rows_dev, early, glu, member_rows);
-                break;
-            case EXL3_DT_F32:
-                e = cudaLaunchKernelEx(&cfg, hadamard_mma_kernel<float>, (const float*)x, rows, n, x_row_stride, pre,
-                                       out, row_src, pre_row, rows_dev, early, glu, member_rows);
-                break;
+            case EXL3_DT_F16: e = launch((const __half*)x); break;
+            case EXL3_DT_BF16: e = launch((const __nv_bfloat16*)x); break;
+            case EXL3_DT_F32: e = launch((const float*)x); break;
             default: return EXL3_E_DTYPE;
         }
         return note_cuda(e);

@@ -48,6 +48,30 @@ def test_fused_group_matches_members(cuda, oracle, rows, k, cb):
         assert rel_err(o.cpu().numpy(), want) <= 1e-3
 
 
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("rows", [17, 24, 63])
+def test_fused_group_with_scales_other_than_signs(cuda, oracle, rows, dtype):
+    """suh holds fp16 multipliers, not only +-1: below 64 rows x * suh is not rounded before the rotation, for the
+    members of a group (51, 72 and 189 rotated rows: both rotation kernels) as for a layer of its own.  The oracle
+    rounds at the same places, so what is left is roundings of xh, y and sums that flip (1e-4); a rounded product
+    would add its own 2^-12 rms, 2.8e-4 and more (5e-4 was seen)."""
+    import ponyexl3_b200
+    from ponyexl3_b200 import EXL3Linear
+    from ponyexl3_b200.fused import FusedEXL3Group
+
+    layers = []
+    for i in range(3):
+        tr, suh, svh, _ = synthetic_layer(4, 1024, 256, seed=970 + i)
+        suh = (suh * np.random.default_rng(i).uniform(0.5, 1.5, 1024)).astype(np.float16)
+        layers.append(ponyexl3_b200.EXL3Layer(f"m{i}", 1024, 256, 4, tr, suh, svh, None))
+    xd = torch.from_numpy(np.random.default_rng(rows).standard_normal((rows, 1024)).astype(np.float32)).cuda().to(getattr(torch, dtype))
+    x = xd.half().cpu().numpy()
+    for o, l in zip(FusedEXL3Group(layers).forward_all(xd), layers):
+        want = oracle.linear_forward(x, l.trellis, 4, 0, l.suh, l.svh, None)
+        for got in (o, EXL3Linear(l)(xd)):
+            assert rel_err(got.cpu().numpy(), want) <= 2.5e-4
+
+
 def test_fused_siblings_share_one_launch_and_refuse_bad_groups(cuda):
     from ponyexl3_b200.fused import FusedEXL3Group, fusable
 
