@@ -120,19 +120,17 @@ __device__ __forceinline__ void had128_warp(float (&v)[4], int lane)
 enum : int { GLU_NONE = 0, GLU_SILU = 1, GLU_GELU = 2 };
 // g / (1 + exp(-g)).  The division is a product with the approximate reciprocal and one correction by the
 // residual (Markstein, IBM J. Res. Dev. 34, 1990), without the division's branch, which kept a rotation from
-// overlapping the elements of a row: SwitchGLU of 4096 tokens 507 -> 499 us, MLP of 300 rows 167 -> 162.  A
-// divisor beyond 2^64 is scaled into the range of the reciprocal, exactly, and an infinite one gives -0 (NaN for
-// an infinite g) as the division does, so that bf16 and fp32 gates of any size are right too.  All 65,536 fp16
-// gates give the division's float (only -0 gives +0).
+// overlapping the elements of a row: SwitchGLU of 4096 tokens 507 -> 499 us, MLP of 300 rows 167 -> 162.  Outside
+// (-87, 87), where the reciprocal would leave fp32, the result is g or -0 (NaN for NaN and minus infinity), so that
+// bf16 and fp32 gates of any size are right too.  All 65,536 fp16 gates give the division's float where that is
+// above 1e-35 (only -0 gives +0).
 __device__ __forceinline__ float silu(float g)
 {
     const float d = 1.f + __expf(-g);
-    const float scale = d > 0x1p64f ? 0x1p-64f : 1.f;
-    const float ds = fminf(d * scale, 3e38f);          // (3e38: its reciprocal is flushed to 0)
     float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(ds));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     const float q = g * r;
-    return d == 1.f ? g : __fmaf_rn(__fmaf_rn(-q, ds, g), r, q) * scale;   // (d is 1 for an infinite g too)
+    return fabsf(g) < 87.f ? __fmaf_rn(__fmaf_rn(-q, d, g), r, q) : g * __saturatef(g);
 }
 __device__ __forceinline__ float glu_value(float g, float u, int mode)
 {
