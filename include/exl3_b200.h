@@ -171,7 +171,9 @@ EXL3_API int exl3_gemv_blocks_counted(const void* x, int x_dtype, int64_t x_row_
  * (decode_full_mlx + matmul, ponyexl3/mlx/gemv_metal.py:630-774, and the striped path).
  * The workspace holds the rotated activations and the partial sums of output tiles that several
  * CTAs share: exl3_gemm_workspace_bytes(rows, in); without room for the latter tiles are not shared.
- * flags: EXL3_FLAG_GLU_* as in exl3_gemv (x rows are [gate (in) | up (in)]). */
+ * flags: EXL3_FLAG_GLU_* as in exl3_gemv (x rows are [gate (in) | up (in)]).  EXL3_FLAG_PDL is taken and has
+ * no effect: a CTA of the GEMM needs a whole SM, so its weights cannot be fetched while an earlier kernel has
+ * it (fetching them during the rotation: decode step of 8 layers, 9 to 16 rows 1430 .. 1495 -> 1440 .. 1506 us). */
 EXL3_API size_t exl3_gemm_workspace_bytes(int64_t rows, int64_t in);
 EXL3_API int exl3_gemm(const void* x, int x_dtype, int64_t rows, int64_t x_row_stride, const uint16_t* trellis,
               int64_t t_in, int64_t t_out, int k, int cb, const uint16_t* suh, const uint16_t* svh,

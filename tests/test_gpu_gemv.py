@@ -220,19 +220,20 @@ def test_more_than_16_rows_go_to_the_gemm(mod, oracle):
     _check(mod, oracle, layer, x)
 
 
-def test_programmatic_launch_chain(mod, oracle):
+@pytest.mark.parametrize("rows", [1, 12, 40])
+def test_programmatic_launch_chain(mod, oracle, rows):
     """Back-to-back layers launched with programmatic stream serialisation give the same
     results as plain launches."""
     layers = [_layer(mod, 4, 1024, 1024, seed=60 + i) for i in range(4)]
     mods = [mod.EXL3Linear(l) for l in layers]
-    x = torch.from_numpy(np.random.default_rng(3).standard_normal((1, 1024)).astype(np.float16)).cuda()
+    x = torch.from_numpy(np.random.default_rng(3).standard_normal((rows, 1024)).astype(np.float16)).cuda()
 
     def chain(pdl):
         h = x
         for m in mods:
             m.pdl = pdl
             h = (m(h).float() * 0.05).half()
-        return h
+        return m((m(h).float() * 0.05).half())
 
     plain = chain(False)
     for _ in range(3):
