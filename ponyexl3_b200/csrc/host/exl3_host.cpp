@@ -140,9 +140,15 @@ Rows rows_of(const at::Tensor& x, int64_t features)
         r.rows = x.size(0);
         r.stride = r.t.stride(0);
     } else {
-        r.t = x.contiguous();
         r.rows = features > 0 ? x.numel() / features : 0;
         r.stride = features;
+        if (x.is_contiguous()) {
+            r.t = x;
+        } else {                                       // a view where the leading dimensions fold into one, else a copy
+            r.t = x.reshape({r.rows, features});
+            if (r.t.stride(1) != 1) r.t = r.t.contiguous();
+            r.stride = r.t.stride(0);
+        }
     }
     // the stride of a single row means nothing (views may carry any number there)
     if (r.rows == 1 && r.stride < features) r.stride = features;

@@ -199,6 +199,22 @@ def test_dtypes_shapes_and_no_parameters(mod, oracle):
     assert rel_err(y2, oracle.linear_forward(x1, layer.trellis, 4, 0, None, None)) <= REL_TOL
 
 
+def test_strided_activations_are_copied_only_where_they_must_be(mod):
+    """Views whose leading dimensions fold into rows of one stride (the last token of every sequence, a column
+    range) are read where they are; others take one copy.  Same bits as from a contiguous tensor."""
+    layer = _layer(mod, 4, 256, 384, seed=12)
+    m = mod.EXL3Linear(layer)
+    big = torch.randn((3, 20, 512), device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).half()
+    allocated = lambda: torch.cuda.memory_stats()["allocation.all.allocated"]
+    for x, allocations in ((big[:, -1:, :256], 1), (big[..., 256:], 1), (big[:, :4, :256], 2), (big[:, 2, 256:], 1),
+                           (big.transpose(0, 1)[..., :256], 2), (big[:1, :, ::2], 2), (big[:, :1, :256].expand(3, 2, 256), 2)):
+        want = m(x.clone(memory_format=torch.contiguous_format))
+        before = allocated()
+        got = m(x)
+        assert allocated() - before == allocations, x.stride()
+        assert got.shape == x.shape[:-1] + (384,) and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("k", [2, 4, 5, 8])
 @pytest.mark.parametrize("cb", [0, 1, 2])
 @pytest.mark.parametrize("rows", [1, 11])
