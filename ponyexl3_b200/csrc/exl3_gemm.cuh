@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "exl3_gemm_plan.h"
 #include "exl3_internal.h"
 #include "exl3_tc.cuh"
 #include "exl3_tma.h"
@@ -736,13 +737,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
 // Bytes of partial sums a dense launch may use: two slots of 128 columns x (tokens of a tile) per CTA.
 inline size_t gemm_tile_partial_bytes(int tok, int ctas) { return (size_t)ctas * 2 * kTsOuts * (size_t)tok * sizeof(float); }
 
-// The launch plan of a dense GEMM (exl3_gemm.cu).
-struct TsPlan {
-    int tok, tiles_m;        // tokens per output tile, tiles of tokens
-    int grid, split;         // CTAs; whether they share tiles
-    int wide;
-};
-TsPlan ts_plan(int64_t rows, int64_t tiles_n, int nks, int sms, size_t partial_bytes, int tok, int tok_wide);
+TsPlan gemm_plan(int64_t rows, int64_t tiles_n, int nks, int sms, size_t partial_bytes, int tok, int tok_wide);
 
 template <int K, int CB, bool TABLE>
 static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, cudaStream_t s)
@@ -780,7 +775,7 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
         grid = std::min(a.n_items, (sms - 1) | 1);
     } else {
         a.tiles_n = a.t_out / 8;
-        const TsPlan plan = ts_plan(a.m, a.tiles_n, nks, sms, a.ts_partial_bytes, L::kTok, L::kTokWide);
+        const TsPlan plan = gemm_plan(a.m, a.tiles_n, nks, sms, a.ts_partial_bytes, L::kTok, L::kTokWide);
         a.ts_tok = plan.tok;
         a.tiles_m = plan.tiles_m;
         a.n_items = a.tiles_m * a.tiles_n;

@@ -1,0 +1,101 @@
+// The launch plan of a dense tensor-core GEMM: tokens per output tile, number of CTAs, whether they share tiles.
+// Host code without CUDA, so that tests can compile it alone.
+//
+// A server sees a new row count on nearly every call, so a plan has to cost about as little as a launch: the exhaustive
+// search over CTA counts, CTAs and segments took 0.1 ms (16 rows) to 24 ms (8191 rows, 17408 columns).  Bounds
+// leave some of the CTA counts, and the segments of a CTA are counted without walking them: 4 to 9 us, with the
+// same choice (tests/test_gemm_plan.py).
+#pragma once
+#include <stdint.h>
+
+#include <algorithm>
+
+namespace exl3 {
+
+struct TsPlan {
+    int tok, tiles_m;        // tokens per output tile, tiles of tokens
+    int grid, split;         // CTAs; whether they share tiles
+    int wide;
+};
+
+// Costs are in k-steps of the slowest CTA: its k-steps, and for each of its segments the hand-over and the
+// epilogue, which the decode warps do themselves.
+constexpr int kTsWholeCost = 6, kTsSharedCost = 10;
+
+// The least that `len` consecutive k-steps can cost, however they lie on tiles of nks.
+inline int64_t ts_least(int64_t len, int nks)
+{
+    return len + kTsWholeCost * (len / nks) + (len % nks ? kTsSharedCost : 0);
+}
+
+// The slowest of g CTAs that take [U c/g, U (c+1)/g) of U = tiles x nks k-steps; `enough` ends the search.
+inline int64_t ts_slowest(int64_t units, int nks, int g, int64_t enough)
+{
+    const int64_t q = units / g, q_tiles = q / nks;
+    const int r = (int)(units % g), q_rest = (int)(q % nks);
+    int at = 0, err = 0;                     // where in its tile a CTA starts; Bresenham's remainder
+    int64_t worst = 0;
+    for (int c = 0; c < g; c++) {
+        err += r;
+        const int more = err >= g;           // U (c+1)/g - U c/g is q or q + 1
+        if (more) err -= g;
+        int end = at + q_rest + more;
+        int64_t ends = q_tiles;              // tile ends inside or at the end of the range
+        if (end >= nks) { end -= nks; ends++; }
+        const int64_t whole = ends - (at != 0 && ends > 0 ? 1 : 0);
+        const int shared = ends == 0 ? 1 : (at != 0) + (end != 0);
+        worst = std::max(worst, q + more + kTsWholeCost * whole + kTsSharedCost * shared);
+        if (worst >= enough) break;
+        at = end;
+    }
+    return worst;
+}
+
+// How many CTAs a launch of `tiles` output tiles of nks k-steps gets, and whether they share tiles.  For shared
+// tiles a count that lets ranges end on tile boundaries saves a segment per CTA, so counts down to half of the SMs
+// are looked at, as far as they can still be the best.  Returns the cost; `enough`: a cost that is of no use.
+inline int64_t ts_deal(int64_t tiles, int nks, int sms, bool room, int64_t enough, int* grid, int* split)
+{
+    const int whole = (int)std::min<int64_t>(tiles, sms);
+    *grid = whole;
+    *split = 0;
+    int64_t best = ((tiles + whole - 1) / whole) * (nks + kTsWholeCost);
+    const int64_t units = tiles * nks;
+    if (!room || tiles >= 64 * (int64_t)sms || units < 4) return best;
+    const int most = (int)std::min<int64_t>(sms, units / 4);
+    for (int g = most; g >= std::max(1, most / 2); g--) {
+        const int64_t least = ts_least((units + g - 1) / g, nks), limit = std::min(best, enough);
+        if (least - 3 >= limit) break;       // (ts_least falls by 3 where a range becomes whole tiles, and only there)
+        if (least >= limit) continue;
+        const int64_t worst = ts_slowest(units, nks, g, limit);
+        if (worst < best) { best = worst; *grid = g; *split = 1; }
+    }
+    return best;
+}
+
+// Tokens per tile: from as few tiles as wide ones allow to as few as ordinary ones need, whichever is cheapest at
+// 340 + 2.6 x tokens clocks a k-step, at least 610 (decoding bounds small tiles, the activations' way from L2
+// large ones).  Of many rows' counts the eight nearest to the ordinary tiles' are looked at, and the widest: further
+// ones differ by less than a tile's share.  Tiles of up to `room` tokens may be shared.
+inline TsPlan ts_plan(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room)
+{
+    TsPlan best = {};
+    double best_cost = 0;
+    auto look = [&](int64_t n) {
+        TsPlan p = {};
+        p.tok = (int)(((rows + n - 1) / n + 15) / 16 * 16);
+        p.wide = p.tok > tok;
+        if (p.tok > tok_wide) return;
+        p.tiles_m = (int)((rows + p.tok - 1) / p.tok);
+        const double clocks = std::max(610.0, 340.0 + 2.6 * p.tok);
+        const int64_t enough = best.tok ? (int64_t)(best_cost / clocks) + 1 : INT64_MAX;     // (rounded up: the exact test follows)
+        const double c = clocks * (double)ts_deal(p.tiles_m * tiles_n, nks, sms, p.tok <= room, enough, &p.grid, &p.split);
+        if (best.tok == 0 || c < best_cost) { best = p; best_cost = c; }
+    };
+    const int64_t few = (rows + tok_wide - 1) / tok_wide, many = (rows + tok - 1) / tok;
+    for (int64_t n = many; n >= few && n >= many - 8; n--) look(n);
+    if (few < many - 8) look(few);
+    return best;
+}
+
+}  // namespace exl3

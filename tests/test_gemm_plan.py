@@ -1,0 +1,70 @@
+"""The launch plan of the dense GEMM (csrc/exl3_gemm_plan.h), compiled for the host: the slowest CTA counted
+without walking its segments, the choice among token and CTA counts, and what a plan costs on the host."""
+
+from __future__ import annotations
+
+import ctypes
+import random
+import subprocess
+import time
+from pathlib import Path
+
+import pytest
+
+HERE = Path(__file__).resolve().parent
+TOKENS = [(256, 384), (240, 368), (224, 368), (208, 352), (192, 336)]      # tokens of an ordinary and a wide tile, K = 4 .. 8
+
+
+@pytest.fixture(scope="module")
+def emul(tmp_path_factory):
+    out = tmp_path_factory.mktemp("emul") / "libgemm_plan_emul.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-o", str(out),
+                    str(HERE / "host_emul" / "gemm_plan_emul.cpp")], check=True)
+    lib = ctypes.CDLL(str(out))
+    i, l = ctypes.c_int, ctypes.c_int64
+    for f in (lib.emul_plan, lib.exhaustive_plan):
+        f.argtypes = [l, l, i, i, i, i, i, ctypes.c_void_p]
+        f.restype = None
+    lib.emul_slowest.argtypes, lib.emul_slowest.restype = [l, i, i, i], l
+    return lib
+
+
+def _plan(f, *args):
+    out = (ctypes.c_int * 5)()
+    f(*args, out)
+    return tuple(out)
+
+
+def test_slowest_cta_equals_the_walk_over_its_segments(emul):
+    rng = random.Random(1)
+    for _ in range(4000):
+        nks = rng.choice([1, 2, 3, 8, 46, 80, 272, rng.randint(1, 300)])
+        units = nks * rng.randint(1, 2000)
+        g = rng.randint(1, min(148, units))
+        assert emul.emul_slowest(units, nks, g, 0) == emul.emul_slowest(units, nks, g, 1), (units, nks, g)
+
+
+def test_choice_equals_the_exhaustive_search(emul):
+    rng = random.Random(2)
+    for n in range(1500):
+        rows = round(2 ** rng.uniform(3, 14 if n % 10 else 17))
+        tiles_n, nks = rng.randint(1, 272), 2 * rng.randint(1, 136)
+        tok, wide = rng.choice(TOKENS)
+        room = rng.choice([0, tok, 384, 384, 384])
+        if rows * tiles_n > 4_000_000:
+            continue
+        args = (rows, tiles_n, nks, rng.choice([148, 148, 148, 132, 20]), tok, wide, room)
+        assert _plan(emul.emul_plan, *args) == _plan(emul.exhaustive_plan, *args), args
+
+
+def test_a_plan_costs_less_than_a_launch(emul):
+    """A new row count is planned anew; an exhaustive search of these takes milliseconds each."""
+    shapes = [(40, 80), (136, 80), (40, 272), (32, 64), (11, 46)]
+    out = (ctypes.c_int * 5)()
+    t0 = time.perf_counter()
+    n = 0
+    for rows in list(range(9, 400, 13)) + list(range(401, 8192, 401)):
+        for tiles_n, nks in shapes:
+            emul.emul_plan(rows, tiles_n, nks, 148, 256, 384, 384, out)
+            n += 1
+    assert (time.perf_counter() - t0) / n < 200e-6
