@@ -207,7 +207,7 @@ template <bool TABLE> struct TsWalk {
     // register.  (Behind a shuffle or a 64-bit division all of the issuing warps' loop control and descriptors
     // lived in ordinary registers and were moved over for every instruction: 5 to 9 % of the kernel.)
     static __device__ __forceinline__ int uniform(int v) { return __reduce_max_sync(0xFFFFFFFFu, v); }
-    int u, u1, u0;
+    int tile0, u, u1, u0;     // dense: the CTA's first tile; next, end and first k-step of its range, counted from that tile's
     // tables: a warp looks at 32 of its CTA's items at a time, one per lane, and takes those in use in turn
     int item;                 // first item not looked at yet
     uint32_t found;           // items in use among those looked at last
@@ -219,11 +219,14 @@ template <bool TABLE> struct TsWalk {
         found = 0;
         const int64_t g = gridDim.x, c = blockIdx.x, nks = a.t_in >> 2;
         if (a.ts_split) {
-            u0 = uniform((int)(a.n_items * nks * c / g));
-            u1 = uniform((int)(a.n_items * nks * (c + 1) / g));
+            const int k0 = (int)(a.n_items * nks * c / g), k1 = (int)(a.n_items * nks * (c + 1) / g);
+            tile0 = uniform(k0 / (int)nks);
+            u0 = uniform(k0 - tile0 * (int)nks);
+            u1 = uniform(k1 - tile0 * (int)nks);
         } else {
-            u0 = uniform((int)(a.n_items * c / g * nks));
-            u1 = uniform((int)(a.n_items * (c + 1) / g * nks));
+            tile0 = uniform((int)(a.n_items * c / g));
+            u0 = 0;
+            u1 = uniform(((int)(a.n_items * (c + 1) / g) - tile0) * (int)nks);
         }
         u = u0;
     }
@@ -268,8 +271,8 @@ template <bool TABLE> struct TsWalk {
         }
         if (u >= u1) return false;
         s.first = u == u0;
-        s.tile = uniform(u / nks);
-        s.k0 = u - s.tile * nks;
+        s.tile = tile0 + uniform(u / nks);
+        s.k0 = u - (s.tile - tile0) * nks;
         s.k1 = min(nks, s.k0 + (u1 - u));
         u += s.k1 - s.k0;
         const int tn = uniform(s.tile / a.tiles_m), tm = s.tile - tn * a.tiles_m;
@@ -778,8 +781,8 @@ static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, 
         const TsPlan plan = gemm_plan(a.m, a.tiles_n, nks, sms, a.ts_partial_bytes, L::kTok, L::kTokWide);
         a.ts_tok = plan.tok;
         a.tiles_m = plan.tiles_m;
+        if (!ts_countable(plan, a.tiles_n, nks)) return EXL3_E_SHAPE;
         a.n_items = a.tiles_m * a.tiles_n;
-        if ((int64_t)a.n_items * nks >= ((int64_t)1 << 31)) return EXL3_E_SHAPE;   // (k-steps are counted in 32 bits)
         a.ts_box_rows = a.ts_tok > 256 ? a.ts_tok / 2 : a.ts_tok;                  // (a box has at most 256 rows)
         a.ts_split = plan.split;
         grid = plan.grid;

@@ -61,7 +61,7 @@ inline int64_t ts_deal(int64_t tiles, int nks, int sms, bool room, int64_t enoug
     *split = 0;
     int64_t best = ((tiles + whole - 1) / whole) * (nks + kTsWholeCost);
     const int64_t units = tiles * nks;
-    if (!room || tiles >= 64 * (int64_t)sms || units < 4) return best;
+    if (!room || tiles >= 64 * (int64_t)sms || units < 4 || units > INT32_MAX) return best;
     const int most = (int)std::min<int64_t>(sms, units / 4);
     for (int g = most; g >= std::max(1, most / 2); g--) {
         const int64_t least = ts_least((units + g - 1) / g, nks), limit = std::min(best, enough);
@@ -96,6 +96,13 @@ inline TsPlan ts_plan(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, 
     for (int64_t n = many; n >= few && n >= many - 8; n--) look(n);
     if (few < many - 8) look(few);
     return best;
+}
+
+// The kernel counts tiles, k-steps where tiles are shared, and the k-steps of one CTA in 32 bits.
+inline bool ts_countable(const TsPlan& p, int64_t tiles_n, int nks)
+{
+    const int64_t tiles = p.tiles_m * tiles_n;
+    return tiles * (p.split ? nks : 1) <= INT32_MAX && (tiles + p.grid - 1) / p.grid * nks <= INT32_MAX;
 }
 
 }  // namespace exl3

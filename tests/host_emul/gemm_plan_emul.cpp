@@ -13,6 +13,11 @@ extern "C" void emul_plan(int64_t rows, int64_t tiles_n, int nks, int sms, int t
     out[0] = p.tok; out[1] = p.tiles_m; out[2] = p.grid; out[3] = p.split; out[4] = p.wide;
 }
 
+extern "C" int emul_countable(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok)
+{
+    return ts_countable(ts_plan(rows, tiles_n, nks, sms, tok, tok_wide, room_tok), tiles_n, nks);
+}
+
 static int64_t slowest(int64_t units, int nks, int g)
 {
     int64_t worst = 0;
@@ -48,7 +53,7 @@ extern "C" void exhaustive_plan(int64_t rows, int64_t tiles_n, int nks, int sms,
         int grid = (int)std::min<int64_t>(tiles, sms), split = 0;
         int64_t cost = ((tiles + grid - 1) / grid) * (nks + 6);
         const int most = (int)std::min<int64_t>(sms, units / 4);
-        if (t <= room_tok && tiles < 64 * (int64_t)sms && units >= 4)
+        if (t <= room_tok && tiles < 64 * (int64_t)sms && units >= 4 && units <= INT32_MAX)
             for (int g = most; g >= std::max(1, most / 2); g--) {
                 const int64_t w = slowest(units, nks, g);
                 if (w < cost) { cost = w; grid = g; split = 1; }

@@ -25,6 +25,7 @@ def emul(tmp_path_factory):
     for f in (lib.emul_plan, lib.exhaustive_plan):
         f.argtypes = [l, l, i, i, i, i, i, ctypes.c_void_p]
         f.restype = None
+    lib.emul_countable.argtypes = [l, l, i, i, i, i, i]
     lib.emul_slowest.argtypes, lib.emul_slowest.restype = [l, i, i, i], l
     return lib
 
@@ -55,6 +56,18 @@ def test_choice_equals_the_exhaustive_search(emul):
             continue
         args = (rows, tiles_n, nks, rng.choice([148, 148, 148, 132, 20]), tok, wide, room)
         assert _plan(emul.emul_plan, *args) == _plan(emul.exhaustive_plan, *args), args
+
+
+def test_every_shape_that_fits_a_gpu_can_be_counted(emul):
+    """rows x in x out beyond 2^31 k-steps of tiles: 42,000 rows of 400,000 x 400,000 (K = 1: 120 GB in all) and the
+    like are dealt in whole tiles, which are counted; k-steps of shared tiles stay within 32 bits."""
+    for rows, inf, outf in ((42_000, 400_000, 400_000), (65_536, 262_144, 262_144), (20_000, 800_000, 500_000), (8_000_000, 4096, 4096),
+                            (1, 16_777_216, 65_536), (1, 65_536, 16_777_216), (500, 2_000_000, 500_000)):
+        for tok, wide in TOKENS:
+            args = (rows, outf // 128, inf // 64, 148, tok, wide, 384)
+            assert emul.emul_countable(*args), args
+            tok_, tiles_m, grid, split, _ = _plan(emul.emul_plan, *args)
+            assert tiles_m * tok_ >= rows and (not split or tiles_m * (outf // 128) * (inf // 64) < 2**31)
 
 
 def test_a_plan_costs_less_than_a_launch(emul):
