@@ -245,11 +245,23 @@ Group group_of(PyObject* const* arg)
     g.total = integer(arg[6]);
     return g;
 }
-// blocks, row_src, suh_row: the group's table for this row count (FusedEXL3Group._table)
-void group_gemv(const Rows& x, int64_t rows, const Group& g, PyObject* blocks, PyObject* row_src, PyObject* suh_row,
-                const at::Tensor& y, unsigned flags, int dev, cudaStream_t s)
+// A Python object that this frame owns.
+struct Owned {
+    PyObject* p;
+    ~Owned() { Py_XDECREF(p); }
+};
+// table: FusedEXL3Group._table, which makes and keeps the block table of a row count: (blocks, row_src, suh_row).
+// Only this path needs one.
+void group_gemv(const Rows& x, int64_t rows, const Group& g, PyObject* table, PyObject* x_object, const at::Tensor& y,
+                unsigned flags, int dev, cudaStream_t s)
 {
-    const at::Tensor& b = tensor(blocks, "blocks");
+    const Owned device{PyObject_GetAttrString(x_object, "device")};
+    if (!device.p) throw PyError();
+    const Owned t{PyObject_CallFunction(table, "LO", (long long)rows, device.p)};
+    if (!t.p) throw PyError();
+    if (!PyTuple_Check(t.p) || PyTuple_GET_SIZE(t.p) != 3) fail(PyExc_TypeError, "a table of three tensors is expected");
+    PyObject *row_src = PyTuple_GET_ITEM(t.p, 1), *suh_row = PyTuple_GET_ITEM(t.p, 2);
+    const at::Tensor& b = tensor(PyTuple_GET_ITEM(t.p, 0), "blocks");
     const Workspace ws = workspace(dev, api.exl3_workspace_bytes(rows * g.members, 16 * g.w.t_in));
     check(api.exl3_gemv_blocks(x.t.data_ptr(), x.dtype, x.stride, rows * g.members, ptr_or_null<int32_t>(row_src, "row_src"),
                                g.suh, ptr_or_null<int32_t>(suh_row, "suh_row"), g.w.trellis, g.w.t_in, g.w.t_out, g.k, g.cb,
@@ -281,7 +293,7 @@ void group_gemm_packed(const Rows& x, const Group& g, PyObject* width_tuple, con
     group_gemm(x, x.rows, g, widths.data(), ptrs.data(), strides.data(), dev, s);
 }
 
-// group_packed(x2d, group..., blocks, row_src, suh_row, flags, widths) -> (rows, total), rows <= 16
+// group_packed(x2d, group..., table, flags, widths) -> (rows, total), rows <= 16
 PyObject* group_packed(PyObject* const* arg)
 {
     const at::Tensor& x = cuda_tensor(arg[0], "x");
@@ -295,9 +307,9 @@ PyObject* group_packed(PyObject* const* arg)
     at::Tensor y = empty_half({r.rows, g.total}, x.device());
     const cudaStream_t s = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
     if (g.members > kMaxMembers || use_gemv(r.rows, g.svh, nullptr, u16(y), g.total))
-        group_gemv(r, r.rows, g, arg[8], arg[9], arg[10], y, (unsigned)integer(arg[11]), dev, s);
+        group_gemv(r, r.rows, g, arg[8], arg[0], y, (unsigned)integer(arg[9]), dev, s);
     else
-        group_gemm_packed(r, g, arg[12], y, dev, s);
+        group_gemm_packed(r, g, arg[10], y, dev, s);
     return THPVariable_Wrap(std::move(y));
 }
 
@@ -325,27 +337,27 @@ PyObject* group_prefill(PyObject* const* arg)
     return t;
 }
 
-// mlp(x2d, group..., blocks, row_src, suh_row, down trellis, k, cb, suh, svh, bias, group flags, down flags)
+// mlp(x2d, group..., table, down trellis, k, cb, suh, svh, bias, group flags, down flags)
 // -> (rows, out): gate|up, then down with the GLU (part of the down flags) applied while it loads.
 PyObject* mlp(PyObject* const* arg)
 {
     const at::Tensor& x = cuda_tensor(arg[0], "x");
     const Group g = group_of(arg + 1);
-    const Weights d = weights(arg[11]);
+    const Weights d = weights(arg[9]);
     const Rows r = rows_of(x, 16 * g.w.t_in);
     const c10::cuda::CUDAGuard guard(x.device());
     const int dev = x.device().index();
     const cudaStream_t s = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-    const int dk = (int)integer(arg[12]), dcb = (int)integer(arg[13]);
-    const uint16_t* suh = ptr_or_null<uint16_t>(arg[14], "suh");
-    const uint16_t* svh = ptr_or_null<uint16_t>(arg[15], "svh");
-    const uint16_t* bias = ptr_or_null<uint16_t>(arg[16], "bias");
-    const unsigned gflags = (unsigned)integer(arg[17]), dflags = (unsigned)integer(arg[18]);
+    const int dk = (int)integer(arg[10]), dcb = (int)integer(arg[11]);
+    const uint16_t* suh = ptr_or_null<uint16_t>(arg[12], "suh");
+    const uint16_t* svh = ptr_or_null<uint16_t>(arg[13], "svh");
+    const uint16_t* bias = ptr_or_null<uint16_t>(arg[14], "bias");
+    const unsigned gflags = (unsigned)integer(arg[15]), dflags = (unsigned)integer(arg[16]);
     const at::Tensor gu = empty_half({r.rows, g.total}, x.device());
     at::Tensor y = empty_half({r.rows, 16 * d.t_out}, x.device());
     const Rows h{gu, r.rows, g.total, EXL3_DT_F16};
     if (use_gemv(r.rows, svh, bias, g.svh, 0)) {
-        group_gemv(r, r.rows, g, arg[8], arg[9], arg[10], gu, gflags, dev, s);
+        group_gemv(r, r.rows, g, arg[8], arg[0], gu, gflags, dev, s);
         gemv(h, r.rows, d, dk, dcb, suh, svh, bias, u16(y), 16 * d.t_out, dflags, dev, s);
     } else {
         const int64_t half = g.total / 2, widths[2] = {half, half}, strides[2] = {g.total, g.total};
@@ -480,9 +492,9 @@ PyMethodDef methods[] = {
     EXL3_METHOD(bind, 3),
     EXL3_METHOD(set_workspace, 3),
     EXL3_METHOD(linear, 9),
-    EXL3_METHOD(group_packed, 13),
+    EXL3_METHOD(group_packed, 11),
     EXL3_METHOD(group_prefill, 9),
-    EXL3_METHOD(mlp, 19),
+    EXL3_METHOD(mlp, 17),
     EXL3_METHOD(switch_glu, 15),
     {nullptr, nullptr, 0, nullptr},
 };

@@ -110,8 +110,8 @@ class FusedEXL3Group(torch.nn.Module):
         return self.in_features * int(self._offsets[-1]) * self.k // 8
 
     def _table(self, rows: int, device: torch.device):
-        """Block table and rotation indices for `rows` activation rows (cached per row count):
-        rotated row sub*rows + r = had(x[r] * suh[sub])."""
+        """Block table and rotation indices of the streamed GEMV for `rows` activation rows (cached per row
+        count): rotated row sub*rows + r = had(x[r] * suh[sub])."""
         t = self._tables.get(rows)
         if t is None:
             nb = len(self._block_sub)
@@ -132,8 +132,7 @@ class FusedEXL3Group(torch.nn.Module):
         if not 1 <= rows <= GEMV_MAX_ROWS:
             raise ValueError("forward_packed serves 1..16 rows")
         return (_lib._host or _lib.host()).group_packed(
-            x2d, *self._native(), *self._table(rows, x2d.device), _lib.FLAG_PDL if self.pdl else 0,
-            tuple(self._out_features))
+            x2d, *self._native(), self._table, _lib.FLAG_PDL if self.pdl else 0, tuple(self._out_features))
 
     def _native(self) -> tuple:
         """What the host extension takes of the group."""

@@ -63,8 +63,7 @@ class EXL3MLPMonolith(torch.nn.Module):
             return torch.empty(lead + (self.out_features,), dtype=torch.float16, device=x.device)
         pdl = _lib.FLAG_PDL if self.pdl else 0
         glu_flag = _lib.FLAG_GLU_GELU if self.activation == "gelu" else _lib.FLAG_GLU_SILU
-        table = g._table(rows, x.device) if rows <= 16 else (None, None, None)
         y = (_lib._host or _lib.host()).mlp(
-            x2d, *g._native(), *table, d._trellis, d.k, d.cb, d._suh, d._svh, d._bias, pdl,
+            x2d, *g._native(), g._table, d._trellis, d.k, d.cb, d._suh, d._svh, d._bias, pdl,
             pdl | glu_flag | (_lib.FLAG_FAST_ACCUM if d.fast_accum else 0))
         return y.reshape(lead + (self.out_features,))
