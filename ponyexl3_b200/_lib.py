@@ -136,20 +136,27 @@ def load() -> ctypes.CDLL:
     return _lib
 
 
+def host_path() -> Path:
+    """File of the host extension.  It is compiled against one PyTorch's C++ interface, so its name carries that
+    version: after an upgrade the old file is not found, instead of loaded."""
+    import sysconfig
+
+    import torch
+
+    return _PKG / "lib" / f"_exl3_host-torch{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
 def host():
     """The native host path of the module calls (``_exl3_host``), bound to the loaded library; raises
-    if it has not been built, as `load` does."""
+    if it has not been built for the installed PyTorch, as `load` does."""
     global _host
     if _host is None:
         import importlib.machinery
         import importlib.util
-        import sysconfig
 
-        import torch  # noqa: F401  (its libraries have to be loaded first)
+        from . import ops       # (imports torch: its libraries have to be loaded first)
 
-        from . import ops
-
-        path = _PKG / "lib" / ("_exl3_host" + sysconfig.get_config_var("EXT_SUFFIX"))
+        path = host_path()
         if not path.exists():
             raise RuntimeError(f"{path} is missing: build it with `python -m ponyexl3_b200.build`")
         loader = importlib.machinery.ExtensionFileLoader("_exl3_host", str(path))

@@ -22,7 +22,6 @@ LIBDIR = PKG / "lib"
 OBJDIR = PKG / "build"
 LIB = LIBDIR / "libexl3b200.so"
 HOST_SRC = CSRC / "host" / "exl3_host.cpp"
-HOST = LIBDIR / ("_exl3_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -88,11 +87,15 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False,
 
 
 def build_host(force: bool = False, verbose: bool = False) -> Path:
-    """Compile the host extension against the installed PyTorch; returns its path."""
-    deps = max(p.stat().st_mtime for p in (HOST_SRC, PKG.parent / "include" / "exl3_b200.h"))
-    if not force and HOST.exists() and HOST.stat().st_mtime >= deps:
-        return HOST
+    """Compile the host extension against the installed PyTorch; returns its path, which names that version."""
     import torch
+
+    from ._lib import host_path
+
+    host = host_path()
+    deps = max(p.stat().st_mtime for p in (HOST_SRC, PKG.parent / "include" / "exl3_b200.h"))
+    if not force and host.exists() and host.stat().st_mtime >= deps:
+        return host
 
     LIBDIR.mkdir(exist_ok=True)
     root = Path(torch.__file__).resolve().parent
@@ -100,13 +103,13 @@ def build_host(force: bool = False, verbose: bool = False) -> Path:
     inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], cuda]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_API_INCLUDE_EXTENSION_H",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in inc), str(HOST_SRC),
-           "-o", str(HOST), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+           "-o", str(host), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
     if verbose:
         print(" ".join(cmd), flush=True)
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed:\n{' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
-    return HOST
+    return host
 
 
 if __name__ == "__main__":

@@ -121,3 +121,16 @@ def test_ops_refuse_cpu_tensors():
         ops.unpack_trellis(torch.zeros((1, 1, 64), dtype=torch.int16), 4)
     with pytest.raises(RuntimeError):
         ops.had_r_128(torch.zeros((1, 128)))
+
+
+def test_host_extension_of_another_pytorch_is_not_loaded(monkeypatch):
+    """The host extension depends on PyTorch's C++ interface: with another version installed the module calls ask
+    for a build instead of loading it."""
+    import torch
+
+    from ponyexl3_b200 import _lib
+
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".other")
+    monkeypatch.setattr(_lib, "_host", None)
+    with pytest.raises(RuntimeError, match="ponyexl3_b200.build"):
+        _lib.host()
