@@ -17,8 +17,9 @@ extern "C" {
 /* max_grid: largest number of virtual CTAs (halves of the 1024-thread CTAs) a streamed GEMV
  * deals its items to (0 = two per SM, the default);
  * fuse_x_bytes: the input rotation runs inside the GEMV when the rotated words of one half fit in
- * this many bytes of shared memory, 0 .. 28,672 (values outside leave it as it is; the default
- * is the maximum; 0 always uses the separate rotation kernel). */
+ * this many bytes of shared memory, 0 .. 32,768 (values outside leave it as it is; the default
+ * is the maximum, of which launches other than block tables of one row each use at most 28,672;
+ * 0 always uses the separate rotation kernel). */
 EXL3_API void exl3_tune_gemv(int max_grid, int fuse_x_bytes);
 
 /* Without effect: they chose between variants of the prefill GEMM (accumulators per tile, pairs of

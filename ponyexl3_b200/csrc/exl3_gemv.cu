@@ -13,7 +13,7 @@ constexpr int kCtasPerSm = 2;           // virtual CTAs: the two halves of the o
 // (K = 2); several rows of a plain layer lose (4 rows, 5120 x 10240, K = 3: 25 -> 27 us).  32 KiB is what leaves
 // the four stages that K = 8 needs.
 constexpr int kFuseXBytes = 28 * 1024, kFuseXBytesTable = 32 * 1024;
-static int g_fuse_x_bytes = kFuseXBytes;
+static int g_fuse_x_bytes = kFuseXBytesTable;   // benchmark cap on both
 constexpr int kXsRowBytesHost = 544;
 
 static int g_gemv_max_grid = 0;          // 0: two virtual CTAs per SM
@@ -24,7 +24,7 @@ void gemv_set_tuning(int max_grid, int fuse_x_bytes)
 {
     g_gemv_max_grid = max_grid > 0 ? std::min(max_grid, kGemvMaxGrid) : 0;
     g_gemv_search_grid = max_grid == 0;      // a forced count is taken as it is
-    if (fuse_x_bytes >= 0 && fuse_x_bytes <= kFuseXBytes) g_fuse_x_bytes = fuse_x_bytes;
+    if (fuse_x_bytes >= 0 && fuse_x_bytes <= kFuseXBytesTable) g_fuse_x_bytes = fuse_x_bytes;
 }
 
 size_t gemv_partial_bytes(int rows)
@@ -91,7 +91,7 @@ GemvPlan gemv_plan(int64_t ncb, int nkb, int rows, bool table, size_t partial_by
     const int64_t range = (items + p.grid - 1) / p.grid;         // longest item range of a virtual CTA
     const int64_t slots = table ? range : std::min<int64_t>(range, nkb);
     p.n_slots = (int)std::min<int64_t>(slots, 1 << 20);
-    const int room = table && rows == 1 && g_fuse_x_bytes == kFuseXBytes ? kFuseXBytesTable : g_fuse_x_bytes;
+    const int room = std::min(g_fuse_x_bytes, table && rows == 1 ? kFuseXBytesTable : kFuseXBytes);
     p.x_fused = rows <= 8 && (slots * rows + 1) * kXsRowBytesHost <= room;
     return p;
 }

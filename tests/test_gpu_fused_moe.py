@@ -263,7 +263,7 @@ def test_decode_with_the_longest_ranges_rotates_in_the_kernel(cuda, k, tokens, w
     try:
         want = m(x, idx).clone()
     finally:
-        _lib.load().exl3_tune_gemv(0, 28 * 1024)
+        _lib.load().exl3_tune_gemv(0, 32 * 1024)
     assert torch.isfinite(got).all() and torch.equal(got, want)
 
 
