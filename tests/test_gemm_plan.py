@@ -70,6 +70,14 @@ def test_every_shape_that_fits_a_gpu_can_be_counted(emul):
             assert tiles_m * tok_ >= rows and (not split or tiles_m * (outf // 128) * (inf // 64) < 2**31)
 
 
+def test_the_gpu_tests_reach_every_form_of_the_kernel(emul):
+    from test_gpu_gemm import FORMS
+
+    for rows, inf, outf, k, cb, form in FORMS:
+        _, tiles_m, grid, _, is_wide = _plan(emul.emul_plan, rows, outf // 128, inf // 64, 148, *TOKENS[max(0, k - 4)], 384)
+        assert form == ("wide" if is_wide else "ahead" if tiles_m * (outf // 128) >= 2 * grid else "plain"), (rows, inf, outf, k)
+
+
 def test_a_plan_costs_less_than_a_launch(emul):
     """A new row count is planned anew; an exhaustive search of these takes milliseconds each."""
     shapes = [(40, 80), (136, 80), (40, 272), (32, 64), (11, 46)]

@@ -72,13 +72,14 @@ def test_fused_group_with_scales_other_than_signs(cuda, oracle, rows, dtype):
             assert rel_err(got.cpu().numpy(), want) <= 2.5e-4
 
 
-def test_block_tables_are_made_only_for_the_gemv(cuda, oracle):
+@pytest.mark.parametrize("k,cb", [(4, 0), (3, 1), (6, 2)])
+def test_block_tables_are_made_only_for_the_gemv(cuda, oracle, k, cb):
     """Up to 8 rows a group runs on the streamed GEMV over a block table; 9 and more take the GEMM, which has none,
     unless the scales are aligned for the GEMV (8 bytes) only."""
     from ponyexl3_b200 import EXL3Linear, EXL3MLPMonolith
     from ponyexl3_b200.fused import FusedEXL3Group
 
-    layers = _members(4, 256, [256, 256], seed=980)
+    layers = _members(k, 256, [256, 256], seed=980, cb=cb)
     grp = FusedEXL3Group(layers)
     mlp = EXL3MLPMonolith.from_fused_gate_up(grp, EXL3Linear(_members(4, 256, [128], seed=985)[0]))
     for rows in (9, 16, 17):
@@ -87,16 +88,16 @@ def test_block_tables_are_made_only_for_the_gemv(cuda, oracle):
         mlp(torch.from_numpy(x).cuda())
         assert not grp._tables
         for o, l in zip(outs, layers):
-            assert rel_err(o.cpu().numpy(), oracle.linear_forward(x, l.trellis, 4, 0, l.suh, l.svh, None)) <= 1e-3
+            assert rel_err(o.cpu().numpy(), oracle.linear_forward(x, l.trellis, k, cb, l.suh, l.svh, None)) <= 1e-3
     odd = torch.empty(grp._svh_cat.numel() + 8, dtype=torch.float16, device="cuda")
     odd[4:-4] = grp._svh_cat
     grp._svh_cat = odd[4:-4]
-    x = np.random.default_rng(1).standard_normal((12, 256)).astype(np.float16)
-    for o, l in zip(grp.forward_all(torch.from_numpy(x).cuda()), layers):
-        assert rel_err(o.cpu().numpy(), oracle.linear_forward(x, l.trellis, 4, 0, l.suh, l.svh, None)) <= 1e-3
-    assert list(grp._tables) == [12]
+    for rows in (9, 12, 16):
+        x = np.random.default_rng(rows).standard_normal((rows, 256)).astype(np.float16)
+        for o, l in zip(grp.forward_all(torch.from_numpy(x).cuda()), layers):
+            assert rel_err(o.cpu().numpy(), oracle.linear_forward(x, l.trellis, k, cb, l.suh, l.svh, None)) <= 1e-3
     mlp(torch.randn((8, 256), device="cuda").half())
-    assert list(grp._tables) == [12, 8]
+    assert list(grp._tables) == [9, 12, 16, 8]
 
 
 def test_fused_siblings_share_one_launch_and_refuse_bad_groups(cuda):

@@ -58,25 +58,11 @@ def test_gemm_all_k_all_codebooks(mod, oracle, k, cb):
 
 @pytest.mark.parametrize("k,cb,bias", [(4, 0, False), (2, 1, True), (5, 2, False), (8, 0, True), (1, 0, False)])
 @pytest.mark.parametrize("rows,inf,outf", [(1024, 256, 256), (1500, 512, 384), (2049, 128, 640)])
-def test_gemm_on_cta_pairs(mod, oracle, rows, inf, outf, k, cb, bias):
-    """The prefill GEMM on pairs of SMs (tcgen05.mma.cta_group::2, 512-row output tiles, each CTA
-    decoding half of the B tile; selected through the tuning hook): whole and ragged row tiles, a
-    last column tile of 128 columns, several tiles per pair, against the oracle; and the one-CTA
-    kernel gives the same bits."""
-    from ponyexl3_b200 import _lib
-
+def test_gemm_many_rows(mod, oracle, rows, inf, outf, k, cb, bias):
+    """Several tiles of tokens, whole and ragged, two to five column tiles, two to eight k-steps."""
     layer = _layer(mod, k, inf, outf, seed=7000 + rows + k, cb=cb, bias=bias)
     x = np.random.default_rng(rows + k).standard_normal((rows, inf)).astype(np.float16)
-    m = mod.EXL3Linear(layer)
-    xd = torch.from_numpy(x).cuda()
-    y_one = m(xd).clone()
-    _lib.load().exl3_tune_gemm_pairs(1)
-    try:
-        _check(mod, oracle, layer, x)
-        y_pair = m(xd).clone()
-    finally:
-        _lib.load().exl3_tune_gemm_pairs(0)
-    assert torch.equal(y_pair, y_one)
+    _check(mod, oracle, layer, x)
 
 
 @pytest.mark.parametrize("rows", [17, 128, 129, 256, 300, 513])
@@ -92,10 +78,10 @@ def test_gemm_ragged_row_counts(mod, oracle, rows):
     (250, 1024, 256, 8, 0),     # K = 8: fewer tokens per tile fit the activation ring, two token tiles
     (257, 1152, 128, 7, 1),     # one row more than a tile, a k-range that is no multiple of the ring
     (700, 128, 640, 1, 0),      # two k-steps per tile, whole tiles
-    (272, 512, 128, 4, 0),      # the smallest wide tile, halves of 144 and 128 tokens
-    (384, 640, 256, 3, 0),      # the largest wide tile
-    (336, 1024, 128, 8, 2),     # ... at K = 8
-    (400, 512, 256, 5, 1),      # two tiles, the second a few tokens short
+    (272, 512, 128, 4, 0),      # two token tiles of 144 and 128
+    (384, 640, 256, 3, 0),      # two of 192
+    (336, 1024, 128, 8, 2),     # two at K = 8
+    (400, 512, 256, 5, 1),      # two, the second a few tokens short
     (1537, 256, 384, 6, 0),     # a last tile of few tokens
 ])
 def test_gemm_tiles_shared_between_ctas(mod, oracle, rows, inf, outf, k, cb):
@@ -107,6 +93,34 @@ def test_gemm_tiles_shared_between_ctas(mod, oracle, rows, inf, outf, k, cb):
     first = m(xd)
     assert all(torch.equal(m(xd), first) for _ in range(3))      # whoever finishes a shared tile
     assert mod.ops.Workspace.get(torch.device("cuda"), 1, 128).status() == 0
+
+
+# Shapes of each form of the kernel (test_gemm_plan.py checks that the plan takes it): tiles of more than the
+# ordinary number of tokens, whose MMAs are two halves; two and more ordinary tiles per CTA; hardly more than one.
+FORMS = [
+    (257, 128, 9600, 4, 0, "wide"),     # the smallest wide tile, halves of 144 and 128 tokens
+    (384, 128, 9600, 4, 1, "wide"),     # the largest
+    (384, 128, 9600, 1, 2, "wide"),
+    (368, 128, 9600, 5, 0, "wide"),     # the largest at K = 5 to 8
+    (225, 128, 9600, 6, 1, "wide"),
+    (352, 128, 9600, 7, 2, "wide"),
+    (193, 128, 9600, 8, 0, "wide"),     # halves of 112 and 96, the second ragged
+    (336, 128, 9600, 8, 1, "wide"),
+    (760, 128, 6400, 4, 0, "wide"),     # two wide tiles of tokens
+    (4625, 128, 1024, 4, 0, "wide"),    # a last tile of one token: its second half is empty
+    (3552, 128, 1024, 8, 2, "wide"),    # a last tile of sixteen
+    (256, 256, 38400, 4, 0, "ahead"),   # two ordinary tiles per CTA and more
+    (17, 256, 38400, 3, 2, "ahead"),
+    (40, 256, 384, 4, 0, "plain"),
+    (300, 256, 384, 8, 1, "plain"),
+]
+
+
+@pytest.mark.parametrize("rows,inf,outf,k,cb,form", FORMS)
+def test_gemm_forms(mod, oracle, rows, inf, outf, k, cb, form):
+    layer = _layer(mod, k, inf, outf, seed=rows + k, cb=cb, bias=rows % 2 == 0)
+    x = np.random.default_rng(rows).standard_normal((rows, inf)).astype(np.float16)
+    _check(mod, oracle, layer, x)
 
 
 def test_gemm_of_many_tiles_per_cta_equals_small_calls(mod):
@@ -142,7 +156,7 @@ def test_gemm_matches_gemv_rows(mod):
     m = mod.EXL3Linear(layer)
     x = torch.from_numpy(np.random.default_rng(7).standard_normal((64, 1024)).astype(np.float16)).cuda()
     big = m(x)
-    small = torch.cat([m(x[i:i + 16]) for i in range(0, 64, 16)])
+    small = torch.cat([mod.ops.gemv(x[i:i + 16], m._trellis, 5, 0, m._suh, m._svh, m._bias) for i in range(0, 64, 16)])
     assert (big.float() - small.float()).norm() / small.float().norm() < 5e-4
 
 

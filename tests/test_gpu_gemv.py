@@ -40,15 +40,24 @@ def _layer(mod, k, inf, outf, seed, cb=0, bias=False):
 
 def _check(mod, oracle, layer, x, tol=REL_TOL):
     m = mod.EXL3Linear(layer)
-    y = m(torch.from_numpy(x).cuda()).cpu().numpy()
     want = oracle.linear_forward(x, layer.trellis, layer.k, layer.codebook_mode, layer.suh,
                                  layer.svh, layer.bias)
-    assert y.shape == want.shape and y.dtype == np.float16
-    assert np.isfinite(y.astype(np.float32)).all()
-    e = rel_err(y, want)
-    assert e <= tol, f"rel err {e}"
+    for y in _results(mod, m, torch.from_numpy(x).cuda()):
+        assert y.shape == want.shape and y.dtype == np.float16
+        assert np.isfinite(y.astype(np.float32)).all()
+        e = rel_err(y, want)
+        assert e <= tol, f"rel err {e}"
     assert mod.ops.Workspace.get(torch.device("cuda"), 1, 128).status() == 0
     return y, want
+
+
+def _results(mod, m, x):
+    """The module's output, and for 9 to 16 rows, which it hands to the GEMM, the streamed GEMV's: that serves them
+    too, through its entry points and where tensors are not aligned for the GEMM."""
+    ys = [m(x)]
+    if 8 < x.shape[0] <= 16:
+        ys.append(mod.ops.gemv(x, m._trellis, m.k, m.cb, m._suh, m._svh, m._bias, fast_accum=m.fast_accum))
+    return [y.cpu().numpy() for y in ys]
 
 
 def test_golden_forwards_from_the_reference(mod, golden):
@@ -114,10 +123,10 @@ def test_config2_full_shapes_other_k_and_codebooks(mod, oracle, k, cb):
     m = mod.EXL3Linear(layer)
     for rows in (1, 8, 16):
         x = np.random.default_rng(100 * k + rows).standard_normal((rows, inf)).astype(np.float16)
-        y = m(torch.from_numpy(x).cuda()).cpu().numpy()
         want = oracle.linear_forward(x, layer.trellis, k, cb, layer.suh, layer.svh, None)
-        e = rel_err(y, want)
-        assert e <= REL_TOL, f"K={k} cb={cb} rows={rows} {inf}x{outf}: rel err {e}"
+        for y in _results(mod, m, torch.from_numpy(x).cuda()):
+            e = rel_err(y, want)
+            assert e <= REL_TOL, f"K={k} cb={cb} rows={rows} {inf}x{outf}: rel err {e}"
     assert mod.ops.Workspace.get(torch.device("cuda"), 1, 128).status() == 0
 
 
@@ -149,9 +158,9 @@ def test_fast_accum_full_shapes(mod, oracle, shape, rows):
     m = mod.EXL3Linear(layer)
     m.fast_accum = True
     x = np.random.default_rng(rows).standard_normal((rows, shape[0])).astype(np.float16)
-    y = m(torch.from_numpy(x).cuda()).cpu().numpy()
     want = oracle.linear_forward(x, layer.trellis, 4, 0, layer.suh, layer.svh, None)
-    assert rel_err(y, want) <= REL_TOL
+    for y in _results(mod, m, torch.from_numpy(x).cuda()):
+        assert rel_err(y, want) <= REL_TOL
 
 
 def test_repeated_calls_are_deterministic_and_counters_rearm(mod, oracle):
@@ -220,14 +229,36 @@ def test_strided_activations_are_copied_only_where_they_must_be(mod):
 @pytest.mark.parametrize("rows", [1, 11])
 def test_fast_accum_mode_stays_within_tolerance(mod, oracle, k, cb, rows):
     """EXL3_FLAG_FAST_ACCUM adds the two fp16 halves of a codebook value inside the fp32
-    accumulation instead of rounding their sum first: same 1e-3 bound."""
+    accumulation instead of rounding their sum first: same 1e-3 bound, other bits where there are
+    two halves (MUL1 has one)."""
     layer = _layer(mod, k, 2048, 512, seed=300 + k + cb, cb=cb)
     m = mod.EXL3Linear(layer)
     m.fast_accum = True
     x = np.random.default_rng(rows).standard_normal((rows, 2048)).astype(np.float16)
-    y = m(torch.from_numpy(x).cuda()).cpu().numpy()
+    xd = torch.from_numpy(x).cuda()
     want = oracle.linear_forward(x, layer.trellis, k, cb, layer.suh, layer.svh, None)
-    assert rel_err(y, want) <= REL_TOL
+    ys = _results(mod, m, xd)
+    assert all(rel_err(y, want) <= REL_TOL for y in ys)
+    plain = mod.ops.gemv(xd, m._trellis, k, cb, m._suh, m._svh, None).cpu().numpy()
+    assert np.array_equal(ys[-1], plain) == (cb == 2)
+
+
+@pytest.mark.parametrize("rows", [9, 16])
+@pytest.mark.parametrize("k,cb", [(4, 0), (3, 1), (8, 2)])
+def test_outputs_aligned_for_the_gemv_only(mod, oracle, k, cb, rows):
+    """The GEMM stores 16 bytes at a time; 9 to 16 rows into an `out` that is aligned to 8 bytes, or whose rows are,
+    stay on the GEMV: the same bits as from it directly, and nothing outside the rows is written."""
+    layer = _layer(mod, k, 512, 256, seed=320 + k, cb=cb, bias=True)
+    m = mod.EXL3Linear(layer)
+    x = torch.from_numpy(np.random.default_rng(rows).standard_normal((rows, 512)).astype(np.float16)).cuda()
+    want = mod.ops.gemv(x, m._trellis, k, cb, m._suh, m._svh, m._bias)
+    assert rel_err(want.cpu().numpy(), oracle.linear_forward(x.cpu().numpy(), layer.trellis, k, cb, layer.suh, layer.svh, layer.bias)) <= REL_TOL
+    for width, first in ((264, 4), (260, 0), (260, 4)):
+        buf = torch.full((rows, width), 7.0, dtype=torch.float16, device="cuda")
+        out = buf[:, first:first + 256]
+        assert m(x, out=out).data_ptr() == out.data_ptr()
+        assert torch.equal(out, want)
+        assert (buf[:, :first] == 7).all() and (buf[:, first + 256:] == 7).all()
 
 
 def test_more_than_16_rows_go_to_the_gemm(mod, oracle):
