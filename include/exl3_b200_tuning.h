@@ -1,8 +1,8 @@
 /*
- * exl3_b200_tuning — benchmark knobs of libexl3b200.so, outside the stable ABI of exl3_b200.h.
+ * exl3_b200_tuning — a benchmark knob of libexl3b200.so, outside the stable ABI of exl3_b200.h.
  *
- * These set process-wide state that every later streamed-GEMV launch reads; they exist for
- * sweeps that look for the best launch shape and are never called on a product path.  They have
+ * It sets process-wide state that every later streamed-GEMV launch reads; it exists for
+ * sweeps that look for the best launch shape and is never called on a product path.  It has
  * no counterpart in the reference.
  */
 #ifndef EXL3_B200_TUNING_H
@@ -21,11 +21,6 @@ extern "C" {
  * is the maximum, of which launches other than block tables of one row each use at most 28,672;
  * 0 always uses the separate rotation kernel). */
 EXL3_API void exl3_tune_gemv(int max_grid, int fuse_x_bytes);
-
-/* Without effect: they chose between variants of the prefill GEMM (accumulators per tile, pairs of
- * SMs), which is one kernel for every shape now.  Kept for callers that link against them. */
-EXL3_API void exl3_tune_gemm(int one_acc_rows);
-EXL3_API void exl3_tune_gemm_pairs(int on);
 
 #ifdef __cplusplus
 }

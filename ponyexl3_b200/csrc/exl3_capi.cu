@@ -1,7 +1,7 @@
 // extern "C" surface of libexl3b200.so: argument validation on the host, then the
-// kernel launchers.  No allocation; the only process-wide state is per-device caches of
-// immutable facts (SM count, function attributes) and the two benchmark knobs of
-// exl3_b200_tuning.h, which no product path sets.
+// kernel launchers.  No allocation of device memory; the only state kept between calls is per-device
+// caches of immutable facts (SM count, function attributes), launch plans per shape and thread, and the
+// benchmark knob of exl3_b200_tuning.h, which no product path sets.
 #include <stdio.h>
 #include <string.h>
 
@@ -702,9 +702,5 @@ void exl3_tune_gemv(int max_grid, int fuse_x_bytes)
 {
     gemv_set_tuning(max_grid, fuse_x_bytes);
 }
-
-// The GEMM these two chose variants of is one kernel now; the names stay for callers that set them.
-void exl3_tune_gemm(int one_acc_rows) { (void)one_acc_rows; }
-void exl3_tune_gemm_pairs(int on) { (void)on; }
 
 }  // extern "C"
