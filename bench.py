@@ -39,8 +39,9 @@ L2_BYTES = 126 * 1024 * 1024
 # dram__bytes_read.sum + dram__bytes_write.sum over packed weight bytes, from the ncu capture of
 # the K=4 batch-1 GEMV 5120 -> 17408
 DRAM_TRAFFIC_RATIO = 1.0028
-# dram read + write per tile of the encoder workload (592 tiles, K=4), from its ncu capture
-ENCODE_DRAM_BYTES_PER_TILE = (97.128867e9 + 159.096134e9) / 592
+# dram read + write and warp instructions per tile of the encoder workload (592 tiles, K=4), from its ncu capture
+ENCODE_DRAM_BYTES_PER_TILE = (151.468288e6 + 1.188942e9) / 592
+ENCODE_WARP_INST_PER_TILE = 5634069510 / 592
 
 
 def packed_bytes(shape, k=K_BITS):
@@ -827,9 +828,9 @@ def run_gemm(args):
 def run_encode(args):
     """The converter's tile search: exact Viterbi encoding of 16x16 tiles of N(0,1) weights at K = 4,
     3INST (one whole wave of tiles per SM and then some).  A step = one exl3_encode_tiles call over
-    592 tiles; value = tiles per second.  The float64 costs of the 148 tiles in flight (1 MiB each)
-    exceed the L2, so the search streams them through DRAM every step: the roofline line reports that
-    traffic against the HBM peak.  The CPU baseline is the C oracle's search on all host cores."""
+    592 tiles; value = tiles per second.  The costs stay in shared memory and the kernel is bound by
+    instruction issue: the roofline line reports warp instructions against four per SM and clock.  The CPU
+    baseline is the C oracle's search on all host cores."""
     import numpy as np
     import torch
 
@@ -883,26 +884,26 @@ def run_encode(args):
         cpu = {"value": m / dt, "unit": "tiles/s", "cores": cores, "kind": "port",
                "sample": f"the first {m} of the {n} tiles through the C oracle's search (each checked against the GPU's "
                          f"states), {dt:.1f} s"}
-    # per pass and step: 65,536 float64 costs read and written, 4,096 back-pointer bytes
-    step_bytes = 2 * 65536 * 8 + (65536 >> k)
+    sm_hz = 1e6 * (clocks.get("sm_mhz") or 1965.0)
+    inst_peak = 4 * torch.cuda.get_device_properties(dev).multi_processor_count * sm_hz
+    inst_rate = ENCODE_WARP_INST_PER_TILE * n / (ms * 1e-3)
     emit({
         "metric": "exl3_trellis_encode_tiles_per_s", "value": n / (ms * 1e-3), "unit": "tiles/s", "n_gpus": 1,
         "steps": steps, "warmup": max(args.warmup, 3), "ms_per_step": ms, "higher_is_better": True,
         "scaling": "strong", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": {"workload": f"trellis encoder: exact Viterbi search of {n} tiles (16x16, N(0,1)), K={k}, 3INST, "
                                "up to 4 pinned passes", "tiles": n, "k": k, "codebook": "3INST",
-                   "l2": "the cost arrays of the 148 tiles in flight (148 MiB) exceed the 126 MB L2"},
-        "roofline": {"bound": "hbm", "achieved": n * 256 * step_bytes / (ms * 1e-3) / 1e9, "peak": 6551.4,
-                     "unit": "GB/s", "frac": n * 256 * step_bytes / (ms * 1e-3) / 1e9 / 6551.4,
+                   "l2": "the back-pointers of a step (1 MiB per tile and pass, 592 tiles) exceed the 126 MB L2"},
+        "roofline": {"bound": "issue", "achieved": inst_rate, "peak": inst_peak, "unit": "warp instructions/s",
+                     "frac": inst_rate / inst_peak,
                      "traffic": ENCODE_DRAM_BYTES_PER_TILE * n,
                      "traffic_unit": "bytes per launch (dram read + write)",
-                     "traffic_note": "ncu capture of this launch: 97.1 GB read + 159.1 GB written for 592 tiles; the "
-                                     "cost arrays of the 148 tiles in flight (148 MiB) do not fit the 126 MB L2, so "
-                                     "every step's costs go through DRAM",
-                     "peak_kind": "of measured",
+                     "traffic_note": "ncu capture of this launch: 0.15 GB read + 1.19 GB written for 592 tiles, the "
+                                     "back-pointers of all passes; costs never leave the SM",
+                     "peak_kind": "four warp instructions per SM and clock at the sampled clock",
                      "kernel": "exl3::encode_kernel",
-                     "note": "achieved counts ONE pass per tile (costs read and written, back-pointers written, "
-                             "per step); tiles take 1-5 passes, which is why the DRAM traffic is higher"},
+                     "note": "instructions per launch from the ncu capture (issue slots 68 % busy while an SM has a "
+                             "tile; SMs are active 74 % of the launch, because tiles take 1-5 passes)"},
         "cpu_baseline": cpu,
         "e2e": {"value": n / e2e_s, "unit": "tiles/s", "h2d_bytes_per_step": n * 256 * 4,
                 "d2h_bytes_per_step": n * 16 * k * 2, "ms_per_step": 1e3 * e2e_s,

@@ -107,8 +107,8 @@ __global__ void __launch_bounds__(256)
                     int early_trigger, int out_mode, int glu, int member_rows)
 {
     rotation_dependency(early_trigger);
-    // 32-bit block arithmetic (the launcher refuses more than 2^31 blocks): the 64-bit divisions
-    // that split a block index into (row, block of the row) cost more than the butterfly itself
+    // 32-bit block arithmetic (the launcher refuses more than 2^31 blocks): 64-bit divisions that split
+    // a block index into (row, block of the row) cost more than the butterfly itself
     const int lane = threadIdx.x & 31;
     const uint32_t nblk = (uint32_t)(n >> 7);
     const uint32_t total = (uint32_t)rows * nblk;

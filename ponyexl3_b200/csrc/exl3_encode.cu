@@ -34,7 +34,7 @@
 //
 // Bound: instruction issue, 8 to 9 warp instructions per 32 states and step, two thirds of the logic
 // pipe's slots busy (the keys, their minimum and the gap are three of them).  592 tiles of a 256 x 592
-// matrix, K = 4: 98.7 -> 10.0 ms (59,000 tiles/s) against a version that kept all 65,536 float64 costs
+// matrix, K = 4: 98.7 -> 9.6 ms (61,000 tiles/s) against a version that kept all 65,536 float64 costs
 // of a tile in L2 and moved 1 MiB per step through it; 148 tiles at K = 2 32 -> 13 ms, K = 8 77 -> 13 ms.
 
 #include <cuda_fp16.h>

@@ -8,10 +8,10 @@
 // the activations (operand B) and the packed words.  Decoding into a swizzled operand tile in shared
 // memory instead costs four scattered stores per tile and 96 bytes of operand reads per clock.
 //
-// Output tile: 128 columns (the width of the output rotation) x up to 256 tokens, k-step 64.
-//   warp 0      packed tiles: one 3-D TMA box of 8 x 4 tiles per k-step (ring w, eight stages)
-//   warp 1      activations: a 128B-swizzled TMA box per k-step (ring x)
-//   warp 2      issues the MMAs: A from tensor memory (eight 32-column stages), B from ring x
+// Output tile: 128 columns (the width of the output rotation) x up to 256 tokens, 384 in the wide form; k-step 64.
+//   warp 0      packed tiles: one 3-D TMA box of 8 x 4 tiles per k-step (ring w, eight stages; four in the wide form)
+//   warp 1      activations: one or more 128B-swizzled TMA boxes per k-step (ring x)
+//   warp 2      issues the MMAs: A from tensor memory (as many 32-column stages as ring w has), B from ring x
 //   warps 4-19  decode, four sets of four warps (a warp may touch the quarter of the tensor-memory
 //               lanes that its index names); the sets take the k-steps in turn
 // then the 16 decode warps finish the tile:
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                                                            : a.y + (int64_t)orow * a.y_row_stride + col0;
                         }
                     };
-                    // (behind the product; a table's launches are quicker with it after: 290 against 280 us as below)
+                    // (here it is done behind the product; SwitchGLU of 200 tokens: 280 us with it further down, 290 here)
                     if (!TABLE) address();
                     // The output scales are fetched behind the product: between the stores below, which might alias
                     // them, the loads would be made and waited for one after the other, and a prefetch into L1 does

@@ -74,9 +74,12 @@ inline int64_t ts_deal(int64_t tiles, int nks, int sms, bool room, int64_t enoug
 }
 
 // Tokens per tile: from as few tiles as wide ones allow to as few as ordinary ones need, whichever is cheapest at
-// 340 + 2.6 x tokens clocks a k-step, at least 610 (decoding bounds small tiles, the activations' way from L2
-// large ones).  Of many rows' counts the eight nearest to the ordinary tiles' are looked at, and the widest: further
-// ones differ by less than a tile's share.  Tiles of up to `room` tokens may be shared.
+// 340 + 2.6 x tokens clocks of 1965 MHz a k-step, at least 610.  That is fitted to the times of whole launches, the
+// lower clock under the power cap included: a wide k-step takes 790 clocks, but 8192 rows run at 1.28 GHz.  One line
+// serves all K: against every other number of tiles (K = 2, 4, 6, 8; 5120 x 5120, 5120 x 17408 and 17408 x 5120;
+// 200 to 4096 rows) the choice is within 3 % of the best, but for 5120 x 5120 at 300 to 1000 rows, where
+// one tile more would be 4 to 10 % faster.  Of many rows' counts the eight nearest to the ordinary tiles' are looked at, and the
+// widest: those between them differ by less than one tile in twenty.  Tiles of up to `room` tokens may be shared.
 inline TsPlan ts_plan(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room)
 {
     TsPlan best = {};

@@ -119,7 +119,7 @@ constexpr int kMoeMaxExperts = 1024;
 // Every CTA counts all pairs per expert (and those in front of its own share of the pairs) in shared memory,
 // scans the counts, and then places its share of the pairs and writes its share of the tables: the
 // counting is cheap to repeat, and no CTA waits for another.  One CTA alone took 133 us for 32,768 pairs
-// over 256 experts, nearly all of it the latency of its scattered stores; 32 take about 8.
+// over 256 experts, nearly all of it the latency of its scattered stores; 32 take 16.
 //
 // Row layout.  The held pairs are sorted by expert; expert e owns sorted positions
 // [seg, seg + cnt).  The rotated rows of the gate/up launch keep an expert's rows together —

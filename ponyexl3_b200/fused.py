@@ -6,8 +6,8 @@ out-tile axis, their ``suh`` rows stacked (each member rotates the input with it
 signs), their ``svh`` concatenated (member widths are multiples of 128, so an output
 rotation block never straddles two members), and ``forward_all`` returns one output per
 member.  On the B200 the group is one streamed GEMV over a block table (``exl3_gemv_blocks``) for up
-to 16 rows, and one rotation launch plus one tensor-core GEMM for all members (``exl3_gemm_members``)
-above that.
+to 8 rows (16 where the scales are not aligned to 16 bytes), and one rotation launch plus one tensor-core
+GEMM for all members (``exl3_gemm_members``) above that.
 """
 
 from __future__ import annotations

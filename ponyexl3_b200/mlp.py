@@ -6,11 +6,12 @@ gate/up sibling group and the down linear, with the same numerics as running the
 and the activation one after the other (``h`` is rounded to fp16 between the GLU and the down
 projection, as there).
 
-Up to 16 rows the call is two streamed-GEMV launches: the sibling group writes ``[gate | up]``,
+Up to 8 rows the call is two streamed-GEMV launches: the sibling group writes ``[gate | up]``,
 and the down projection reads that buffer as it is, applying ``act(gate) * up`` while it loads
 its activations (EXL3_FLAG_GLU_*), so there is no activation kernel and no ``h`` buffer in
 between.  More rows take the tensor-core GEMM the same way: rotation and GEMM for gate and up together,
-then a rotation that applies the GLU while it loads, and the GEMM of the down projection.
+then a rotation that applies the GLU while it loads, and the GEMM of the down projection.  (9 to 16 rows
+stay on the GEMV where scales or biases are not aligned to 16 bytes.)
 """
 
 from __future__ import annotations
