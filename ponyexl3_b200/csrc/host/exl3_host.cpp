@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <algorithm>
+#include <mutex>
 #include <string>
 
 #include "../../../include/exl3_b200.h"
@@ -61,6 +62,28 @@ void check(int rc, const char* what)
     Py_XDECREF(r);
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, what);
     throw PyError();
+}
+
+// Allocations, copies and launches run without the interpreter's lock, as PyTorch's own do: a launch waits while
+// the stream's queue is full, and what the GPU waits for may be another Python thread's work.
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+
+// One library call.  The calls of a device's threads go one at a time: the launches of one call use the workspace
+// one after the other, and another call's may not come in between on the same stream.
+std::mutex launching[kMaxDevices];
+template <typename F> void launch(int dev, const char* what, F&& call)
+{
+    if (dev < 0 || dev >= kMaxDevices) fail(PyExc_ValueError, "device index out of range");
+    int rc;
+    {
+        const NoGil unlocked;
+        const std::lock_guard<std::mutex> one(launching[dev]);
+        rc = call();
+    }
+    check(rc, what);
 }
 
 const at::Tensor& tensor(PyObject* o, const char* name)
@@ -112,8 +135,22 @@ Workspace workspace(int dev, size_t need)
     return workspaces[dev];
 }
 
-at::Tensor empty_half(at::IntArrayRef sizes, const at::Device& d) { return at::empty(sizes, at::TensorOptions().dtype(at::kHalf).device(d)); }
-at::Tensor empty_int(int64_t n, const at::Device& d) { return at::empty({n}, at::TensorOptions().dtype(at::kInt).device(d)); }
+at::Tensor empty_half(at::IntArrayRef sizes, const at::Device& d)
+{
+    const NoGil unlocked;
+    return at::empty(sizes, at::TensorOptions().dtype(at::kHalf).device(d));
+}
+at::Tensor empty_int(int64_t n, const at::Device& d)
+{
+    const NoGil unlocked;
+    return at::empty({n}, at::TensorOptions().dtype(at::kInt).device(d));
+}
+at::Tensor dense(const at::Tensor& t)
+{
+    if (t.is_contiguous()) return t;
+    const NoGil unlocked;
+    return t.contiguous();
+}
 
 struct Weights {
     const uint16_t* trellis;
@@ -136,7 +173,7 @@ Rows rows_of(const at::Tensor& x, int64_t features)
     Rows r;
     r.dtype = dtype_code(x);
     if (x.dim() == 2) {
-        r.t = x.stride(1) == 1 ? x : x.contiguous();
+        r.t = x.stride(1) == 1 ? x : dense(x);
         r.rows = x.size(0);
         r.stride = r.t.stride(0);
     } else {
@@ -145,6 +182,7 @@ Rows rows_of(const at::Tensor& x, int64_t features)
         if (x.is_contiguous()) {
             r.t = x;
         } else {                                       // a view where the leading dimensions fold into one, else a copy
+            const NoGil unlocked;
             r.t = x.reshape({r.rows, features});
             if (r.t.stride(1) != 1) r.t = r.t.contiguous();
             r.stride = r.t.stride(0);
@@ -159,16 +197,20 @@ void gemv(const Rows& x, int64_t rows, const Weights& w, int k, int cb, const ui
           const uint16_t* bias, uint16_t* y, int64_t y_stride, unsigned flags, int dev, cudaStream_t s)
 {
     const Workspace ws = workspace(dev, api.exl3_workspace_bytes(rows, 16 * w.t_in));
-    check(api.exl3_gemv(x.t.data_ptr(), x.dtype, (int)rows, x.stride, w.trellis, w.t_in, w.t_out, k, cb, suh, svh, bias, y,
-                        y_stride, ws.ptr, ws.bytes, flags, (exl3_stream_t)s), "exl3_gemv");
+    launch(dev, "exl3_gemv", [&] {
+        return api.exl3_gemv(x.t.data_ptr(), x.dtype, (int)rows, x.stride, w.trellis, w.t_in, w.t_out, k, cb, suh,
+                             svh, bias, y, y_stride, ws.ptr, ws.bytes, flags, (exl3_stream_t)s);
+    });
 }
 
 void gemm(const Rows& x, int64_t rows, const Weights& w, int k, int cb, const uint16_t* suh, const uint16_t* svh,
           const uint16_t* bias, uint16_t* y, int64_t y_stride, int dev, cudaStream_t s)
 {
     const Workspace ws = workspace(dev, api.exl3_gemm_workspace_bytes(rows, 16 * w.t_in));
-    check(api.exl3_gemm(x.t.data_ptr(), x.dtype, rows, x.stride, w.trellis, w.t_in, w.t_out, k, cb, suh, svh, bias, y,
-                        y_stride, ws.ptr, ws.bytes, 0, (exl3_stream_t)s), "exl3_gemm");
+    launch(dev, "exl3_gemm", [&] {
+        return api.exl3_gemm(x.t.data_ptr(), x.dtype, rows, x.stride, w.trellis, w.t_in, w.t_out, k, cb, suh, svh,
+                             bias, y, y_stride, ws.ptr, ws.bytes, 0, (exl3_stream_t)s);
+    });
 }
 
 // GEMV or GEMM.  Nine to sixteen rows take a second MMA and a rotation kernel in the GEMV, and the GEMM is as
@@ -260,22 +302,27 @@ void group_gemv(const Rows& x, int64_t rows, const Group& g, PyObject* table, Py
     const Owned t{PyObject_CallFunction(table, "LO", (long long)rows, device.p)};
     if (!t.p) throw PyError();
     if (!PyTuple_Check(t.p) || PyTuple_GET_SIZE(t.p) != 3) fail(PyExc_TypeError, "a table of three tensors is expected");
-    PyObject *row_src = PyTuple_GET_ITEM(t.p, 1), *suh_row = PyTuple_GET_ITEM(t.p, 2);
     const at::Tensor& b = tensor(PyTuple_GET_ITEM(t.p, 0), "blocks");
+    const int32_t* row_src = ptr_or_null<int32_t>(PyTuple_GET_ITEM(t.p, 1), "row_src");
+    const int32_t* suh_row = ptr_or_null<int32_t>(PyTuple_GET_ITEM(t.p, 2), "suh_row");
+    const int32_t* blocks = static_cast<const int32_t*>(b.data_ptr());
     const Workspace ws = workspace(dev, api.exl3_workspace_bytes(rows * g.members, 16 * g.w.t_in));
-    check(api.exl3_gemv_blocks(x.t.data_ptr(), x.dtype, x.stride, rows * g.members, ptr_or_null<int32_t>(row_src, "row_src"),
-                               g.suh, ptr_or_null<int32_t>(suh_row, "suh_row"), g.w.trellis, g.w.t_in, g.w.t_out, g.k, g.cb,
-                               static_cast<const int32_t*>(b.data_ptr()), b.size(0), (int)rows, g.svh, nullptr, u16(y),
-                               g.total, 0, ws.ptr, ws.bytes, flags, (exl3_stream_t)s), "exl3_gemv_blocks");
+    launch(dev, "exl3_gemv_blocks", [&] {
+        return api.exl3_gemv_blocks(x.t.data_ptr(), x.dtype, x.stride, rows * g.members, row_src, g.suh, suh_row,
+                                    g.w.trellis, g.w.t_in, g.w.t_out, g.k, g.cb, blocks, b.size(0), (int)rows, g.svh,
+                                    nullptr, u16(y), g.total, 0, ws.ptr, ws.bytes, flags, (exl3_stream_t)s);
+    });
 }
 // All members into the columns of one (rows, total) matrix (packed), or one matrix each.
 void group_gemm(const Rows& x, int64_t rows, const Group& g, const int64_t* widths, const uint64_t* y, const int64_t* strides,
                 int dev, cudaStream_t s)
 {
     const Workspace ws = workspace(dev, api.exl3_gemm_workspace_bytes(rows * g.members, 16 * g.w.t_in));
-    check(api.exl3_gemm_members(x.t.data_ptr(), x.dtype, rows, x.stride, g.w.trellis, g.w.t_in, g.w.t_out, g.k, g.cb, g.suh,
-                                g.svh, (int)g.members, widths, y, strides, ws.ptr, ws.bytes, 0, (exl3_stream_t)s),
-          "exl3_gemm_members");
+    launch(dev, "exl3_gemm_members", [&] {
+        return api.exl3_gemm_members(x.t.data_ptr(), x.dtype, rows, x.stride, g.w.trellis, g.w.t_in, g.w.t_out, g.k,
+                                     g.cb, g.suh, g.svh, (int)g.members, widths, y, strides, ws.ptr, ws.bytes, 0,
+                                     (exl3_stream_t)s);
+    });
 }
 
 // All members side by side in one (rows, total) matrix.
@@ -364,8 +411,10 @@ PyObject* mlp(PyObject* const* arg)
         const uint64_t base = reinterpret_cast<uint64_t>(gu.data_ptr()), ptrs[2] = {base, base + 2 * (uint64_t)half};
         group_gemm(r, r.rows, g, widths, ptrs, strides, dev, s);
         const Workspace ws = workspace(dev, api.exl3_gemm_workspace_bytes(r.rows, 16 * d.t_in));
-        check(api.exl3_gemm(gu.data_ptr(), EXL3_DT_F16, r.rows, g.total, d.trellis, d.t_in, d.t_out, dk, dcb, suh, svh, bias,
-                            u16(y), 16 * d.t_out, ws.ptr, ws.bytes, dflags, (exl3_stream_t)s), "exl3_gemm");
+        launch(dev, "exl3_gemm", [&] {
+            return api.exl3_gemm(gu.data_ptr(), EXL3_DT_F16, r.rows, g.total, d.trellis, d.t_in, d.t_out, dk, dcb,
+                                 suh, svh, bias, u16(y), 16 * d.t_out, ws.ptr, ws.bytes, dflags, (exl3_stream_t)s);
+        });
     }
     return THPVariable_Wrap(std::move(y));
 }
@@ -383,8 +432,11 @@ PyObject* switch_glu(PyObject* const* arg)
     const int64_t E = integer(arg[8]), H = integer(arg[9]), D = 16 * gu.t_in;
     const int k = (int)integer(arg[10]), cb = (int)integer(arg[11]);
     const unsigned glu = (unsigned)integer(arg[12]), flags = (unsigned)integer(arg[13]);
-    if (idx.scalar_type() != at::kInt && idx.scalar_type() != at::kLong) idx = idx.to(at::kLong);
-    if (!idx.is_contiguous()) idx = idx.contiguous();
+    if (idx.scalar_type() != at::kInt && idx.scalar_type() != at::kLong) {
+        const NoGil unlocked;
+        idx = idx.to(at::kLong);
+    }
+    idx = dense(idx);
     const int64_t R = idx.size(0), kk = idx.size(1), n = R * kk;
     const int bytes = idx.scalar_type() == at::kInt ? 4 : 8;
     const Rows r = rows_of(x, D);
@@ -402,16 +454,22 @@ PyObject* switch_glu(PyObject* const* arg)
         const at::Tensor tab = empty_int(4 * (n_gu + n_dn) + 5 * n, device);
         int32_t* blocks_gu = static_cast<int32_t*>(tab.data_ptr());
         int32_t *blocks_dn = blocks_gu + 4 * n_gu, *row_src = blocks_dn + 4 * n_dn, *suh_row = row_src + 2 * n, *sel = suh_row + 2 * n;
-        check(api.exl3_moe_decode_tables(idx.data_ptr(), bytes, (int)n, (int)kk, (int)E, D, H, blocks_gu, row_src, suh_row,
-                                         blocks_dn, sel, flags, es), "exl3_moe_decode_tables");
+        launch(dev, "exl3_moe_decode_tables", [&] {
+            return api.exl3_moe_decode_tables(idx.data_ptr(), bytes, (int)n, (int)kk, (int)E, D, H, blocks_gu,
+                                              row_src, suh_row, blocks_dn, sel, flags, es);
+        });
         Workspace ws = workspace(dev, api.exl3_workspace_bytes(2 * n, D));
-        check(api.exl3_gemv_blocks(r.t.data_ptr(), r.dtype, r.stride, 2 * n, row_src, gu_suh, suh_row, gu.trellis, gu.t_in,
-                                   gu.t_out, k, cb, blocks_gu, n_gu, 1, gu_svh, nullptr, u16(ygu), 2 * H, 0, ws.ptr, ws.bytes,
-                                   flags, es), "exl3_gemv_blocks");
+        launch(dev, "exl3_gemv_blocks", [&] {
+            return api.exl3_gemv_blocks(r.t.data_ptr(), r.dtype, r.stride, 2 * n, row_src, gu_suh, suh_row,
+                                        gu.trellis, gu.t_in, gu.t_out, k, cb, blocks_gu, n_gu, 1, gu_svh, nullptr,
+                                        u16(ygu), 2 * H, 0, ws.ptr, ws.bytes, flags, es);
+        });
         ws = workspace(dev, api.exl3_workspace_bytes(n, H));
-        check(api.exl3_gemv_blocks(ygu.data_ptr(), EXL3_DT_F16, 2 * H, n, nullptr, dn_suh, sel, dn.trellis, dn.t_in, dn.t_out,
-                                   k, cb, blocks_dn, n_dn, 1, dn_svh, nullptr, u16(y), D, 0, ws.ptr, ws.bytes, flags | glu, es),
-              "exl3_gemv_blocks");
+        launch(dev, "exl3_gemv_blocks", [&] {
+            return api.exl3_gemv_blocks(ygu.data_ptr(), EXL3_DT_F16, 2 * H, n, nullptr, dn_suh, sel, dn.trellis,
+                                        dn.t_in, dn.t_out, k, cb, blocks_dn, n_dn, 1, dn_svh, nullptr, u16(y), D, 0,
+                                        ws.ptr, ws.bytes, flags | glu, es);
+        });
     } else {
         // tables, rotation, gate|up, rotation with the GLU on load, down stored back into pair order
         const int64_t slots = n / 256 + E, ct_h = (H + 255) / 256, ct_d = (D + 255) / 256;
@@ -420,16 +478,23 @@ PyObject* switch_glu(PyObject* const* arg)
         int32_t* tiles_gu = static_cast<int32_t*>(tab.data_ptr());
         int32_t *tiles_dn = tiles_gu + 8 * n_gu, *order = tiles_dn + 8 * n_dn, *row_src = order + n, *suh_gu = row_src + 2 * n,
                 *suh_dn = suh_gu + 2 * n;
-        check(api.exl3_moe_prefill_tables(idx.data_ptr(), bytes, (int)n, (int)kk, (int)E, D, H, order, row_src, suh_gu, suh_dn,
-                                          tiles_gu, tiles_dn, 0, es), "exl3_moe_prefill_tables");
+        launch(dev, "exl3_moe_prefill_tables", [&] {
+            return api.exl3_moe_prefill_tables(idx.data_ptr(), bytes, (int)n, (int)kk, (int)E, D, H, order, row_src,
+                                               suh_gu, suh_dn, tiles_gu, tiles_dn, 0, es);
+        });
         const unsigned hint = (unsigned)std::min<int64_t>(n / E, 0xFFFF) << 16;      // rows of an expert
         Workspace ws = workspace(dev, api.exl3_gemm_workspace_bytes(2 * n, D));
-        check(api.exl3_gemm_tiles(r.t.data_ptr(), r.dtype, r.stride, 2 * n, row_src, gu_suh, suh_gu, gu.trellis, gu.t_in,
-                                  gu.t_out, k, cb, tiles_gu, n_gu, gu_svh, u16(ygu), 2 * H, nullptr, ws.ptr, ws.bytes, hint, es),
-              "exl3_gemm_tiles");
+        launch(dev, "exl3_gemm_tiles", [&] {
+            return api.exl3_gemm_tiles(r.t.data_ptr(), r.dtype, r.stride, 2 * n, row_src, gu_suh, suh_gu,
+                                       gu.trellis, gu.t_in, gu.t_out, k, cb, tiles_gu, n_gu, gu_svh, u16(ygu), 2 *
+                                       H, nullptr, ws.ptr, ws.bytes, hint, es);
+        });
         ws = workspace(dev, api.exl3_gemm_workspace_bytes(n, H));
-        check(api.exl3_gemm_tiles(ygu.data_ptr(), EXL3_DT_F16, 2 * H, n, nullptr, dn_suh, suh_dn, dn.trellis, dn.t_in, dn.t_out,
-                                  k, cb, tiles_dn, n_dn, dn_svh, u16(y), D, order, ws.ptr, ws.bytes, glu | hint, es), "exl3_gemm_tiles");
+        launch(dev, "exl3_gemm_tiles", [&] {
+            return api.exl3_gemm_tiles(ygu.data_ptr(), EXL3_DT_F16, 2 * H, n, nullptr, dn_suh, suh_dn, dn.trellis,
+                                       dn.t_in, dn.t_out, k, cb, tiles_dn, n_dn, dn_svh, u16(y), D, order, ws.ptr,
+                                       ws.bytes, glu | hint, es);
+        });
     }
     return THPVariable_Wrap(std::move(y));
 }

@@ -267,6 +267,91 @@ def test_more_than_16_rows_go_to_the_gemm(mod, oracle):
     _check(mod, oracle, layer, x)
 
 
+def test_a_full_queue_does_not_stop_other_threads(mod):
+    """A launch waits while the stream's queue is full (some thousand launches behind a kernel of half a second
+    here); the interpreter goes on with other threads meanwhile."""
+    import threading
+    import time
+
+    m = mod.EXL3Linear(_layer(mod, 4, 128, 128, seed=5))
+    x = torch.randn((1, 128), device="cuda").half()
+    want = m(x).clone()
+    torch.cuda.synchronize()
+    done, longest = [], 0.0
+
+    def enqueue():
+        torch.cuda._sleep(1_000_000_000)
+        done.append([m(x) for _ in range(4000)][-1])
+
+    worker = threading.Thread(target=enqueue)
+    start = last = time.perf_counter()
+    worker.start()
+    while worker.is_alive():
+        time.sleep(0.001)
+        now = time.perf_counter()
+        longest, last = max(longest, now - last), now
+    torch.cuda.synchronize()
+    assert torch.equal(done[0], want)
+    assert last - start > 0.3, "the queue was never full"
+    assert longest < 0.15
+
+
+def test_calls_of_several_threads_keep_their_workspace_apart(mod):
+    """Threads that call on one stream share the device's workspace: the rotation and the GEMM of one call are not
+    separated by another's."""
+    import threading
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    one = lambda n: torch.ones(n, device="cuda").half()
+    mods = [mod.EXL3Linear.from_device_tensors(
+        trellis=torch.randint(-32768, 32768, (64, 16, 64), dtype=torch.int16, device="cuda", generator=g), k=4, cb=0,
+        suh=one(1024), svh=one(256)) for _ in range(4)]
+    xs = [torch.randn((40, 1024), device="cuda", generator=g).half() for _ in range(4)]
+    want = [m(x).clone() for m, x in zip(mods, xs)]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        for _ in range(300):
+            if not torch.equal(mods[i](xs[i]), want[i]):
+                bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+@pytest.mark.parametrize("rows", [1, 12, 40])
+def test_calls_behind_a_fork_in_a_captured_graph(mod, oracle, rows):
+    """A call whose input comes from another stream, captured: its kernels are programmatic dependents of what is in
+    front of them, here the join of two streams, and read nothing before both are complete."""
+    layer = _layer(mod, 4, 512, 384, seed=90)
+    m = mod.EXL3Linear(layer)
+    src = torch.zeros((rows, 512), device="cuda").half()
+    m(src)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        main = torch.cuda.current_stream()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(500_000)                     # the input is late
+            x = src * 1
+        y0 = m(src)                                        # meanwhile, a call on the main stream
+        main.wait_stream(side)
+        y = m(x)
+        y2 = m(x)
+    for seed in range(3):
+        src.copy_(torch.from_numpy(np.random.default_rng(seed).standard_normal((rows, 512)).astype(np.float16)))
+        graph.replay()
+        torch.cuda.synchronize()
+        want = oracle.linear_forward(src.cpu().numpy(), layer.trellis, 4, 0, layer.suh, layer.svh, None)
+        assert rel_err(y.cpu().numpy(), want) <= REL_TOL and torch.equal(y, y0) and torch.equal(y, y2)
+
+
 @pytest.mark.parametrize("rows", [1, 12, 40])
 def test_programmatic_launch_chain(mod, oracle, rows):
     """Back-to-back layers launched with programmatic stream serialisation give the same
