@@ -98,6 +98,10 @@ class FusedEXL3Group(torch.nn.Module):
         g.pdl = False
         return g
 
+    def __setstate__(self, state: dict) -> None:
+        super().__setstate__(state)
+        self._set_spans()               # groups pickled by earlier versions do not hold them
+
     def _set_spans(self) -> None:
         ends = [int(v) for v in self._offsets]
         self._spans, self._total = list(zip(ends[:-1], ends[1:])), ends[-1]

@@ -134,3 +134,18 @@ def test_host_extension_of_another_pytorch_is_not_loaded(monkeypatch):
     monkeypatch.setattr(_lib, "_host", None)
     with pytest.raises(RuntimeError, match="ponyexl3_b200.build"):
         _lib.host()
+
+
+def test_groups_pickled_by_earlier_versions_load():
+    """What a group keeps beside its tensors is computed again where a pickle does not hold it."""
+    import torch
+
+    from ponyexl3_b200 import FusedEXL3Group
+
+    grp = FusedEXL3Group.from_device_tensors(
+        trellis=torch.zeros((8, 24, 64), dtype=torch.int16), k=4, cb=0, suh_stack=torch.ones((2, 128)).half(),
+        svh_cat=torch.ones(384).half(), out_features=[256, 128])
+    state = {k: v for k, v in grp.__dict__.items() if k not in ("_spans", "_total")}
+    old = FusedEXL3Group.__new__(FusedEXL3Group)
+    old.__setstate__(state)
+    assert old._spans == [(0, 256), (256, 384)] and old._native()[-1] == 384
