@@ -410,9 +410,9 @@ EXL3_API int exl3_moe_prefill_tables_range(const void* indices, int index_bytes,
  * matrix to it); states: (n_tiles, 256) the 16-bit window of every codeword; packed (may be
  * NULL): (n_tiles, 16K) the packed tiles as stored on disk (pack_trellis_tile,
  * ponyexl3/ref/trellis.py:12-50).  max_pins: pinned passes after the free one (the reference's
- * default is 4).  The workspace holds the back-pointers (at K = 1 also the costs) of the tiles in
- * flight, 8.5 MiB each, and a tile counter: exl3_encode_workspace_bytes(n_tiles) is enough for one tile per SM; a smaller
- * workspace (at least one slot) only lowers the number of tiles in flight. */
+ * default is 4).  The workspace holds the back-pointers (and, at K = 1 and for weights beyond 1e13, the
+ * costs) of the tiles in flight, 8.5 MiB each, and two tile counters: exl3_encode_workspace_bytes(n_tiles)
+ * is enough for one tile per SM; a smaller workspace (at least one slot) only lowers the number of tiles in flight. */
 EXL3_API size_t exl3_encode_workspace_bytes(int64_t n_tiles);
 EXL3_API int exl3_encode_tiles(const float* w, int64_t n_tiles, int k, int cb, int max_pins, uint16_t* states,
                                uint16_t* packed, void* workspace, size_t workspace_bytes, exl3_stream_t stream);

@@ -49,10 +49,14 @@ namespace exl3 {
 
 constexpr int kEncStates = 65536;
 constexpr int kEncThreads = 512;
-constexpr size_t kEncCounterBytes = 256;                 // tile counter in front of the slots
+constexpr size_t kEncCounterBytes = 256;                 // two tile counters in front of the slots
 constexpr size_t kEncBackBytes = 256 * (size_t)(kEncStates / 2);
-constexpr size_t kEncCostBytes = 2 * (size_t)(kEncStates / 2) * sizeof(double);   // K = 1 only
+constexpr size_t kEncCostBytes = 2 * (size_t)(kEncStates / 2) * sizeof(double);   // K = 1, and odd tiles
 constexpr size_t kEncSlotBytes = kEncBackBytes + kEncCostBytes;
+
+// With weights up to here a path costs less than 256 x 1e26, far from the 1e30 of states that the pinned one cannot
+// reach, which a cost can therefore be told from, and every cost is a number.
+constexpr float kEncLargest = 1e13f;
 
 struct EncodeArgs {
     const float* w;        // (n_tiles, 256) codeword order
@@ -60,7 +64,7 @@ struct EncodeArgs {
     int max_pins;
     uint16_t* states;      // (n_tiles, 256) the 16-bit window of every codeword
     uint32_t* packed;      // NULL or (n_tiles, 8K) packed tile words
-    unsigned* counter;     // tiles handed out so far
+    unsigned* counter;     // tiles handed out so far by this kernel
     uint8_t* slots;        // gridDim.x workspace slots
 };
 
@@ -72,6 +76,7 @@ struct EncodeShared {
     uint32_t words[64];
     unsigned smin[3];
     int fin, pin, done;
+    int odd;                           // a weight of the tile is not finite or beyond kEncLargest
     unsigned tile;
 };
 
@@ -178,20 +183,19 @@ __device__ __forceinline__ int64_t next_tile(EncodeShared& sh, const EncodeArgs&
     if (tid == 0) sh.tile = atomicAdd(a.counter, 1u);
     __syncthreads();
     const int64_t tile = sh.tile;
+    bool odd = false;
     if (tile < a.n_tiles) {
-        if (tid < 256) sh.w[tid] = a.w[tile * 256 + tid];
+        if (tid < 256) {
+            const float w = a.w[tile * 256 + tid];
+            sh.w[tid] = w;
+            odd = !(fabsf(w) < kEncLargest);
+        }
         if (tid == 0) { sh.pin = -1; sh.done = 0; }
     }
+    const int any_odd = __syncthreads_or(odd);
+    if (tid == 0) sh.odd = any_odd;
     __syncthreads();
     return tile;
-}
-
-// The larger one; NaN if either is (a NaN weight makes all costs NaN, and then index 0 wins everywhere).
-__device__ __forceinline__ float fmax_nan(float a, float b)
-{
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
 }
 
 // (k & ~(J - 1)) | j as one three-input operation (written in C, ptxas made two of it).
@@ -268,6 +272,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
     for (;;) {
         const int64_t tile = next_tile(sh, a);
         if (tile >= a.n_tiles) return;
+        if (sh.odd) continue;                            // encode_odd_kernel's
         for (int pass = 0; pass <= a.max_pins; pass++) {
             const int pin = sh.pin;
             for (int b = tid; b < NB; b += kEncThreads) {
@@ -281,7 +286,6 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
             if (tid == 0) sh.smin[1] = 0x7F800000u;
             __syncthreads();
             double off = 0.0;                            // lower bound of every m_t[b]
-            bool tame = true;                            // all weights so far are small against the 1e30 of the unreachable
             for (int t = 0; t < 255; t++) {
                 const int cur = E::kInPlace ? 0 : (t & 1), nxt = E::kInPlace ? 0 : cur ^ 1;
                 const int rot = E::kInPlace ? (K * t) % LB : 0;
@@ -290,7 +294,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                 double* mdn = md0 + nxt * NB;
                 float* mfn = mf0 + nxt * NB;
                 const float w = sh.w[t];
-                tame = tame && fabsf(w) < 1e6f;
+                const bool tame = fabsf(w) < 1e6f;
                 // costs in mfc are relative to the bound of the step before
                 const float near = (float)off * 9.3e-10f;   // 2^-30: closer than this, float64 roundings decide
                 if (t > 0) {
@@ -387,7 +391,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                             const uint32_t b = (h << K) | (l0 + i);
                             // in place, base b' = (h << K) | l of the next step takes the address of h | l << (LB - K)
                             const uint32_t at = E::kInPlace ? slot(h | (i << (LB - K)), rot) : slot(b, 0);
-                            const float rel = fmax_nan((float)(val[i] - off), 0.f);
+                            const float rel = fmaxf((float)(val[i] - off), 0.f);
                             mdn[at] = val[i];
                             mfn[at] = rel;
                             low_new = min(low_new, __float_as_uint(rel));
@@ -422,6 +426,65 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                 }
                 final_state(sh, bc, bs, kEncThreads / 32);
             }
+            if (tid < 32) walk_back<K>(sh, back, pass);
+            __syncthreads();
+            if (sh.done) break;
+        }
+        store_tile<K>(sh, a, tile);
+    }
+}
+
+// The tiles that encode_kernel leaves (K >= 2), with weights that are no numbers or beyond kEncLargest: in float64
+// throughout, the costs in the slot (L2).  Not worth more: such a tile has no good path, only a defined one.  In
+// encode_kernel, carrying NaN and telling such costs from the 1e30 took 1 % (K = 4) to 3 % (K = 6) from every tile; as a
+// launch behind it, looking all tiles through takes 5 us of 9 ms.
+template <int K, int CB> __global__ void __launch_bounds__(kEncThreads, 1) encode_odd_kernel(const EncodeArgs a)
+{
+    constexpr int NB = kEncStates >> K, J = 1 << K, LB = 16 - K;
+    __shared__ EncodeShared sh;
+    const int tid = threadIdx.x;
+    uint8_t* back = a.slots + (size_t)blockIdx.x * kEncSlotBytes;
+    double* cost0 = reinterpret_cast<double*>(back + kEncBackBytes);
+    double* cost1 = cost0 + NB;
+    for (;;) {
+        const int64_t tile = next_tile(sh, a);
+        if (tile >= a.n_tiles) return;
+        if (!sh.odd) continue;
+        for (int pass = 0; pass <= a.max_pins; pass++) {
+            const int pin = sh.pin;
+            for (int b = tid; b < NB; b += kEncThreads) {
+                const bool home = pin >= 0 && b == (pin & (NB - 1));
+                __stcg(cost0 + b, pin < 0 || home ? 0.0 : 1e30);
+                __stcg(back + b, (uint8_t)(home ? pin >> LB : 0));
+            }
+            __syncthreads();
+            double* cur = cost0;
+            double* nxt = cost1;
+            for (int t = 0; t < 255; t++) {
+                const double wd = (double)sh.w[t];
+                for (int b = tid; b < NB; b += kEncThreads) {
+                    double best = 0.0;
+                    int bj = 0;
+#pragma unroll 1
+                    for (int j = 0; j < J; j++) {
+                        const double v = __dadd_rn(__ldcg(cur + ((b >> K) | (j << (LB - K)))),
+                                                   sq_err((double)codebook_f32<CB>((uint32_t)(b | (j << LB))), wd));
+                        if (j == 0 || v < best) { best = v; bj = j; }
+                    }
+                    __stcg(nxt + b, best);
+                    __stcg(back + (size_t)(t + 1) * NB + b, (uint8_t)bj);
+                }
+                __syncthreads();
+                double* tmp = cur; cur = nxt; nxt = tmp;
+            }
+            const double wd = (double)sh.w[255];
+            double bc = 0.0;
+            int bs = -1;
+            for (int s = tid; s < kEncStates; s += kEncThreads) {
+                const double v = __dadd_rn(__ldcg(cur + (s >> K)), sq_err((double)codebook_f32<CB>((uint32_t)s), wd));
+                if (bs < 0 || v < bc) { bc = v; bs = s; }
+            }
+            final_state(sh, bc, bs, kEncThreads / 32);
             if (tid < 32) walk_back<K>(sh, back, pass);
             __syncthreads();
             if (sh.done) break;
@@ -510,6 +573,11 @@ template <int K, int CB> static int launch_encode(const EncodeArgs& a, unsigned 
             attr_set[dev] = true;
         }
         encode_kernel<K, CB><<<slots, kEncThreads, EncodeSplit<K>::kSmem, s>>>(a);
+        const int rc = check_launch();
+        if (rc) return rc;
+        EncodeArgs odd = a;
+        odd.counter = a.counter + 1;
+        encode_odd_kernel<K, CB><<<slots, kEncThreads, 0, s>>>(odd);
         return check_launch();
     }
 }
@@ -563,7 +631,7 @@ extern "C" int exl3_encode_tiles(const float* w, int64_t n_tiles, int k, int cb,
         a.n_tiles = std::min<int64_t>(kMost, n_tiles - t0);
         a.states = states + t0 * 256;
         a.packed = packed ? reinterpret_cast<uint32_t*>(packed) + t0 * 8 * k : nullptr;
-        int rc = note_cuda(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), s));
+        int rc = note_cuda(cudaMemsetAsync(a.counter, 0, 2 * sizeof(unsigned), s));
         if (rc) return rc;
         switch (k) {
             case 1: rc = launch_encode_k<1>(a, cb, (unsigned)slots, s); break;

@@ -73,7 +73,7 @@ def test_encoder_of_weights_without_measure(ops, oracle, k, cb):
     """Squared errors of the size of the 1e30 that marks unreachable states and beyond the range of fp32, infinite
     weights and NaN, each at the start, in the middle and at the end of a tile: the states of the oracle's search."""
     rng = np.random.default_rng(60 + k)
-    w = rng.standard_normal((8, 256)).astype(np.float32)
+    w = rng.standard_normal((11, 256)).astype(np.float32)
     w[0, 5] = 1e16
     w[1, 100] = np.nan
     w[2, 30] = np.inf
@@ -82,8 +82,10 @@ def test_encoder_of_weights_without_measure(ops, oracle, k, cb):
     w[5, [0, 255]] = 4e17, 1e16
     w[6, [0, 128]] = np.nan, -np.inf
     w[7, 255] = np.nan
-    states, _ = ops.quantize_tiles(torch.from_numpy(w).cuda(), k, cb)
-    for t in range(8):
+    w[9, ::5] = 9.9e12                                    # the largest weights of the ordinary search, one more beyond
+    w[10, 17] = -1.1e13
+    states, _ = ops.quantize_tiles(torch.from_numpy(w).cuda(), k, cb, max_tiles_in_flight=3)
+    for t in range(11):
         want, _ = oracle.quantize_tile(w[t], k, cb)
         assert (_u16(states)[t] == want).all(), f"tile {t}"
 
