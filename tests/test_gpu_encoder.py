@@ -90,6 +90,23 @@ def test_encoder_of_weights_without_measure(ops, oracle, k, cb):
         assert (_u16(states)[t] == want).all(), f"tile {t}"
 
 
+@pytest.mark.parametrize("k,cb,max_pins", [(1, 2, 4), (2, 0, 4), (2, 2, 1), (3, 1, 0), (4, 0, 0), (4, 2, 4), (5, 0, 64), (6, 2, 0),
+                                           (7, 2, 4), (8, 2, 4), (8, 0, 0)])
+def test_encoder_free_and_pinned_paths(ops, oracle, k, cb, max_pins):
+    """The searches that one pass over a tile answers, and the tiles it leaves to the search from the start: MUL1's thousand
+    values tie at every third tile of K = 8, small multiples of one number tie nearly everywhere; no pinned pass, one, many."""
+    rng = np.random.default_rng(200 + 10 * k + cb)
+    w = rng.standard_normal((10, 256)).astype(np.float32)
+    w[3] = np.round(w[3] * 4) / 4
+    w[4, 64:] = 0.25
+    w[5, :200] = 0.0
+    states, packed = ops.quantize_tiles(torch.from_numpy(w).cuda(), k, cb, max_pins=max_pins, max_tiles_in_flight=7)
+    for t in range(10):
+        want, _ = oracle.quantize_tile(w[t], k, cb, max_pins)
+        assert (_u16(states)[t] == want).all(), f"tile {t}"
+        assert (_u16(packed)[t] == oracle.pack_trellis_tile((want & ((1 << k) - 1)).astype(np.uint16), k)).all()
+
+
 def test_quantised_matrix_decodes_to_the_chosen_codebook_values(ops, oracle):
     k, cb = 3, 0
     rng = np.random.default_rng(3)
