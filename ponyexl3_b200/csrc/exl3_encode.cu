@@ -40,10 +40,11 @@
 //     chain of L2 round trips it took 90 K); a pinned path is only walked to where it meets the one before.
 // Tiles are handed out by a counter.
 //
-// Bound: instruction issue (57 % of the slots, the logic pipe 55 %), 8.5 warp instructions per 32 states and step (the keys,
-// their minimum and the gap are three of them).  592 tiles of a 256 x 592 matrix, K = 4: 10.0 -> 4.2 ms against
-// the search from the start; 518 tiles at K = 2, 3, 5, 6, 7, 8 (3INST): 29.0, 12.5, 7.0, 7.2, 7.9, 10.2 -> 10.2, 5.3, 3.5,
-// 3.3, 3.5, 6.1 ms (K = 8: with one tile left to encode_kernel).
+// Bound: instruction issue (some 60 % of the slots, the logic pipe as busy), 8 warp instructions per 32 states and step (the
+// keys, their minimum and the gap are three of them).  592 tiles of a 256 x 592 matrix, K = 4: 10.0 -> 3.8 ms
+// against the search from the start; at K = 2, 3, 5, 6, 7, 8 (3INST) 9.4, 4.9, 3.4, 3.2, 3.4, 6.4 ms (518 tiles of the
+// search from the start: 29.0, 12.5, 7.0, 7.2, 7.9, 10.2; K = 8 leaves one tile to encode_kernel).  1024 threads of half the
+// registers, for more warps to choose from, took 4.3 ms at K = 4.
 
 #include <cuda_fp16.h>
 
@@ -204,7 +205,7 @@ template <int MARK = -1> __device__ __forceinline__ int64_t next_tile(EncodeShar
         unsigned t;
         do {
             t = atomicAdd(a.counter, 1u);
-        } while (MARK >= 0 && t < a.n_tiles && !(a.states[(int64_t)t * 256] == 0xFFFF && a.states[(int64_t)t * 256 + 1] == MARK));
+        } while (MARK >= 0 && t < a.n_tiles && !(a.states[(int64_t)t * 256] == 0xFFFF && (int)a.states[(int64_t)t * 256 + 1] == MARK));
         sh.tile = t;
         sh.pin = -1;
         sh.done = 0;
@@ -227,36 +228,40 @@ template <int J> __device__ __forceinline__ uint32_t key_with_index(uint32_t k, 
 // How the 65,536 (b, n) pairs of a step of the backward search are dealt to the threads.  The bases b with the same
 // h = b mod 2^(16-2K) have the same successors, (h << K) | n.
 template <int K> struct SearchSplit {
+    static constexpr int NT = kEncThreads;               // threads
+    static constexpr int kPairs = kEncStates / NT;       // pairs per thread
     static constexpr int NB = kEncStates >> K;           // bases
     static constexpr int J = 1 << K;
     static constexpr int HB = 16 - 2 * K;                // bits of h
     static constexpr int NH = 1 << HB;                   // groups
-    static constexpr int NG = NH < kEncThreads ? NH : kEncThreads;
+    static constexpr int JT = J < kPairs ? J : kPairs;   // n values per thread and base
+    static constexpr int TB = J / JT;                    // threads of a base: more than one for the largest K
+    static constexpr int NG = NH < NT ? NH : NT;
     static constexpr int G = NH / NG;                    // groups per thread
-    static constexpr int JT = J < 128 ? J : 128;         // n values per thread and base (K = 8: two threads a base)
-    static constexpr int L = 128 / JT / G;               // bases per thread and group: (l0 + T i) << HB | h, i < L
+    static constexpr int L = kPairs / JT / G;            // bases per thread and group: (l0 + T i) << HB | h, i < L
     static constexpr int T = J / L;
     static constexpr int JC = JT < 16 ? JT : 16;         // n values per turn
+    static constexpr int BL = L < 4 ? L : 4;             // bases whose costs are made at a time (all of them at once spill)
     static constexpr bool kInPlace = K == 2;
     static constexpr size_t kCost = (size_t)NB * (kInPlace ? 1 : 2) * (sizeof(double) + sizeof(float));
     static constexpr int kChunk = 32768;                 // bytes of pointers fetched at a time by the walk
     static constexpr int kRowBytes = NB;                 // pointers of a step
     static constexpr int kRows = kChunk / kRowBytes;     // ... steps
     static constexpr size_t kSmem = kCost > 2 * kChunk ? kCost : 2 * kChunk;
-    static constexpr int kThreads = kEncThreads;
+    static constexpr int kThreads = NT;
     // The byte of a step's row that holds base b's pointer (a thread's L pointers lie side by side), and the pointer in it.
     static __device__ __forceinline__ uint32_t at(uint32_t b)
     {
-        if (K == 8) return b;
+        if (TB > 1) return b;
         const uint32_t h = b & (NH - 1), q = b >> HB;
-        return ((h >> 9) * kEncThreads + (q % T) * NG + (h & (NG - 1))) * L + q / T;
+        return ((h / NG) * NT + (q % T) * NG + (h & (NG - 1))) * L + q / T;
     }
     static __device__ __forceinline__ uint32_t pick(uint8_t byte, uint32_t) { return byte; }
 };
 // K = 1: 1024 threads, a pointer is a bit.
 template <> struct SearchSplit<1> {
     static constexpr int NB = kEncStates / 2, J = 2, HB = 14, NH = 1 << HB;
-    static constexpr int kThreads = 1024, kRowBytes = NB / 8;
+    static constexpr int NT = 1024, kThreads = 1024, kRowBytes = NB / 8;
     static constexpr int kChunk = 32768, kRows = kChunk / kRowBytes;
     static constexpr size_t kSmem = 2 * kChunk;
     static __device__ __forceinline__ uint32_t at(uint32_t b) { return b >> 3; }
@@ -314,24 +319,24 @@ __device__ __forceinline__ void leave_tile(const EncodeArgs& a, int64_t tile, in
     atomicAdd(a.left + why, 1u);
 }
 
-// No path costs more than the sum of (|w| + 4)^2, because every value of the codebooks is less than 4.  Two paths whose
-// float64 costs, summed in any order, are further apart than 2^-42 of the cost are in the right order; a decision
-// that fp32 leaves unsure, or by less than twice the number returned here (2^-41 of that sum), is made in float64, and
-// noted if it is closer than that.  Below 0: the tile is not for this search.
-__device__ __forceinline__ float close_bound(EncodeShared& sh)
+// What a tile's paths should cost at most: far more than K bits usually leave, and what lies beyond the bulk of the
+// codebooks.  (A tile whose path costs more is in doubt.)  Two paths whose float64 costs, summed in any order, are
+// further apart than 2^-42 of the cost are in the right order; a decision that fp32 leaves unsure, or by less than
+// twice `close`, 2^-41 of the bound, is made in float64, and noted if it is closer than that.  False: the tile is not for this search.
+__device__ __forceinline__ bool cost_bound(EncodeShared& sh, float per_weight, float& bound)
 {
     const int tid = threadIdx.x;
-    const float w = tid < 256 ? sh.w[tid] : 0.f;
-    float sum = tid < 256 ? (fabsf(w) + 4.f) * (fabsf(w) + 4.f) : 0.f;
+    const float w = tid < 256 ? sh.w[tid] : 0.f, over = fmaxf(fabsf(w) - 2.5f, 0.f);
+    float sum = over * over;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     if ((tid & 31) == 0) sh.sums[tid >> 5] = sum;
     if (tid == 0) sh.n_close = 0;
-    if (__syncthreads_or(!(fabsf(w) < kEncLargest))) return -1.f;
-    float total = 0.f;
+    if (__syncthreads_or(!(fabsf(w) < kEncLargest))) return false;
+    bound = 256.f * per_weight;
 #pragma unroll
-    for (int i = 0; i < 8; i++) total += sh.sums[i];
-    return total * 4.6e-13f;
+    for (int i = 0; i < 8; i++) bound += sh.sums[i];
+    return true;
 }
 __device__ __forceinline__ void note_close(EncodeShared& sh, int t, uint32_t base, double gap)
 {
@@ -345,7 +350,7 @@ __device__ __forceinline__ void note_close(EncodeShared& sh, int t, uint32_t bas
 // The paths of a tile from the pointers of all its bases, `cost` giving a base's cost to the end of the tile: the free
 // path, then the pinned ones until one closes.  False: a decision on one of them is too close to be told.
 template <int K, int CB, typename Cost>
-__device__ __forceinline__ bool search_paths(EncodeShared& sh, uint8_t* stage, const uint8_t* ptr, int max_pins, Cost&& cost)
+__device__ __forceinline__ bool search_paths(EncodeShared& sh, uint8_t* stage, const uint8_t* ptr, int max_pins, float bound, Cost&& cost)
 {
     using E = SearchSplit<K>;
     constexpr int NB = E::NB, kWarps = E::kThreads / 32;
@@ -399,7 +404,7 @@ __device__ __forceinline__ bool search_paths(EncodeShared& sh, uint8_t* stage, c
         double total = 0.0;
 #pragma unroll
         for (int i = 0; i < 8; i++) total += sh.red_c[i];
-        bool doubt = sh.n_close > kEncClose || (pass == 0 && unsure_start);
+        bool doubt = sh.n_close > kEncClose || (pass == 0 && unsure_start) || !(total <= (double)bound);
         for (int i = tid; i < min(sh.n_close, kEncClose); i += E::kThreads) {
             const uint32_t at = sh.close_at[i];
             if ((uint32_t)(sh.states[at >> 16] >> K) == (at & 0xFFFFu) && !(sh.close_gap[i] > total * 2.3e-13)) doubt = true;
@@ -414,7 +419,7 @@ template <int K, int CB>
 __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs a)
 {
     using E = SearchSplit<K>;
-    constexpr int NB = E::NB, J = E::J, L = E::L, G = E::G, JC = E::JC, HB = E::HB, LB = 16 - K;
+    constexpr int NB = E::NB, J = E::J, L = E::L, G = E::G, JC = E::JC, BL = E::BL, HB = E::HB, LB = 16 - K;
     // Two fp32 keys whose bit patterns differ by less than this may be in the wrong order: the low K
     // bits hold n (2^K units), the arithmetic before is off by at most four units on either side; twice
     // that, rounded up.
@@ -427,9 +432,12 @@ __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs
     uint8_t* ptr = a.slots + (size_t)blockIdx.x * kEncSlotBytes;
 
     const uint32_t h0 = (uint32_t)tid & (E::NG - 1);
-    const uint32_t l0 = K == 8 ? (uint32_t)((tid & 15) | ((tid >> 5) << 4)) : (uint32_t)(tid / E::NG);
-    const uint32_t n_first = K == 8 ? 128u * ((tid >> 4) & 1) : 0u;
-    auto base = [&](int g, int i) -> uint32_t { return ((l0 + E::T * i) << HB) | (h0 + 512u * g); };
+    const uint32_t l0 = (uint32_t)(tid / E::NG);
+    // several threads of a base are lanes 32 / TB apart
+    constexpr int kLanes = 32 / E::TB;
+    const uint32_t b_own = (uint32_t)((tid & (kLanes - 1)) | ((tid >> 5) * kLanes));
+    const uint32_t n_first = (uint32_t)(((tid & 31) / kLanes) * E::JT);
+    auto base = [&](int g, int i) -> uint32_t { return E::TB > 1 ? b_own : ((l0 + E::T * i) << HB) | (h0 + E::NG * g); };
 
     uint32_t cbr[G * L][E::JT / 2];
 #pragma unroll
@@ -459,12 +467,15 @@ __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs
         const int64_t tile = next_tile(sh, a);
         if (tile >= a.n_tiles) return;
         if (tid == 0) sh.smin[0] = sh.smin[1] = 0x7F800000u;
-        for (int b = tid; b < NB; b += kEncThreads) { md0[b] = 0.0; mf0[b] = 0.f; }
-        const float close = close_bound(sh);
-        if (close < 0.f) {
+        for (int b = tid; b < NB; b += E::NT) { md0[b] = 0.0; mf0[b] = 0.f; }
+        float bound;
+        if (!cost_bound(sh, 32.f / (float)(1 << (2 * K)), bound)) {
             if (tid == 0) leave_tile(a, tile, kEncOdd);
             continue;
         }
+        const double close = (double)bound * 0x1p-41;
+        // ... so fp32 keys of at least `near` decide if their bit patterns are kGap apart: that is 2^-20 of them or more
+        const uint32_t near = __float_as_uint(bound * 0x1p-20f);
 
         double off = 0.0;                                // lower bound of every cost of the step
 #pragma unroll 1
@@ -484,11 +495,11 @@ __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs
             uint32_t low_new = 0x7F800000u;
 #pragma unroll
             for (int g = 0; g < G; g++) {
-                const uint32_t row = (h0 + 512u * g) << K;       // the successors of this group
-                uint32_t m1[L], m2[L];
-#pragma unroll
-                for (int c = 0; c < E::JT / JC; c++) {
-                    uint64_t mf2[JC / 2];
+                const uint32_t row = (E::TB > 1 ? b_own & (E::NH - 1) : h0 + E::NG * g) << K;       // the successors of this group
+                uint8_t* pp = ptr + (size_t)t * NB + (E::TB > 1 ? b_own : (uint32_t)(E::NT * g + tid) * L);
+                uint32_t pk[(L + 3) / 4];
+                uint64_t mf2[JC / 2];
+                auto load = [&](int c) {
                     if constexpr (E::kInPlace) {
 #pragma unroll
                         for (int q = 0; q < JC / 2; q++)
@@ -502,91 +513,101 @@ __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs
                             mf2[2 * q + 1] = f32x2(v.z, v.w);
                         }
                     }
+                };
+                if (E::JT == JC) load(0);
 #pragma unroll
-                    for (int i = 0; i < L; i++) {
-                        uint32_t key[JC];
+                for (int i0 = 0; i0 < L; i0 += BL) {
+                    uint32_t m1[BL], m2[BL];
 #pragma unroll
-                        for (int q = 0; q < JC / 2; q++) {
-                            uint32_t pair = cbr[g * L + i][c * (JC / 2) + q];
-                            asm volatile("" : "+r"(pair));   // converted here: hoisted, 128 floats spill
-                            const float2 cf = __half22float2(u32_as_h2(pair));
-                            const uint64_t d = add_f32x2(f32x2(cf.x, cf.y), nw);
-                            const uint64_t k2 = fma_f32x2(d, d, mf2[q]);
-                            const uint32_t n = c * JC + 2 * q;
-                            key[2 * q] = key_with_index<J>((uint32_t)k2, n);
-                            key[2 * q + 1] = key_with_index<J>((uint32_t)(k2 >> 32), n + 1);
-                        }
-                        uint32_t lo = key[0];
+                    for (int c = 0; c < E::JT / JC; c++) {
+                        if (E::JT != JC) load(c);
 #pragma unroll
-                        for (int q = 1; q < JC; q++) lo = min(lo, key[q]);
-                        // gap to the runner-up: the winner itself wraps to the largest number
-                        uint32_t gap = 0xFFFFFFFFu;
+                        for (int i = 0; i < BL; i++) {
+                            uint32_t key[JC];
 #pragma unroll
-                        for (int q = 0; q < JC; q++) gap = __viaddmin_u32(key[q], ~lo, gap);
-                        const uint32_t up = lo + 1u + gap;
-                        if (c == 0) {
-                            m1[i] = lo;
-                            m2[i] = up;
-                        } else {
-                            m2[i] = min(max(m1[i], lo), min(m2[i], up));
-                            m1[i] = min(m1[i], lo);
+                            for (int q = 0; q < JC / 2; q++) {
+                                uint32_t pair = cbr[g * L + i0 + i][c * (JC / 2) + q];
+                                asm volatile("" : "+r"(pair));   // converted here: hoisted, the floats spill
+                                const float2 cf = __half22float2(u32_as_h2(pair));
+                                const uint64_t d = add_f32x2(f32x2(cf.x, cf.y), nw);
+                                const uint64_t k2 = fma_f32x2(d, d, mf2[q]);
+                                const uint32_t n = c * JC + 2 * q;
+                                key[2 * q] = key_with_index<J>((uint32_t)k2, n);
+                                key[2 * q + 1] = key_with_index<J>((uint32_t)(k2 >> 32), n + 1);
+                            }
+                            uint32_t lo = key[0];
+#pragma unroll
+                            for (int q = 1; q < JC; q++) lo = min(lo, key[q]);
+                            // gap to the runner-up: the winner itself wraps to the largest number
+                            uint32_t gap = 0xFFFFFFFFu;
+#pragma unroll
+                            for (int q = 0; q < JC; q++) gap = __viaddmin_u32(key[q], ~lo, gap);
+                            const uint32_t up = lo + 1u + gap;
+                            if (c == 0) {
+                                m1[i] = lo;
+                                m2[i] = up;
+                            } else {
+                                m2[i] = min(max(m1[i], lo), min(m2[i], up));
+                                m1[i] = min(m1[i], lo);
+                            }
                         }
                     }
-                }
-                // the winners' costs in float64, all bases at once; then the bases where fp32 could not decide
-                double val[L];
-                uint32_t bn[L], unsure = 0;
-                const double wd = (double)w;
+                    // the winners' costs in float64, several bases at once; then the bases where fp32 could not decide
+                    double val[BL];
+                    uint32_t bn[BL], unsure = 0;
+                    const double wd = (double)w;
 #pragma unroll
-                for (int i = 0; i < L; i++) {
-                    uint32_t lo = m1[i], up = m2[i];
-                    if (K == 8) {                        // the other half of the n values
-                        lo |= n_first;                   // (the low bits hold 0 .. 127 so far)
-                        up |= n_first;
-                        const uint32_t lo2 = __shfl_xor_sync(0xFFFFFFFFu, lo, 16), up2 = __shfl_xor_sync(0xFFFFFFFFu, up, 16);
-                        up = min(max(lo, lo2), min(up, up2));
-                        lo = min(lo, lo2);
+                    for (int i = 0; i < BL; i++) {
+                        uint32_t lo = m1[i], up = m2[i];
+                        if constexpr (E::TB > 1) {       // the other threads' n values
+                            lo |= n_first;               // (the low bits hold 0 .. JT - 1 so far)
+                            up |= n_first;
+#pragma unroll
+                            for (int o = kLanes; o < 32; o <<= 1) {
+                                const uint32_t lo2 = __shfl_xor_sync(0xFFFFFFFFu, lo, o), up2 = __shfl_xor_sync(0xFFFFFFFFu, up, o);
+                                up = min(max(lo, lo2), min(up, up2));
+                                lo = min(lo, lo2);
+                            }
+                        }
+                        bn[i] = lo & (J - 1);
+                        const uint32_t s = (base(g, i0 + i) << K) | bn[i];
+                        val[i] = __dadd_rn(mdc[slot(row | bn[i], rot)], sq_err((double)codebook_f32<CB>(s), wd));
+                        if (up - lo < kGap || up < near) unsure |= 1u << i;
                     }
-                    bn[i] = lo & (J - 1);
-                    const uint32_t s = (base(g, i) << K) | bn[i];
-                    val[i] = __dadd_rn(mdc[slot(row | bn[i], rot)], sq_err(half_as_f64(decode_one<CB>(s)), wd));
-                    if (up - lo < kGap || __uint_as_float(up) - __uint_as_float(lo) < 2.f * close) unsure |= 1u << i;
-                }
-                if (unsure) {
+                    if (unsure) {
 #pragma unroll
-                    for (int i = 0; i < L; i++) {
-                        if (!((unsure >> i) & 1u)) continue;
-                        const uint32_t s = base(g, i) << K;
-                        double second = 1e300;
-                        bn[i] = 0;
-                        val[i] = __dadd_rn(mdc[slot(row, rot)], sq_err(half_as_f64(decode_one<CB>(s)), wd));
+                        for (int i = 0; i < BL; i++) {
+                            if (!((unsure >> i) & 1u)) continue;
+                            const uint32_t s = base(g, i0 + i) << K;
+                            double second = 1e300;
+                            bn[i] = 0;
+                            val[i] = __dadd_rn(mdc[slot(row, rot)], sq_err((double)codebook_f32<CB>(s), wd));
 #pragma unroll 4
-                        for (int q = 1; q < J; q++) {
-                            const double v = __dadd_rn(mdc[slot(row | (uint32_t)q, rot)], sq_err(half_as_f64(decode_one<CB>(s | (uint32_t)q)), wd));
-                            // (final states with equal errors: the first of them, in whatever order the costs are summed)
-                            if (v < val[i]) { second = val[i]; val[i] = v; bn[i] = q; }
-                            else if (v < second && (u > 0 || v > val[i])) second = v;
+                            for (int q = 1; q < J; q++) {
+                                const double v = __dadd_rn(mdc[slot(row | (uint32_t)q, rot)], sq_err((double)codebook_f32<CB>(s | (uint32_t)q), wd));
+                                // (final states with equal errors: the first of them, in whatever order the costs are summed)
+                                if (v < val[i]) { second = val[i]; val[i] = v; bn[i] = q; }
+                                else if (v < second && (u > 0 || v > val[i])) second = v;
+                            }
+                            if (second - val[i] < close && n_first == 0) note_close(sh, t, base(g, i0 + i), second - val[i]);
                         }
-                        if (second - val[i] < (double)close && (K != 8 || n_first == 0)) note_close(sh, t, base(g, i), second - val[i]);
+                    }
+                    if (n_first == 0) {
+#pragma unroll
+                        for (int i = 0; i < BL; i++) {
+                            // in place, base (i << HB) | h of the next step takes the address of (h << K) | i
+                            const uint32_t ad = E::kInPlace ? slot(row | (i0 + i), rot) : base(g, i0 + i);
+                            const uint32_t af = E::kInPlace ? ad : first_f + (i0 + i) * (E::T << HB) + E::NG * g;
+                            const float rel = fmaxf((float)(val[i] - off), 0.f);
+                            mdn[ad] = val[i];
+                            mfn[af] = rel;
+                            low_new = min(low_new, __float_as_uint(rel));
+                            const int q = i0 + i;
+                            pk[q >> 2] = (q & 3) ? pk[q >> 2] | (bn[i] << (8 * (q & 3))) : bn[i];
+                        }
                     }
                 }
-                if (K != 8 || n_first == 0) {
-#pragma unroll
-                    for (int i = 0; i < L; i++) {
-                        // in place, base (i << HB) | h of the next step takes the address of (h << K) | i
-                        const uint32_t ad = E::kInPlace ? slot(row | i, rot) : base(g, i);
-                        const uint32_t af = E::kInPlace ? ad : first_f + i * (E::T << HB) + 512u * g;
-                        const float rel = fmaxf((float)(val[i] - off), 0.f);
-                        mdn[ad] = val[i];
-                        mfn[af] = rel;
-                        low_new = min(low_new, __float_as_uint(rel));
-                    }
-                    uint8_t* pp = ptr + (size_t)t * NB + (K == 8 ? l0 : (uint32_t)(512 * g + tid) * L);
-                    uint32_t pk[(L + 3) / 4];
-#pragma unroll
-                    for (int i = 0; i < (L + 3) / 4; i++) pk[i] = 0u;
-#pragma unroll
-                    for (int i = 0; i < L; i++) pk[i >> 2] |= bn[i] << (8 * (i & 3));
+                if (n_first == 0) {
                     if constexpr (L == 8) __stcg(reinterpret_cast<uint2*>(pp), make_uint2(pk[0], pk[1]));
                     else if constexpr (L == 4) __stcg(reinterpret_cast<uint32_t*>(pp), pk[0]);
                     else if constexpr (L == 2) __stcg(reinterpret_cast<uint16_t*>(pp), (uint16_t)pk[0]);
@@ -598,7 +619,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs
             __syncthreads();
         }
         constexpr int end_rot = E::kInPlace ? (K * 256) % LB : 0;
-        if (search_paths<K, CB>(sh, smem, ptr, a.max_pins, [&](uint32_t b) { return md0[slot(b, end_rot)]; })) store_tile<K>(sh, a, tile);
+        if (search_paths<K, CB>(sh, smem, ptr, a.max_pins, bound, [&](uint32_t b) { return md0[slot(b, end_rot)]; })) store_tile<K>(sh, a, tile);
         else if (tid == 0) leave_tile(a, tile, kEncDoubt);
     }
 }
@@ -975,11 +996,12 @@ template <int CB> __global__ void __launch_bounds__(kEncThreads1, 1) search_kern
         const int64_t tile = next_tile(sh, a);
         if (tile >= a.n_tiles) return;
         for (int b = tid; b < NB; b += kEncThreads1) __stcg(cost0 + b, 0.0);
-        const float close = close_bound(sh);
-        if (close < 0.f) {
+        float bound;
+        if (!cost_bound(sh, 8.f, bound)) {
             if (tid == 0) leave_tile(a, tile, kEncDoubt);
             continue;
         }
+        const double close = (double)bound * 0x1p-41;
 #pragma unroll 1
         for (int u = 0; u < 256; u++) {
             const int t = 255 - u;
@@ -997,7 +1019,7 @@ template <int CB> __global__ void __launch_bounds__(kEncThreads1, 1) search_kern
                     const double v1 = __dadd_rn(c.y, sq_err(half_as_f64(__high2half(u32_as_h2(pair))), wd));
                     const double gap = fabs(v1 - v0);
                     // (final states with equal errors: the first of them, in whatever order the costs are summed)
-                    if (gap < (double)close && (u > 0 || gap > 0.0)) note_close(sh, t, b, gap);
+                    if (gap < close && (u > 0 || gap > 0.0)) note_close(sh, t, b, gap);
                     __stcg(nxt + b, v1 < v0 ? v1 : v0);
                     const uint32_t bits = __ballot_sync(0xFFFFFFFFu, v1 < v0);
                     if ((tid & 31) == 0) __stcg(row + (b >> 5), bits);
@@ -1005,7 +1027,7 @@ template <int CB> __global__ void __launch_bounds__(kEncThreads1, 1) search_kern
             }
             __syncthreads();
         }
-        if (search_paths<1, CB>(sh, smem, ptr, a.max_pins, [&](uint32_t b) { return __ldcg(cost0 + b); })) store_tile<1>(sh, a, tile);
+        if (search_paths<1, CB>(sh, smem, ptr, a.max_pins, bound, [&](uint32_t b) { return __ldcg(cost0 + b); })) store_tile<1>(sh, a, tile);
         else if (tid == 0) leave_tile(a, tile, kEncDoubt);
     }
 }
@@ -1044,7 +1066,7 @@ template <int K, int CB> static int launch_encode(const EncodeArgs& a, unsigned 
             if (e != cudaSuccess) return note_cuda(e);
             attr_set[dev] = true;
         }
-        search_kernel<K, CB><<<slots, kEncThreads, SearchSplit<K>::kSmem, s>>>(a);
+        search_kernel<K, CB><<<slots, SearchSplit<K>::NT, SearchSplit<K>::kSmem, s>>>(a);
         int rc = check_launch();
         if (rc) return rc;
         EncodeArgs rest = a;
