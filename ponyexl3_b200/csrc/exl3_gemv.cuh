@@ -170,7 +170,11 @@ __device__ __forceinline__ unsigned atom_inc_acq_rel(unsigned* p, unsigned bound
     return old;
 }
 
-template <int K, int CB, int NMMA, bool FAST, bool XFUSED>
+// PAIRED: two virtual CTAs per column block, that is, a block's two contributors are the halves of one CTA and the second
+// leaves its sums in shared memory for the first (through the workspace, as other split blocks do, 5120 -> 17408 at 1 and 8
+// rows takes 29.9 and 33.0 us, this way 28.1 and 31.0).  A kernel of its own, because the same code as a branch moved the
+// times of all other launches by up to 0.2 us in either direction.
+template <int K, int CB, int NMMA, bool FAST, bool XFUSED, bool PAIRED>
 __global__ void __launch_bounds__(kGemvThreads, 1)
     gemv_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap tm_w,
                 const __grid_constant__ CUtensorMap tm_x)
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
     // The launch must match the plan the host made: every thread of every CTA takes the same
     // branch here, so a mismatch ends the grid before any barrier is touched.
     if (dynamic_smem_bytes() < (uint32_t)(a.stage0_off + 2 * ns * stage_bytes) || ns < kGroups || ns > kMaxStages ||
-        (int)gridDim.x * 2 < G || G < 1 ||
+        (int)gridDim.x * 2 < G || G < 1 || (PAIRED && G != 2 * ncb) ||
         (XFUSED && (a.blocks ? (I + G - 1) / G : min((I + G - 1) / G, (int64_t)nkb)) > a.n_slots)) {
         if (tid == 0) atomicOr(a.status, ST_BAD_LAUNCH);
         return;
@@ -616,7 +620,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
         // and the contributor that completes the count finishes the block.
         bool finish = true;
         int c_first = 0, n_contrib = 0, slot_first = 0;
-        if (seg_len == nkb) {
+        if (PAIRED || seg_len == nkb) {
             for (int i = tidh; i < nv; i += kHalfThreads) {
                 const int o = (i >> 7) * kYStride + (i & 127);
                 float f = ybuf[o];
@@ -624,7 +628,14 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
                 for (int cc = 1; cc < L::kCopies; cc++) f += ybuf[o + cc * L::kYCopy];
                 ybuf[o] = f;
             }
-            named_bar_sync(hbar, kHalfThreads);
+            if (!PAIRED) {
+                named_bar_sync(hbar, kHalfThreads);
+            } else if (half == 0) {
+                asm volatile("bar.sync 3, %0;" ::"n"(kGemvThreads) : "memory");
+            } else {
+                asm volatile("bar.arrive 3, %0;" ::"n"(kGemvThreads) : "memory");
+                return;                                // a half has one segment
+            }
         } else {
             if ((size_t)(2 * c + 2) * nv * sizeof(float) > a.partial_bytes) {   // never true for a launch as planned
                 if (tidh == 0) atomicOr(a.status, ST_BAD_LAUNCH);
@@ -669,10 +680,10 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
                 const bool biased = a.bias && sv_off >= 0 && !a.raw_out;
                 if (scaled) sv = *reinterpret_cast<const uint2*>(a.svh + sv_off + 4 * lane);
                 if (biased) bv = *reinterpret_cast<const uint2*>(a.bias + sv_off + 4 * lane);
-                if (seg_len == nkb) {
+                if (PAIRED || seg_len == nkb) {
                     const int o = n * kYStride + 4 * lane;
 #pragma unroll
-                    for (int q = 0; q < 4; q++) v[q] = ybuf[o + q];
+                    for (int q = 0; q < 4; q++) v[q] = PAIRED ? ybuf[o + q] + ybuf[o + q + L::kYBytes / 4] : ybuf[o + q];
                 } else {
                     // the contributors' sums, in virtual-CTA order
                     v[0] = v[1] = v[2] = v[3] = 0.f;
@@ -773,15 +784,16 @@ static int launch_gemv_t(GemvArgs a, bool pdl, cudaStream_t s)
     a.stage0_off = stage0;
     const size_t smem = (size_t)stage0 + 2 * (size_t)stages * stage_bytes;
 
-    static bool attr_set[kMaxDevices] = {};  // per device
+    const bool paired = plan.grid == 2 * a.ncb && !a.ncb_dev;
+    const auto kernel = paired ? gemv_kernel<K, CB, NMMA, FAST, XFUSED, true> : gemv_kernel<K, CB, NMMA, FAST, XFUSED, false>;
+    static bool attr_set[kMaxDevices][2] = {};  // per device
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxDevices) return EXL3_E_UNSUPPORTED;
-    if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemv_kernel<K, CB, NMMA, FAST, XFUSED>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes);
+    if (!attr_set[dev][paired]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes);
         if (e != cudaSuccess) return note_cuda(e);
-        attr_set[dev] = true;
+        attr_set[dev][paired] = true;
     }
     CUtensorMap tm_w, tm_x;
     {
@@ -816,7 +828,7 @@ static int launch_gemv_t(GemvArgs a, bool pdl, cudaStream_t s)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     a.early_weights = pdl || !XFUSED;   // behind the rotation kernel all earlier work is complete already
-    return note_cuda(cudaLaunchKernelEx(&cfg, gemv_kernel<K, CB, NMMA, FAST, XFUSED>, a, tm_w, tm_x));
+    return note_cuda(cudaLaunchKernelEx(&cfg, kernel, a, tm_w, tm_x));
 }
 
 template <int K, int CB> static int launch_gemv_kc(const GemvArgs& a, bool pdl, cudaStream_t s)

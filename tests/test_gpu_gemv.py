@@ -370,3 +370,18 @@ def test_programmatic_launch_chain(mod, oracle, rows):
     plain = chain(False)
     for _ in range(3):
         assert torch.equal(chain(True), plain)
+
+
+@pytest.mark.parametrize("rows", [1, 3, 8, 16])
+@pytest.mark.parametrize("k,inf,outf", [(4, 256, 640), (4, 384, 1152), (3, 2176, 384), (8, 640, 1280)])
+def test_gemv_two_halves_per_block(mod, oracle, k, inf, outf, rows):
+    """As many virtual CTAs as twice the column blocks: both contributors of a block are halves of one CTA and hand over in shared
+    memory (even and odd numbers of k-blocks, ranges shorter and longer than the four groups)."""
+    from ponyexl3_b200 import _lib
+    layer = _layer(mod, k, inf, outf, 900 + rows, bias=True)
+    x = np.random.default_rng(rows).standard_normal((rows, inf)).astype(np.float16)
+    _lib.load().exl3_tune_gemv(2 * (outf // 128), -1)
+    try:
+        _check(mod, oracle, layer, x)
+    finally:
+        _lib.load().exl3_tune_gemv(0, -1)
