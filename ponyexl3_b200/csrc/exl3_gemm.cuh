@@ -9,9 +9,9 @@
 // memory instead costs four scattered stores per tile and 96 bytes of operand reads per clock.
 //
 // Output tile: 128 columns (the width of the output rotation) x up to 256 tokens, 384 in the wide form; k-step 64.
-//   warp 0      packed tiles: one 3-D TMA box of 8 x 4 tiles per k-step (ring w, eight stages; four in the wide form)
+//   warp 0      packed tiles: one 3-D TMA box of 8 x 4 tiles per k-step (ring w, as deep as shared memory allows)
 //   warp 1      activations: one or more 128B-swizzled TMA boxes per k-step (ring x)
-//   warp 2      issues the MMAs: A from tensor memory (as many 32-column stages as ring w has), B from ring x
+//   warp 2      issues the MMAs: A from tensor memory (eight 32-column stages; four in the wide form), B from ring x
 //   warps 4-19  decode, four sets of four warps (a warp may touch the quarter of the tensor-memory
 //               lanes that its index names); the sets take the k-steps in turn
 // then the 16 decode warps finish the tile:
@@ -45,8 +45,10 @@ constexpr int kTsThreads = 32 * (kTsFirstDecodeWarp + kTsDecodeWarps);
 constexpr int kTsOuts = 128, kTsStepTiles = 4;      // k-step: 4 tile rows
 constexpr int kTsMaxTok = 256, kTsWideTok = 384;    // tokens of a tile; of a wide one
 constexpr int kTsStages = 8;                        // barriers of the k-steps in flight
-// Three forms of the kernel.
+// Four forms of the kernel.
 //   PLAIN  for CTAs with hardly more than one tile.
+//   JOINT  PLAIN where the two to eight CTAs of a tile are a thread-block cluster: each adds up a share of the tokens
+//          from the others' sums, which they write into its shared memory, and finishes them.
 //   AHEAD  decodes k-steps of the next tile before it finishes one.
 //   WIDE   AHEAD with up to 384 tokens a tile: the weights are decoded once for all of them, and decoding
 //          is what bounds the kernel.
@@ -54,13 +56,13 @@ constexpr int kTsStages = 8;                        // barriers of the k-steps i
 // while the one before is finished) or one of up to 256, and eight stages of weights; WIDE has one of 384 and
 // four stages.  (Four stages with 256 tokens were slower for every shape: a set of decode warps then waits for
 // the MMAs of its own k-step before it can decode the next.)
-enum : int { TS_PLAIN = 0, TS_AHEAD = 1, TS_WIDE = 2 };
+enum : int { TS_PLAIN = 0, TS_AHEAD = 1, TS_WIDE = 2, TS_JOINT = 3 };
 template <int MODE> struct TsForm {
-    static constexpr bool kAhead = MODE != TS_PLAIN, kWide = MODE == TS_WIDE;
-    static constexpr int kStages = kWide ? 4 : 8;   // stages of ring w and of the weights in tensor memory
+    static constexpr bool kAhead = MODE == TS_AHEAD || MODE == TS_WIDE, kWide = MODE == TS_WIDE, kJoint = MODE == TS_JOINT;
+    static constexpr int kStages = kWide ? 4 : 8;   // stages of the weights in tensor memory
     static constexpr int kACol0 = kWide ? 384 : 256;
 };
-constexpr int kTsMaxXStages = 8;
+constexpr int kTsMaxWStages = 12;
 constexpr int kTsCtrlBytes = 1024;
 constexpr int kTsHBytes = 128 * 128 * 2, kTsYBytes = 128 * 128 * 2;
 constexpr int kTsHOff = kTsCtrlBytes, kTsYOff = kTsHOff + kTsHBytes, kTsWOff = kTsYOff + kTsYBytes;
@@ -69,8 +71,7 @@ constexpr int kTsSmemBytes = 227 * 1024;
 template <int K> struct TsLayout {
     static constexpr int kTileWords = 8 * K;
     static constexpr int kWBytes = 32 * kTileWords * 4;                 // 8 x 4 packed tiles: K KiB
-    template <int MODE> static constexpr int xoff() { return kTsWOff + TsForm<MODE>::kStages * kWBytes; }
-    template <int MODE> static constexpr int xroom() { return kTsSmemBytes - xoff<MODE>(); }
+    static constexpr int kRoom = kTsSmemBytes - kTsWOff;                // of the two rings
     // tokens per tile of a dense launch: at least four stages of activations have to fit, three wide ones
     static constexpr int kTok = std::min(kTsMaxTok, kTsSmemBytes - kTsWOff - 8 * kWBytes >= 512 * kTsMaxTok
                                                         ? kTsMaxTok
@@ -101,13 +102,20 @@ struct TsWait {
 
 // ---- tensor memory as an operand and as a destination of registers ------------------------------------
 // D[tmem] (+)= A[tmem] * B[smem]; issued by ONE thread.
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                              uint32_t accumulate)
+// The four products of a k-step of 64 (16 k = 8 columns of A, 32 bytes of B each), in one
+// statement: the issuing warp shares its scheduler with the decode warps, and what it takes to issue a k-step is
+// what a short k-step takes.
+__device__ __forceinline__ void tc_mma_kstep(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
-        "{\n.reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "{\n.reg .pred p, t;\n.reg .b32 a1, a2, a3;\n.reg .b64 b1, b2, b3;\n"
+        "setp.ne.b32 p, %4, 0;\nsetp.eq.b32 t, 0, 0;\n"
+        "add.s32 a1, %1, 8;\nadd.s32 a2, %1, 16;\nadd.s32 a3, %1, 24;\n"
+        "add.s64 b1, %2, 2;\nadd.s64 b2, %2, 4;\nadd.s64 b3, %2, 6;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n}\n" ::"r"(d_tmem),
         "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
@@ -190,6 +198,31 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t smem_addr)
 }
 constexpr uint32_t kIdescMajorA = 1u << 15;          // A is MN-major
 
+// ---- the output rotation of 128 tokens: D2 = Y H ---------------------------------------------------------
+// B operand H[n][k] = (-1)^popcount(n & k), K-major: two 64-wide halves of k, 128 rows of 128 bytes each.  (As H64 and
+// -H64, half of it, with products of 64 columns: room for more packed tiles, but MLP of 300 rows 188.6 -> 190.8 us.)
+__device__ __forceinline__ void store_sylvester(uint8_t* h_mat, int thread, int threads)
+{
+    for (int i = thread; i < 2048; i += threads) {
+        const int kh = i >> 10, n = (i >> 3) & 127, ch = i & 7;
+        const uint32_t flip = (__popc(n & (64 * kh + 8 * ch)) & 1) ? 0x80008000u : 0u;
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            w[j] = flip ^ (0x3C003C00u | ((__popc(n & (2 * j)) & 1) ? 0x8000u : 0u) | ((__popc(n & (2 * j + 1)) & 1) ? 0x80000000u : 0u));
+        *reinterpret_cast<uint4*>(h_mat + kh * 16384 + n * 128 + ((ch ^ (n & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+// Issued by ONE thread; `done` gets one arrival when the product is complete.
+__device__ __forceinline__ void rotate_tile(uint32_t d_tmem, uint32_t y_buf, uint32_t h_mat, uint32_t done)
+{
+    const uint64_t yd = smem_desc_mn_sw128(y_buf), hd = smem_desc_sw128(h_mat);
+#pragma unroll
+    for (int kk = 0; kk < 8; kk++)
+        tc_mma_f16(d_tmem, yd + 128 * kk, hd + (kk >> 2) * 1024 + (kk & 3) * 2, mma_idesc_f16(128, 128) | kIdescMajorA, kk > 0 ? 1u : 0u);
+    tc_commit(done);
+}
+
 // One stretch of k-steps of one output tile.
 struct TsSeg {
     int m0, rows;            // first row of xh, rows in use
@@ -259,9 +292,9 @@ template <bool TABLE> struct TsWalk {
             }
             const int l = __ffs(found) - 1;
             found &= found - 1;
-            s.m0 = __shfl_sync(0xFFFFFFFFu, p.x, l);
-            s.rows = __shfl_sync(0xFFFFFFFFu, p.y, l);
-            s.tn0 = __shfl_sync(0xFFFFFFFFu, p.z, l);
+            s.m0 = uniform(__shfl_sync(0xFFFFFFFFu, p.x, l));
+            s.rows = uniform(__shfl_sync(0xFFFFFFFFu, p.y, l));
+            s.tn0 = uniform(__shfl_sync(0xFFFFFFFFu, p.z, l));
             s.sv_off = __shfl_sync(0xFFFFFFFFu, p.w, l);
             s.y_col = __shfl_sync(0xFFFFFFFFu, q.x, l);
             s.y_row_delta = __shfl_sync(0xFFFFFFFFu, q.z, l);
@@ -292,7 +325,61 @@ template <bool TABLE> struct TsWalk {
     }
 };
 
-template <int K, int CB, bool TABLE, int MODE>
+// Last step of a tile's finishing: D2 (lane = token) scaled, biased and stored; this warp's 32 columns.  `drained` is called when
+// tensor memory has been read.
+template <typename Drained>
+__device__ __forceinline__ void store_rotated(const GemmArgs& a, const TsSeg& sg, bool used, int orow, uint32_t lane_base, int set,
+                                              uint64_t* h_full, uint32_t hpar, const TsWait& wait, Drained&& drained)
+{
+    __half* yp = nullptr;
+    if (used) {
+        const int col0 = sg.y_col + 32 * set;
+        yp = a.n_members > 1 ? a.member_y[sg.member] + (int64_t)orow * a.member_stride[sg.member] + col0
+                             : a.y + (int64_t)orow * a.y_row_stride + col0;
+    }
+    // The output scales are fetched behind the product: between the stores below, which might alias
+    // them, the loads would be made and waited for one after the other, and a prefetch into L1 does
+    // not help.
+    uint4 sv[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        sv[c] = a.svh ? ldg_nc_128(a.svh + sg.sv_off + 32 * set + 8 * c)
+                      : make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
+    wait(h_full, hpar);
+    tc_fence_after_sync();
+    float f[32];
+    tmem_ld_32cols(lane_base + 32 * set, f);
+    drained();
+    if (!used) return;
+    const uint64_t scale = f32x2(EXL3_HAD_SCALE, EXL3_HAD_SCALE);
+    uint4 held16 = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const uint32_t sw4[4] = {sv[c].x, sv[c].y, sv[c].z, sv[c].w};
+        uint32_t h[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 w2 = __half22float2(u32_as_h2(sw4[i]));
+            h[i] = f16_pair(mul_f32x2(mul_f32x2(f32x2(f[8 * c + 2 * i], f[8 * c + 2 * i + 1]), scale), f32x2(w2.x, w2.y)));
+        }
+        if (a.bias) {
+            const uint4 bv = __ldg(reinterpret_cast<const uint4*>(a.bias + sg.sv_off + 32 * set + 8 * c));
+            const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) h[i] = h2_as_u32(__hadd2(u32_as_h2(h[i]), u32_as_h2(bw[i])));
+        }
+        const uint4 ov = make_uint4(h[0], h[1], h[2], h[3]);
+        if (!a.y_wide) {
+            *reinterpret_cast<uint4*>(yp + 8 * c) = ov;
+        } else if (c & 1) {
+            st_global_256(yp + 8 * (c - 1), held16, ov);   // whole sectors
+        } else {
+            held16 = ov;
+        }
+    }
+}
+
+template <int K, int CB, int MODE>
 __global__ void __launch_bounds__(kTsThreads, 1)
     gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w)
 {
@@ -300,9 +387,9 @@ __global__ void __launch_bounds__(kTsThreads, 1)
     using F = TsForm<MODE>;
     constexpr int NS = F::kStages;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* w_full = reinterpret_cast<uint64_t*>(smem);      // packed tiles landed                      [8]
-    uint64_t* w_empty = w_full + kTsStages;                   // ... read by the set's four warps          [8]
-    uint64_t* full = w_empty + kTsStages;                     // weights decoded AND activations landed    [8]
+    uint64_t* w_full = reinterpret_cast<uint64_t*>(smem);      // packed tiles landed                     [12]
+    uint64_t* w_empty = w_full + kTsMaxWStages;               // ... read by the set's four warps         [12]
+    uint64_t* full = w_empty + kTsMaxWStages;                   // weights decoded AND activations landed    [8]
     uint64_t* empty = full + kTsStages;                       // the k-step's MMAs are done                [8]
     uint64_t* d_full = empty + kTsStages;                      // a segment's sums are complete             [2]
     uint64_t* d_empty = d_full + 2;                            // ... and drained                          [2]
@@ -312,35 +399,43 @@ __global__ void __launch_bounds__(kTsThreads, 1)
     const TsWait wait{reinterpret_cast<volatile int*>(tmem_slot + 1), a.status};
     uint8_t* h_mat = smem + kTsHOff;
     uint8_t* y_buf = smem + kTsYOff;
-    uint8_t* w_ring = smem + kTsWOff;
-    uint8_t* x_ring = smem + L::template xoff<MODE>();
+    uint8_t* recv = smem + kTsWOff;                            // JOINT: sums from the tile's other CTAs
+    uint8_t* w_ring = smem + kTsWOff + (F::kJoint ? a.ts_recv_bytes : 0);
+    const int nw = a.ts_w_stages;                              // depth of ring w, a multiple of the sets
+    uint8_t* x_ring = w_ring + nw * L::kWBytes;
 
-    const int tid = threadIdx.x, warp = TsWalk<TABLE>::uniform(tid >> 5), lane = tid & 31;
+    using Walk = TsWalk<false>;
+    const int tid = threadIdx.x, warp = Walk::uniform(tid >> 5), lane = tid & 31;
     const int nx = a.stages, x_bytes = a.ts_x_bytes;           // depth and stage size of ring x
-    TsWalk<TABLE> walk;
+    Walk walk;
     walk.start(a);
     TsSeg sg;
 
-    if (tid == 0) {
-        *wait.abort_word = 0;
-        for (int s = 0; s < kTsStages; s++) {
-            mbar_init(smem_u32(&w_full[s]), 1);
-            mbar_init(smem_u32(&w_empty[s]), 4);
-            mbar_init(smem_u32(&full[s]), 5);                  // a set's four warps and the activations' copy
-            mbar_init(smem_u32(&empty[s]), 1);
+    if (warp == 0) {                                           // (one thread's 40 to 60 barriers took 0.3 us)
+        if (lane < nw) {
+            mbar_init(smem_u32(&w_full[lane]), 1);
+            mbar_init(smem_u32(&w_empty[lane]), 4);
         }
-        for (int s = 0; s < 2; s++) {
-            mbar_init(smem_u32(&d_full[s]), 1);
-            mbar_init(smem_u32(&d_empty[s]), kTsDecodeWarps);
+        if (lane < kTsStages) {
+            mbar_init(smem_u32(&full[lane]), 5);               // a set's four warps and the activations' copy
+            mbar_init(smem_u32(&empty[lane]), 1);
         }
-        mbar_init(smem_u32(h_full), 1);
+        if (lane < 2) {
+            mbar_init(smem_u32(&d_full[lane]), 1);
+            mbar_init(smem_u32(&d_empty[lane]), kTsDecodeWarps);
+        }
+        if (lane == 0) {
+            mbar_init(smem_u32(h_full), 1);
+            *wait.abort_word = 0;
+        }
         mbar_fence_init();
     }
     if (warp == 2) tmem_alloc(smem_u32(tmem_slot), 512);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = (uint32_t)TsWalk<TABLE>::uniform((int)*tmem_slot);
+    const uint32_t tmem_base = (uint32_t)Walk::uniform((int)*tmem_slot);
+    if (F::kJoint) cluster_arrive_relaxed();                   // "my shared memory is there"
     griddep_launch_dependents();
 
     // The three single-issuer roles run as whole warps with one elected lane issuing: loop control,
@@ -350,7 +445,6 @@ __global__ void __launch_bounds__(kTsThreads, 1)
         // ------------------------------------------------------------------ packed tiles ----
         const bool leader = elect_one();
         if (leader) tma_prefetch_desc(&tm_w);
-        if (TABLE) griddep_wait();                        // the table belongs to an earlier kernel
         int s = 0;
         uint32_t parity = 1;                                   // (a wait for the phase before the first passes)
         while (walk.next(a, sg)) {
@@ -361,7 +455,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                     mbar_arrive_expect_tx(bar, L::kWBytes);
                     tma_load_3d(smem_u32(w_ring) + s * L::kWBytes, &tm_w, 0, sg.tn0, kTsStepTiles * ks, bar);
                 }
-                if (++s == NS) { s = 0; parity ^= 1u; }
+                if (++s == nw) { s = 0; parity ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -392,7 +486,6 @@ __global__ void __launch_bounds__(kTsThreads, 1)
     } else if (warp == 2) {
         // -------------------------------------------------------------------- MMA issuer ----
         const bool leader = elect_one();
-        if (TABLE) griddep_wait();
         int xs = 0, as = 0, db = 0, v = 0;
         uint32_t dpar = 1;
         const uint32_t x0 = smem_u32(x_ring);
@@ -409,18 +502,9 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                 const uint64_t xd = smem_desc_sw128(x0 + (uint32_t)(xs * x_bytes));
                 wait(&full[v & (kTsStages - 1)], (uint32_t)(v / kTsStages) & 1u);
                 tc_fence_after_sync();
-                if (leader) {                                  // 16 k = 8 columns of A, 32 bytes of B
-                    tc_mma_f16_ts(d_tmem, at, xd, idesc, accum);
-                    tc_mma_f16_ts(d_tmem, at + 8, xd + 2, idesc, 1u);
-                    tc_mma_f16_ts(d_tmem, at + 16, xd + 4, idesc, 1u);
-                    tc_mma_f16_ts(d_tmem, at + 24, xd + 6, idesc, 1u);
-                    if (F::kWide && n1 > 0) {
-                        const uint64_t xe = xd + (uint64_t)(8 * n0);           // n0 rows of 128 bytes further
-                        tc_mma_f16_ts(d_tmem + n0, at, xe, idesc1, accum);
-                        tc_mma_f16_ts(d_tmem + n0, at + 8, xe + 2, idesc1, 1u);
-                        tc_mma_f16_ts(d_tmem + n0, at + 16, xe + 4, idesc1, 1u);
-                        tc_mma_f16_ts(d_tmem + n0, at + 24, xe + 6, idesc1, 1u);
-                    }
+                if (leader) {
+                    tc_mma_kstep(d_tmem, at, xd, idesc, accum);
+                    if (F::kWide && n1 > 0) tc_mma_kstep(d_tmem + n0, at, xd + (uint64_t)(8 * n0), idesc1, accum);   // n0 rows of 128 bytes further
                     tc_commit(smem_u32(&empty[v & (kTsStages - 1)]));
                 }
                 accum = 1u;
@@ -439,27 +523,12 @@ __global__ void __launch_bounds__(kTsThreads, 1)
         const int nks = a.t_in >> 2;
         LaneWords<K> lw;
         lw.init(lane);
-        // H[n][k] = (-1)^popcount(n & k), K-major: two 64-wide halves of k, 128 rows of 128 bytes each
-        {
-            uint32_t w4[4];                                        // the low three bits of k: the same for all of a thread's pieces
-            const int n_low = (dt >> 3) & 7;
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                w4[j] = 0x3C003C00u | ((__popc(n_low & (2 * j)) & 1) ? 0x8000u : 0u) | ((__popc(n_low & (2 * j + 1)) & 1) ? 0x80000000u : 0u);
-#pragma unroll
-            for (int i = dt; i < 2048; i += 512) {
-                const int kh = i >> 10, n = (i >> 3) & 127, ch = i & 7;
-                const uint32_t flip = (__popc(n & (64 * kh + 8 * ch)) & 1) ? 0x80008000u : 0u;
-                *reinterpret_cast<uint4*>(h_mat + kh * 16384 + n * 128 + ((ch ^ (n & 7)) << 4)) =
-                    make_uint4(w4[0] ^ flip, w4[1] ^ flip, w4[2] ^ flip, w4[3] ^ flip);
-            }
-        }
-        if (TABLE) griddep_wait();
+        store_sylvester(h_mat, dt, 512);
         // A set decodes its k-steps in order, whatever tiles they belong to.  With AHEAD the warps decode as many
         // k-steps of the next tile as there are stages before they finish one, so that the tensor core has work
-        // in the meantime (SwitchGLU of 4096 tokens 546 -> 524 us); a CTA with hardly more than one tile is 1 us
-        // quicker without.
-        int kc = 0, v = set;                                       // end of the current tile's k-steps; next one of this set
+        // in the meantime; a CTA with hardly more than one tile is 1 us quicker without.
+        int kc = 0, v = set, ws = set;                             // end of the current tile's k-steps; next one of this set, its ring stage
+        uint32_t w_par = 0;
         int db = 0;
         uint32_t dpar = 0, hpar = 0;
         TsSeg nx_sg;
@@ -471,51 +540,79 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             kc += n_steps;
             const int v_end = kc + (F::kAhead && more ? min(NS, nx_sg.k1 - nx_sg.k0) : 0);
             for (; v < v_end; v += kTsSets) {
-                // Four or eight stages, four sets: a stage always belongs to the same set.  (With another number a
-                // set could look at a barrier two phases early and read a stale parity.)
+                // Four sets, and a multiple of them in stages of ring w and of tensor memory: a stage always belongs to the
+                // same set.  (With another number a set could look at a barrier two phases early and read a stale parity.)
                 const int st = v & (NS - 1), vb = v - NS;      // vb: the k-step that had the stage before
-                wait(&w_full[st], (uint32_t)(v / NS) & 1u);
-                // tile columns 2q, 2q + 1 of all four tile rows
-                const uint32_t* wt = reinterpret_cast<const uint32_t*>(w_ring + st * L::kWBytes) + 2 * q * L::kTileWords;
-                uint32_t pw[2][4][K == 4 ? 4 : 3];
+                wait(&w_full[ws], w_par);
+                const uint32_t* wt = reinterpret_cast<const uint32_t*>(w_ring + ws * L::kWBytes) + 2 * q * L::kTileWords;
+                auto tile_frag = [&](const uint32_t (&cw)[8], uint32_t* f) {
+                    f[0] = decode_pair_rt<CB>(cw[0], cw[1], xc);
+                    f[1] = decode_pair_rt<CB>(cw[4], cw[5], xc);
+                    f[2] = decode_pair_rt<CB>(cw[2], cw[3], xc);
+                    f[3] = decode_pair_rt<CB>(cw[6], cw[7], xc);
+                };
+                auto await_operand = [&]() {
+                    if (vb >= 0) wait(&empty[vb & (kTsStages - 1)], (uint32_t)(vb / kTsStages) & 1u);
+                    tc_fence_after_sync();
+                };
+                const uint32_t a_tmem = tmem_base + ((uint32_t)(32 * q) << 16) + F::kACol0 + 32 * st;
+                // Tile columns 2q, 2q + 1 of all four tile rows, one after the other: half the code leaves the issuing warps and
+                // a short call's start more of the instruction cache (512 x 512 8.4 -> 7.9 us).  The wide form, whose sets
+                // mostly wait for MMAs, reads all words first and is 2 % quicker with it (an MLP of 300 rows).
+                if constexpr (F::kWide) {
+                    uint32_t pw[2][4][K == 4 ? 4 : 3];
 #pragma unroll
-                for (int h = 0; h < 2; h++)
+                    for (int h = 0; h < 2; h++)
 #pragma unroll
-                    for (int tk = 0; tk < 4; tk++) {
-                        const uint32_t* tw = wt + (tk * 8 + h) * L::kTileWords;
-                        if (K == 4) {
-                            pw[h][tk][0] = tw[lane];
-                            pw[h][tk][1] = tw[prev_word];
-                            pw[h][tk][2] = reinterpret_cast<const uint16_t*>(tw)[2 * lane];        // the two 16-bit aligned
-                            pw[h][tk][3] = reinterpret_cast<const uint16_t*>(tw)[2 * lane + 1];    // windows
-                        } else {
-                            pw[h][tk][0] = tw[lw.i0];
-                            pw[h][tk][1] = tw[lw.i1];
-                            pw[h][tk][2] = LaneWords<K>::kThree ? tw[lw.i2] : 0u;
+                        for (int tk = 0; tk < 4; tk++) {
+                            const uint32_t* tw = wt + (tk * 8 + h) * L::kTileWords;
+                            if constexpr (K == 4) {
+                                pw[h][tk][0] = tw[lane];
+                                pw[h][tk][1] = tw[prev_word];
+                                pw[h][tk][2] = reinterpret_cast<const uint16_t*>(tw)[2 * lane];        // the two 16-bit aligned
+                                pw[h][tk][3] = reinterpret_cast<const uint16_t*>(tw)[2 * lane + 1];    // windows
+                            } else {
+                                pw[h][tk][0] = tw[lw.i0];
+                                pw[h][tk][1] = tw[lw.i1];
+                                pw[h][tk][2] = LaneWords<K>::kThree ? tw[lw.i2] : 0u;
+                            }
                         }
-                    }
-                if (vb >= 0) wait(&empty[vb & (kTsStages - 1)], (uint32_t)(vb / kTsStages) & 1u);
-                tc_fence_after_sync();
+                    await_operand();
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    uint32_t frag[16];
+                    for (int h = 0; h < 2; h++) {
+                        uint32_t frag[16];
 #pragma unroll
-                    for (int tk = 0; tk < 4; tk++) {
-                        uint32_t cw[8];
-                        if constexpr (K == 4) lane_codewords_k4_halves(pw[h][tk][0], pw[h][tk][1], pw[h][tk][2], pw[h][tk][3], cw);
-                        else lane_codewords<K>(pw[h][tk][0], pw[h][tk][1], pw[h][tk][2], lw.sh, cw);
-                        frag[4 * tk + 0] = decode_pair_rt<CB>(cw[0], cw[1], xc);
-                        frag[4 * tk + 1] = decode_pair_rt<CB>(cw[4], cw[5], xc);
-                        frag[4 * tk + 2] = decode_pair_rt<CB>(cw[2], cw[3], xc);
-                        frag[4 * tk + 3] = decode_pair_rt<CB>(cw[6], cw[7], xc);
+                        for (int tk = 0; tk < 4; tk++) {
+                            const auto& p = pw[h][tk];
+                            uint32_t cw[8];
+                            if constexpr (K == 4) lane_codewords_k4_halves(p[0], p[1], p[2], p[3], cw);
+                            else lane_codewords<K>(p[0], p[1], p[2], lw.sh, cw);
+                            tile_frag(cw, frag + 4 * tk);
+                        }
+                        tmem_st_16x32cols(a_tmem + ((uint32_t)(16 * h) << 16), frag);
                     }
-                    tmem_st_16x32cols(tmem_base + ((uint32_t)(32 * q + 16 * h) << 16) + F::kACol0 + 32 * st, frag);
+                } else {
+#pragma unroll 1
+                    for (int h = 0; h < 2; h++) {
+                        uint32_t frag[16];
+#pragma unroll
+                        for (int tk = 0; tk < 4; tk++) {
+                            const uint32_t* tw = wt + (tk * 8 + h) * L::kTileWords;
+                            uint32_t cw[8];
+                            if constexpr (K == 4) lane_codewords_k4(tw[lane], tw[prev_word], cw);
+                            else lane_codewords<K>(tw[lw.i0], tw[lw.i1], LaneWords<K>::kThree ? tw[lw.i2] : 0u, lw.sh, cw);
+                            tile_frag(cw, frag + 4 * tk);
+                        }
+                        if (h == 0) await_operand();
+                        tmem_st_16x32cols(a_tmem + ((uint32_t)(16 * h) << 16), frag);
+                    }
                 }
                 // Only now is it certain that the packed words have been read: the stores above depend on them.  (With
                 // the slot given back before the wait for `empty`, some loads were found to take place after it, and
-                // to see the words of eight k-steps later.)
+                // to see the words of a later k-step.)
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&w_empty[st]));
+                if (lane == 0) mbar_arrive(smem_u32(&w_empty[ws]));
+                if ((ws += kTsSets) >= nw) { ws = set; w_par ^= 1u; }
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -525,11 +622,6 @@ __global__ void __launch_bounds__(kTsThreads, 1)
             // ---- finish the tile: what it needs from global memory first ----
             const int out = 32 * q + lane;                         // this thread's column of the tile
             const int n16 = (sg.rows + 15) >> 4;
-            auto out_row = [&](int tg) {                           // output row of this thread's token
-                const int row = 128 * tg + out, grow = sg.m0 + row + sg.y_row_delta;
-                return a.y_row_map && row < sg.rows ? a.y_row_map[grow] : grow;
-            };
-            int orow = out_row(0);
             // a shared tile's first and last contributor (64-bit divisions, done behind the last MMAs)
             int cf = 0, cl = 0, slot_first = 0;
             if (n_steps != nks && dt == 0) {
@@ -551,6 +643,64 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&d_empty[db]));
             };
+            if constexpr (F::kJoint) {
+                // The tile's CTAs share its tokens out, sixteen at a time: chunk ch is CTA ch % n's.  The sums go to their
+                // owners as they lie in tensor memory, [source][chunk][four tokens][column].
+                const int n = a.ts_joint, rank = (int)(blockIdx.x % (unsigned)n), most = (a.ts_tok / 16 + n - 1) / n;
+                cluster_wait();
+                for (int ch = set; ch < n16; ch += kTsSets) {
+                    const int owner = ch % n;
+                    if (owner == rank) continue;
+                    float f[16];
+                    tmem_ld_16cols(lane_base + 16 * ch, f);
+                    const int src = rank < owner ? rank : rank - 1;
+                    const uint32_t dst = cluster_address(smem_u32(recv) + (uint32_t)(((src * most + ch / n) * 4 * kTsOuts + out) * 16), owner);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) st_cluster_f32x4(dst + i * kTsOuts * 16, make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]));
+                }
+                __syncwarp();
+                cluster_sync();
+                const int own = n16 > rank ? (n16 - rank + n - 1) / n : 0;
+                if (own == 0) continue;                            // (nothing follows: a CTA has one tile)
+                for (int o = set; o < own; o += kTsSets) {
+                    float v[16], f[16];
+                    tmem_ld_16cols(lane_base + 16 * (rank + o * n), v);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) f[i] = 0.f;
+                    for (int j = 0; j < n; j++) {                  // in CTA order
+                        if (j == rank) {
+#pragma unroll
+                            for (int i = 0; i < 16; i++) f[i] += v[i];
+                            continue;
+                        }
+                        const float4* part = reinterpret_cast<const float4*>(recv) + ((j < rank ? j : j - 1) * most + o) * 4 * kTsOuts + out;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const float4 u = part[i * kTsOuts];
+                            f[4 * i] += u.x; f[4 * i + 1] += u.y; f[4 * i + 2] += u.z; f[4 * i + 3] += u.w;
+                        }
+                    }
+                    uint32_t hv[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) hv[i] = h2_as_u32(__floats2half2_rn(f[2 * i], f[2 * i + 1]));
+                    uint8_t* row = y_buf + (o >> 2) * 16384 + out * 128;
+                    const int piece = 2 * (o & 3), sw = out & 7;
+                    *reinterpret_cast<uint4*>(row + ((piece ^ sw) << 4)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+                    *reinterpret_cast<uint4*>(row + (((piece + 1) ^ sw) << 4)) = make_uint4(hv[4], hv[5], hv[6], hv[7]);
+                }
+                fence_proxy_async_smem();
+                tc_fence_before_sync();
+                named_bar_sync(1, 512);
+                if (warp == kTsFirstDecodeWarp) {
+                    tc_fence_after_sync();
+                    if (elect_one()) rotate_tile(d_tmem, smem_u32(y_buf), smem_u32(h_mat), smem_u32(h_full));
+                    __syncwarp();
+                }
+                const int row = 16 * (rank + (out >> 4) * n) + (out & 15);       // lane = token now
+                const bool used = out < 16 * own && row < sg.rows;
+                store_rotated(a, sg, used, sg.m0 + row + sg.y_row_delta, lane_base, set, h_full, hpar, wait, [] {});
+                continue;
+            }
             bool finish = true;
             int c_first = 0, n_contrib = 1;
             if (n_steps != nks) {
@@ -636,75 +786,13 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                     named_bar_sync(1, 512);
                     if (warp == kTsFirstDecodeWarp) {
                         tc_fence_after_sync();
-                        const uint64_t yd = smem_desc_mn_sw128(smem_u32(y_buf)), hd = smem_desc_sw128(smem_u32(h_mat));
-                        if (elect_one()) {
-#pragma unroll
-                            for (int kk = 0; kk < 8; kk++)
-                                tc_mma_f16(d_tmem, yd + 128 * kk, hd + (kk >> 2) * 1024 + (kk & 3) * 2,
-                                           mma_idesc_f16(128, 128) | kIdescMajorA, kk > 0 ? 1u : 0u);
-                            tc_commit(smem_u32(h_full));
-                        }
+                        if (elect_one()) rotate_tile(d_tmem, smem_u32(y_buf), smem_u32(h_mat), smem_u32(h_full));
                         __syncwarp();
                     }
                     const bool used = 128 * tg + out < sg.rows;    // lane = token now
-                    __half* yp = nullptr;
-                    auto address = [&]() {
-                        if (!used) return;
-                        const int col0 = sg.y_col + 32 * set;
-                        if (a.n_peer > 0) {      // the row belongs to the GPU that holds its token
-                            const int pr = orow / a.rows_per_peer;
-                            yp = a.y_peer[pr] + (int64_t)(orow - pr * a.rows_per_peer) * a.y_row_stride + col0;
-                        } else {
-                            yp = !TABLE && a.n_members > 1 ? a.member_y[sg.member] + (int64_t)orow * a.member_stride[sg.member] + col0
-                                                           : a.y + (int64_t)orow * a.y_row_stride + col0;
-                        }
-                    };
-                    // (here it is done behind the product; SwitchGLU of 200 tokens: 280 us with it further down, 290 here)
-                    if (!TABLE) address();
-                    // The output scales are fetched behind the product: between the stores below, which might alias
-                    // them, the loads would be made and waited for one after the other, and a prefetch into L1 does
-                    // not help (SwitchGLU of 200 tokens 298 -> 284 us).
-                    uint4 sv[4];
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        sv[c] = a.svh ? ldg_nc_128(a.svh + sg.sv_off + 32 * set + 8 * c)
-                                      : make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
-                    wait(h_full, hpar);
+                    store_rotated(a, sg, used, sg.m0 + 128 * tg + out + sg.y_row_delta, lane_base, set, h_full, hpar, wait,
+                                  [&] { if (128 * tg + 128 >= sg.rows) release_d(); });    // the last reads of D
                     hpar ^= 1u;
-                    tc_fence_after_sync();
-                    float f[32];
-                    tmem_ld_32cols(lane_base + 32 * set, f);
-                    if (128 * tg + 128 >= sg.rows) release_d();    // the last reads of D
-                    if (TABLE) address();
-                    if (used) {
-                        const uint64_t scale = f32x2(EXL3_HAD_SCALE, EXL3_HAD_SCALE);
-                        uint4 held16 = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-                        for (int c = 0; c < 4; c++) {
-                            const uint32_t sw4[4] = {sv[c].x, sv[c].y, sv[c].z, sv[c].w};
-                            uint32_t h[4];
-#pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                const float2 w2 = __half22float2(u32_as_h2(sw4[i]));
-                                h[i] = f16_pair(mul_f32x2(mul_f32x2(f32x2(f[8 * c + 2 * i], f[8 * c + 2 * i + 1]), scale), f32x2(w2.x, w2.y)));
-                            }
-                            if (a.bias) {
-                                const uint4 bv = __ldg(reinterpret_cast<const uint4*>(a.bias + sg.sv_off + 32 * set + 8 * c));
-                                const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-                                for (int i = 0; i < 4; i++) h[i] = h2_as_u32(__hadd2(u32_as_h2(h[i]), u32_as_h2(bw[i])));
-                            }
-                            const uint4 ov = make_uint4(h[0], h[1], h[2], h[3]);
-                            if (!a.y_wide) {
-                                *reinterpret_cast<uint4*>(yp + 8 * c) = ov;
-                            } else if (c & 1) {
-                                st_global_256(yp + 8 * (c - 1), held16, ov);   // whole sectors, also into another GPU
-                            } else {
-                                held16 = ov;
-                            }
-                        }
-                    }
-                    if (128 * tg + 128 < sg.rows) orow = out_row(tg + 1);
                 }
             }
             release_d();
@@ -714,26 +802,23 @@ __global__ void __launch_bounds__(kTsThreads, 1)
         }
     }
     __syncwarp();
+    if (F::kJoint && warp < kTsFirstDecodeWarp) {              // all threads take part in the cluster's barriers
+        cluster_wait();
+        cluster_sync();
+    }
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 2) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
-    if (a.n_peer > 0 && tid == 0) {
-        // Rows were stored into other GPUs' memory: every CTA is counted on a local counter (the
-        // barrier above orders the CTA's stores before this thread's fence), and the CTA that
-        // completes the count announces this GPU's rows to every peer.
-        __threadfence();
-        const unsigned done = atomicAdd(a.done_ctr, 1u) + 1u;
-        if (done == gridDim.x) {
-            atomicExch(a.done_ctr, 0u);           // re-armed for the next launch on this workspace
-            __threadfence_system();
-            for (int p = 0; p < a.n_peer; p++)
-                asm volatile("red.relaxed.sys.global.add.u32 [%0], 1;" ::"l"(a.ctr_peer[p]) : "memory");
-        }
-    }
 }
+
+}  // namespace exl3
+
+#include "exl3_gemm_tiles.cuh"
+
+namespace exl3 {
 
 // ---- host side ----------------------------------------------------------------------------------
 
@@ -742,75 +827,138 @@ inline size_t gemm_tile_partial_bytes(int tok, int ctas) { return (size_t)ctas *
 
 TsPlan gemm_plan(int64_t rows, int64_t tiles_n, int nks, int sms, size_t partial_bytes, int tok, int tok_wide);
 
-template <int K, int CB, bool TABLE>
-static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, cudaStream_t s)
+inline int gemm_tensor_maps(CUtensorMap* tm_x, CUtensorMap* tm_w, const GemmArgs& a, int tile_words, const __half* xh, const uint32_t* trellis)
 {
-    using L = TsLayout<K>;
-    static bool attr_set[kMaxDevices] = {};
+    const uint64_t in = (uint64_t)a.t_in * 16;
+    const uint64_t xdims[2] = {in, (uint64_t)a.xh_rows};
+    const uint64_t xstrides[1] = {in * 2};
+    const uint32_t xbox[2] = {64u, (uint32_t)a.ts_box_rows};
+    const int rc = make_tensor_map(tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, xh, xdims, xstrides, xbox, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    const uint64_t dims[3] = {(uint64_t)tile_words, (uint64_t)a.t_out, (uint64_t)a.t_in};
+    const uint64_t strides[2] = {(uint64_t)tile_words * 4, (uint64_t)a.t_out * tile_words * 4};
+    const uint32_t box[3] = {(uint32_t)tile_words, 8u, (uint32_t)kTsStepTiles};
+    return make_tensor_map(tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, trellis, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
+// Makes a kernel's whole shared memory available, once per device.
+template <typename Kernel> static int gemm_shared_memory(Kernel kernel, bool (&done)[kMaxDevices])
+{
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxDevices) return EXL3_E_UNSUPPORTED;
-    if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, TS_AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
-        if (e == cudaSuccess && !TABLE)
-            e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, TABLE ? TS_AHEAD : TS_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
-        if (e == cudaSuccess && !TABLE)
-            e = cudaFuncSetAttribute(gemm_kernel<K, CB, TABLE, TABLE ? TS_AHEAD : TS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes);
-        if (e != cudaSuccess) return note_cuda(e);
-        attr_set[dev] = true;
+    if (done[dev]) return EXL3_OK;
+    const int rc = note_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmemBytes));
+    if (rc == EXL3_OK) done[dev] = true;
+    return rc;
+}
+
+struct JointLaunch {
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = {};
+    JointLaunch(int grid, int n, cudaStream_t s)
+    {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)n;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(kTsThreads);
+        cfg.dynamicSmemBytes = kTsSmemBytes;
+        cfg.stream = s;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
     }
+};
+// Clusters of n CTAs that the device holds at a time (a cluster lies in one part of the chip); asked once.
+template <typename Kernel> static int gemm_clusters(Kernel kernel, int n)
+{
+    static int known[kMaxDevices][kTsJointMost + 1] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= kMaxDevices || n < 1 || n > kTsJointMost) return 0;
+    int& k = known[dev][n];
+    if (k == 0) {
+        JointLaunch l(n, n, nullptr);
+        l.cfg.numAttrs = 1;
+        int c = 0;
+        if (cudaOccupancyMaxActiveClusters(&c, kernel, &l.cfg) != cudaSuccess) { cudaGetLastError(); c = 0; }
+        k = c > 0 ? c : -1;
+    }
+    return k;
+}
+
+template <int K, int CB> static int launch_gemm_tiles_t(GemmArgs a, const __half* xh, const uint32_t* trellis, cudaStream_t s)
+{
+    static bool attr_set[kMaxDevices] = {};
+    int rc = gemm_shared_memory(gemm_tiles_kernel<K, CB>, attr_set);
+    if (rc) return rc;
+    a.cb_xor = 0x3B603B60u;
+    a.ts_split = 0;
+    // Rows of a tile: what nearly all tiles need if the caller says how many rows a tile has on average (the activation
+    // ring is as deep as its stages are small, and up to 192 there are two accumulators), the table's 256 if not.  Tiles
+    // with more are taken in parts.
+    a.ts_tok = kTsMaxTok;
+    a.ts_box_rows = 64;
+    if (a.rows_hint > 0 && a.rows_hint < 200) {
+        const double most = a.rows_hint + 2.5 * std::sqrt((double)a.rows_hint);
+        a.ts_tok = std::max(64, std::min(kTsMaxTok, ((int)most + 31) / 32 * 32));
+        a.ts_box_rows = 32;
+    }
+    a.n_items = 2 * a.n_tiles_tab * ((kTsMaxTok + a.ts_tok - 1) / a.ts_tok);
+    a.ts_x_bytes = (a.ts_tok + a.ts_box_rows - 1) / a.ts_box_rows * a.ts_box_rows * 128;
+    a.stages = std::min(kGtMaxXStages, (kTsSmemBytes - gt_x_off<K>()) / a.ts_x_bytes);
+    a.ts_dbuf = a.ts_tok <= kGtTokTwice ? 2 : 1;
+    CUtensorMap tm_x, tm_w;
+    rc = gemm_tensor_maps(&tm_x, &tm_w, a, TsLayout<K>::kTileWords, xh, trellis);
+    if (rc) return rc;
+    // an odd stride: which items are in use repeats with a period of 2 or 4
+    const int grid = std::min(a.n_items, (device_sm_count() - 1) | 1);
+    return launch_kernel(gemm_tiles_kernel<K, CB>, dim3((unsigned)grid), dim3(kGtThreads), kTsSmemBytes, s, true, a, tm_x, tm_w);
+}
+
+template <int K, int CB> static int launch_gemm_t(GemmArgs a, const __half* xh, const uint32_t* trellis, cudaStream_t s)
+{
+    using L = TsLayout<K>;
+    static bool attr_set[4][kMaxDevices] = {};
+    int rc = gemm_shared_memory(gemm_kernel<K, CB, TS_PLAIN>, attr_set[TS_PLAIN]);
+    if (rc == EXL3_OK) rc = gemm_shared_memory(gemm_kernel<K, CB, TS_AHEAD>, attr_set[TS_AHEAD]);
+    if (rc == EXL3_OK) rc = gemm_shared_memory(gemm_kernel<K, CB, TS_WIDE>, attr_set[TS_WIDE]);
+    if (rc == EXL3_OK) rc = gemm_shared_memory(gemm_kernel<K, CB, TS_JOINT>, attr_set[TS_JOINT]);
+    if (rc) return rc;
     a.cb_xor = 0x3B603B60u;
     const int sms = device_sm_count(), nks = a.t_in / kTsStepTiles;
-    int grid, mode = TS_AHEAD;
-    a.ts_split = 0;
-    if (TABLE) {
-        // Rows of a tile: what nearly all tiles need if the caller says how many rows a tile has on average
-        // (the activation ring is as deep as its stages are small), the table's 256 if not.
-        a.ts_tok = kTsMaxTok;
-        a.ts_box_rows = 64;
-        if (a.rows_hint > 0 && a.rows_hint < 200) {
-            const double most = a.rows_hint + 2.5 * std::sqrt((double)a.rows_hint);
-            a.ts_tok = std::max(128, std::min(kTsMaxTok, ((int)most + 31) / 32 * 32));
-            a.ts_box_rows = 32;
-        }
-        a.n_items = 2 * a.n_tiles_tab * (a.ts_tok < kTsMaxTok ? 2 : 1);
-        // an odd stride: which items are in use repeats with a period of 2 or 4
-        grid = std::min(a.n_items, (sms - 1) | 1);
-    } else {
-        a.tiles_n = a.t_out / 8;
-        const TsPlan plan = gemm_plan(a.m, a.tiles_n, nks, sms, a.ts_partial_bytes, L::kTok, L::kTokWide);
-        a.ts_tok = plan.tok;
-        a.tiles_m = plan.tiles_m;
-        if (!ts_countable(plan, a.tiles_n, nks)) return EXL3_E_SHAPE;
-        a.n_items = a.tiles_m * a.tiles_n;
-        a.ts_box_rows = a.ts_tok > 256 ? a.ts_tok / 2 : a.ts_tok;                  // (a box has at most 256 rows)
-        a.ts_split = plan.split;
-        grid = plan.grid;
-        mode = plan.wide ? TS_WIDE : a.n_items >= 2 * grid ? TS_AHEAD : TS_PLAIN;
-    }
+    a.tiles_n = a.t_out / 8;
+    TsPlan plan = gemm_plan(a.m, a.tiles_n, nks, sms, a.ts_partial_bytes, L::kTok, L::kTokWide);
+    a.ts_joint = ts_joint(plan, a.tiles_n, nks, sms);
+    while (a.ts_joint && gemm_clusters(gemm_kernel<K, CB, TS_JOINT>, a.ts_joint) < plan.tiles_m * a.tiles_n)
+        a.ts_joint = ts_joint(plan, a.tiles_n, nks, sms, a.ts_joint - 1);
+    if (a.ts_joint) { plan.grid = (int)(plan.tiles_m * a.tiles_n) * a.ts_joint; plan.split = 1; }
+    a.ts_tok = plan.tok;
+    a.tiles_m = plan.tiles_m;
+    if (!ts_countable(plan, a.tiles_n, nks)) return EXL3_E_SHAPE;
+    a.n_items = a.tiles_m * a.tiles_n;
+    a.ts_box_rows = a.ts_tok > 256 ? a.ts_tok / 2 : a.ts_tok;                      // (a box has at most 256 rows)
+    a.ts_split = plan.split;
+    const int mode = a.ts_joint ? TS_JOINT : plan.wide ? TS_WIDE : a.n_items >= 2 * plan.grid ? TS_AHEAD : TS_PLAIN;
     a.ts_x_bytes = (a.ts_tok + a.ts_box_rows - 1) / a.ts_box_rows * a.ts_box_rows * 128;
-    a.stages = std::min(kTsStages, (mode == TS_WIDE ? L::template xroom<TS_WIDE>() : L::template xroom<TS_AHEAD>()) / a.ts_x_bytes);
+    // Ring x has up to eight stages beside eight of ring w (four in the wide form); what is left goes to ring w, up to three
+    // stages per set (more do not pay: 28 stages delay the first activations behind them, 17408 -> 512 16.4 -> 17.4 us).
+    a.ts_recv_bytes = a.ts_joint ? (a.ts_tok / 16 + a.ts_joint - 1) / a.ts_joint * (a.ts_joint - 1) * 8192 : 0;   // (at most 64 KiB)
+    const int room = L::kRoom - a.ts_recv_bytes;
+    a.stages = std::min(kTsStages, (room - (mode == TS_WIDE ? 4 : 8) * L::kWBytes) / a.ts_x_bytes);
+    a.ts_w_stages = std::min(kTsMaxWStages, (room - a.stages * a.ts_x_bytes) / L::kWBytes) / kTsSets * kTsSets;
     a.ts_dbuf = a.ts_tok <= 128 ? 2 : 1;
     CUtensorMap tm_x, tm_w;
-    {
-        const uint64_t in = (uint64_t)a.t_in * 16;
-        const uint64_t xdims[2] = {in, (uint64_t)a.xh_rows};
-        const uint64_t xstrides[1] = {in * 2};
-        const uint32_t xbox[2] = {64u, (uint32_t)a.ts_box_rows};
-        int rc = make_tensor_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, xh, xdims, xstrides, xbox,
-                                 CU_TENSOR_MAP_SWIZZLE_128B);
-        if (rc) return rc;
-        const uint64_t dims[3] = {(uint64_t)L::kTileWords, (uint64_t)a.t_out, (uint64_t)a.t_in};
-        const uint64_t strides[2] = {(uint64_t)L::kTileWords * 4, (uint64_t)a.t_out * L::kTileWords * 4};
-        const uint32_t box[3] = {(uint32_t)L::kTileWords, 8u, (uint32_t)kTsStepTiles};
-        rc = make_tensor_map(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, trellis, dims, strides, box,
-                             CU_TENSOR_MAP_SWIZZLE_NONE);
-        if (rc) return rc;
+    rc = gemm_tensor_maps(&tm_x, &tm_w, a, L::kTileWords, xh, trellis);
+    if (rc) return rc;
+    if (mode == TS_JOINT) {
+        const JointLaunch l(plan.grid, a.ts_joint, s);
+        return note_cuda(cudaLaunchKernelEx(&l.cfg, gemm_kernel<K, CB, TS_JOINT>, (const GemmArgs)a, (const CUtensorMap)tm_x, (const CUtensorMap)tm_w));
     }
-    const auto kernel = TABLE || mode == TS_AHEAD ? gemm_kernel<K, CB, TABLE, TS_AHEAD>
-                        : mode == TS_WIDE         ? gemm_kernel<K, CB, TABLE, TABLE ? TS_AHEAD : TS_WIDE>
-                                                  : gemm_kernel<K, CB, TABLE, TABLE ? TS_AHEAD : TS_PLAIN>;
-    return launch_kernel(kernel, dim3((unsigned)grid), dim3(kTsThreads), kTsSmemBytes, s, true, a, tm_x, tm_w);
+    const auto kernel = mode == TS_AHEAD ? gemm_kernel<K, CB, TS_AHEAD> : mode == TS_WIDE ? gemm_kernel<K, CB, TS_WIDE> : gemm_kernel<K, CB, TS_PLAIN>;
+    return launch_kernel(kernel, dim3((unsigned)plan.grid), dim3(kTsThreads), kTsSmemBytes, s, true, a, tm_x, tm_w);
 }
 
 template <int K>
@@ -818,11 +966,11 @@ int launch_gemm_k(const GemmArgs& a, int cb, const __half* xh, const uint32_t* t
 {
     switch (cb) {
         case CB_3INST:
-            return a.tile_tab ? launch_gemm_t<K, CB_3INST, true>(a, xh, trellis, s) : launch_gemm_t<K, CB_3INST, false>(a, xh, trellis, s);
+            return a.tile_tab ? launch_gemm_tiles_t<K, CB_3INST>(a, xh, trellis, s) : launch_gemm_t<K, CB_3INST>(a, xh, trellis, s);
         case CB_MCG:
-            return a.tile_tab ? launch_gemm_t<K, CB_MCG, true>(a, xh, trellis, s) : launch_gemm_t<K, CB_MCG, false>(a, xh, trellis, s);
+            return a.tile_tab ? launch_gemm_tiles_t<K, CB_MCG>(a, xh, trellis, s) : launch_gemm_t<K, CB_MCG>(a, xh, trellis, s);
         case CB_MUL1:
-            return a.tile_tab ? launch_gemm_t<K, CB_MUL1, true>(a, xh, trellis, s) : launch_gemm_t<K, CB_MUL1, false>(a, xh, trellis, s);
+            return a.tile_tab ? launch_gemm_tiles_t<K, CB_MUL1>(a, xh, trellis, s) : launch_gemm_t<K, CB_MUL1>(a, xh, trellis, s);
         default: return EXL3_E_CODEBOOK;
     }
 }

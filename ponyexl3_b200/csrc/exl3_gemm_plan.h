@@ -101,6 +101,22 @@ inline TsPlan ts_plan(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, 
     return best;
 }
 
+// CTAs per tile where a tile's CTAs should be a cluster (two to eight of them, of one tile and at least four k-steps each)
+// instead of what the plan says, or 0: up to 128 tokens, and where the longer ranges of k-steps of a whole number of CTAs
+// per tile cost less than the hand-over through the workspace.  us at 9, 40, 77, 128 rows, through the workspace / as
+// clusters, K = 4: 5120 x 5120 (three) 15.5, 19.3, 17.7, 19.7 / 15.4, 18.5, 15.9, 17.1; 4096 x 1024 (eight) 10.8, 15.6, 16.5, 22.2 /
+// 10.6, 11.6, 11.3, 12.1; 2048 x 2048 (eight) 9.4, 12.7, 13.0, 14.0 / 9.3, 10.6, 10.3, 11.4.
+constexpr int kTsJointCost = 4, kTsJointMost = 8, kTsJointTok = 128;
+inline int ts_joint(const TsPlan& p, int64_t tiles_n, int nks, int sms, int most = kTsJointMost)
+{
+    const int64_t tiles = p.tiles_m * tiles_n;
+    if (!p.split || p.tok > kTsJointTok || 2 * tiles > sms) return 0;
+    const int n = (int)std::min<int64_t>(std::min<int64_t>(most, sms / tiles), nks / 4);
+    if (n < 2) return 0;
+    const int64_t shared = ts_slowest(tiles * nks, nks, p.grid, INT64_MAX), joint = (nks + n - 1) / n + kTsJointCost;
+    return joint <= shared ? n : 0;
+}
+
 // The kernel counts tiles, k-steps where tiles are shared, and the k-steps of one CTA in 32 bits.
 inline bool ts_countable(const TsPlan& p, int64_t tiles_n, int nks)
 {

@@ -186,6 +186,9 @@ struct GemmArgs {
     int ts_tok;               // tokens per output tile
     int ts_x_bytes;           // bytes of one stage of the activation ring
     int ts_box_rows;          // rows of one activation TMA box
+    int ts_w_stages;          // depth of the ring of packed tiles (dense launches)
+    int ts_joint;             // CTAs of a tile, which are a cluster; 0: they are not
+    int ts_recv_bytes;        // shared memory for the sums that they exchange
     int ts_dbuf;              // accumulators in tensor memory
     // sibling groups: member i has the column blocks [member_end[i - 1], member_end[i]) of the trellis, the
     // rotated rows [i m, (i + 1) m) and an output matrix of its own

@@ -7,6 +7,11 @@
 using namespace exl3;
 
 // out: tok, tiles_m, grid, split, wide.  Shared tiles have room up to room_tok tokens.
+extern "C" int emul_joint(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok, int most)
+{
+    return ts_joint(ts_plan(rows, tiles_n, nks, sms, tok, tok_wide, room_tok), tiles_n, nks, sms, most);
+}
+
 extern "C" void emul_plan(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok, int* out)
 {
     const TsPlan p = ts_plan(rows, tiles_n, nks, sms, tok, tok_wide, room_tok);

@@ -89,3 +89,22 @@ def test_a_plan_costs_less_than_a_launch(emul):
             emul.emul_plan(rows, tiles_n, nks, 148, 256, 384, 384, out)
             n += 1
     assert (time.perf_counter() - t0) / n < 200e-6
+
+
+def test_clusters_of_a_tile(emul):
+    """Where the CTAs of a tile become a cluster: up to eight of them with at least four k-steps each, all on the chip at a time, no
+    tile of more than 128 tokens, and never more CTAs than asked for."""
+    emul.emul_joint.argtypes = [ctypes.c_int64, ctypes.c_int64] + [ctypes.c_int] * 6
+    rng = random.Random(7)
+    taken = set()
+    for _ in range(3000):
+        rows, tiles_n, nks = rng.randint(9, 400), rng.randint(1, 160), 2 * rng.randint(1, 136)
+        most = rng.randint(1, 8)
+        args = (rows, tiles_n, nks, 148, 256, 384, rng.choice([0, 384]))
+        tok, tiles_m, _, split, _ = _plan(emul.emul_plan, *args)
+        n = emul.emul_joint(*args, most)
+        taken.add(n)
+        assert n == 0 or (2 <= n <= most and 4 * n <= nks and split and tok <= 128 and tiles_m * tiles_n * n <= 148), (args, n)
+    assert taken == {0, 2, 3, 4, 5, 6, 7, 8}
+    assert emul.emul_joint(77, 40, 80, 148, 256, 384, 384, 8) == 3      # 5120 x 5120: three CTAs of 27 k-steps
+    assert emul.emul_joint(77, 136, 80, 148, 256, 384, 384, 8) == 0     # 5120 x 17408: a CTA per tile

@@ -95,6 +95,24 @@ def test_gemm_tiles_shared_between_ctas(mod, oracle, rows, inf, outf, k, cb):
     assert mod.ops.Workspace.get(torch.device("cuda"), 1, 128).status() == 0
 
 
+@pytest.mark.parametrize("rows", [9, 16, 33, 100, 128])
+@pytest.mark.parametrize("inf,outf,k,cb", [
+    (2048, 384, 4, 0),          # eight CTAs of four k-steps per tile; more CTAs than pieces of 16 tokens, and as many
+    (2048, 2560, 5, 1),         # seven
+    (1152, 5120, 3, 2),         # three
+    (896, 8192, 8, 0),          # two, the deepest packed tiles
+])
+def test_gemm_tiles_of_clusters(mod, oracle, rows, inf, outf, k, cb):
+    """The CTAs of a tile as a cluster that shares out its tokens: repeatable, and nothing left behind in shared memory."""
+    layer = _layer(mod, k, inf, outf, seed=rows + inf, cb=cb, bias=rows % 2 == 1)
+    x = np.random.default_rng(rows).standard_normal((rows, inf)).astype(np.float16)
+    _check(mod, oracle, layer, x)
+    m = mod.EXL3Linear(layer)
+    xd = torch.from_numpy(x).cuda()
+    first = m(xd)
+    assert all(torch.equal(m(xd), first) for _ in range(3))
+
+
 # Shapes of each form of the kernel (test_gemm_plan.py checks that the plan takes it): tiles of more than the
 # ordinary number of tokens, whose MMAs are two halves; two and more ordinary tiles per CTA; hardly more than one.
 FORMS = [
