@@ -69,6 +69,9 @@ extern "C" {
                                    the gate|up output as it is, with no activation launch in between
                                    (the reference folds the GLU into its down kernel the same way,
                                    ponyexl3/mlx/exl3_moe.py:374-422; activations :62-75) */
+#define EXL3_FLAG_ROW_PAIRS 16u /* exl3_moe_prefill_tables: the gate row of sorted position p is rotated row p, its up row
+                                   n_pairs + p.  exl3_gemm_tiles: rows r and r + xh_rows / 2 have the same row_src (which
+                                   is required, and xh_rows even), so that a row of x is read once for both */
 
 typedef void* exl3_stream_t;    /* cudaStream_t */
 
@@ -205,7 +208,7 @@ EXL3_API int exl3_gemm_members(const void* x, int x_dtype, int64_t rows, int64_t
  * y row that computed row r + y_row_delta is stored to — the last projection of a MoE call
  * writes straight back into (token, slot) order instead of sorted order.
  * flags >> 16 (optional): average rows of the tiles in use, which sizes the stages of the activation
- * ring; any value gives the same results.
+ * ring; any value gives the same results.  EXL3_FLAG_ROW_PAIRS: see there.
  * Replaces the segmented trellis GEMM of the reference, inner_mm_seg_mlx with its expert block
  * table, ponyexl3/mlx/gemv_metal.py:1519-1741 and ponyexl3/mlx/exl3_moe.py:79-99,685-768. */
 EXL3_API int exl3_gemm_tiles(const void* x, int x_dtype, int64_t x_row_stride, int64_t xh_rows,
@@ -381,7 +384,7 @@ EXL3_API int exl3_moe_decode_tables_range(const void* indices, int index_bytes, 
  *   row_src_gu, suh_row_gu (2*n_pairs): the rotated rows of the gate/up launch; an expert with
  *     sorted positions [seg, seg + cnt) has its gate rows at [2 seg, 2 seg + cnt) and its up rows
  *     at [2 seg + cnt, 2 seg + 2 cnt), and both kinds of tiles store to the [gate | up] row of
- *     the sorted position;
+ *     the sorted position (EXL3_FLAG_ROW_PAIRS: all gate rows, then all up rows);
  *   suh_row_dn (n_pairs); tiles_gu (2 * slots * ceil(h/256), 8): gate tiles then up tiles;
  *   tiles_dn (slots * ceil(d/256), 8); slots = n_pairs / 256 + num_experts (unused ones are empty).
  * n_pairs <= 2^20, num_experts <= 1024. */
@@ -411,7 +414,7 @@ EXL3_API int exl3_moe_prefill_tables_range(const void* indices, int index_bytes,
  * NULL): (n_tiles, 16K) the packed tiles as stored on disk (pack_trellis_tile,
  * ponyexl3/ref/trellis.py:12-50).  max_pins: pinned passes after the free one (the reference's
  * default is 4).  The workspace holds the back-pointers (and, at K = 1 and for weights beyond 1e13, the
- * costs) of the tiles in flight, 8.5 MiB each, and two tile counters: exl3_encode_workspace_bytes(n_tiles)
+ * costs) of the tiles in flight, 8.5 MiB each, and a few counters: exl3_encode_workspace_bytes(n_tiles)
  * is enough for one tile per SM; a smaller workspace (at least one slot) only lowers the number of tiles in flight. */
 EXL3_API size_t exl3_encode_workspace_bytes(int64_t n_tiles);
 EXL3_API int exl3_encode_tiles(const float* w, int64_t n_tiles, int k, int cb, int max_pins, uint16_t* states,

@@ -204,6 +204,9 @@ __global__ void __launch_bounds__(256)
 // the rows of a sibling group that one by one would be few enough for the butterfly kernel, which does not round
 // it (multipliers of 0.5 to 1.5, 40 rows: 5.0e-4 off the oracle without, 7e-5 with it).  A group of 5120 + 2 x 1024
 // columns and 24 to 63 rows takes 19.4 .. 21.0 us without, 19.6 .. 21.2 with it, 23.1 .. 27.2 by the butterfly kernel.
+//
+// COPIES: output rows r, r + base, r + 2 base, .. are the same row of x with other multipliers (gate and up of a
+// SwitchGLU, the members of a sibling group), and a block's loads of x serve all of them.
 template <typename T> struct Load8;
 template <> struct Load8<__half> {
     static __device__ __forceinline__ uint4 at(const __half* p) { return *reinterpret_cast<const uint4*>(p); }
@@ -243,14 +246,15 @@ __device__ __forceinline__ void split_product(uint32_t& x, uint32_t p, uint32_t&
     rest = h2_as_u32(__hfma2(x2, p2, __hneg2(h)));
 }
 
-template <typename T, bool SPLIT>
+template <typename T, bool SPLIT, bool COPIES>
 __global__ void __launch_bounds__(256, 2)
     hadamard_mma_kernel(const T* __restrict__ x, int64_t rows, int64_t n, int64_t x_row_stride,
                         const __half* __restrict__ pre, __half* __restrict__ out,
                         const int32_t* __restrict__ row_src, const int32_t* __restrict__ pre_row,
-                        const int32_t* __restrict__ rows_dev, int early_trigger, int glu, int member_rows)
+                        const int32_t* __restrict__ rows_dev, int early_trigger, int glu, int member_rows, int copies)
 {
     rotation_dependency(early_trigger);
+    if (COPIES) rows /= copies;
     if (rows_dev) {           // the number of rows in use was left on the device by an earlier kernel
         const int64_t r = *rows_dev;
         rows = r < 0 ? 0 : (r < rows ? r : rows);
@@ -275,8 +279,8 @@ __global__ void __launch_bounds__(256, 2)
         const bool ok0 = r0 < rows, ok1 = r1 < rows;
         const int64_t col = (int64_t)cb * 128 + 8 * t;
         // (see hadamard_kernel)
-        const int64_t mb0 = member_rows && ok0 ? (uint32_t)r0 / (uint32_t)member_rows : 0;
-        const int64_t mb1 = member_rows && ok1 ? (uint32_t)r1 / (uint32_t)member_rows : 0;
+        const int64_t mb0 = !COPIES && member_rows && ok0 ? (uint32_t)r0 / (uint32_t)member_rows : 0;
+        const int64_t mb1 = !COPIES && member_rows && ok1 ? (uint32_t)r1 / (uint32_t)member_rows : 0;
         uint4 xa[4], xb[4];
         {
             const int64_t s0 = ok0 ? (row_src ? row_src[r0] : r0 - mb0 * member_rows) : 0;
@@ -305,79 +309,87 @@ __global__ void __launch_bounds__(256, 2)
                 }
             }
         }
-        uint4 la[4], lb[4];                                  // SPLIT: the second parts
-        if (SPLIT && !pre)
+        const int n_copies = COPIES ? copies : 1;
+#pragma unroll 1
+        for (int v = 0; v < n_copies; v++) {
+            const int64_t o0 = COPIES ? r0 + v * rows : r0, o1 = COPIES ? r1 + v * rows : r1;
+            uint4 la[4], lb[4];                                  // SPLIT: the second parts
+            uint4 ya[4], yb[4];                                  // the products
 #pragma unroll
-            for (int q = 0; q < 4; q++) la[q] = lb[q] = make_uint4(0u, 0u, 0u, 0u);
-        if (pre) {
-            const __half* q0 = pre + (ok0 && pre_row ? (int64_t)pre_row[r0] : mb0) * n + col;
-            const __half* q1 = pre + (ok1 && pre_row ? (int64_t)pre_row[r1] : mb1) * n + col;
+            for (int q = 0; q < 4; q++) { ya[q] = xa[q]; yb[q] = xb[q]; }
+            if (SPLIT && !pre)
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const uint4 a = *reinterpret_cast<const uint4*>(q0 + 32 * q);
-                const uint4 b = *reinterpret_cast<const uint4*>(q1 + 32 * q);
-                if constexpr (SPLIT) {
-                    split_product(xa[q].x, a.x, la[q].x); split_product(xa[q].y, a.y, la[q].y);
-                    split_product(xa[q].z, a.z, la[q].z); split_product(xa[q].w, a.w, la[q].w);
-                    split_product(xb[q].x, b.x, lb[q].x); split_product(xb[q].y, b.y, lb[q].y);
-                    split_product(xb[q].z, b.z, lb[q].z); split_product(xb[q].w, b.w, lb[q].w);
-                    continue;
-                }
-                xa[q].x = h2_as_u32(__hmul2(u32_as_h2(xa[q].x), u32_as_h2(a.x)));
-                xa[q].y = h2_as_u32(__hmul2(u32_as_h2(xa[q].y), u32_as_h2(a.y)));
-                xa[q].z = h2_as_u32(__hmul2(u32_as_h2(xa[q].z), u32_as_h2(a.z)));
-                xa[q].w = h2_as_u32(__hmul2(u32_as_h2(xa[q].w), u32_as_h2(a.w)));
-                xb[q].x = h2_as_u32(__hmul2(u32_as_h2(xb[q].x), u32_as_h2(b.x)));
-                xb[q].y = h2_as_u32(__hmul2(u32_as_h2(xb[q].y), u32_as_h2(b.y)));
-                xb[q].z = h2_as_u32(__hmul2(u32_as_h2(xb[q].z), u32_as_h2(b.z)));
-                xb[q].w = h2_as_u32(__hmul2(u32_as_h2(xb[q].w), u32_as_h2(b.w)));
-            }
-        }
-        // c[2 q + s][nt]: columns 32 q' + 8 t + 4 s' + 2 nt + {0, 1} of rows g (first pair) and g + 8, for the
-        // 16-point transform of group (q, s); the butterflies turn (q, s) into (q', s')
-        uint64_t c[8][2][2];
+                for (int q = 0; q < 4; q++) la[q] = lb[q] = make_uint4(0u, 0u, 0u, 0u);
+            if (pre) {
+                const __half* q0 = pre + (ok0 && pre_row ? (int64_t)pre_row[o0] : mb0 + v) * n + col;
+                const __half* q1 = pre + (ok1 && pre_row ? (int64_t)pre_row[o1] : mb1 + v) * n + col;
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-#pragma unroll
-            for (int s = 0; s < 2; s++) {
-                const uint32_t af[4] = {s ? xa[q].z : xa[q].x, s ? xb[q].z : xb[q].x, s ? xa[q].w : xa[q].y, s ? xb[q].w : xb[q].y};
-#pragma unroll
-                for (int nt = 0; nt < 2; nt++) {
-                    float d[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_16816(d, af, hb[nt][0], hb[nt][1]);
+                for (int q = 0; q < 4; q++) {
+                    const uint4 a = *reinterpret_cast<const uint4*>(q0 + 32 * q);
+                    const uint4 b = *reinterpret_cast<const uint4*>(q1 + 32 * q);
                     if constexpr (SPLIT) {
-                        const uint32_t lf[4] = {s ? la[q].z : la[q].x, s ? lb[q].z : lb[q].x, s ? la[q].w : la[q].y, s ? lb[q].w : lb[q].y};
-                        mma_16816(d, lf, hb[nt][0], hb[nt][1]);
+                        split_product(ya[q].x, a.x, la[q].x); split_product(ya[q].y, a.y, la[q].y);
+                        split_product(ya[q].z, a.z, la[q].z); split_product(ya[q].w, a.w, la[q].w);
+                        split_product(yb[q].x, b.x, lb[q].x); split_product(yb[q].y, b.y, lb[q].y);
+                        split_product(yb[q].z, b.z, lb[q].z); split_product(yb[q].w, b.w, lb[q].w);
+                        continue;
                     }
-                    c[2 * q + s][nt][0] = f32x2(d[0], d[1]);
-                    c[2 * q + s][nt][1] = f32x2(d[2], d[3]);
+                    ya[q].x = h2_as_u32(__hmul2(u32_as_h2(ya[q].x), u32_as_h2(a.x)));
+                    ya[q].y = h2_as_u32(__hmul2(u32_as_h2(ya[q].y), u32_as_h2(a.y)));
+                    ya[q].z = h2_as_u32(__hmul2(u32_as_h2(ya[q].z), u32_as_h2(a.z)));
+                    ya[q].w = h2_as_u32(__hmul2(u32_as_h2(ya[q].w), u32_as_h2(a.w)));
+                    yb[q].x = h2_as_u32(__hmul2(u32_as_h2(yb[q].x), u32_as_h2(b.x)));
+                    yb[q].y = h2_as_u32(__hmul2(u32_as_h2(yb[q].y), u32_as_h2(b.y)));
+                    yb[q].z = h2_as_u32(__hmul2(u32_as_h2(yb[q].z), u32_as_h2(b.z)));
+                    yb[q].w = h2_as_u32(__hmul2(u32_as_h2(yb[q].w), u32_as_h2(b.w)));
                 }
             }
-        const uint64_t minus = f32x2(-1.f, -1.f), scale = f32x2(EXL3_HAD_SCALE, EXL3_HAD_SCALE);
-#pragma unroll
-        for (int h = 1; h < 8; h <<= 1)
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                if (i & h) continue;
-#pragma unroll
-                for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-                    for (int r = 0; r < 2; r++) {
-                        const uint64_t u = c[i][nt][r], v = c[i + h][nt][r];
-                        c[i][nt][r] = add_f32x2(u, v);
-                        c[i + h][nt][r] = fma_f32x2(v, minus, u);
-                    }
-            }
-        auto put = [&](int64_t row, int r) {
-            __half* o = out + row * n + col;
+            // c[2 q + s][nt]: columns 32 q' + 8 t + 4 s' + 2 nt + {0, 1} of rows g (first pair) and g + 8, for the
+            // 16-point transform of group (q, s); the butterflies turn (q, s) into (q', s')
+            uint64_t c[8][2][2];
 #pragma unroll
             for (int q = 0; q < 4; q++)
-                *reinterpret_cast<uint4*>(o + 32 * q) =
-                    make_uint4(f16_pair(mul_f32x2(c[2 * q][0][r], scale)), f16_pair(mul_f32x2(c[2 * q][1][r], scale)),
-                               f16_pair(mul_f32x2(c[2 * q + 1][0][r], scale)), f16_pair(mul_f32x2(c[2 * q + 1][1][r], scale)));
-        };
-        if (ok0) put(r0, 0);
-        if (ok1) put(r1, 1);
+#pragma unroll
+                for (int s = 0; s < 2; s++) {
+                    const uint32_t af[4] = {s ? ya[q].z : ya[q].x, s ? yb[q].z : yb[q].x, s ? ya[q].w : ya[q].y, s ? yb[q].w : yb[q].y};
+#pragma unroll
+                    for (int nt = 0; nt < 2; nt++) {
+                        float d[4] = {0.f, 0.f, 0.f, 0.f};
+                        mma_16816(d, af, hb[nt][0], hb[nt][1]);
+                        if constexpr (SPLIT) {
+                            const uint32_t lf[4] = {s ? la[q].z : la[q].x, s ? lb[q].z : lb[q].x, s ? la[q].w : la[q].y, s ? lb[q].w : lb[q].y};
+                            mma_16816(d, lf, hb[nt][0], hb[nt][1]);
+                        }
+                        c[2 * q + s][nt][0] = f32x2(d[0], d[1]);
+                        c[2 * q + s][nt][1] = f32x2(d[2], d[3]);
+                    }
+                }
+            const uint64_t minus = f32x2(-1.f, -1.f), scale = f32x2(EXL3_HAD_SCALE, EXL3_HAD_SCALE);
+#pragma unroll
+            for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    if (i & h) continue;
+#pragma unroll
+                    for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+                        for (int r = 0; r < 2; r++) {
+                            const uint64_t u = c[i][nt][r], v = c[i + h][nt][r];
+                            c[i][nt][r] = add_f32x2(u, v);
+                            c[i + h][nt][r] = fma_f32x2(v, minus, u);
+                        }
+                }
+            auto put = [&](int64_t row, int r) {
+                __half* o = out + row * n + col;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    *reinterpret_cast<uint4*>(o + 32 * q) =
+                        make_uint4(f16_pair(mul_f32x2(c[2 * q][0][r], scale)), f16_pair(mul_f32x2(c[2 * q][1][r], scale)),
+                                   f16_pair(mul_f32x2(c[2 * q + 1][0][r], scale)), f16_pair(mul_f32x2(c[2 * q + 1][1][r], scale)));
+            };
+            if (ok0) put(o0, 0);
+            if (ok1) put(o1, 1);
+        }
     }
 }
 
@@ -457,7 +469,7 @@ int launch_table(int cb, __half* table, cudaStream_t s)
 int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t x_row_stride,
                     const __half* pre, const __half* post, __half* out, const int32_t* row_src,
                     const int32_t* pre_row, const int32_t* post_row, bool pdl, int out_mode,
-                    cudaStream_t s, int glu, const int32_t* rows_dev, int member_rows)
+                    cudaStream_t s, int glu, const int32_t* rows_dev, int member_rows, bool row_pairs)
 {
     if (rows * (n >> 7) >= ((int64_t)1 << 31)) return EXL3_E_RANGE;   // the kernel counts blocks in 32 bits
     // Many rows into a plain fp16 matrix (the prefill GEMM's operand): 16-row blocks on the tensor cores.
@@ -468,7 +480,10 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
                      x_row_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
                      (!pre || (reinterpret_cast<uintptr_t>(pre) & 15) == 0) && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     if (rows_dev && !mma) return EXL3_E_UNSUPPORTED;
-    const int g = mma ? grid_for(((rows + 15) >> 4) * (n >> 7), 8) : grid_for(rows * (n >> 7), 8);
+    // Rows that share a row of x: worth it where there are blocks enough without splitting them (below, 592 x 4 warps).
+    int copies = !mma || rows_dev || glu ? 1 : row_pairs ? 2 : member_rows >= kHadamardMmaMinRows ? (int)(rows / member_rows) : 1;
+    if (((rows / copies + 15) >> 4) * (n >> 7) < 4 * 16 * (int64_t)device_sm_count()) copies = 1;
+    const int g = mma ? grid_for(((rows / copies + 15) >> 4) * (n >> 7), 8) : grid_for(rows * (n >> 7), 8);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g);
     cfg.blockDim = dim3(256);
@@ -485,8 +500,8 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
         const bool split = member_rows > 0 && member_rows < kHadamardMmaMinRows;
         auto launch = [&](auto* xt) {
             using T = std::remove_const_t<std::remove_pointer_t<decltype(xt)>>;
-            return cudaLaunchKernelEx(&cfg, split ? hadamard_mma_kernel<T, true> : hadamard_mma_kernel<T, false>, xt, rows, n,
-                                      x_row_stride, pre, out, row_src, pre_row, rows_dev, early, glu, member_rows);
+            const auto kernel = copies > 1 ? hadamard_mma_kernel<T, false, true> : split ? hadamard_mma_kernel<T, true, false> : hadamard_mma_kernel<T, false, false>;
+            return cudaLaunchKernelEx(&cfg, kernel, xt, rows, n, x_row_stride, pre, out, row_src, pre_row, rows_dev, early, glu, member_rows, copies);
         };
         switch (x_dtype) {
             case EXL3_DT_F16: e = launch((const __half*)x); break;

@@ -600,6 +600,7 @@ static int gemm_tiles_impl(const void* x, int x_dtype, int64_t x_row_stride, int
     if (t_in <= 0 || t_out_total <= 0 || t_in % 8 || t_out_total % 8) return EXL3_E_SHAPE;
     if (t_in > (1 << 24) || t_out_total > (1 << 24)) return EXL3_E_SHAPE;
     if (xh_rows < 1 || xh_rows > (1 << 30)) return EXL3_E_ROWS;
+    if ((flags & EXL3_FLAG_ROW_PAIRS) && (!row_src || xh_rows % 2)) return EXL3_E_ROWS;
     if (n_tiles < 0 || n_tiles > (1 << 24)) return EXL3_E_SHAPE;
     const int64_t in = 16 * t_in;
     const int glu = glu_mode(flags);
@@ -621,7 +622,8 @@ static int gemm_tiles_impl(const void* x, int x_dtype, int64_t x_row_stride, int
     __half* xh = reinterpret_cast<__half*>(ws + kWsScratch);
     cudaStream_t s = (cudaStream_t)stream;
     rc = launch_hadamard(x, x_dtype, xh_rows, in, x_row_stride, reinterpret_cast<const __half*>(suh),
-                         nullptr, xh, row_src, suh_row, nullptr, false, HAD_OUT_F16, s, glu, peers.xh_rows_dev);
+                         nullptr, xh, row_src, suh_row, nullptr, false, HAD_OUT_F16, s, glu, peers.xh_rows_dev, 0,
+                         (flags & EXL3_FLAG_ROW_PAIRS) != 0);
     if (rc) return rc;
     GemmArgs a = {};
     a.svh = reinterpret_cast<const __half*>(svh);

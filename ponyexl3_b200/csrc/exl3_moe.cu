@@ -112,6 +112,7 @@ struct MoePrefillArgs {
     int32_t* tiles_gu;     // (2 * slots * ceil(H/256), 8)
     int32_t* tiles_dn;     // (slots * ceil(D/256), 8)
     int32_t* counts;       // NULL, or {rotated gate/up rows in use, sorted positions in use}
+    int pairs;             // gate row p and up row n + p for sorted position p, instead of an expert's rows together
 };
 
 constexpr int kMoeMaxExperts = 1024;
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(1024) moe_prefill_tables_kernel(const MoePrefi
         const int pos = seg[e] + i;
         a.order[pos] = s;
         const int tok = s / a.kk;
-        const int rg = 2 * seg[e] + i, ru = rg + count[e];
+        const int rg = a.pairs ? pos : 2 * seg[e] + i, ru = rg + (a.pairs ? a.n : count[e]);
         a.row_src_gu[rg] = tok;
         a.row_src_gu[ru] = tok;
         a.suh_row_gu[rg] = 2 * e;
@@ -220,11 +221,11 @@ __global__ void __launch_bounds__(1024) moe_prefill_tables_kernel(const MoePrefi
         }
         if (j < ct_h) {
             put(a.tiles_gu, slot * ct_h + j, row0, row_end, e * (a.H / 16) + 16 * j, e * 2 * a.H + 256 * j, 256 * j,
-                min(a.H - 256 * j, 256), sg);
+                min(a.H - 256 * j, 256), a.pairs ? 0 : sg);
         } else if (j < 2 * ct_h) {
             j -= ct_h;
             put(a.tiles_gu, (a.slots + slot) * ct_h + j, row0, row_end, (E_here + e) * (a.H / 16) + 16 * j,
-                e * 2 * a.H + a.H + 256 * j, a.H + 256 * j, min(a.H - 256 * j, 256), sg + cnt);
+                e * 2 * a.H + a.H + 256 * j, a.H + 256 * j, min(a.H - 256 * j, 256), a.pairs ? a.n : sg + cnt);
         } else {
             j -= 2 * ct_h;
             put(a.tiles_dn, slot * ct_d + j, row0, row_end, e * (a.D / 16) + 16 * j, e * a.D + 256 * j, 256 * j,
@@ -304,6 +305,7 @@ static int moe_prefill_tables_impl(const void* indices, int index_bytes, int n_p
     a.order = order; a.row_src_gu = row_src_gu; a.suh_row_gu = suh_row_gu; a.suh_row_dn = suh_row_dn;
     a.tiles_gu = tiles_gu; a.tiles_dn = tiles_dn;
     a.counts = counts;
+    a.pairs = !counts && (flags & EXL3_FLAG_ROW_PAIRS) != 0;
     return launch_kernel(moe_prefill_tables_kernel, dim3((unsigned)std::max(1, std::min(32, n_pairs / 512))), dim3(1024), 0, (cudaStream_t)stream,
                          (flags & EXL3_FLAG_PDL) != 0, a);
 }

@@ -480,14 +480,14 @@ PyObject* switch_glu(PyObject* const* arg)
                 *suh_dn = suh_gu + 2 * n;
         launch(dev, "exl3_moe_prefill_tables", [&] {
             return api.exl3_moe_prefill_tables(idx.data_ptr(), bytes, (int)n, (int)kk, (int)E, D, H, order, row_src,
-                                               suh_gu, suh_dn, tiles_gu, tiles_dn, 0, es);
+                                               suh_gu, suh_dn, tiles_gu, tiles_dn, EXL3_FLAG_ROW_PAIRS, es);
         });
-        const unsigned hint = (unsigned)std::min<int64_t>(n / E, 0xFFFF) << 16;      // rows of an expert
+        const unsigned hint = (unsigned)std::max<int64_t>(1, std::min<int64_t>(n / E, 0xFFFF)) << 16;      // rows of an expert
         Workspace ws = workspace(dev, api.exl3_gemm_workspace_bytes(2 * n, D));
         launch(dev, "exl3_gemm_tiles", [&] {
             return api.exl3_gemm_tiles(r.t.data_ptr(), r.dtype, r.stride, 2 * n, row_src, gu_suh, suh_gu,
                                        gu.trellis, gu.t_in, gu.t_out, k, cb, tiles_gu, n_gu, gu_svh, u16(ygu), 2 *
-                                       H, nullptr, ws.ptr, ws.bytes, hint, es);
+                                       H, nullptr, ws.ptr, ws.bytes, hint | EXL3_FLAG_ROW_PAIRS, es);
         });
         ws = workspace(dev, api.exl3_gemm_workspace_bytes(n, H));
         launch(dev, "exl3_gemm_tiles", [&] {

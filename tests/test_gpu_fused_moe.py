@@ -152,6 +152,29 @@ def test_switch_glu_decode_matches_oracle(cuda, oracle, tokens, k, cb, act):
     assert rel_err(y.cpu().numpy().reshape(tokens, kk, D), want) <= 2e-3
 
 
+def test_rows_of_x_read_once_for_all_their_copies(cuda):
+    """Many rows: the rotation reads a row of x once for gate and up, or for all members of a group, and the result is what
+    fewer rows give, whose copies are rotated one by one (16-row blocks x 128 columns below and above 64 per SM)."""
+    from ponyexl3_b200 import EXL3Linear
+    from ponyexl3_b200.fused import FusedEXL3Group
+
+    E, D, H, kk = 16, 512, 128, 8
+    sw = _switch(_experts(E, D, H, 4, seed=81), 4, 0)
+    rng = np.random.default_rng(6)
+    T = 4801
+    x = torch.from_numpy((rng.standard_normal((T, D)) * 0.5).astype(np.float16)).cuda()
+    idx = torch.from_numpy(np.stack([rng.permutation(E)[:kk] for _ in range(T)])).cuda()
+    y = sw(x[None], idx[None])
+    assert torch.equal(y, torch.cat([sw(x[None, i:i + 700], idx[None, i:i + 700]) for i in range(0, T, 700)], 1))
+    layers = _members(4, 2048, [256, 128, 384], seed=82)
+    x = torch.from_numpy(rng.standard_normal((9497, 2048)).astype(np.float32)).cuda().bfloat16()
+    for got, l in zip(FusedEXL3Group(layers).forward_all(x), layers):
+        want = EXL3Linear(l)(x)
+        # the group's launch deals its tiles to other CTAs, whose fp32 sums are added in another order: some of the fp16
+        # values that are rotated on the way out flip by an ulp (2^-11); a wrong row or multiplier would be of order 1
+        assert rel_err(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 2 ** -11
+
+
 def test_switch_glu_prefill_matches_oracle_and_decode(cuda, oracle):
     E, D, H, kk, k = 8, 256, 128, 2, 4
     w = _experts(E, D, H, k, seed=77)

@@ -104,3 +104,38 @@ def test_prefill_tables_of_an_expert_range(lib, lo, hi, n_tokens):
         assert g[2] == e * (H // 16) and u[2] == (e_here + e) * (H // 16) and dn[2] == e * (D // 16)
     for g, u, dn in zip(t_g[len(tiles):], t_u[len(tiles):], t_d[len(tiles):]):
         assert g[0] >= g[1] and u[0] >= u[1] and dn[0] >= dn[1]                             # unused slots are empty
+
+
+@pytest.mark.parametrize("n_tokens", [3, 96, 700])
+def test_prefill_tables_with_all_gate_rows_before_all_up_rows(lib, n_tokens):
+    """EXL3_FLAG_ROW_PAIRS: the gate row of sorted position p is row p, its up row n + p, and tiles say so; the rest is
+    as without the flag."""
+    E, kk, D, H = 16, 4, 512, 384
+    idx = _routing(n_tokens, kk, E, 3 + n_tokens)
+    n = len(idx)
+    slots, ct_h, ct_d = n // 256 + E, (H + 255) // 256, (D + 255) // 256
+    d = torch.device("cuda")
+    idd = torch.from_numpy(idx).to(d)
+    z = lambda *s: torch.full(s, -7, dtype=torch.int32, device=d)
+
+    def tables(flags):
+        order, rs, sr, sd, tgu, tdn = z(n), z(2 * n), z(2 * n), z(n), z(2 * slots * ct_h, 8), z(slots * ct_d, 8)
+        lib.check(lib.load().exl3_moe_prefill_tables(
+            idd.data_ptr(), 8, n, kk, E, D, H, order.data_ptr(), rs.data_ptr(), sr.data_ptr(), sd.data_ptr(),
+            tgu.data_ptr(), tdn.data_ptr(), flags, torch.cuda.current_stream().cuda_stream), "tables")
+        return [t.cpu() for t in (order, rs, sr, sd, tgu, tdn)]
+
+    order, rs, sr, sd, tgu, tdn = tables(16)
+    _, _, _, sd0, tgu0, tdn0 = tables(0)
+    assert sorted(order.tolist()) == list(range(n))
+    assert torch.equal(sd, sd0) and torch.equal(tdn, tdn0)
+    assert rs.tolist() == 2 * [s // kk for s in order.tolist()]
+    assert sr.tolist() == [2 * idx[s] for s in order.tolist()] + [2 * idx[s] + 1 for s in order.tolist()]
+    # a tile's rotated rows less its shift are sorted positions: the same as without the flag, and so is all else
+    half, shift = slots * ct_h, -tgu[:, 6]
+    used = tgu0[:, 0] < tgu0[:, 1]
+    assert bool((shift[:half][used[:half]] == 0).all()) and bool((shift[half:][used[half:]] == n).all())
+    for t in (tgu, tgu0):
+        t[:, :2] += t[:, 6:7]
+        t[:, 6] = 0
+    assert torch.equal(tgu[used], tgu0[used]) and bool((tgu[~used, 0] >= tgu[~used, 1]).all())
