@@ -72,6 +72,8 @@ extern "C" {
 #define EXL3_FLAG_ROW_PAIRS 16u /* exl3_moe_prefill_tables: the gate row of sorted position p is rotated row p, its up row
                                    n_pairs + p.  exl3_gemm_tiles: rows r and r + xh_rows / 2 have the same row_src (which
                                    is required, and xh_rows even), so that a row of x is read once for both */
+#define EXL3_FLAG_WIDE_SCALES 32u /* exl3_gemm_tiles: x * suh goes into the rotation as it is, not rounded to fp16, whatever
+                                   the number of rows; so does the GEMV's (no difference for multipliers of +-1) */
 
 typedef void* exl3_stream_t;    /* cudaStream_t */
 

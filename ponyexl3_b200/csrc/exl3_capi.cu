@@ -623,7 +623,7 @@ static int gemm_tiles_impl(const void* x, int x_dtype, int64_t x_row_stride, int
     cudaStream_t s = (cudaStream_t)stream;
     rc = launch_hadamard(x, x_dtype, xh_rows, in, x_row_stride, reinterpret_cast<const __half*>(suh),
                          nullptr, xh, row_src, suh_row, nullptr, false, HAD_OUT_F16, s, glu, peers.xh_rows_dev, 0,
-                         (flags & EXL3_FLAG_ROW_PAIRS) != 0);
+                         (flags & EXL3_FLAG_ROW_PAIRS) != 0, (flags & EXL3_FLAG_WIDE_SCALES) != 0);
     if (rc) return rc;
     GemmArgs a = {};
     a.svh = reinterpret_cast<const __half*>(svh);

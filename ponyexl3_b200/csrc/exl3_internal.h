@@ -68,7 +68,8 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
                     const int32_t* pre_row, const int32_t* post_row, bool pdl, int out_mode,
                     cudaStream_t s, int glu = 0, const int32_t* rows_dev = nullptr,   // glu: x rows are [gate (n) | up (n)], see glu_value
                     int member_rows = 0,    // > 0: output row r is row r % member_rows of x with row r / member_rows of pre
-                    bool row_pairs = false);   // row_src is the same for rows r and r + rows / 2
+                    bool row_pairs = false,    // row_src is the same for rows r and r + rows / 2
+                    bool wide_scales = false); // x * pre unrounded also where the tensor cores rotate
 
 // One logical 128-column output block of a streamed GEMV: where its weights, activations,
 // output scales and results live.  NULL descriptor table = the identity mapping of a plain

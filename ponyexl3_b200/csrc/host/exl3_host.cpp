@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <string>
 
@@ -420,6 +421,20 @@ PyObject* mlp(PyObject* const* arg)
 }
 
 // ---- stacked-expert SwitchGLU ---------------------------------------------------------------------------------
+// Few tokens: every (token, slot) pair as a one-row problem, which decodes an expert's weights once per pair, or the
+// pairs sorted by expert, which decodes them once per expert but has two more launches and longer tables.  With pairs
+// spread evenly over the experts the one takes about 20 + 0.88 n us for n pairs (2048 / 512 dims, K = 4), the other 30 + 0.88 u
+// for the u experts that get any; with 1024 / 256 dims 14 + 0.28 n and 29 + 0.29 u: the line lies where n - u pays for what the
+// second has more.  us by pairs / by expert at 16 tokens, top-8: 256 experts 132 / 118, 128 131 / 98, 64 131 / 82 (2048 / 512);
+// 50 / 58, 49 / 54, 48 / 44 (1024 / 256); at 8 tokens 77 / 89, 76 / 75, 76 / 69.
+// (More than 1024 experts or 2^20 pairs have no tables by expert.)
+bool by_expert(int64_t pairs, int64_t experts, int64_t d, int64_t h)
+{
+    if (experts > 1024 || pairs > (1 << 20)) return false;
+    const double e = (double)experts, hit = experts > 1 ? e * -std::expm1((double)pairs * std::log1p(-1.0 / e)) : 1.0;
+    return (double)pairs - hit > 8.0 + 3.7e7 / (3.0 * (double)d * (double)h);
+}
+
 // switch_glu(x2d, indices (R, k), gu_trellis, gu_suh, gu_svh, dn_trellis, dn_suh, dn_svh, experts, hidden, k, cb,
 //            glu flag, flags, decode) -> (R, k, D)
 PyObject* switch_glu(PyObject* const* arg)
@@ -448,7 +463,7 @@ PyObject* switch_glu(PyObject* const* arg)
     const at::Tensor ygu = empty_half({n, 2 * H}, device);
     at::Tensor y = empty_half({R, kk, D}, device);
     if (n == 0) return THPVariable_Wrap(std::move(y));
-    if (PyObject_IsTrue(arg[14])) {
+    if (PyObject_IsTrue(arg[14]) && !by_expert(n, E, D, H)) {
         // tables, gate|up, down with the GLU on load
         const int64_t gb = H / 128, db = D / 128, n_gu = n * 2 * gb, n_dn = n * db;
         const at::Tensor tab = empty_int(4 * (n_gu + n_dn) + 5 * n, device);
@@ -483,17 +498,18 @@ PyObject* switch_glu(PyObject* const* arg)
                                                suh_gu, suh_dn, tiles_gu, tiles_dn, EXL3_FLAG_ROW_PAIRS, es);
         });
         const unsigned hint = (unsigned)std::max<int64_t>(1, std::min<int64_t>(n / E, 0xFFFF)) << 16;      // rows of an expert
+        const unsigned wide = PyObject_IsTrue(arg[14]) ? EXL3_FLAG_WIDE_SCALES : 0u;      // few tokens: what the GEMV would give
         Workspace ws = workspace(dev, api.exl3_gemm_workspace_bytes(2 * n, D));
         launch(dev, "exl3_gemm_tiles", [&] {
             return api.exl3_gemm_tiles(r.t.data_ptr(), r.dtype, r.stride, 2 * n, row_src, gu_suh, suh_gu,
                                        gu.trellis, gu.t_in, gu.t_out, k, cb, tiles_gu, n_gu, gu_svh, u16(ygu), 2 *
-                                       H, nullptr, ws.ptr, ws.bytes, hint | EXL3_FLAG_ROW_PAIRS, es);
+                                       H, nullptr, ws.ptr, ws.bytes, hint | wide | EXL3_FLAG_ROW_PAIRS, es);
         });
         ws = workspace(dev, api.exl3_gemm_workspace_bytes(n, H));
         launch(dev, "exl3_gemm_tiles", [&] {
             return api.exl3_gemm_tiles(ygu.data_ptr(), EXL3_DT_F16, 2 * H, n, nullptr, dn_suh, suh_dn, dn.trellis,
                                        dn.t_in, dn.t_out, k, cb, tiles_dn, n_dn, dn_svh, u16(y), D, order, ws.ptr,
-                                       ws.bytes, glu | hint, es);
+                                       ws.bytes, glu | hint | wide, es);
         });
     }
     return THPVariable_Wrap(std::move(y));

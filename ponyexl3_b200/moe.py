@@ -12,8 +12,9 @@ mlx_lm's SwitchGLU; routing and the weighted sum stay in the block.
 Decode-class calls (few tokens) run two streamed GEMVs over block tables built on the device
 from the routing indices — every (token, slot) pair is its own one-row problem against its
 expert's column range (the reference's mapped GEMV, exl3_moe.py:634-683).  Prefill-class
-calls sort the pairs by expert and run the tensor-core GEMM over a table of expert tiles
-(the reference's segmented trellis GEMM, exl3_moe.py:685-768).
+calls, and few tokens whose pairs crowd on few experts, sort the pairs by expert and run the
+tensor-core GEMM over a table of expert tiles (the reference's segmented trellis GEMM,
+exl3_moe.py:685-768).
 """
 
 from __future__ import annotations

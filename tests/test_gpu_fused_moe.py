@@ -152,6 +152,37 @@ def test_switch_glu_decode_matches_oracle(cuda, oracle, tokens, k, cb, act):
     assert rel_err(y.cpu().numpy().reshape(tokens, kk, D), want) <= 2e-3
 
 
+@pytest.mark.parametrize("k,tokens", [(4, 6), (4, 16), (1, 13), (6, 16)])
+def test_switch_glu_few_tokens_by_expert(cuda, oracle, k, tokens):
+    """Pairs that crowd on few experts: 6 tokens of 8 experts lie below the line between the two paths (48 - 8 < 55),
+    13 and 16 above it (104 - 8, 128 - 8)."""
+    E, D, H, kk = 8, 512, 512, 8
+    w = _experts(E, D, H, k, seed=60 + k)
+    rng = np.random.default_rng(tokens)
+    x = (rng.standard_normal((tokens, D)) * 0.5).astype(np.float16)
+    idx = np.stack([rng.permutation(E)[:kk] for _ in range(tokens)]).astype(np.int64)
+    y = _switch(w, k, 0)(torch.from_numpy(x).cuda()[None], torch.from_numpy(idx).cuda()[None])
+    want = oracle.switch_glu(x, idx, **w, k=k, cb=0)
+    assert rel_err(y.cpu().numpy().reshape(tokens, kk, D), want) <= 2e-3
+
+
+def test_few_tokens_by_expert_keep_scales_unrounded(cuda, oracle):
+    """Multipliers other than +-1: below 17 tokens x * suh is not rounded before the rotation on either path, so sixteen
+    tokens at once are no further from the oracle than by fours (one row per pair).  Roundings that flip along the chain
+    leave both 3e-4; a rounded product adds 2.8e-4 to 5e-4 in each of two projections, 1.6 times as much and more."""
+    E, D, H, kk, T = 8, 512, 512, 8, 16
+    w = _experts(E, D, H, 4, seed=90)
+    rng = np.random.default_rng(7)
+    for n in ("gu_suh", "dn_suh"):
+        w[n] = (w[n] * rng.uniform(0.5, 1.5, w[n].shape)).astype(np.float16)
+    x = (rng.standard_normal((T, D)) * 0.5).astype(np.float16)
+    idx = np.stack([rng.permutation(E)[:kk] for _ in range(T)]).astype(np.int64)
+    sw, xd, idd = _switch(w, 4, 0), torch.from_numpy(x).cuda()[None], torch.from_numpy(idx).cuda()[None]
+    want = oracle.switch_glu(x, idx, **w, k=4, cb=0)
+    err = lambda y: rel_err(y.cpu().numpy().reshape(T, kk, D), want)
+    assert err(sw(xd, idd)) <= 1.25 * err(torch.cat([sw(xd[:, i:i + 4], idd[:, i:i + 4]) for i in range(0, T, 4)], 1))
+
+
 def test_rows_of_x_read_once_for_all_their_copies(cuda):
     """Many rows: the rotation reads a row of x once for gate and up, or for all members of a group, and the result is what
     fewer rows give, whose copies are rotated one by one (16-row blocks x 128 columns below and above 64 per SM)."""
