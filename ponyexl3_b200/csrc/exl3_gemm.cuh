@@ -72,7 +72,8 @@ template <int K> struct TsLayout {
     static constexpr int kTileWords = 8 * K;
     static constexpr int kWBytes = 32 * kTileWords * 4;                 // 8 x 4 packed tiles: K KiB
     static constexpr int kRoom = kTsSmemBytes - kTsWOff;                // of the two rings
-    // tokens per tile of a dense launch: at least four stages of activations have to fit, three wide ones
+    // tokens per tile of a dense launch: at least four stages of activations have to fit, three wide ones (beside a cluster's
+    // exchange of sums ts_joint sees to it)
     static constexpr int kTok = std::min(kTsMaxTok, kTsSmemBytes - kTsWOff - 8 * kWBytes >= 512 * kTsMaxTok
                                                         ? kTsMaxTok
                                                         : (kTsSmemBytes - kTsWOff - 8 * kWBytes) / 512 / 16 * 16);
@@ -931,9 +932,10 @@ template <int K, int CB> static int launch_gemm_t(GemmArgs a, const __half* xh, 
     const int sms = device_sm_count(), nks = a.t_in / kTsStepTiles;
     a.tiles_n = a.t_out / 8;
     TsPlan plan = gemm_plan(a.m, a.tiles_n, nks, sms, a.ts_partial_bytes, L::kTok, L::kTokWide);
-    a.ts_joint = ts_joint(plan, a.tiles_n, nks, sms);
+    const TsRings rings = {L::kRoom, L::kWBytes};
+    a.ts_joint = ts_joint(plan, a.tiles_n, nks, sms, rings);
     while (a.ts_joint && gemm_clusters(gemm_kernel<K, CB, TS_JOINT>, a.ts_joint) < plan.tiles_m * a.tiles_n)
-        a.ts_joint = ts_joint(plan, a.tiles_n, nks, sms, a.ts_joint - 1);
+        a.ts_joint = ts_joint(plan, a.tiles_n, nks, sms, rings, a.ts_joint - 1);
     if (a.ts_joint) { plan.grid = (int)(plan.tiles_m * a.tiles_n) * a.ts_joint; plan.split = 1; }
     a.ts_tok = plan.tok;
     a.tiles_m = plan.tiles_m;
@@ -945,10 +947,10 @@ template <int K, int CB> static int launch_gemm_t(GemmArgs a, const __half* xh, 
     a.ts_x_bytes = (a.ts_tok + a.ts_box_rows - 1) / a.ts_box_rows * a.ts_box_rows * 128;
     // Ring x has up to eight stages beside eight of ring w (four in the wide form); what is left goes to ring w, up to three
     // stages per set (more do not pay: 28 stages delay the first activations behind them, 17408 -> 512 16.4 -> 17.4 us).
-    a.ts_recv_bytes = a.ts_joint ? (a.ts_tok / 16 + a.ts_joint - 1) / a.ts_joint * (a.ts_joint - 1) * 8192 : 0;   // (at most 64 KiB)
-    const int room = L::kRoom - a.ts_recv_bytes;
-    a.stages = std::min(kTsStages, (room - (mode == TS_WIDE ? 4 : 8) * L::kWBytes) / a.ts_x_bytes);
-    a.ts_w_stages = std::min(kTsMaxWStages, (room - a.stages * a.ts_x_bytes) / L::kWBytes) / kTsSets * kTsSets;
+    a.ts_recv_bytes = ts_recv_bytes(a.ts_tok, a.ts_joint);
+    a.stages = ts_x_stages(rings, a.ts_recv_bytes, mode == TS_WIDE ? 4 : 8, a.ts_x_bytes, kTsStages);
+    a.ts_w_stages = std::min(kTsMaxWStages, (L::kRoom - a.ts_recv_bytes - a.stages * a.ts_x_bytes) / L::kWBytes) / kTsSets * kTsSets;
+    if (a.stages < kTsLeastStages || a.ts_w_stages < kTsSets) return EXL3_E_UNSUPPORTED;        // (never for a plan as above: no ring, no launch)
     a.ts_dbuf = a.ts_tok <= 128 ? 2 : 1;
     CUtensorMap tm_x, tm_w;
     rc = gemm_tensor_maps(&tm_x, &tm_w, a, L::kTileWords, xh, trellis);

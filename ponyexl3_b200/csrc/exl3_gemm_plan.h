@@ -101,20 +101,42 @@ inline TsPlan ts_plan(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, 
     return best;
 }
 
+// Shared memory for the rings of a dense launch, and what a k-step's packed tiles take of it.
+struct TsRings {
+    int room, w_bytes;
+};
+// Bytes into which a CTA of a cluster of n gets the other CTAs' sums: up to ceil(tok / 16 / n) pieces of sixteen tokens
+// x 128 columns from each.
+inline int ts_recv_bytes(int tok, int n) { return n ? (tok / 16 + n - 1) / n * (n - 1) * 16 * 128 * 4 : 0; }
+// Stages of the activation ring beside them and w_stages of packed tiles.
+inline int ts_x_stages(const TsRings& r, int recv_bytes, int w_stages, int x_bytes, int most)
+{
+    return std::min(most, (r.room - recv_bytes - w_stages * r.w_bytes) / x_bytes);
+}
+
 // CTAs per tile where a tile's CTAs should be a cluster (two to eight of them, of one tile and at least four k-steps each)
 // instead of what the plan says, or 0: up to 128 tokens, and where the longer ranges of k-steps of a whole number of CTAs
 // per tile cost less than the hand-over through the workspace.  us at 9, 40, 77, 128 rows, through the workspace / as
 // clusters, K = 4: 5120 x 5120 (three) 15.5, 19.3, 17.7, 19.7 / 15.4, 18.5, 15.9, 17.1; 4096 x 1024 (eight) 10.8, 15.6, 16.5, 22.2 /
 // 10.6, 11.6, 11.3, 12.1; 2048 x 2048 (eight) 9.4, 12.7, 13.0, 14.0 / 9.3, 10.6, 10.3, 11.4.
-constexpr int kTsJointCost = 4, kTsJointMost = 8, kTsJointTok = 128;
-inline int ts_joint(const TsPlan& p, int64_t tiles_n, int nks, int sms, int most = kTsJointMost)
+// The sums that they exchange take the rings' memory, most of it at 128 tokens and six or seven CTAs (80 and 96 of
+// 162 KiB).  As many CTAs are taken as leave three stages of activations beside eight of packed tiles: us with two, three and four
+// stages at 128 rows, 2048 -> 2560, K = 5 (seven, six, four CTAs) 12.0, 11.2, 11.2; 4096 -> 2816, K = 6 (six, five, four) 14.6, 13.7,
+// 13.8.  Two stages are enough where fewer CTAs would not be worth it: 4096 -> 1024, K = 8 (eight) 12.6, through the workspace 22.3.
+constexpr int kTsJointCost = 4, kTsJointMost = 8, kTsJointTok = 128, kTsJointStages = 3, kTsLeastStages = 2;
+inline int ts_joint(const TsPlan& p, int64_t tiles_n, int nks, int sms, const TsRings& r, int most = kTsJointMost)
 {
     const int64_t tiles = p.tiles_m * tiles_n;
     if (!p.split || p.tok > kTsJointTok || 2 * tiles > sms) return 0;
-    const int n = (int)std::min<int64_t>(std::min<int64_t>(most, sms / tiles), nks / 4);
-    if (n < 2) return 0;
-    const int64_t shared = ts_slowest(tiles * nks, nks, p.grid, INT64_MAX), joint = (nks + n - 1) / n + kTsJointCost;
-    return joint <= shared ? n : 0;
+    most = (int)std::min<int64_t>(std::min<int64_t>(most, sms / tiles), nks / 4);
+    if (most < 2) return 0;
+    const int64_t shared = ts_slowest(tiles * nks, nks, p.grid, INT64_MAX);
+    for (int least = kTsJointStages; least >= kTsLeastStages; least--) {
+        int n = most;
+        while (n >= 2 && ts_x_stages(r, ts_recv_bytes(p.tok, n), 8, 128 * p.tok, least) < least) n--;
+        if (n >= 2 && (nks + n - 1) / n + kTsJointCost <= shared) return n;
+    }
+    return 0;
 }
 
 // The kernel counts tiles, k-steps where tiles are shared, and the k-steps of one CTA in 32 bits.

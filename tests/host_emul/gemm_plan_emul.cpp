@@ -6,12 +6,31 @@
 
 using namespace exl3;
 
-// out: tok, tiles_m, grid, split, wide.  Shared tiles have room up to room_tok tokens.
-extern "C" int emul_joint(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok, int most)
+extern "C" int emul_joint(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok, int room, int w_bytes, int most)
 {
-    return ts_joint(ts_plan(rows, tiles_n, nks, sms, tok, tok_wide, room_tok), tiles_n, nks, sms, most);
+    return ts_joint(ts_plan(rows, tiles_n, nks, sms, tok, tok_wide, room_tok), tiles_n, nks, sms, TsRings{room, w_bytes}, most);
 }
 
+// Every number of CTAs that may be asked for, over 16 .. 256 rows, up to sms / 2 column tiles and 2 .. most_nks k-steps: the fewest
+// stages of activations beside eight of packed tiles that a cluster is left with, and clusters seen by size (seen[2 .. 8]).
+extern "C" int emul_joint_stages(int most_nks, int sms, int tok, int tok_wide, int room, int w_bytes, int* seen)
+{
+    int least = 1 << 20;
+    for (int rows = 16; rows <= 256; rows += 16)
+        for (int tiles_n = 1; tiles_n <= sms / 2; tiles_n++)
+            for (int nks = 2; nks <= most_nks; nks += 2) {
+                const TsPlan p = ts_plan(rows, tiles_n, nks, sms, tok, tok_wide, tok_wide);
+                for (int most = 8; most >= 2; most--) {
+                    const int n = ts_joint(p, tiles_n, nks, sms, TsRings{room, w_bytes}, most);
+                    if (!n) continue;
+                    seen[n]++;
+                    least = std::min(least, (room - ts_recv_bytes(p.tok, n) - 8 * w_bytes) / (128 * p.tok));
+                }
+            }
+    return least;
+}
+
+// out: tok, tiles_m, grid, split, wide.  Shared tiles have room up to room_tok tokens.
 extern "C" void emul_plan(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok, int* out)
 {
     const TsPlan p = ts_plan(rows, tiles_n, nks, sms, tok, tok_wide, room_tok);

@@ -98,7 +98,7 @@ def test_gemm_tiles_shared_between_ctas(mod, oracle, rows, inf, outf, k, cb):
 @pytest.mark.parametrize("rows", [9, 16, 33, 100, 128])
 @pytest.mark.parametrize("inf,outf,k,cb", [
     (2048, 384, 4, 0),          # eight CTAs of four k-steps per tile; more CTAs than pieces of 16 tokens, and as many
-    (2048, 2560, 5, 1),         # seven
+    (2048, 2560, 5, 1),         # seven, or as many as the device holds twenty clusters of
     (1152, 5120, 3, 2),         # three
     (896, 8192, 8, 0),          # two, the deepest packed tiles
 ])
@@ -111,6 +111,37 @@ def test_gemm_tiles_of_clusters(mod, oracle, rows, inf, outf, k, cb):
     xd = torch.from_numpy(x).cuda()
     first = m(xd)
     assert all(torch.equal(m(xd), first) for _ in range(3))
+
+
+# Clusters of each size, by rows (test_gemm_plan.py checks that the plan takes them): where the exchanged sums are largest, at
+# 113 to 128 tokens a tile, and where the packed tiles are.
+CLUSTERS = [
+    (1792, 1024, 4, 1, 77, 7),
+    (1792, 1024, 4, 0, 128, 6),
+    (1792, 1024, 5, 2, 121, 5),
+    (1536, 1024, 6, 0, 100, 5),
+    (1536, 1024, 6, 0, 90, 6),
+    (1792, 1024, 7, 0, 113, 4),
+    (1920, 2048, 7, 1, 128, 4),
+    (1792, 1024, 7, 2, 256, 4),         # two tiles of tokens
+    (1792, 1024, 8, 2, 112, 7),
+    (1792, 1024, 8, 0, 128, 4),
+    (1920, 2048, 8, 1, 120, 4),
+    (4096, 1024, 8, 0, 128, 8),         # two stages of activations
+    (4096, 1024, 8, 2, 9, 8),
+]
+
+
+@pytest.mark.parametrize("inf,outf,k,cb,rows,n", CLUSTERS)
+def test_gemm_clusters_beside_the_rings(mod, oracle, inf, outf, k, cb, rows, n):
+    layer = _layer(mod, k, inf, outf, seed=rows + inf + k, cb=cb, bias=rows % 2 == 1)
+    x = np.random.default_rng(rows).standard_normal((rows, inf)).astype(np.float16)
+    _check(mod, oracle, layer, x)
+    m = mod.EXL3Linear(layer)
+    xd = torch.from_numpy(x).cuda()
+    first = m(xd)
+    assert all(torch.equal(m(xd), first) for _ in range(3))
+    assert mod.ops.Workspace.get(torch.device("cuda"), 1, 128).status() == 0
 
 
 # Shapes of each form of the kernel (test_gemm_plan.py checks that the plan takes it): tiles of more than the
