@@ -202,16 +202,21 @@ constexpr uint32_t kIdescMajorA = 1u << 15;          // A is MN-major
 // ---- the output rotation of 128 tokens: D2 = Y H ---------------------------------------------------------
 // B operand H[n][k] = (-1)^popcount(n & k), K-major: two 64-wide halves of k, 128 rows of 128 bytes each.  (As H64 and
 // -H64, half of it, with products of 64 columns: room for more packed tiles, but MLP of 300 rows 188.6 -> 190.8 us.)
+// (The decode warps do this before they decode.  A word's pattern depends on the low three bits of n, which are the same for
+// all of a thread's pieces if `threads` is a multiple of 64: 8 of the 12 bit counts a thread are made once.  With all 36, at a
+// quarter of the ordinary rate, every launch took 0.2 to 0.4 us longer: 6784 -> 768 at 330 rows 28.5 us, this way 28.1.)
 __device__ __forceinline__ void store_sylvester(uint8_t* h_mat, int thread, int threads)
 {
+    uint32_t w[4];
+    const int n_low = (thread >> 3) & 7;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        w[j] = 0x3C003C00u | ((__popc(n_low & (2 * j)) & 1) ? 0x8000u : 0u) | ((__popc(n_low & (2 * j + 1)) & 1) ? 0x80000000u : 0u);
+#pragma unroll
     for (int i = thread; i < 2048; i += threads) {
         const int kh = i >> 10, n = (i >> 3) & 127, ch = i & 7;
         const uint32_t flip = (__popc(n & (64 * kh + 8 * ch)) & 1) ? 0x80008000u : 0u;
-        uint32_t w[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            w[j] = flip ^ (0x3C003C00u | ((__popc(n & (2 * j)) & 1) ? 0x8000u : 0u) | ((__popc(n & (2 * j + 1)) & 1) ? 0x80000000u : 0u));
-        *reinterpret_cast<uint4*>(h_mat + kh * 16384 + n * 128 + ((ch ^ (n & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(h_mat + kh * 16384 + n * 128 + ((ch ^ (n & 7)) << 4)) = make_uint4(w[0] ^ flip, w[1] ^ flip, w[2] ^ flip, w[3] ^ flip);
     }
 }
 // Issued by ONE thread; `done` gets one arrival when the product is complete.
