@@ -355,8 +355,10 @@ __device__ __forceinline__ bool search_paths(EncodeShared& sh, uint8_t* stage, c
     using E = SearchSplit<K>;
     constexpr int NB = E::NB, kWarps = E::kThreads / 32;
     const int tid = threadIdx.x;
-    // The free path starts at the cheapest base.  Bases of a group whose first codewords have the same value cost the
-    // same to the bit, and the lowest wins, in whatever order the costs are summed, if the paths behind are one.
+    // The free path starts at the cheapest base.  Bases of a group whose first codewords have the same error cost the
+    // same to the bit, and the lowest wins, in whatever order the costs are summed, if the paths behind are one.  (Totals that
+    // are the same to the bit do not say so: the search from the start compares the first errors alone, and two that
+    // differ by less than the total's last place decide it.)
     uint32_t b0;
     bool unsure_start;
     {
@@ -386,7 +388,9 @@ __device__ __forceinline__ bool search_paths(EncodeShared& sh, uint8_t* stage, c
         bool other = false;
         if (tid < E::J) {
             const uint32_t b = ((uint32_t)tid << E::HB) | (b0 & (E::NH - 1));
-            other = cost(b) == bc && E::pick(__ldcg(ptr + E::at(b)), b) != E::pick(__ldcg(ptr + E::at(b0)), b0);
+            const uint32_t s = (b << K) | E::pick(__ldcg(ptr + E::at(b)), b), s0 = (b0 << K) | E::pick(__ldcg(ptr + E::at(b0)), b0);
+            auto first = [&](uint32_t state) { return sq_err((double)codebook_f32<CB>(state), (double)sh.w[0]); };
+            other = cost(b) == bc && ((s ^ s0) & (E::J - 1) || first(s) != first(s0));
         }
         unsure_start = __syncthreads_or(other) || !(second - bc > bc * 2.3e-13);       // 2^-42
     }

@@ -107,6 +107,29 @@ def test_encoder_free_and_pinned_paths(ops, oracle, k, cb, max_pins):
         assert (_u16(packed)[t] == oracle.pack_trellis_tile((want & ((1 << k) - 1)).astype(np.uint16), k)).all()
 
 
+@pytest.mark.parametrize("k,cb", [(3, 0), (4, 0), (6, 0), (6, 1)])
+def test_encoder_where_first_errors_differ_below_the_total(ops, oracle, k, cb):
+    """Codewords +a and -a in front of one path and a first weight of 1e-18 to 1e-15: both starts cost the same to the bit, but
+    the search from the start sees the first error alone, and without a pinned pass its choice stays."""
+    C = oracle.codebook_table(cb).astype(np.float64)
+    G = C.reshape(1 << k, 1 << (16 - k))             # a column: the states with the same low bits
+    a = np.abs(G).min(0)
+    both = np.flatnonzero((G == a).any(0) & (G == -a).any(0) & (a > 0))
+    tiles = []
+    for seed in range(12):
+        rng = np.random.default_rng(seed)
+        w, s = np.zeros(256), int(rng.choice(both))
+        w[0] = rng.choice([-1, 1]) * 10.0 ** rng.uniform(-18, -15)
+        for t in range(1, 256):
+            s = ((s << k) | int(rng.integers(1 << k))) & 0xFFFF
+            w[t] = C[s] + rng.standard_normal() * 0.3 * 2.0 ** -k
+        tiles.append(w.astype(np.float32))
+    for max_pins in (0, 4):
+        states, _ = ops.quantize_tiles(torch.from_numpy(np.stack(tiles)).cuda(), k, cb, max_pins=max_pins)
+        for t, w in enumerate(tiles):
+            assert (_u16(states)[t] == oracle.quantize_tile(w, k, cb, max_pins)[0]).all(), f"tile {t}"
+
+
 def test_quantised_matrix_decodes_to_the_chosen_codebook_values(ops, oracle):
     k, cb = 3, 0
     rng = np.random.default_rng(3)
