@@ -243,6 +243,10 @@ template <int K> struct SearchSplit {
     static constexpr int JC = JT < 16 ? JT : 16;         // n values per turn
     static constexpr int BL = L < 4 ? L : 4;             // bases whose costs are made at a time (all of them at once spill)
     static constexpr bool kInPlace = K == 2;
+    // Every how many steps a tile with too many close decisions is left.  At K = 8 MUL1's thousand values tie at most bases of a
+    // zero weight: 592 tiles of zeros take 50 ms this way, 70 with the whole search before they are left (48.6 by the search from
+    // the start alone), and others 1 % longer.  At lower K such tiles are few, or fill the list up late.
+    static constexpr int kLook = K == 8 ? 16 : 256;
     static constexpr size_t kCost = (size_t)NB * (kInPlace ? 1 : 2) * (sizeof(double) + sizeof(float));
     static constexpr int kChunk = 32768;                 // bytes of pointers fetched at a time by the walk
     static constexpr int kRowBytes = NB;                 // pointers of a step
@@ -320,10 +324,12 @@ __device__ __forceinline__ void leave_tile(const EncodeArgs& a, int64_t tile, in
 }
 
 // What a tile's paths should cost at most: far more than K bits usually leave, and what lies beyond the bulk of the
-// codebooks.  (A tile whose path costs more is in doubt.)  Two paths whose float64 costs, summed in any order, are
-// further apart than 2^-42 of the cost are in the right order; a decision that fp32 leaves unsure, or by less than
-// twice `close`, 2^-41 of the bound, is made in float64, and noted if it is closer than that.  False: the tile is not for this search.
-__device__ __forceinline__ bool cost_bound(EncodeShared& sh, float per_weight, float& bound)
+// codebooks, twice where one or two bits cannot follow large weights of changing sign.  (A tile whose path costs more is in
+// doubt.  592 tiles of standard deviation 10, K = 1 with 3INST and K = 2 with MUL1: 38.9 and 25.3 ms without the 2, 11.3 and 8.2
+// with it.)  Two paths whose float64 costs, summed in any order, are further apart than 2^-42 of the cost are in the right
+// order; a decision that fp32 leaves unsure, or by less than twice `close`, 2^-41 of the bound, is made in float64, and noted
+// if it is closer than that.  False: the tile is not for this search.
+__device__ __forceinline__ bool cost_bound(EncodeShared& sh, float per_weight, float per_outlier, float& bound)
 {
     const int tid = threadIdx.x;
     const float w = tid < 256 ? sh.w[tid] : 0.f, over = fmaxf(fabsf(w) - 2.5f, 0.f);
@@ -335,7 +341,7 @@ __device__ __forceinline__ bool cost_bound(EncodeShared& sh, float per_weight, f
     if (__syncthreads_or(!(fabsf(w) < kEncLargest))) return false;
     bound = 256.f * per_weight;
 #pragma unroll
-    for (int i = 0; i < 8; i++) bound += sh.sums[i];
+    for (int i = 0; i < 8; i++) bound += per_outlier * sh.sums[i];
     return true;
 }
 __device__ __forceinline__ void note_close(EncodeShared& sh, int t, uint32_t base, double gap)
@@ -345,6 +351,13 @@ __device__ __forceinline__ void note_close(EncodeShared& sh, int t, uint32_t bas
         sh.close_at[at] = ((uint32_t)t << 16) | base;
         sh.close_gap[at] = gap;
     }
+}
+
+// For all threads, between two steps: whether more decisions have been noted than there is room for, which leaves the tile
+// in doubt whatever comes.
+__device__ __forceinline__ bool too_close(EncodeShared& sh)
+{
+    return __syncthreads_or(sh.n_close > kEncClose);
 }
 
 // The paths of a tile from the pointers of all its bases, `cost` giving a base's cost to the end of the tile: the free
@@ -473,7 +486,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs
         if (tid == 0) sh.smin[0] = sh.smin[1] = 0x7F800000u;
         for (int b = tid; b < NB; b += E::NT) { md0[b] = 0.0; mf0[b] = 0.f; }
         float bound;
-        if (!cost_bound(sh, 32.f / (float)(1 << (2 * K)), bound)) {
+        if (!cost_bound(sh, 32.f / (float)(1 << (2 * K)), K == 2 ? 2.f : 1.f, bound)) {
             if (tid == 0) leave_tile(a, tile, kEncOdd);
             continue;
         }
@@ -482,6 +495,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs
         const uint32_t near = __float_as_uint(bound * 0x1p-20f);
 
         double off = 0.0;                                // lower bound of every cost of the step
+        bool left = false;
 #pragma unroll 1
         for (int u = 0; u < 256; u++) {
             const int t = 255 - u;
@@ -621,9 +635,11 @@ __global__ void __launch_bounds__(kEncThreads, 1) search_kernel(const EncodeArgs
             low_new = __reduce_min_sync(0xFFFFFFFFu, low_new);
             if ((tid & 31) == 0) atomicMin(&sh.smin[(u + 1) % 3], low_new);
             __syncthreads();
+            if constexpr (E::kLook < 256)
+                if (u % E::kLook == E::kLook - 1 && (left = too_close(sh))) break;
         }
         constexpr int end_rot = E::kInPlace ? (K * 256) % LB : 0;
-        if (search_paths<K, CB>(sh, smem, ptr, a.max_pins, bound, [&](uint32_t b) { return md0[slot(b, end_rot)]; })) store_tile<K>(sh, a, tile);
+        if (!left && search_paths<K, CB>(sh, smem, ptr, a.max_pins, bound, [&](uint32_t b) { return md0[slot(b, end_rot)]; })) store_tile<K>(sh, a, tile);
         else if (tid == 0) leave_tile(a, tile, kEncDoubt);
     }
 }
@@ -1001,7 +1017,7 @@ template <int CB> __global__ void __launch_bounds__(kEncThreads1, 1) search_kern
         if (tile >= a.n_tiles) return;
         for (int b = tid; b < NB; b += kEncThreads1) __stcg(cost0 + b, 0.0);
         float bound;
-        if (!cost_bound(sh, 8.f, bound)) {
+        if (!cost_bound(sh, 8.f, 2.f, bound)) {
             if (tid == 0) leave_tile(a, tile, kEncDoubt);
             continue;
         }

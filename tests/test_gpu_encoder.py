@@ -107,6 +107,20 @@ def test_encoder_free_and_pinned_paths(ops, oracle, k, cb, max_pins):
         assert (_u16(packed)[t] == oracle.pack_trellis_tile((want & ((1 << k) - 1)).astype(np.uint16), k)).all()
 
 
+@pytest.mark.parametrize("k,cb", [(1, 0), (1, 2), (2, 2), (4, 2), (8, 2)])
+def test_encoder_of_tiles_it_leaves_early_and_of_large_weights(ops, oracle, k, cb):
+    """Zeros, whose decisions are all ties: more than are noted, in the first steps or (a tile's front) in the last ones; weights far
+    beyond the codebook; an ordinary tile behind them on the same slot."""
+    w = np.random.default_rng(300 + k).standard_normal((6, 256)).astype(np.float32)
+    w[0] = 0.0
+    w[1, :3] = 0.0
+    w[2, 128:] = 0.0
+    w[3:5] *= 10.0
+    states, _ = ops.quantize_tiles(torch.from_numpy(w).cuda(), k, cb, max_tiles_in_flight=1)
+    for t in range(6):
+        assert (_u16(states)[t] == oracle.quantize_tile(w[t], k, cb)[0]).all(), f"tile {t}"
+
+
 @pytest.mark.parametrize("k,cb", [(3, 0), (4, 0), (6, 0), (6, 1)])
 def test_encoder_where_first_errors_differ_below_the_total(ops, oracle, k, cb):
     """Codewords +a and -a in front of one path and a first weight of 1e-18 to 1e-15: both starts cost the same to the bit, but
