@@ -321,8 +321,10 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
                 for (int q = 0; q < 4; q++) la[q] = lb[q] = make_uint4(0u, 0u, 0u, 0u);
             if (pre) {
-                const __half* q0 = pre + (ok0 && pre_row ? (int64_t)pre_row[o0] : mb0 + v) * n + col;
-                const __half* q1 = pre + (ok1 && pre_row ? (int64_t)pre_row[o1] : mb1 + v) * n + col;
+                // (without pre_row, only the members of a group have multipliers of their own; a row out of use has the first ones)
+                const int64_t mv = COPIES && member_rows ? v : 0;
+                const __half* q0 = pre + (ok0 && pre_row ? (int64_t)pre_row[o0] : mb0 + mv) * n + col;
+                const __half* q1 = pre + (ok1 && pre_row ? (int64_t)pre_row[o1] : mb1 + mv) * n + col;
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const uint4 a = *reinterpret_cast<const uint4*>(q0 + 32 * q);

@@ -139,3 +139,36 @@ def test_prefill_tables_with_all_gate_rows_before_all_up_rows(lib, n_tokens):
         t[:, :2] += t[:, 6:7]
         t[:, 6] = 0
     assert torch.equal(tgu[used], tgu0[used]) and bool((tgu[~used, 0] >= tgu[~used, 1]).all())
+
+
+def _tile_gemm(lib, x, xh_rows, row_src, suh, tile, flags, rows_dev=None, seed=0):
+    """One tile of 128 columns through exl3_gemm_tiles (rows_dev: through exl3_gemm_tiles_peers, without peers)."""
+    from ponyexl3_b200 import ops
+
+    n_in = x.shape[1]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    trellis = torch.randint(-32768, 32768, (n_in // 16, 8, 64), dtype=torch.int16, device="cuda", generator=g)
+    y = torch.zeros((tile[1], 128), dtype=torch.float16, device="cuda")
+    tiles = torch.tensor([[tile[0], tile[1], 0, 0, 0, 128, 0, 0]], dtype=torch.int32, device="cuda")
+    L = lib.load()
+    ws = ops.Workspace.get_bytes(x.device, int(L.exl3_gemm_workspace_bytes(xh_rows, n_in)))
+    args = (row_src.data_ptr(), suh.data_ptr(), None, trellis.data_ptr(), n_in // 16, 8, 4, 0, tiles.data_ptr(), 1, None, y.data_ptr(), 128, None)
+    tail = (ws.buf.data_ptr(), ws.nbytes, flags, torch.cuda.current_stream().cuda_stream)
+    if rows_dev is None:
+        lib.check(L.exl3_gemm_tiles(x.data_ptr(), 0, n_in, xh_rows, *args, *tail), "tiles")
+    else:
+        lib.check(L.exl3_gemm_tiles_peers(x.data_ptr(), 0, n_in, xh_rows, rows_dev.data_ptr(), *args, None, None, 0, 0, *tail), "tiles")
+    return y[tile[0]:]
+
+
+@pytest.mark.parametrize("half", [1000, 37881])
+def test_row_pairs_without_a_multiplier_row(lib, half):
+    """EXL3_FLAG_ROW_PAIRS without suh_row: the first row of suh is all rows', below and above the number of rows from which a row of
+    x is read once for two (the rows behind the last have one row of multipliers, too)."""
+    x = torch.randn((64, 512), device="cuda").half()
+    row_src = (torch.arange(half, dtype=torch.int32, device="cuda") % 64).repeat(2)
+    suh = torch.stack([torch.where(torch.rand(512, device="cuda") < 0.5, -1.0, 1.0), torch.full((512,), 3.0, device="cuda")]).half()
+    for tile in ((0, 64), (2 * half - 64, 2 * half)):
+        plain, pairs = (_tile_gemm(lib, x, 2 * half, row_src, suh, tile, flags) for flags in (0, 16))
+        assert torch.equal(plain, pairs)
