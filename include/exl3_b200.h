@@ -73,7 +73,8 @@ extern "C" {
                                    n_pairs + p.  exl3_gemm_tiles: rows r and r + xh_rows / 2 have the same row_src (which
                                    is required, and xh_rows even), so that a row of x is read once for both */
 #define EXL3_FLAG_WIDE_SCALES 32u /* exl3_gemm_tiles: x * suh goes into the rotation as it is, not rounded to fp16, whatever
-                                   the number of rows; so does the GEMV's (no difference for multipliers of +-1) */
+                                   the number of rows; so does the GEMV's (no difference for multipliers of +-1).
+                                   exl3_gemm_tiles_peers with xh_rows_dev: x itself is rounded to fp16 */
 
 typedef void* exl3_stream_t;    /* cudaStream_t */
 

@@ -203,7 +203,8 @@ __global__ void __launch_bounds__(256)
 // x * pre is rounded to fp16, which is exact for +-1 only.  With SPLIT it is two fp16 parts and two products: for
 // the rows of a sibling group that one by one would be few enough for the butterfly kernel, which does not round
 // it (multipliers of 0.5 to 1.5, 40 rows: 5.0e-4 off the oracle without, 7e-5 with it).  A group of 5120 + 2 x 1024
-// columns and 24 to 63 rows takes 19.4 .. 21.0 us without, 19.6 .. 21.2 with it, 23.1 .. 27.2 by the butterfly kernel.
+// columns and 24 to 63 rows takes 19.4 .. 21.0 us without, 19.6 .. 21.2 with it, 23.1 .. 27.2 by the butterfly kernel.  (And for
+// EXL3_FLAG_WIDE_SCALES where the number of rows is on the device, which the butterfly kernel does not read.)
 //
 // COPIES: output rows r, r + base, r + 2 base, .. are the same row of x with other multipliers (gate and up of a
 // SwitchGLU, the members of a sibling group), and a block's loads of x serve all of them.
@@ -500,7 +501,7 @@ int launch_hadamard(const void* x, int x_dtype, int64_t rows, int64_t n, int64_t
     const int early = pdl ? 1 : 0;
     cudaError_t e;
     if (mma) {
-        const bool split = member_rows > 0 && member_rows < kHadamardMmaMinRows;
+        const bool split = (member_rows > 0 && member_rows < kHadamardMmaMinRows) || wide_scales;
         auto launch = [&](auto* xt) {
             using T = std::remove_const_t<std::remove_pointer_t<decltype(xt)>>;
             const auto kernel = copies > 1 ? hadamard_mma_kernel<T, false, true> : split ? hadamard_mma_kernel<T, true, false> : hadamard_mma_kernel<T, false, false>;

@@ -172,3 +172,16 @@ def test_row_pairs_without_a_multiplier_row(lib, half):
     for tile in ((0, 64), (2 * half - 64, 2 * half)):
         plain, pairs = (_tile_gemm(lib, x, 2 * half, row_src, suh, tile, flags) for flags in (0, 16))
         assert torch.equal(plain, pairs)
+
+
+def test_wide_scales_with_a_row_count_on_the_device(lib):
+    """EXL3_FLAG_WIDE_SCALES where the tensor cores rotate whatever the number of rows: multipliers of 0.5 to 1.5 are not rounded
+    with x.  Against the rotation that multiplies in fp32, what is left is roundings of the rotated rows that flip; a rounded
+    product is 2^-12 rms and more off."""
+    x = torch.randn((200, 1024), device="cuda").half()
+    row_src = torch.arange(200, dtype=torch.int32, device="cuda")
+    suh = (torch.rand((1, 1024), device="cuda") + 0.5).half()
+    rows = torch.tensor([200], dtype=torch.int32, device="cuda")
+    want = _tile_gemm(lib, x, 200, row_src, suh, (0, 200), 32).float()
+    err = lambda flags: float((_tile_gemm(lib, x, 200, row_src, suh, (0, 200), flags, rows).float() - want).norm() / want.norm())
+    assert err(32) <= 2 ** -13 and err(0) >= 2 ** -12, (err(32), err(0))
