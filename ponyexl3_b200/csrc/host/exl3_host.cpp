@@ -463,7 +463,9 @@ PyObject* switch_glu(PyObject* const* arg)
     const at::Tensor ygu = empty_half({n, 2 * H}, device);
     at::Tensor y = empty_half({R, kk, D}, device);
     if (n == 0) return THPVariable_Wrap(std::move(y));
-    if (PyObject_IsTrue(arg[14]) && !by_expert(n, E, D, H)) {
+    // (the tile kernel wants the output scales on 16 bytes, where the GEMV takes 8)
+    const bool tiles_take_scales = (reinterpret_cast<uintptr_t>(gu_svh) | reinterpret_cast<uintptr_t>(dn_svh)) % 16 == 0;
+    if (PyObject_IsTrue(arg[14]) && !(tiles_take_scales && by_expert(n, E, D, H))) {
         // tables, gate|up, down with the GLU on load
         const int64_t gb = H / 128, db = D / 128, n_gu = n * 2 * gb, n_dn = n * db;
         const at::Tensor tab = empty_int(4 * (n_gu + n_dn) + 5 * n, device);

@@ -166,6 +166,24 @@ def test_switch_glu_few_tokens_by_expert(cuda, oracle, k, tokens):
     assert rel_err(y.cpu().numpy().reshape(tokens, kk, D), want) <= 2e-3
 
 
+@pytest.mark.parametrize("name", ["_gu_svh", "_dn_svh"])
+def test_few_tokens_with_scales_on_eight_bytes(cuda, oracle, name):
+    """Output scales aligned for the GEMV only: sixteen tokens on few experts stay with it (the tile kernel refuses them)."""
+    E, D, H, kk, T = 8, 512, 512, 8, 16
+    w = _experts(E, D, H, 4, seed=95)
+    sw = _switch(w, 4, 0)
+    t = getattr(sw, name)
+    odd = torch.empty(t.numel() + 8, dtype=t.dtype, device="cuda")[4:-4]
+    odd.copy_(t.reshape(-1))
+    setattr(sw, name, odd.view(t.shape))
+    assert odd.data_ptr() % 16 == 8
+    rng = np.random.default_rng(T)
+    x = (rng.standard_normal((T, D)) * 0.5).astype(np.float16)
+    idx = np.stack([rng.permutation(E)[:kk] for _ in range(T)]).astype(np.int64)
+    y = sw(torch.from_numpy(x).cuda()[None], torch.from_numpy(idx).cuda()[None])
+    assert rel_err(y.cpu().numpy().reshape(T, kk, D), oracle.switch_glu(x, idx, **w, k=4, cb=0)) <= 2e-3
+
+
 def test_few_tokens_by_expert_keep_scales_unrounded(cuda, oracle):
     """Multipliers other than +-1: below 17 tokens x * suh is not rounded before the rotation on either path, so sixteen
     tokens at once are no further from the oracle than by fours (one row per pair).  Roundings that flip along the chain
