@@ -93,7 +93,7 @@ def build_host(force: bool = False, verbose: bool = False) -> Path:
     from ._lib import host_path
 
     host = host_path()
-    deps = max(p.stat().st_mtime for p in (HOST_SRC, PKG.parent / "include" / "exl3_b200.h"))
+    deps = max(p.stat().st_mtime for p in (HOST_SRC, CSRC / "exl3_moe_plan.h", PKG.parent / "include" / "exl3_b200.h"))
     if not force and host.exists() and host.stat().st_mtime >= deps:
         return host
 

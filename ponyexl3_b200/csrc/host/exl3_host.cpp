@@ -14,11 +14,11 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <algorithm>
-#include <cmath>
 #include <mutex>
 #include <string>
 
 #include "../../../include/exl3_b200.h"
+#include "../exl3_moe_plan.h"
 
 namespace {
 
@@ -421,18 +421,17 @@ PyObject* mlp(PyObject* const* arg)
 }
 
 // ---- stacked-expert SwitchGLU ---------------------------------------------------------------------------------
-// Few tokens: every (token, slot) pair as a one-row problem, which decodes an expert's weights once per pair, or the
-// pairs sorted by expert, which decodes them once per expert but has two more launches and longer tables.  With pairs
-// spread evenly over the experts the one takes about 20 + 0.88 n us for n pairs (2048 / 512 dims, K = 4), the other 30 + 0.88 u
-// for the u experts that get any; with 1024 / 256 dims 14 + 0.28 n and 29 + 0.29 u: the line lies where n - u pays for what the
-// second has more.  us by pairs / by expert at 16 tokens, top-8: 256 experts 132 / 118, 128 131 / 98, 64 131 / 82 (2048 / 512);
-// 50 / 58, 49 / 54, 48 / 44 (1024 / 256); at 8 tokens 77 / 89, 76 / 75, 76 / 69.
-// (More than 1024 experts or 2^20 pairs have no tables by expert.)
-bool by_expert(int64_t pairs, int64_t experts, int64_t d, int64_t h)
+// Few tokens by expert instead of by pairs (exl3_moe_plan.h), remembered for the shapes seen last: some us to find out, 0.02 to look up.
+// The tile kernel wants the output scales on 16 bytes, where the GEMV takes 8.
+bool by_expert(int64_t pairs, int64_t experts, int64_t d, int64_t h, int k, const uint16_t* gu_svh, const uint16_t* dn_svh)
 {
-    if (experts > 1024 || pairs > (1 << 20)) return false;
-    const double e = (double)experts, hit = experts > 1 ? e * -std::expm1((double)pairs * std::log1p(-1.0 / e)) : 1.0;
-    return (double)pairs - hit > 8.0 + 3.7e7 / (3.0 * (double)d * (double)h);
+    if ((reinterpret_cast<uintptr_t>(gu_svh) | reinterpret_cast<uintptr_t>(dn_svh)) % 16) return false;
+    struct Slot { int64_t pairs, experts, d, h; int k; bool answer; };
+    static thread_local Slot memo[16] = {};
+    Slot& m = memo[((uint64_t)pairs * 0x9E3779B97F4A7C15u ^ (uint64_t)k * 0xC2B2AE3D27D4EB4Fu) >> 60];
+    if (m.pairs != pairs || m.experts != experts || m.d != d || m.h != h || m.k != k)
+        m = Slot{pairs, experts, d, h, k, exl3::moe_by_expert(pairs, experts, d, h, k)};
+    return m.answer;
 }
 
 // switch_glu(x2d, indices (R, k), gu_trellis, gu_suh, gu_svh, dn_trellis, dn_suh, dn_svh, experts, hidden, k, cb,
@@ -463,9 +462,7 @@ PyObject* switch_glu(PyObject* const* arg)
     const at::Tensor ygu = empty_half({n, 2 * H}, device);
     at::Tensor y = empty_half({R, kk, D}, device);
     if (n == 0) return THPVariable_Wrap(std::move(y));
-    // (the tile kernel wants the output scales on 16 bytes, where the GEMV takes 8)
-    const bool tiles_take_scales = (reinterpret_cast<uintptr_t>(gu_svh) | reinterpret_cast<uintptr_t>(dn_svh)) % 16 == 0;
-    if (PyObject_IsTrue(arg[14]) && !(tiles_take_scales && by_expert(n, E, D, H))) {
+    if (PyObject_IsTrue(arg[14]) && !by_expert(n, E, D, H, k, gu_svh, dn_svh)) {
         // tables, gate|up, down with the GLU on load
         const int64_t gb = H / 128, db = D / 128, n_gu = n * 2 * gb, n_dn = n * db;
         const at::Tensor tab = empty_int(4 * (n_gu + n_dn) + 5 * n, device);
