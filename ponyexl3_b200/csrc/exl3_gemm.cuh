@@ -204,15 +204,17 @@ constexpr uint32_t kIdescMajorA = 1u << 15;          // A is MN-major
 // -H64, half of it, with products of 64 columns: room for more packed tiles, but MLP of 300 rows 188.6 -> 190.8 us.)
 // (The decode warps do this before they decode.  A word's pattern depends on the low three bits of n, which are the same for
 // all of a thread's pieces if `threads` is a multiple of 64: 8 of the 12 bit counts a thread are made once.  With all 36, at a
-// quarter of the ordinary rate, every launch took 0.2 to 0.4 us longer: 6784 -> 768 at 330 rows 28.5 us, this way 28.1.)
-__device__ __forceinline__ void store_sylvester(uint8_t* h_mat, int thread, int threads)
+// quarter of the ordinary rate, every launch took 0.2 to 0.4 us longer: 6784 -> 768 at 330 rows 28.5 us, this way 28.1.  UNROLL
+// pieces at a time: all four in the forms whose tail is long; one in JOINT, which runs for a tile only and is the quicker
+// the less code it has to fetch, K = 1, 5120 x 5120 at 77 rows 16.9 / 16.6.)
+template <int UNROLL> __device__ __forceinline__ void store_sylvester(uint8_t* h_mat, int thread, int threads)
 {
     uint32_t w[4];
     const int n_low = (thread >> 3) & 7;
 #pragma unroll
     for (int j = 0; j < 4; j++)
         w[j] = 0x3C003C00u | ((__popc(n_low & (2 * j)) & 1) ? 0x8000u : 0u) | ((__popc(n_low & (2 * j + 1)) & 1) ? 0x80000000u : 0u);
-#pragma unroll
+#pragma unroll UNROLL
     for (int i = thread; i < 2048; i += threads) {
         const int kh = i >> 10, n = (i >> 3) & 127, ch = i & 7;
         const uint32_t flip = (__popc(n & (64 * kh + 8 * ch)) & 1) ? 0x80008000u : 0u;
@@ -529,7 +531,7 @@ __global__ void __launch_bounds__(kTsThreads, 1)
         const int nks = a.t_in >> 2;
         LaneWords<K> lw;
         lw.init(lane);
-        store_sylvester(h_mat, dt, 512);
+        store_sylvester<F::kJoint ? 1 : 4>(h_mat, dt, 512);
         // A set decodes its k-steps in order, whatever tiles they belong to.  With AHEAD the warps decode as many
         // k-steps of the next tile as there are stages before they finish one, so that the tensor core has work
         // in the meantime; a CTA with hardly more than one tile is 1 us quicker without.
