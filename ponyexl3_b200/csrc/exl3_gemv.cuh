@@ -634,7 +634,11 @@ __global__ void __launch_bounds__(kGemvThreads, 1)
                 asm volatile("bar.sync 3, %0;" ::"n"(kGemvThreads) : "memory");
             } else {
                 asm volatile("bar.arrive 3, %0;" ::"n"(kGemvThreads) : "memory");
+#ifdef EXL3_PROFILE
+                finish = false;                        // its stamps are still to be written
+#else
                 return;                                // a half has one segment
+#endif
             }
         } else {
             if ((size_t)(2 * c + 2) * nv * sizeof(float) > a.partial_bytes) {   // never true for a launch as planned
