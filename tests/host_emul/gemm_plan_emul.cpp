@@ -6,9 +6,14 @@
 
 using namespace exl3;
 
-extern "C" int emul_joint(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok, int room, int w_bytes, int most)
+extern "C" int emul_joint_beside(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok, int room, int w_bytes, int most)
 {
     return ts_joint(ts_plan(rows, tiles_n, nks, sms, tok, tok_wide, room_tok), tiles_n, nks, sms, TsRings{room, w_bytes}, most);
+}
+// K = 4
+extern "C" int emul_joint(int64_t rows, int64_t tiles_n, int nks, int sms, int tok, int tok_wide, int room_tok, int most)
+{
+    return emul_joint_beside(rows, tiles_n, nks, sms, tok, tok_wide, room_tok, 162 * 1024, 4096, most);
 }
 
 // Every number of CTAs that may be asked for, over 16 .. 256 rows, up to sms / 2 column tiles and 2 .. most_nks k-steps: the fewest

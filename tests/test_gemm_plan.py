@@ -96,7 +96,7 @@ def test_a_plan_costs_less_than_a_launch(emul):
 def test_clusters_of_a_tile(emul):
     """Where the CTAs of a tile become a cluster: up to eight of them with at least four k-steps each, all on the chip at a time, no
     tile of more than 128 tokens, and never more CTAs than asked for."""
-    emul.emul_joint.argtypes = [ctypes.c_int64, ctypes.c_int64] + [ctypes.c_int] * 8
+    emul.emul_joint.argtypes = [ctypes.c_int64, ctypes.c_int64] + [ctypes.c_int] * 6
     rng = random.Random(7)
     taken = set()
     for _ in range(3000):
@@ -104,12 +104,12 @@ def test_clusters_of_a_tile(emul):
         most = rng.randint(1, 8)
         args = (rows, tiles_n, nks, 148, 256, 384, rng.choice([0, 384]))
         tok, tiles_m, _, split, _ = _plan(emul.emul_plan, *args)
-        n = emul.emul_joint(*args, ROOM, 4096, most)
+        n = emul.emul_joint(*args, most)
         taken.add(n)
         assert n == 0 or (2 <= n <= most and 4 * n <= nks and split and tok <= 128 and tiles_m * tiles_n * n <= 148), (args, n)
     assert taken == {0, 2, 3, 4, 5, 6, 7, 8}
-    assert emul.emul_joint(77, 40, 80, 148, 256, 384, 384, ROOM, 4096, 8) == 3      # 5120 x 5120: three CTAs of 27 k-steps
-    assert emul.emul_joint(77, 136, 80, 148, 256, 384, 384, ROOM, 4096, 8) == 0     # 5120 x 17408: a CTA per tile
+    assert emul.emul_joint(77, 40, 80, 148, 256, 384, 384, 8) == 3      # 5120 x 5120: three CTAs of 27 k-steps
+    assert emul.emul_joint(77, 136, 80, 148, 256, 384, 384, 8) == 0     # 5120 x 17408: a CTA per tile
 
 
 @pytest.mark.parametrize("k", range(1, 9))
@@ -126,6 +126,6 @@ def test_the_gpu_tests_reach_clusters_of_each_size(emul):
     """By the number of k-steps, so that a device that holds fewer clusters of the largest sizes does not change them."""
     from test_gpu_gemm import CLUSTERS
 
-    emul.emul_joint.argtypes = [ctypes.c_int64, ctypes.c_int64] + [ctypes.c_int] * 8
+    emul.emul_joint_beside.argtypes = [ctypes.c_int64, ctypes.c_int64] + [ctypes.c_int] * 8
     for inf, outf, k, cb, rows, n in CLUSTERS:
-        assert emul.emul_joint(rows, outf // 128, inf // 64, 148, *TOKENS[max(0, k - 4)], 384, ROOM, 1024 * k, 8) == n, (inf, outf, k, rows)
+        assert emul.emul_joint_beside(rows, outf // 128, inf // 64, 148, *TOKENS[max(0, k - 4)], 384, ROOM, 1024 * k, 8) == n, (inf, outf, k, rows)

@@ -152,6 +152,20 @@ def test_switch_glu_decode_matches_oracle(cuda, oracle, tokens, k, cb, act):
     assert rel_err(y.cpu().numpy().reshape(tokens, kk, D), want) <= 2e-3
 
 
+@pytest.mark.parametrize("k,tokens", [(4, 6), (4, 16), (1, 13), (6, 16)])
+def test_switch_glu_few_tokens_by_expert(cuda, oracle, k, tokens):
+    """Pairs that crowd on few experts: 6 tokens of 8 experts lie below the line between the two paths (48 - 8 < 55),
+    13 and 16 above it (104 - 8, 128 - 8)."""
+    E, D, H, kk = 8, 512, 512, 8
+    w = _experts(E, D, H, k, seed=60 + k)
+    rng = np.random.default_rng(tokens)
+    x = (rng.standard_normal((tokens, D)) * 0.5).astype(np.float16)
+    idx = np.stack([rng.permutation(E)[:kk] for _ in range(tokens)]).astype(np.int64)
+    y = _switch(w, k, 0)(torch.from_numpy(x).cuda()[None], torch.from_numpy(idx).cuda()[None])
+    want = oracle.switch_glu(x, idx, **w, k=k, cb=0)
+    assert rel_err(y.cpu().numpy().reshape(tokens, kk, D), want) <= 2e-3
+
+
 # K, tokens, experts, dims, top-k, and whether they go by expert (test_moe_plan.py checks that they do)
 FEW_TOKENS = [
     (4, 6, 8, 512, 512, 8, False),
@@ -164,7 +178,7 @@ FEW_TOKENS = [
 
 
 @pytest.mark.parametrize("k,tokens,E,D,H,kk,by_expert", FEW_TOKENS)
-def test_switch_glu_few_tokens_by_expert(cuda, oracle, k, tokens, E, D, H, kk, by_expert):
+def test_switch_glu_few_tokens_on_both_sides_of_the_line(cuda, oracle, k, tokens, E, D, H, kk, by_expert):
     """Pairs that crowd on few experts, on both sides of the line between the two paths."""
     w = _experts(E, D, H, k, seed=60 + k)
     rng = np.random.default_rng(tokens)

@@ -98,7 +98,7 @@ def test_gemm_tiles_shared_between_ctas(mod, oracle, rows, inf, outf, k, cb):
 @pytest.mark.parametrize("rows", [9, 16, 33, 100, 128])
 @pytest.mark.parametrize("inf,outf,k,cb", [
     (2048, 384, 4, 0),          # eight CTAs of four k-steps per tile; more CTAs than pieces of 16 tokens, and as many
-    (2048, 2560, 5, 1),         # seven, or as many as the device holds twenty clusters of
+    (2048, 2560, 5, 1),         # seven
     (1152, 5120, 3, 2),         # three
     (896, 8192, 8, 0),          # two, the deepest packed tiles
 ])
