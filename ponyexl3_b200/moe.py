@@ -163,14 +163,15 @@ class EXL3SwitchGLU(torch.nn.Module):
             suh_gu.data_ptr(), suh_dn.data_ptr(), tiles_gu.data_ptr(), tiles_dn.data_ptr(), counts.data_ptr(),
             0, stream), "exl3_moe_prefill_tables_range")
         rows_gu, rows_dn = counts[0:1], counts[1:2]
+        hint = max(1, n // total)       # rows of an expert
         ygu = torch.empty((n, 2 * H), dtype=torch.float16, device=dev)
         ops.gemm_tiles(x2d, xh_rows=2 * n, row_src=row_src, suh=self._gu_suh, suh_row=suh_gu,
                        trellis=self._gu_trellis, k=self.k, cb=self.cb, tiles=tiles_gu, svh=self._gu_svh, y=ygu,
-                       xh_rows_dev=rows_gu)
+                       xh_rows_dev=rows_gu, rows_hint=hint)
         # the down launch reads [gate | up] as it is and applies the GLU while it rotates the rows
         ops.gemm_tiles(ygu, xh_rows=n, row_src=None, suh=self._dn_suh, suh_row=suh_dn, trellis=self._dn_trellis,
                        k=self.k, cb=self.cb, tiles=tiles_dn, svh=self._dn_svh, y=None, y_row_map=order,
-                       glu=self.activation, xh_rows_dev=rows_dn, peers=peers)
+                       glu=self.activation, xh_rows_dev=rows_dn, peers=peers, rows_hint=hint)
 
     @torch.no_grad()
     def prefill_range(self, x2d: torch.Tensor, indices: torch.Tensor, expert_range, peers) -> None:

@@ -344,13 +344,13 @@ def gemm_tiles(x2d: torch.Tensor, *, xh_rows: int, row_src: torch.Tensor | None,
                suh: torch.Tensor | None, suh_row: torch.Tensor | None, trellis: torch.Tensor, k: int,
                cb: int, tiles: torch.Tensor, svh: torch.Tensor | None, y: torch.Tensor | None,
                y_row_map: torch.Tensor | None = None, glu: str | None = None,
-               xh_rows_dev: torch.Tensor | None = None, peers=None) -> torch.Tensor | None:
+               xh_rows_dev: torch.Tensor | None = None, peers=None, rows_hint: int = 0) -> torch.Tensor | None:
     """Tensor-core GEMM over a tile table (see exl3_gemm_tiles in the header).  `tiles` is an
     int32 CUDA tensor (n_tiles, 8); `y` (rows, cols) fp16 is written in place.
     glu: x2d rows are [gate | up] and the input is fp16(act(gate) * up).
     xh_rows_dev: int32 CUDA scalar, rotated rows in use.  peers = (y_ptrs, counter_ptrs, n,
     rows_per_peer, row_stride): the output rows go to the GPUs that own them (y may be None), see
-    exl3_gemm_tiles_peers."""
+    exl3_gemm_tiles_peers.  rows_hint: average rows of the tiles in use, 0 if not known."""
     _need_cuda(x2d, "x")
     t_in, t_out_total, _ = trellis.shape
     if x2d.shape[1] != t_in * 16 * (2 if glu is not None else 1):
@@ -363,7 +363,7 @@ def gemm_tiles(x2d: torch.Tensor, *, xh_rows: int, row_src: torch.Tensor | None,
     lib = _lib.load()
     ws = Workspace.get_bytes(x2d.device, int(lib.exl3_gemm_workspace_bytes(xh_rows, t_in * 16)))
     ptr = lambda t: None if t is None else t.data_ptr()
-    flags = _GLU_FLAGS[glu]
+    flags = _GLU_FLAGS[glu] | min(rows_hint, 0xFFFF) << 16
     if peers is None and xh_rows_dev is None:
         _lib.check(lib.exl3_gemm_tiles(
             x2d.data_ptr(), _DTYPES[x2d.dtype], x2d.stride(0), xh_rows, ptr(row_src), ptr(suh),
