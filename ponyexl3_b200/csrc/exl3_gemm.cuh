@@ -24,8 +24,8 @@
 // Work is dealt in k-steps: CTA c takes the k-steps [U c/G, U (c+1)/G) of the tiles laid end to end, so a
 // layer with few tiles still uses every SM.  A tile that several CTAs share is finished by the one that
 // ends last: each writes its fp32 sums to its own slot of the workspace and counts itself; the last
-// one adds the slots in CTA order, so the result does not depend on who came last.  Grouped launches
-// (a tile table) take whole tiles in turn.
+// one adds the slots in CTA order, so the result does not depend on who came last.  (A cluster's CTAs exchange
+// their sums instead, see JOINT.)  Launches over a tile table have a kernel of their own, exl3_gemm_tiles.cuh.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets ST_TC_TIMEOUT, the thread stops waiting (so
 // named barriers still meet) and the tensor memory is freed at the end.
@@ -564,9 +564,12 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                     tc_fence_after_sync();
                 };
                 const uint32_t a_tmem = tmem_base + ((uint32_t)(32 * q) << 16) + F::kACol0 + 32 * st;
-                // Tile columns 2q, 2q + 1 of all four tile rows, one after the other: half the code leaves the issuing warps and
-                // a short call's start more of the instruction cache (512 x 512 8.4 -> 7.9 us).  The wide form, whose sets
-                // mostly wait for MMAs, reads all words first and is 2 % quicker with it (an MLP of 300 rows).
+                // Tile columns 2q, 2q + 1 of all four tile rows, one after the other.  As a loop, half the code leaves the issuing
+                // warps and a short call's start more of the instruction cache: for JOINT, whose CTAs have few k-steps, and for
+                // K = 1.  Elsewhere the loop costs long ranges more than it gives short ones: us as a loop / unrolled / before
+                // there was a loop, 5120 x 17408: K = 3, 200 rows 39.9 / 38.9 / 38.9, K = 5, 64 rows 35.1 / 33.0 / 35.6; 512 x 512,
+                // K = 5, 64 rows 8.2 / 8.2 / 8.3.  The wide form, whose sets mostly wait for MMAs, reads all words first and is 2 %
+                // quicker with it (an MLP of 300 rows).
                 if constexpr (F::kWide) {
                     uint32_t pw[2][4][K == 4 ? 4 : 3];
 #pragma unroll
@@ -600,7 +603,8 @@ __global__ void __launch_bounds__(kTsThreads, 1)
                         tmem_st_16x32cols(a_tmem + ((uint32_t)(16 * h) << 16), frag);
                     }
                 } else {
-#pragma unroll 1
+                    constexpr int kUnroll = F::kJoint || K == 1 ? 1 : 2;
+#pragma unroll kUnroll
                     for (int h = 0; h < 2; h++) {
                         uint32_t frag[16];
 #pragma unroll
