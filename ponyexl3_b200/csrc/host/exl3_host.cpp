@@ -498,13 +498,16 @@ PyObject* switch_glu(PyObject* const* arg)
         });
         const unsigned hint = (unsigned)std::max<int64_t>(1, std::min<int64_t>(n / E, 0xFFFF)) << 16;      // rows of an expert
         const unsigned wide = PyObject_IsTrue(arg[14]) ? EXL3_FLAG_WIDE_SCALES : 0u;      // few tokens: what the GEMV would give
-        Workspace ws = workspace(dev, api.exl3_gemm_workspace_bytes(2 * n, D));
+        // The tile kernel keeps nothing but the rotated rows in the workspace.  Few tokens ask for what their way by pairs does, so
+        // that a call which fits the workspace (one that is captured behind a warm-up of other sizes) does not make it grow.
+        auto scratch = [&](int64_t rows, int64_t in) { return wide ? api.exl3_workspace_bytes(rows, in) : api.exl3_gemm_workspace_bytes(rows, in); };
+        Workspace ws = workspace(dev, scratch(2 * n, D));
         launch(dev, "exl3_gemm_tiles", [&] {
             return api.exl3_gemm_tiles(r.t.data_ptr(), r.dtype, r.stride, 2 * n, row_src, gu_suh, suh_gu,
                                        gu.trellis, gu.t_in, gu.t_out, k, cb, tiles_gu, n_gu, gu_svh, u16(ygu), 2 *
                                        H, nullptr, ws.ptr, ws.bytes, hint | wide | EXL3_FLAG_ROW_PAIRS, es);
         });
-        ws = workspace(dev, api.exl3_gemm_workspace_bytes(n, H));
+        ws = workspace(dev, scratch(n, H));
         launch(dev, "exl3_gemm_tiles", [&] {
             return api.exl3_gemm_tiles(ygu.data_ptr(), EXL3_DT_F16, 2 * H, n, nullptr, dn_suh, suh_dn, dn.trellis,
                                        dn.t_in, dn.t_out, k, cb, tiles_dn, n_dn, dn_svh, u16(y), D, order, ws.ptr,

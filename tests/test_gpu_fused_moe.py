@@ -189,6 +189,30 @@ def test_switch_glu_few_tokens_on_both_sides_of_the_line(cuda, oracle, k, tokens
     assert rel_err(y.cpu().numpy().reshape(tokens, kk, D), want) <= 2e-3
 
 
+def test_few_tokens_by_expert_do_not_grow_the_workspace(cuda, oracle):
+    """Sixteen tokens on few experts fit the scratch that their way by pairs takes: a call captured behind a warm-up of one token
+    must not allocate and clear a new workspace inside the graph."""
+    from ponyexl3_b200 import _lib, ops
+
+    dev = torch.cuda.current_device()
+    old = ops.Workspace._per_device.pop(dev, None)
+    if old is not None:
+        ops.Workspace._retired.setdefault(dev, []).append(old)
+    _lib.host().set_workspace(dev, 0, 0)
+    E, D, H, kk = 8, 512, 512, 8
+    w = _experts(E, D, H, 4, seed=97)
+    sw = _switch(w, 4, 0)
+    rng = np.random.default_rng(97)
+    x = (rng.standard_normal((16, D)) * 0.5).astype(np.float16)
+    idx = np.stack([rng.permutation(E)[:kk] for _ in range(16)]).astype(np.int64)
+    xd, idd = torch.from_numpy(x).cuda()[None], torch.from_numpy(idx).cuda()[None]
+    sw(xd[:, :1], idd[:, :1])
+    before = ops.Workspace._per_device[dev]
+    y = sw(xd, idd)
+    assert ops.Workspace._per_device[dev] is before
+    assert rel_err(y.cpu().numpy().reshape(16, kk, D), oracle.switch_glu(x, idx, **w, k=4, cb=0)) <= 2e-3
+
+
 @pytest.mark.parametrize("name", ["_gu_svh", "_dn_svh"])
 def test_few_tokens_with_scales_on_eight_bytes(cuda, oracle, name):
     """Output scales aligned for the GEMV only: sixteen tokens on few experts stay with it (the tile kernel refuses them)."""
