@@ -18,9 +18,9 @@
 // B_0) and every pinned one (the path from the pinned base), where the reference's recursion from the start needs a
 // pass of 255 steps for each: two for most tiles, up to five.  The sums are rounded in another order, so a result
 // is only taken if it cannot depend on that: every decision on the path is further from its runner-up than the
-// rounding of float64 sums of that size (2^-42), or tied in a way that both orders resolve alike.  Tiles where that
-// fails (exact ties: one tile in some thousands at K <= 6, one in three at K = 8 with MUL1's thousand values) are marked, and
-// encode_kernel searches them from the start, in the reference's order.
+// rounding of float64 sums of that size (2^-42), or a tie of equal errors at either end of the path, where both orders take
+// the first.  Tiles where that fails (exact ties: one tile in some thousands at K <= 6, one in three at K = 8 with MUL1's
+// thousand values) are marked, and encode_kernel searches them from the start, in the reference's order.
 //
 // The 2^K bases with the same b mod 2^(16-2K) share their successors, so all that a step hands on is one cost per base,
 // 2^(16-K) numbers instead of 65,536.  For K >= 2 they fit the SM's shared memory and a tile is searched by
@@ -105,14 +105,8 @@ __device__ __forceinline__ double sq_err(double c, double w)
     const double d = c - w;
     return __dmul_rn(d, d);
 }
-// fp16 -> float64 with integer operations (a value of the codebook is finite): the conversion
-// instructions run at an eighth of the rate.
-__device__ __forceinline__ double half_as_f64(__half h)
-{
-    const uint32_t f = __float_as_uint(__half2float(h));       // at most eleven significant bits
-    const uint32_t hi = (f & 0x7FFFFFFFu) ? (f & 0x80000000u) | (((f & 0x7FFFFFFFu) >> 3) + 0x38000000u) : f;
-    return __hiloint2double((int)hi, 0);
-}
+// (Converted to float64 by the instruction, here and below: as six integer ones, 592 tiles of K = 1 took 11.2 ms for 10.5, and
+// tiles of zeros at K = 8 with MUL1, which the search from the start answers, 50.2 for 43.9.)
 template <int CB> __device__ __forceinline__ float codebook_f32(uint32_t s) { return __half2float(decode_one<CB>(s)); }
 
 // The cheapest final state, the lowest index among equals, over the CTA; (bc, bs) is the thread's own.
@@ -244,8 +238,8 @@ template <int K> struct SearchSplit {
     static constexpr int BL = L < 4 ? L : 4;             // bases whose costs are made at a time (all of them at once spill)
     static constexpr bool kInPlace = K == 2;
     // Every how many steps a tile with too many close decisions is left.  At K = 8 MUL1's thousand values tie at most bases of a
-    // zero weight: 592 tiles of zeros take 50 ms this way, 70 with the whole search before they are left (48.6 by the search from
-    // the start alone), and others 1 % longer.  At lower K such tiles are few, or fill the list up late.
+    // zero weight: 592 tiles of zeros take 44 ms this way, nearly all of it the search from the start, and 20 more with the whole
+    // search before they are left; others take 1 % longer.  At lower K such tiles are few, or fill the list up late.
     static constexpr int kLook = K == 8 ? 16 : 256;
     static constexpr size_t kCost = (size_t)NB * (kInPlace ? 1 : 2) * (sizeof(double) + sizeof(float));
     static constexpr int kChunk = 32768;                 // bytes of pointers fetched at a time by the walk
@@ -807,7 +801,7 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                         }
                         bj[i] = lo & (J - 1);
                         const uint32_t s = ((h << K) | (l0 + i)) | (bj[i] << LB);
-                        val[i] = __dadd_rn(mdc[pred_slot(h, hs, bj[i], rot)], sq_err(half_as_f64(decode_one<CB>(s)), wd));
+                        val[i] = __dadd_rn(mdc[pred_slot(h, hs, bj[i], rot)], sq_err((double)codebook_f32<CB>(s), wd));
                         if (up - lo < kGap || __uint_as_float(up) < near) unsure |= 1u << i;
                     }
                     if (unsure) {
@@ -820,11 +814,11 @@ __global__ void __launch_bounds__(kEncThreads, 1) encode_kernel(const EncodeArgs
                                 val[i] = 1e30;
                                 continue;
                             }
-                            val[i] = __dadd_rn(mdc[pred_slot(h, hs, 0, rot)], sq_err(half_as_f64(decode_one<CB>(b)), wd));
+                            val[i] = __dadd_rn(mdc[pred_slot(h, hs, 0, rot)], sq_err((double)codebook_f32<CB>(b), wd));
 #pragma unroll 1
                             for (int q = 1; q < J; q++) {
                                 const uint32_t sq = b | ((uint32_t)q << LB);
-                                const double v = __dadd_rn(mdc[pred_slot(h, hs, (uint32_t)q, rot)], sq_err(half_as_f64(decode_one<CB>(sq)), wd));
+                                const double v = __dadd_rn(mdc[pred_slot(h, hs, (uint32_t)q, rot)], sq_err((double)codebook_f32<CB>(sq), wd));
                                 if (v < val[i]) { val[i] = v; bj[i] = q; }
                             }
                         }
@@ -1035,8 +1029,8 @@ template <int CB> __global__ void __launch_bounds__(kEncThreads1, 1) search_kern
 #pragma unroll
                 for (int g = 0; g < 2; g++) {
                     const uint32_t b = (uint32_t)(h | (g << E::HB)), pair = decode_pair<CB>(2 * b, 2 * b + 1);
-                    const double v0 = __dadd_rn(c.x, sq_err(half_as_f64(__low2half(u32_as_h2(pair))), wd));
-                    const double v1 = __dadd_rn(c.y, sq_err(half_as_f64(__high2half(u32_as_h2(pair))), wd));
+                    const double v0 = __dadd_rn(c.x, sq_err((double)__low2float(u32_as_h2(pair)), wd));
+                    const double v1 = __dadd_rn(c.y, sq_err((double)__high2float(u32_as_h2(pair)), wd));
                     const double gap = fabs(v1 - v0);
                     // (final states with equal errors: the first of them, in whatever order the costs are summed)
                     if (gap < close && (u > 0 || gap > 0.0)) note_close(sh, t, b, gap);
